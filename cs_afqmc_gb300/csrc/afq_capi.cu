@@ -10,7 +10,9 @@
 
 #include "afq_common.cuh"
 #include "afq_adjoint.cuh"
+#include "afq_digits.cuh"
 #include "afq_kernels.cuh"
+#include "afq_prof.cuh"
 #include "afq_tangent.cuh"
 #include "afq_tc.cuh"
 
@@ -22,6 +24,18 @@ void afq_set_error(const char* fmt, ...) {
   vsnprintf(g_err, sizeof(g_err), fmt, ap);
   va_end(ap);
 }
+
+// FP64 contractions of a context (afq_digits.cuh): operands sliced once (chol, rc) and the
+// scratch of the walker-dependent ones.
+struct DigCtx {
+  afq::DigOp chol;  // vhs: rows (p, q), K = g
+  afq::DigOp rc;    // force bias: rows g, K = (i, p)
+  afq::DigOp xa;    // [2 nw] x nchol
+  afq::DigOp ga;    // [2 nw] x ktot
+  afq::DigPlan fb;  // K ranges of the force bias
+  double2* fb_part;
+  int* status;
+};
 
 struct afq_ctx {
   afq_dims d;
@@ -48,6 +62,7 @@ struct afq_ctx {
   double* cum;
   double2* free_scr;  // free projection: spin constants and QR norm factors [4][nw]
   afq::TcState tc;  // tensor-core (mixed precision) operands and plans
+  DigCtx dg;        // digit-sliced FP64 operands and plans
   // Inside afq_propagate_phaseless only (mixed path): 1 when the operand buffers already
   // hold G, its operands and the walker operand of the current walkers, else 0.
   int gstate;
@@ -65,6 +80,7 @@ struct Layout {
 };
 
 struct Sizes {
+  size_t dg, dg_chol[2], dg_rc[2], dg_xa[2], dg_ga[2], dg_part, dg_status;  // digits: [tiles, row exponents]
   size_t green, fb, xt, shift, fbt, vhs, ovl_new, ene, epart, rccat, wcopy, sr_idx, cum, free_scr, tc, total;
 };
 
@@ -137,6 +153,24 @@ int derive(const afq_dims* d, afq_ctx_dev* c, int* nw_chunk, int* e_chunks, int*
   return 0;
 }
 
+// Shapes of the sliced FP64 operands (no pointers). The plan assumes the full part's 152 SMs, so
+// that workspace sizes do not depend on where they are asked for.
+constexpr int kPlanSms = 152;
+void dig_dims(const afq_ctx_dev& c, DigCtx* g) {
+  const int nn = c.norb * c.norb;
+  auto op = [](afq::DigOp& o, int rows, int K, int tr) {
+    o.rows = rows;
+    o.K = K;
+    o.tr = tr;
+  };
+  op(g->chol, nn, c.nchol, afq::dig_tr(c.nw, nn, 1, kPlanSms));
+  op(g->rc, c.nchol, c.ktot, afq::dig_tr(c.nw, c.nchol, (c.ktot + 15) / 16, kPlanSms));
+  op(g->xa, 2 * c.nw, c.nchol, afq::kDigTile);
+  op(g->ga, 2 * c.nw, c.ktot, afq::kDigTile);
+  const int tiles = ((2 * c.nw + afq::kDigTile - 1) / afq::kDigTile) * ((c.nchol + g->rc.tr - 1) / g->rc.tr);
+  g->fb = afq::dig_plan(tiles, g->rc.kb(), kPlanSms, 8);
+}
+
 Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chunks, size_t welem,
                 Layout* L) {
   Sizes s;
@@ -157,6 +191,21 @@ Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chu
   s.free_scr = L->take(4 * nw * C16);
   s.tc = L->take(d->precision == AFQ_PREC_MIXED ? afq::tc_workspace_bytes(c, nw_chunk, d->mixed_config)
                                                 : 256);
+  if (d->precision == AFQ_PREC_FP64) {
+    DigCtx g;
+    dig_dims(c, &g);
+    auto take = [&](size_t (&o)[2], const afq::DigOp& op) {
+      o[0] = L->take(afq::dig_bytes(op.rows, op.K, op.tr));
+      o[1] = L->take(afq::dig_exps(op.rows, op.tr));
+    };
+    s.dg = L->off;
+    take(s.dg_chol, g.chol);
+    take(s.dg_rc, g.rc);
+    take(s.dg_xa, g.xa);
+    take(s.dg_ga, g.ga);
+    s.dg_status = L->take(256);
+    s.dg_part = L->take(afq::dig_partial_bytes(c.nw, c.nchol, g.fb.splits));
+  }
   s.total = L->off;
   return s;
 }
@@ -183,13 +232,28 @@ int green(afq_ctx* c, const void* wu, const void* wd, double2* g, double2* ovl, 
   return 0;
 }
 
-int force_bias_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
+// out [nw][nchol] = alpha g . rc^T (FP64), alpha = 2 (RHF, one slab) or 1
+int fb_gemm(afq_ctx* c, const double2* g, const afq::DigOp& rc, double2* out, cudaStream_t st) {
   const afq_ctx_dev& d = c->dev;
-  double2 alpha = c2(d.energy_mode == 0 ? 2.0 : 1.0, 0.0);
-  const double* B = d.nspin_g == 2 ? c->rccat : d.rot_chol[0];
-  if (!is_fp64(c)) return afq::tc_force_bias(c->tc, d, out, st);
-  return afq::launch_gemm_cr(false, d.nw, d.nchol, d.ktot, c->green, d.ktot, B, d.ktot, out, d.nchol,
-                             alpha, st);
+  CHECK(afq::dig_slice_cplx_rows(c->dg.ga, g, d.ktot, 1.0, st));
+  return afq::dig_gemm_c(afq::K_FB, c->dg.ga, rc, d.nw, d.nchol, out, d.nchol, 0, d.energy_mode == 0 ? 1 : 0, c->dg.fb,
+                         c->dg.fb_part, c->dg.status, st);
+}
+
+// vhs [nwc][norb^2] = i sqrt(dt) x . chol (FP64)
+int vhs_gemm(afq_ctx* c, const double2* x, int nwc, double2* vhs, cudaStream_t st) {
+  const afq_ctx_dev& d = c->dev;
+  const int nn = d.norb * d.norb;
+  afq::DigOp a = c->dg.xa;
+  a.rows = 2 * nwc;
+  CHECK(afq::dig_slice_cplx_rows(a, x, d.nchol, sqrt(d.dt), st));
+  return afq::dig_gemm_c(afq::K_VHS, a, c->dg.chol, nwc, nn, vhs, nn, 1, 0, afq::DigPlan{1, a.kb()}, nullptr,
+                         c->dg.status, st);
+}
+
+int force_bias_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
+  if (!is_fp64(c)) return afq::tc_force_bias(c->tc, c->dev, out, st);
+  return fb_gemm(c, c->green, c->dg.rc, out, st);
 }
 
 int energy_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
@@ -232,15 +296,12 @@ int propagate_impl(afq_ctx* c, afq_walker_state* s, const double* fields, cudaSt
   const int nb = d.nw / c->nw_chunk;
   for (int b = 0; b < nb; ++b) {
     const int w0 = b * c->nw_chunk;
-    double sq = sqrt(d.dt);
-    CHECK(afq::launch_gemm_cr(true, c->nw_chunk, d.norb * d.norb, d.nchol, c->xt + (size_t)w0 * d.nchol,
-                              d.nchol, c->h.chol, (long)d.norb * d.norb, c->vhs, (long)d.norb * d.norb,
-                              c2(0.0, sq), st));
+    CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
     CHECK(afq::launch_taylor_f64<double>(d, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
   }
   CHECK(green(c, s->walkers_up, s->walkers_dn, nullptr, c->ovl_new, false, st));
   return afq::launch_weights(d, c->shift, c->fbt, 1, c->ovl_new, reinterpret_cast<double2*>(s->overlaps),
-                             s->weights, s->scalars, st);
+                             s->weights, s->scalars, st, c->dg.status);
 }
 
 int qr_impl(afq_ctx* c, afq_walker_state* s, cudaStream_t st) {
@@ -272,11 +333,9 @@ int free_step(afq_ctx* c, afq_walker_state* s, const double* fields, double ene0
   double2* ovl = reinterpret_cast<double2*>(s->overlaps);
   CHECK(afq::launch_free_prep(d, fields, ene0, c->xt, consts, st));
   const int nb = d.nw / c->nw_chunk;
-  const long nn = (long)d.norb * d.norb;
   for (int b = 0; b < nb; ++b) {
     const int w0 = b * c->nw_chunk;
-    CHECK(afq::launch_gemm_cr(true, c->nw_chunk, d.norb * d.norb, d.nchol, c->xt + (size_t)w0 * d.nchol, d.nchol,
-                              c->h.chol, nn, c->vhs, nn, c2(0.0, sqrt(d.dt)), st));
+    CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
     CHECK(afq::launch_taylor_f64<double>(d, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
   }
   CHECK(afq::launch_free_scale(d, consts, s->walkers_up, s->walkers_dn, st));
@@ -305,7 +364,7 @@ int check_free(const afq_ctx* c) {
 // Tangent workspace of afq_propagate_phaseless_jvp, carved like the main workspace.
 struct TSizes {
   size_t dw[2], wold[2], dgreen, dfb, dxt, dshift, dfbt, dvhs, dlo, dlo_new, dweights, dscalars, dene, dpart,
-      dsum, drccat, total;
+      dsum, drccat, drc_d, drc_e, total;  // drc_*: sliced drccat
 };
 
 TSizes tangent_sizes(const afq_ctx_dev& c, int nw_chunk, int e_chunks, Layout* L) {
@@ -329,38 +388,32 @@ TSizes tangent_sizes(const afq_ctx_dev& c, int nw_chunk, int e_chunks, Layout* L
   s.dpart = L->take(nw * e_chunks * 5 * C16);
   s.dsum = L->take(sizeof(double));
   s.drccat = L->take(c.nspin_g == 2 ? (size_t)c.nchol * c.ktot * sizeof(double) : 256);
+  DigCtx g;
+  dig_dims(c, &g);
+  s.drc_d = L->take(afq::dig_bytes(g.rc.rows, g.rc.K, g.rc.tr));
+  s.drc_e = L->take(afq::dig_exps(g.rc.rows, g.rc.tr));
   s.total = L->off;
   return s;
 }
 
 // One phaseless step with tangents (propagate_impl's FP64 branch, each stage followed by
 // its tangent).
-int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, const double* fields,
-                  cudaStream_t st) {
+int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, const afq::DigOp& drc,
+                  const double* fields, cudaStream_t st) {
   const afq_ctx_dev& d = c->dev;
   CHECK(afq::t_launch_green(d, t, s->walkers_up, s->walkers_dn, c->green, t.dgreen, c->ovl_new, t.dlo_new, st));
   CHECK(force_bias_from_green(c, c->fb, st));
-  {
-    const double2 alpha = c2(d.energy_mode == 0 ? 2.0 : 1.0, 0.0);
-    const double* B = d.nspin_g == 2 ? c->rccat : d.rot_chol[0];
-    CHECK(afq::launch_gemm_cr(false, d.nw, d.nchol, d.ktot, t.dgreen, d.ktot, B, d.ktot, t.dfb, d.nchol, alpha,
-                              st));
-    if (t.drccat) {  // orbital rotation: + alpha G dRC^T (t.dxt as scratch, rewritten below)
-      CHECK(afq::launch_gemm_cr(false, d.nw, d.nchol, d.ktot, c->green, d.ktot, t.drccat, d.ktot, t.dxt, d.nchol,
-                                alpha, st));
-      CHECK(afq::t_launch_add((long)d.nw * d.nchol, t.dxt, t.dfb, st));
-    }
+  CHECK(fb_gemm(c, t.dgreen, c->dg.rc, t.dfb, st));
+  if (t.drccat) {  // orbital rotation: + alpha G dRC^T (t.dxt as scratch, rewritten below)
+    CHECK(fb_gemm(c, c->green, drc, t.dxt, st));
+    CHECK(afq::t_launch_add((long)d.nw * d.nchol, t.dxt, t.dfb, st));
   }
   CHECK(afq::t_launch_field_shifts(d, fields, c->fb, t.dfb, c->xt, t.dxt, c->shift, t.dshift, c->fbt, t.dfbt, st));
   const int nb = d.nw / c->nw_chunk;
-  const long nn = (long)d.norb * d.norb;
-  const double2 isq = c2(0.0, sqrt(d.dt));
   for (int b = 0; b < nb; ++b) {
     const int w0 = b * c->nw_chunk;
-    CHECK(afq::launch_gemm_cr(true, c->nw_chunk, d.norb * d.norb, d.nchol, c->xt + (size_t)w0 * d.nchol, d.nchol,
-                              c->h.chol, nn, c->vhs, nn, isq, st));
-    CHECK(afq::launch_gemm_cr(true, c->nw_chunk, d.norb * d.norb, d.nchol, t.dxt + (size_t)w0 * d.nchol, d.nchol,
-                              c->h.chol, nn, t.dvhs, nn, isq, st));
+    CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
+    CHECK(vhs_gemm(c, t.dxt + (size_t)w0 * d.nchol, c->nw_chunk, t.dvhs, st));
     CHECK(afq::t_launch_taylor(d, t, w0, c->nw_chunk, c->vhs, t.dvhs, s->walkers_up, s->walkers_dn, st));
   }
   CHECK(afq::t_launch_green(d, t, s->walkers_up, s->walkers_dn, nullptr, nullptr, c->ovl_new, t.dlo_new, st));
@@ -374,6 +427,29 @@ int copy_d2d(void* dst, const void* src, size_t bytes, cudaStream_t st, const ch
   return 0;
 }
 
+// Sliced operands of the backward sweep: Cholesky vectors with rows g (field cotangents from V
+// cotangents), rot_chol with rows (i, p) (G cotangents), the V cotangents, and the K ranges of
+// the field cotangents (K = norb^2).
+struct AdjOps {
+  afq::DigOp cn, rt, va;
+  afq::DigPlan xtb;
+};
+AdjOps adj_ops(const afq_ctx_dev& c, int nwc) {
+  AdjOps o;
+  const int nn = c.norb * c.norb, kb = (nn + 15) / 16;
+  o.cn.rows = c.nchol;
+  o.cn.K = nn;
+  o.cn.tr = afq::dig_tr(nwc, c.nchol, kb, kPlanSms);
+  o.rt.rows = c.ktot;
+  o.rt.K = c.nchol;
+  o.rt.tr = afq::dig_tr(c.nw, c.ktot, 1, kPlanSms);
+  o.va.rows = 2 * nwc;
+  o.va.K = nn;
+  o.xtb = afq::dig_plan(((2 * nwc + afq::kDigTile - 1) / afq::kDigTile) * ((c.nchol + o.cn.tr - 1) / o.cn.tr), kb,
+                        kPlanSms, 16);
+  return o;
+}
+
 // Workspace of afq_propagate_phaseless_vjp: the recorded forward sweep (snapshots of the
 // walker state before every step, after the last step of an energy block and after its QR;
 // shifted fields and shift terms of every step; local energies of every block; SR indices)
@@ -381,6 +457,8 @@ int copy_d2d(void* dst, const void* src, size_t bytes, cudaStream_t st, const ch
 struct AdjSizes {
   size_t snap_w, snap_wt, snap_ov, snap_sc, t_xt, t_sh, t_fbt, t_ene, t_idx;
   size_t wb, wb2, wbar, lbar, lbar2, gpend, gene, fbb, xtb, shb, fbtb, vbar, tay, ebar, scal, beb, bwb, total;
+  size_t dg_end, part;
+  size_t dg, cn_d, cn_e, rt_d, rt_e, va_d, va_e;  // digits: chol (rows g), rot_chol^T, V cotangents
   size_t wslab;  // walker elements of one snapshot, both slabs
   int nblk, nsteps, nsnap;
 };
@@ -418,6 +496,16 @@ AdjSizes adjoint_sizes(const afq_ctx_dev& c, int nw_chunk, int n_prop, int n_ene
   s.scal = L->take(8 * sizeof(double));
   s.beb = L->take((size_t)s.nblk * sizeof(double));
   s.bwb = L->take((size_t)s.nblk * sizeof(double));
+  const AdjOps o = adj_ops(c, nw_chunk);
+  s.dg = L->off;
+  s.cn_d = L->take(afq::dig_bytes(o.cn.rows, o.cn.K, o.cn.tr));
+  s.cn_e = L->take(afq::dig_exps(o.cn.rows, o.cn.tr));
+  s.rt_d = L->take(afq::dig_bytes(o.rt.rows, o.rt.K, o.rt.tr));
+  s.rt_e = L->take(afq::dig_exps(o.rt.rows, o.rt.tr));
+  s.va_d = L->take(afq::dig_bytes(o.va.rows, o.va.K));
+  s.va_e = L->take(afq::dig_exps(o.va.rows));
+  s.dg_end = L->off;
+  s.part = L->take(afq::dig_partial_bytes(nw_chunk, c.nchol, o.xtb.splits));
   s.total = L->off;
   return s;
 }
@@ -562,6 +650,26 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
       afq_set_error("rot_chol concat: %s", cudaGetErrorString(e));
       delete c;
       return (int)e;
+    }
+  }
+  if (dims->precision == AFQ_PREC_FP64) {
+    dig_dims(c->dev, &c->dg);
+    auto at = [&](afq::DigOp& o, const size_t (&off)[2]) {
+      o.d = reinterpret_cast<unsigned char*>(ws + off[0]);
+      o.e = reinterpret_cast<int*>(ws + off[1]);
+    };
+    at(c->dg.chol, sz.dg_chol);
+    at(c->dg.rc, sz.dg_rc);
+    at(c->dg.xa, sz.dg_xa);
+    at(c->dg.ga, sz.dg_ga);
+    c->dg.status = reinterpret_cast<int*>(ws + sz.dg_status);
+    c->dg.fb_part = reinterpret_cast<double2*>(ws + sz.dg_part);
+    int e = zero(ws + sz.dg, sz.dg_part - sz.dg, st);  // padding stays zero
+    if (!e) e = afq::dig_slice_real_cols(c->dg.chol, ham->chol, (long)dims->norb * dims->norb, st);
+    if (!e) e = afq::dig_slice_real_rows(c->dg.rc, dev.nspin_g == 2 ? c->rccat : ham->rot_chol_up, dev.ktot, st);
+    if (e) {
+      delete c;
+      return e;
     }
   }
   if (dims->precision == AFQ_PREC_MIXED) {
@@ -780,6 +888,10 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
   } else if (rot) {
     t.drccat = in->drot_chol_up;
   }
+  afq::DigOp drc = ctx->dg.rc;
+  drc.d = reinterpret_cast<unsigned char*>(tw + ts.drc_d);
+  drc.e = reinterpret_cast<int*>(tw + ts.drc_e);
+  if (t.drccat) CHECK(afq::dig_slice_real_rows(drc, t.drccat, d.ktot, st));
   double2* ovl = reinterpret_cast<double2*>(state->overlaps);
   const size_t welems[2] = {(size_t)d.nw * d.norb * d.kslab[0], (size_t)d.nw * d.norb * d.kslab[1]};
   void* wslab[2] = {state->walkers_up, state->walkers_dn};
@@ -792,7 +904,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
     for (int eb = 0; eb < n_ene_blocks; ++eb, ++blk) {
       for (int p = 0; p < n_prop_steps; ++p) {
         const double* f = fields + ((size_t)blk * n_prop_steps + p) * step_elems;
-        CHECK(propagate_jvp(ctx, state, t, f, st));
+        CHECK(propagate_jvp(ctx, state, t, drc, f, st));
       }
       for (int k = 0; k < d.nslab; ++k)
         CHECK(copy_d2d(t.wold[k], wslab[k], welems[k] * sizeof(double2), st, "walker copy before QR"));
@@ -979,8 +1091,17 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
   CHECK(afq::a_launch_end(blk, block_energy, block_weight, a, st));
   const int nwc = ctx->nw_chunk, nb = d.nw / nwc;
   const long nn = (long)d.norb * d.norb;
-  const double sq = sqrt(d.dt);
   const double* brc = d.nspin_g == 2 ? ctx->rccat : d.rot_chol[0];
+  AdjOps ao = adj_ops(d, nwc);
+  ao.cn.d = reinterpret_cast<unsigned char*>(base + as.cn_d);
+  ao.cn.e = reinterpret_cast<int*>(base + as.cn_e);
+  ao.rt.d = reinterpret_cast<unsigned char*>(base + as.rt_d);
+  ao.rt.e = reinterpret_cast<int*>(base + as.rt_e);
+  ao.va.d = reinterpret_cast<unsigned char*>(base + as.va_d);
+  ao.va.e = reinterpret_cast<int*>(base + as.va_e);
+  CHECK(zero(base + as.dg, as.dg_end - as.dg, st));
+  CHECK(afq::dig_slice_real_rows(ao.cn, ctx->h.chol, nn, st));
+  CHECK(afq::dig_slice_real_cols(ao.rt, brc, d.ktot, st));
   const double alpha = d.energy_mode == 0 ? 2.0 : 1.0;
   bool gp = false;  // a.gpend holds the pending G cotangent of the current point
   for (int b = blk - 1; b >= 0; --b) {
@@ -1015,20 +1136,21 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
                                 a.wb[1], st, gt));
       for (int k = 0; k < nb; ++k) {
         const int w0 = k * nwc;
-        CHECK(afq::launch_gemm_cr(true, nwc, (int)nn, d.nchol, tp.xt(step) + (size_t)w0 * d.nchol, d.nchol,
-                                  ctx->h.chol, nn, ctx->vhs, nn, c2(0.0, sq), st));
+        CHECK(vhs_gemm(ctx, tp.xt(step) + (size_t)w0 * d.nchol, nwc, ctx->vhs, st));
         CHECK(afq::a_launch_taylor(d, a, w0, nwc, ctx->vhs, tp.w(start, 0), tp.w(start, 1), st));
         if (cg) CHECK(afq::a_launch_chol_grad(d, a, nwc, tp.xt(step) + (size_t)w0 * d.nchol, st));
-        CHECK(afq::launch_gemm_cr(false, nwc, d.nchol, (int)nn, a.vbar, nn, ctx->h.chol, nn,
-                                  a.xtb + (size_t)w0 * d.nchol, d.nchol, c2(0.0, -sq), st));
+        CHECK(afq::dig_slice_cplx_rows(ao.va, a.vbar, nn, sqrt(d.dt), st));
+        CHECK(afq::dig_gemm_c(afq::K_FB, ao.va, ao.cn, nwc, d.nchol, a.xtb + (size_t)w0 * d.nchol, d.nchol, 3, 0,
+                              ao.xtb, reinterpret_cast<double2*>(base + as.part), ctx->dg.status, st));
       }
       CHECK(afq::a_launch_field(d, a, tp.xt(step), st));
       if (rot) {  // fb = alpha rot_chol G(W_start): rot_chol-bar += alpha Re(fb-bar^H G)
         CHECK(afq::launch_green<double>(d, tp.w(start, 0), tp.w(start, 1), ctx->green, nullptr, true, st));
         CHECK(afq::a_launch_rc_fb(d, a, ctx->green, alpha, st));
       }
-      CHECK(afq::launch_gemm_cr(true, d.nw, d.ktot, d.nchol, a.fbb, d.nchol, brc, d.ktot, a.gpend, d.ktot,
-                                c2(alpha, 0.0), st));
+      CHECK(afq::dig_slice_cplx_rows(ctx->dg.xa, a.fbb, d.nchol, 1.0, st));
+      CHECK(afq::dig_gemm_c(afq::K_VHS, ctx->dg.xa, ao.rt, d.nw, d.ktot, a.gpend, d.ktot, 0,
+                            d.energy_mode == 0 ? 1 : 0, afq::DigPlan{1, ctx->dg.xa.kb()}, nullptr, ctx->dg.status, st));
       gp = true;
       swap_slabs(a.wb, a.wb2);
       double2* t = a.lbar;

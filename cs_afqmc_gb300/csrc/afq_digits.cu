@@ -1,0 +1,753 @@
+// Sliced FP64 contractions: slicing kernels, the digit GEMM and its launchers (afq_digits.cuh).
+
+#include <math.h>
+
+#include "afq_common.cuh"
+#include "afq_digits.cuh"
+#include "afq_prof.cuh"
+#include "afq_ptx.cuh"
+
+namespace afq {
+
+// ======================================================================================
+// digits
+// ======================================================================================
+
+// Position of the leading bit of |x| above 2^-1074 (0 for zero); 2098 for NaN and infinities
+AFQ_D unsigned dig_key(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  const unsigned ef = (unsigned)(b >> 52);
+  return ef ? ef + 51u : 63u - (unsigned)__clzll((long long)(b | 1ull));
+}
+
+// exponent e with |x| < 2^e for every x of a row whose largest key is `key`
+AFQ_D int dig_row_exp(unsigned key) { return key >= 2098u ? kDigBad : (int)key - 1073; }
+
+// x 2^(56 - e) rounded to an integer (|x| < 2^e); e = kDigBad gives 0
+AFQ_D long long dig_fixed(double x, int e) {
+  const long long b = __double_as_longlong(x);
+  const int ef = (int)((b >> 52) & 0x7ff);
+  long long m = b & 0xfffffffffffffll;
+  if (ef) m |= 1ll << 52;
+  const int sh = 4 + (ef ? ef : 1) - 1023 - e;  // m << sh < 2^56
+  long long q;
+  if (e == kDigBad || sh < -58) q = 0;
+  else if (sh >= 0) q = m << sh;
+  else q = (m + (1ll << (-sh - 1))) >> -sh;
+  return b < 0 ? -q : q;
+}
+
+// sum_{k<7} 64 * 128^k: makes the seven lower digits of q + offset non-negative
+constexpr long long kDigOffset = 64ll * (((1ll << 49) - 1) / 127);
+
+// Digit j of q times its weight as an FP32 value (exact; its upper 16 bits are the BF16 value).
+template <int J>
+AFQ_D unsigned dig_f32(long long qo) {
+  constexpr float s = 1.0f / (float)(1ll << (7 + 7 * J));
+  if (J == 0) {
+    const int u = (int)(qo >> 49) + 128;
+    return __float_as_uint(fmaf(__uint_as_float(0x4B000000u | (unsigned)u), s, -(8388608.0f + 128.0f) * s));
+  }
+  const unsigned u = (unsigned)(qo >> (49 - 7 * J)) & 127u;
+  return __float_as_uint(fmaf(__uint_as_float(0x4B000000u | u), s, -(8388608.0f + 64.0f) * s));
+}
+
+template <int J>
+AFQ_D uint4 dig_chunk(const long long (&qo)[8], unsigned flip) {
+  uint4 w;
+  w.x = __byte_perm(dig_f32<J>(qo[0]), dig_f32<J>(qo[1]), 0x7632) ^ flip;
+  w.y = __byte_perm(dig_f32<J>(qo[2]), dig_f32<J>(qo[3]), 0x7632) ^ flip;
+  w.z = __byte_perm(dig_f32<J>(qo[4]), dig_f32<J>(qo[5]), 0x7632) ^ flip;
+  w.w = __byte_perm(dig_f32<J>(qo[6]), dig_f32<J>(qo[7]), 0x7632) ^ flip;
+  return w;
+}
+
+// Writes the eight digits of eight consecutive k of one row. base: the row tile's K block,
+// row: within the tile, half: k & 8. flip = 0x80008000 stores the negated values as well or
+// instead.
+AFQ_D void dig_store(const long long (&q)[8], unsigned char* base, int tr, int row, int half, unsigned flip = 0) {
+  long long qo[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) qo[i] = q[i] + kDigOffset;
+  unsigned char* r = base + row * 128;
+  const int x = row & 7;
+  auto at = [&](int j) -> uint4* {
+    return reinterpret_cast<uint4*>(r + (j >> 2) * (tr * 128) + (((((j & 3) << 1) | half) ^ x) << 4));
+  };
+  *at(0) = dig_chunk<0>(qo, flip);
+  *at(1) = dig_chunk<1>(qo, flip);
+  *at(2) = dig_chunk<2>(qo, flip);
+  *at(3) = dig_chunk<3>(qo, flip);
+  *at(4) = dig_chunk<4>(qo, flip);
+  *at(5) = dig_chunk<5>(qo, flip);
+  *at(6) = dig_chunk<6>(qo, flip);
+  *at(7) = dig_chunk<7>(qo, flip);
+}
+
+AFQ_D unsigned char* dig_block(unsigned char* d, int row, int kblk, int kb, int tr) {
+  return d + ((size_t)(row / tr) * kb + kblk) * ((size_t)tr * 256);
+}
+
+AFQ_D unsigned block_max_u(unsigned v, unsigned* red) {
+  v = __reduce_max_sync(0xffffffffu, v);
+  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[wid] = v;
+  __syncthreads();
+  unsigned m = red[0];
+  for (int i = 1; i < nw; ++i) m = max(m, red[i]);
+  return m;
+}
+
+// One CTA per complex row: lane pairs hold the two halves of a K block, so each 32-byte
+// sector of the digit tile is written by one instruction.
+__global__ void __launch_bounds__(128) k_dig_cplx_rows(const double2* __restrict__ src, long ld, int K, int kb,
+                                                       double mul, unsigned char* __restrict__ d,
+                                                       int* __restrict__ e) {
+  __shared__ unsigned red[2][4];
+  const int m = blockIdx.x;
+  const double2* s = src + (size_t)m * ld;
+  unsigned er = 0, ei = 0;
+  for (int k = threadIdx.x; k < K; k += blockDim.x) {
+    const double2 v = s[k];
+    er = max(er, dig_key(v.x * mul));
+    ei = max(ei, dig_key(v.y * mul));
+  }
+  const int xr = dig_row_exp(block_max_u(er, red[0])), xi = dig_row_exp(block_max_u(ei, red[1]));
+  if (threadIdx.x == 0) {
+    e[2 * m] = xr;
+    e[2 * m + 1] = xi;
+  }
+  const int row = (2 * m) & (kDigTile - 1);
+  for (int t = threadIdx.x; t < 2 * kb; t += blockDim.x) {
+    long long qr[8], qi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = 8 * t + i;
+      const double2 v = k < K ? s[k] : c2(0.0, 0.0);
+      qr[i] = dig_fixed(v.x * mul, xr);
+      qi[i] = dig_fixed(v.y * mul, xi);
+    }
+    unsigned char* b = dig_block(d, 2 * m, t >> 1, kb, kDigTile);
+    dig_store(qr, b, kDigTile, row, t & 1);
+    dig_store(qi, b, kDigTile, row + 1, t & 1);
+  }
+}
+
+__global__ void __launch_bounds__(128) k_dig_real_rows(const double* __restrict__ src, long ld, int K, int kb, int tr,
+                                                       unsigned char* __restrict__ d, int* __restrict__ e) {
+  __shared__ unsigned red[4];
+  const int m = blockIdx.x;
+  const double* s = src + (size_t)m * ld;
+  unsigned er = 0;
+  for (int k = threadIdx.x; k < K; k += blockDim.x) er = max(er, dig_key(s[k]));
+  const int xr = dig_row_exp(block_max_u(er, red));
+  if (threadIdx.x == 0) e[m] = xr;
+  for (int t = threadIdx.x; t < 2 * kb; t += blockDim.x) {
+    long long q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = 8 * t + i;
+      q[i] = dig_fixed(k < K ? s[k] : 0.0, xr);
+    }
+    dig_store(q, dig_block(d, m, t >> 1, kb, tr), tr, m % tr, t & 1);
+  }
+}
+
+// src [K][ld]: lanes along the rows (contiguous), the eight warps split K.
+__global__ void __launch_bounds__(256) k_dig_real_cols(const double* __restrict__ src, long ld, int rows, int K,
+                                                       int kb, int tr, unsigned char* __restrict__ d,
+                                                       int* __restrict__ e) {
+  __shared__ unsigned red[8][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
+  const bool in = row < rows;
+  unsigned er = 0;
+  if (in)
+    for (int k = wid; k < K; k += 8) er = max(er, dig_key(src[(size_t)k * ld + row]));
+  red[wid][lane] = er;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) er = max(er, red[i][lane]);
+  const int x = dig_row_exp(er);
+  if (!in) return;
+  if (wid == 0) e[row] = x;
+  for (int t = wid; t < 2 * kb; t += 8) {
+    long long q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = 8 * t + i;
+      q[i] = dig_fixed(k < K ? src[(size_t)k * ld + row] : 0.0, x);
+    }
+    dig_store(q, dig_block(d, row, t >> 1, kb, tr), tr, row % tr, t & 1);
+  }
+}
+
+// ======================================================================================
+// the digit GEMM
+// ======================================================================================
+
+// i_c: the integer sums of the groups. Returns sum_c i_c 2^(-14-7c) 2^e rounded to FP64, from
+// H = i_0 2^21 + i_1 2^14 + i_2 2^7 + i_3 and L, the same of groups 4..7.
+AFQ_D double dig_combine(long long H, long long L, int e) {
+  const long long hi = H + (L >> 28);
+  const int sgn = (int)(hi >> 63);  // sign of the whole sum: the rest is non-negative
+  unsigned lo = (unsigned)L & 0xfffffffu;
+  unsigned long long a = (unsigned long long)(hi ^ sgn);  // |sum| = a 2^28 + lo, sum < 0: complement + 1
+  lo = ((lo ^ (unsigned)sgn) & 0xfffffffu) - (unsigned)sgn;
+  a += lo >> 28;
+  lo &= 0xfffffffu;
+  if (a == 0) {  // below 2^28 units: shift up (exact)
+    if (lo == 0) return e > kDigBad / 2 ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+    a = lo;
+    lo = 0;
+    e -= 28;
+  }
+  const int lz = __clzll((long long)a);  // a has at most 46 bits: lz >= 18
+  const unsigned long long m = (a << lz) | (((unsigned long long)lo << 36) >> (64 - lz));
+  const unsigned long long r = (m >> 11) + ((m >> 10) & 1ull);
+  const int be = 28 - lz + e + 1022;  // biased exponent - 1: r carries the hidden bit
+  if (be < 0 || be > 2044) {          // outside the normal range, or a bad row
+    if (e > kDigBad / 2) return __longlong_as_double(0x7ff8000000000000ll);
+    const double v = scalbn((double)r, be - 1022 - 52);
+    return sgn ? -v : v;
+  }
+  return __hiloint2double((int)((unsigned)(r >> 32) + ((unsigned)be << 20)) | (sgn & (int)0x80000000), (int)(unsigned)r);
+}
+
+// Integer sums of groups C..C+3 of one element, i_C 2^21 + i_(C+1) 2^14 + i_(C+2) 2^7 + i_(C+3).
+// Fast form: v 2^(14+7c) + 1.5 2^23 holds the integer in its low mantissa bits while it is
+// below 2^22 in size (one FFMA instead of a conversion at a quarter of the rate); `over`
+// collects a nonzero value above bit 22 when one is not.
+template <int C>
+AFQ_D unsigned dig_magic(float v, unsigned& over) {
+  constexpr float s = (float)(1ll << (14 + 7 * (C < 7 ? C : 6)));
+  const unsigned b = __float_as_uint(fmaf(C < 7 ? v : v * 128.0f, s, 12582912.0f));
+  over |= b ^ 0x4B000000u;
+  return b;
+}
+constexpr long long kDigMagic = 0x4B400000ll * ((1ll << 21) + (1ll << 14) + (1ll << 7) + 1ll);
+template <int C>
+AFQ_D long long dig_quad_fast(float a, float b, float c, float d, unsigned& over) {
+  const unsigned i0 = dig_magic<C>(a, over), i1 = dig_magic<C + 1>(b, over), i2 = dig_magic<C + 2>(c, over),
+                 i3 = dig_magic<C + 3>(d, over);
+  const unsigned long long x = (unsigned long long)i0 * (1u << 21) + (unsigned long long)i1 * (1u << 14) +
+                               (unsigned long long)i2 * (1u << 7) + i3;
+  return (long long)(x - (unsigned long long)kDigMagic);
+}
+template <int C>
+AFQ_D int dig_int(float v) {
+  constexpr float s = (float)(1ll << (14 + 7 * (C < 7 ? C : 6)));
+  return __float2int_rn(C < 7 ? v * s : v * s * 128.0f);
+}
+template <int C>
+__device__ __noinline__ long long dig_quad_slow(float a, float b, float c, float d) {
+  return ((long long)dig_int<C>(a) << 21) + ((long long)dig_int<C + 1>(b) << 14) +
+         ((long long)dig_int<C + 2>(c) << 7) + (long long)dig_int<C + 3>(d);
+}
+template <int C>
+AFQ_D long long dig_quad(float a, float b, float c, float d) {
+  unsigned over = 0;
+  const long long x = dig_quad_fast<C>(a, b, c, d, over);
+  return (over >> 23) ? dig_quad_slow<C>(a, b, c, d) : x;
+}
+
+struct DigGemm {
+  const unsigned char *a, *b;
+  const int *ea, *eb;
+  int kba, kbb;    // K blocks per row tile in the layouts
+  int kb;          // K blocks contracted
+  int mt, nt, nb;  // row tiles, column tiles, batch entries
+  int a_bt, b_bt;  // row tiles per batch entry (0: one operand for all entries)
+  int tr;          // B rows per tile
+  int splits, kps; // K ranges, K blocks per range
+  int stages;
+  uint32_t idesc;
+};
+
+struct DigWhere {
+  int batch, m, n, split;
+  bool add;  // a later K segment of the same range: add to what is there
+};
+
+constexpr int kDigThreads = 320;
+constexpr int kDigABlock = kDigTile * 256;  // bytes of an A K block
+constexpr int kDigRing = 196608;
+constexpr int kDigSmem = 1024 + kDigRing + 256;
+constexpr int kDigMaxStages = 5;
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   ptx::smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(ptx::smem_u32(bar))
+               : "memory");
+}
+
+// Persistent over (K range, batch entry, column tile, row tile). Warp 0 loads K blocks
+// (A 32 KB + B) with bulk copies, warp 1 issues the MMAs, warps 2..9 combine and store: warp w
+// reads TMEM lanes 32 (w % 4).. and half of the columns.
+//
+// WIDE (128 columns): four accumulators of 128 columns fill the tensor memory, so a range is
+// contracted twice, first groups 4..7 (26 products), then 0..3 (10 products of the first four
+// digits only). A tcgen05.mma of M 128, N 128, K 16 takes 64 cycles and reads 8 KB of shared
+// memory, both at their limits; with N = 64 it is bound by the 6 KB it reads, so the wide form
+// needs about half the tensor time per flop. Narrow (tr <= 64 columns): all eight accumulators
+// at once, two sets when tr <= 32. Narrow tiles serve the batched products (tr = one walker's
+// columns) and problems with too few wide tiles for the SMs.
+template <bool WIDE, class Epi>
+__global__ void __launch_bounds__(kDigThreads, 1)
+    k_gemm_digits(const DigGemm g, const __grid_constant__ typename Epi::Params ep, int* status) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kDigRing);
+  uint64_t* empty = full + kDigMaxStages;
+  uint64_t* accfull = empty + kDigMaxStages;  // [2]
+  uint64_t* accempty = accfull + 2;           // [2]
+  uint64_t* done = accempty + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tr = g.tr, bblock = tr * 256, unit = kDigABlock + bblock;
+  constexpr int PASSES = WIDE ? 2 : 1;
+  const int acols = WIDE ? 128 : tr <= 32 ? 32 : 64;  // columns between accumulators
+  const int nbuf = !WIDE && tr <= 32 ? 2 : 1;
+  const int mn = g.mt * g.nt * g.nb, ntiles = mn * g.splits;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < g.stages; ++s) {
+      ptx::mbar_init(&full[s], 1);
+      ptx::mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(&accfull[i], 1);
+      ptx::mbar_init(&accempty[i], 8);
+    }
+    ptx::mbar_init(done, 1);
+    ptx::fence_mbar_init();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(tmem_holder, 512);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = *tmem_holder;
+  bool ok = true;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        const int ks = tile / mn, x = tile % mn;
+        const int m = x % g.mt, n = (x / g.mt) % g.nt, b = x / (g.mt * g.nt);
+        const int ka = ks * g.kps, kz = min(g.kb, ka + g.kps);
+        const unsigned char* pa = g.a + (size_t)(b * g.a_bt + m) * g.kba * kDigABlock;
+        const unsigned char* pb = g.b + (size_t)(b * g.b_bt + n) * g.kbb * bblock;
+        for (int k0 = ka; k0 < kz && ok; k0 += kDigSegBlocks) {
+          const int k1 = min(kz, k0 + kDigSegBlocks);
+          for (int pass = 0; pass < PASSES && ok; ++pass) {
+            const uint32_t da = WIDE && pass == 1 ? kDigABlock / 2 : kDigABlock;
+            const uint32_t db = WIDE && pass == 1 ? bblock / 2 : bblock;
+            for (int k = k0; k < k1; ++k, ++it) {
+              const int s = it % g.stages, r = it / g.stages;
+              if (r > 0 && !ptx::mbar_wait(&empty[s], (r - 1) & 1)) {
+                ok = false;
+                break;
+              }
+              unsigned char* u = smem + s * unit;
+              ptx::mbar_expect_tx(&full[s], da + db);
+              bulk_load(u, pa + (size_t)k * kDigABlock, da, &full[s]);
+              bulk_load(u + kDigABlock, pb + (size_t)k * bblock, db, &full[s]);
+            }
+          }
+        }
+      }
+      // never leave a copy in flight
+      for (int j = it - 1; j >= 0 && j >= it - g.stages; --j)
+        if (!ptx::mbar_wait(&full[j % g.stages], (j / g.stages) & 1)) ok = false;
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int it = 0, run = 0;
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        const int ka = (tile / mn) * g.kps, kz = min(g.kb, ka + g.kps);
+        for (int k0 = ka; k0 < kz && ok; k0 += kDigSegBlocks) {
+          const int k1 = min(kz, k0 + kDigSegBlocks);
+          for (int pass = 0; pass < PASSES && ok; ++pass, ++run) {
+            const int buf = run % nbuf, use = run / nbuf;
+            if (use > 0 && !ptx::mbar_wait(&accempty[buf], (use - 1) & 1)) {
+              ok = false;
+              break;
+            }
+            ptx::tc_fence_after();
+            const uint32_t acc = tmem + (uint32_t)(buf * 256);
+            for (int k = k0; k < k1; ++k, ++it) {
+              const int s = it % g.stages, r = it / g.stages;
+              if (!ptx::mbar_wait(&full[s], r & 1)) {
+                ok = false;
+                break;
+              }
+              ptx::tc_fence_after();
+              const uint32_t ua = ptx::smem_u32(smem + s * unit), ub = ua + kDigABlock;
+              const uint64_t da = ptx::desc_kmajor_sw128(ua), db = ptx::desc_kmajor_sw128(ub);
+              const uint64_t qa = (kDigABlock / 2) >> 4, qb = (uint64_t)(bblock / 2) >> 4;
+              auto group = [&](int c, uint32_t d) {
+#pragma unroll
+                for (int i = 0; i <= c; ++i) {
+                  const int j = c - i;
+                  ptx::mma_f16(d, da + (i >> 2) * qa + (i & 3) * 2, db + (j >> 2) * qb + (j & 3) * 2, g.idesc,
+                               (k > k0 || i > 0) ? 1u : 0u);
+                }
+              };
+              if constexpr (WIDE) {
+                if (pass == 0) {
+#pragma unroll
+                  for (int c = 4; c < 8; ++c) group(c, acc + (uint32_t)((c - 4) * 128));
+                } else {
+#pragma unroll
+                  for (int c = 0; c < 4; ++c) group(c, acc + (uint32_t)(c * 128));
+                }
+              } else {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) group(c, acc + (uint32_t)(c * acols));
+              }
+              ptx::mma_commit(&empty[s]);
+            }
+            ptx::mma_commit(&accfull[buf]);
+          }
+        }
+      }
+      ptx::mma_commit(done);
+      if (!ptx::mbar_wait(done, 0)) ok = false;
+    }
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2, r = q * 32 + lane;
+    const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+    int run = 0;
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+      DigWhere w;
+      w.split = tile / mn;
+      const int x = tile % mn;
+      w.m = x % g.mt;
+      w.n = (x / g.mt) % g.nt;
+      w.batch = x / (g.mt * g.nt);
+      const int ka = w.split * g.kps, kz = min(g.kb, ka + g.kps);
+      const int er = g.ea[(size_t)(w.batch * g.a_bt + w.m) * kDigTile + r];
+      const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * tr;
+      for (int k0 = ka; k0 < kz && ok; k0 += kDigSegBlocks) {
+        w.add = k0 > ka;
+        if constexpr (WIDE) {
+          long long L[64];
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[0], run & 1))) {
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t src = tmem + lane_off + (uint32_t)(half * 64);
+#pragma unroll
+          for (int c0 = 0; c0 < 64; c0 += 8) {
+            float v[4][8];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ptx::tmem_ld8p(src + (uint32_t)(c * 128 + c0), v[c]);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) L[c0 + j] = dig_quad<4>(v[0][j], v[1][j], v[2][j], v[3][j]);
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&accempty[0]);
+          ++run;
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[0], run & 1))) {
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+#pragma unroll
+          for (int c0 = 0; c0 < 64; c0 += 8) {
+            float v[4][8];
+            double o[8];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ptx::tmem_ld8p(src + (uint32_t)(c * 128 + c0), v[c]);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              o[j] = dig_combine(dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]), L[c0 + j],
+                                 er + eb[half * 64 + c0 + j] + ep.shift);
+            Epi::store(ep, w, r, half * 64 + c0, o);
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&accempty[0]);
+          ++run;
+        } else {
+          const int buf = run % nbuf, use = run / nbuf;
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[buf], use & 1))) {
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const int hc = tr >> 1;
+          const uint32_t src = tmem + lane_off + (uint32_t)(buf * 256 + half * hc);
+          for (int c0 = 0; c0 < hc; c0 += 8) {
+            float v[8][8];
+            double o[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) ptx::tmem_ld8p(src + (uint32_t)(c * acols + c0), v[c]);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              o[j] = dig_combine(dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]),
+                                 dig_quad<4>(v[4][j], v[5][j], v[6][j], v[7][j]),
+                                 er + eb[half * hc + c0 + j] + ep.shift);
+            Epi::store(ep, w, r, half * hc + c0, o);
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
+          ++run;
+        }
+      }
+    }
+  }
+  if (!ok) atomicOr(status, 4);
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, 512);
+  }
+}
+
+// Complex results: rows 2m / 2m + 1 of D are the real and imaginary parts of row m of C.
+// Neighbouring lanes exchange halves so that each stores whole complex numbers.
+struct EpiDigC {
+  struct Params {
+    double2* c;
+    int M, N, tr;
+    long ldc, split_stride;
+    int rot, shift;  // C = i^rot 2^shift D
+  };
+  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[8]) {
+    const int m = (w.m * kDigTile + r) >> 1, odd = r & 1, n0 = w.n * p.tr + col0;
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const double x = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+      const double re = odd ? x : v[j], im = odd ? v[j + 1] : x;
+      const int n = n0 + j + odd;
+      double2 o = c2(re, im);
+      if (p.rot == 1) o = c2(-im, re);
+      if (p.rot == 3) o = c2(im, -re);
+      if (m < p.M && n < p.N) {
+        double2* dst = p.c + (size_t)w.split * p.split_stride + (size_t)m * p.ldc + n;
+        if (w.add) o = cadd(o, *dst);
+        *dst = o;
+      }
+    }
+  }
+};
+
+struct EpiDigR {
+  struct Params {
+    double* d;
+    int M, N, tr;
+    long ldd;
+    int shift;
+  };
+  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[8]) {
+    const int m = w.m * kDigTile + r, n0 = w.n * p.tr + col0;
+    if (m >= p.M) return;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (n0 + j < p.N) {
+        double* dst = p.d + (size_t)m * p.ldd + n0 + j;
+        *dst = w.add ? *dst + v[j] : v[j];
+      }
+  }
+};
+
+// C = sum of the partial results of a split contraction
+__global__ void k_dig_sum(long M, long N, int splits, long sst, const double2* __restrict__ part,
+                          double2* __restrict__ c, long ldc) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < M * N; i += (long)gridDim.x * blockDim.x) {
+    double2 a = part[i];
+    for (int s = 1; s < splits; ++s) a = cadd(a, part[i + s * sst]);
+    c[(i / N) * ldc + i % N] = a;
+  }
+}
+
+// ======================================================================================
+// host launchers
+// ======================================================================================
+
+static int dig_err(const char* what) {
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    afq_set_error("%s: %s", what, cudaGetErrorString(e));
+    return (int)e;
+  }
+  return 0;
+}
+
+int dig_sms() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    cudaGetLastError();
+    sms = 148;
+  }
+  return sms;
+}
+
+int dig_slice_cplx_rows(const DigOp& op, const double2* src, long ld, double mul, cudaStream_t st) {
+  {
+    ProfScope _ps(K_PREP, st);
+    k_dig_cplx_rows<<<op.rows / 2, 128, 0, st>>>(src, ld, op.K, op.kb(), mul, op.d, op.e);
+  }
+  return dig_err("slice rows");
+}
+
+int dig_slice_real_rows(const DigOp& op, const double* src, long ld, cudaStream_t st) {
+  {
+    ProfScope _ps(K_PREP, st);
+    k_dig_real_rows<<<op.rows, 128, 0, st>>>(src, ld, op.K, op.kb(), op.tr, op.d, op.e);
+  }
+  return dig_err("slice rows");
+}
+
+int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_t st) {
+  {
+    ProfScope _ps(K_PREP, st);
+    k_dig_real_cols<<<(op.rows + 31) / 32, 256, 0, st>>>(src, ld, op.rows, op.K, op.kb(), op.tr, op.d, op.e);
+  }
+  return dig_err("slice columns");
+}
+
+template <bool WIDE, class Epi>
+static int launch_digits(int cls, DigGemm g, const typename Epi::Params& ep, int* status, cudaStream_t st) {
+  const int unit = kDigABlock + g.tr * 256;
+  g.stages = kDigRing / unit < kDigMaxStages ? kDigRing / unit : kDigMaxStages;
+  g.idesc = ptx::idesc_f16(128, g.tr, 1);
+  const long tiles = (long)g.mt * g.nt * g.nb * g.splits;
+  const int sms = dig_sms();
+  auto kfn = k_gemm_digits<WIDE, Epi>;
+  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kDigSmem);
+  if (e != cudaSuccess) {
+    afq_set_error("digit GEMM: shared-memory attribute: %s", cudaGetErrorString(e));
+    return (int)e;
+  }
+  {
+    ProfScope _ps(cls, st);
+    kfn<<<(unsigned)(tiles < sms ? tiles : sms), kDigThreads, kDigSmem, st>>>(g, ep, status);
+  }
+  return dig_err("digit GEMM");
+}
+
+static DigGemm dig_args(const DigOp& A, const DigOp& B) {
+  DigGemm g;
+  g.a = A.d;
+  g.b = B.d;
+  g.ea = A.e;
+  g.eb = B.e;
+  g.kba = A.kb();
+  g.kbb = B.kb();
+  g.kb = g.kba < g.kbb ? g.kba : g.kbb;
+  g.mt = (A.rows + kDigTile - 1) / kDigTile;
+  g.nt = (B.rows + B.tr - 1) / B.tr;
+  g.nb = 1;
+  g.a_bt = g.b_bt = 0;
+  g.tr = B.tr;
+  g.splits = 1;
+  g.kps = g.kb;
+  g.stages = 0;
+  g.idesc = 0;
+  return g;
+}
+
+int dig_tr(int M, int N, int kb, int sms) {
+  const int mt = (2 * M + kDigTile - 1) / kDigTile, need = (N + 15) / 16 * 16;
+  const int tr = mt * ((N + 63) / 64) * (kb < 8 ? kb : 8) * 2 >= sms ? 64 : 32;
+  return need < tr ? need : tr;
+}
+
+// The count of K ranges that gives the fewest (rounds of tiles over the SMs) x (K blocks per
+// range + 2 for a range's epilogue).
+DigPlan dig_plan(int tiles, int kb, int sms, int max_splits) {
+  DigPlan best{1, kb};
+  long cost = -1;
+  for (int s = 1; s <= max_splits && s <= kb; ++s) {
+    const int kps = (kb + s - 1) / s, used = (kb + kps - 1) / kps;
+    const long c = (long)((tiles * (long)used + sms - 1) / sms) * (kps + 2 * ((kps + kDigSegBlocks - 1) / kDigSegBlocks));
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = DigPlan{used, kps};
+    }
+  }
+  return best;
+}
+
+size_t dig_partial_bytes(int M, int N, int splits) {
+  return splits > 1 ? (size_t)splits * M * N * sizeof(double2) : 256;
+}
+
+int dig_gemm_c(int cls, const DigOp& A, const DigOp& B, int M, int N, double2* C, long ldc, int rot, int shift,
+               const DigPlan& plan, double2* part, int* status, cudaStream_t st) {
+  DigGemm g = dig_args(A, B);
+  g.mt = (2 * M + kDigTile - 1) / kDigTile;
+  g.nt = (N + B.tr - 1) / B.tr;
+  g.splits = plan.splits;
+  g.kps = plan.kps;
+  const bool split = plan.splits > 1;
+  EpiDigC::Params ep{split ? part : C, M, N, B.tr, split ? (long)N : ldc, (long)M * N, rot, shift};
+  int rc = B.tr == 128 ? launch_digits<true, EpiDigC>(cls, g, ep, status, st)
+                       : launch_digits<false, EpiDigC>(cls, g, ep, status, st);
+  if (rc || !split) return rc;
+  {
+    ProfScope _ps(cls, st);
+    const long n = (long)M * N;
+    k_dig_sum<<<(unsigned)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096), 256, 0, st>>>(M, N, plan.splits, n, part,
+                                                                                          C, ldc);
+  }
+  return dig_err("digit GEMM sum");
+}
+
+int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D, long ldd, int* status,
+               cudaStream_t st) {
+  DigGemm g = dig_args(A, B);
+  EpiDigR::Params ep{D, M, N, B.tr, ldd, 0};
+  return B.tr == 128 ? launch_digits<true, EpiDigR>(cls, g, ep, status, st)
+                     : launch_digits<false, EpiDigR>(cls, g, ep, status, st);
+}
+
+}  // namespace afq
+
+extern "C" size_t afq_test_gemm_digits_bytes(int M, int N, int K, int tr) {
+  return afq::dig_bytes(M, K) + afq::dig_bytes(N, K, tr) + afq::dig_exps(M) + afq::dig_exps(N, tr) + 1024;
+}
+
+extern "C" int afq_test_gemm_digits(const double* a, const double* b, double* d, int M, int N, int K, int tr,
+                                    void* scratch, int* status, void* stream) {
+  using namespace afq;
+  if (!a || !b || !d || !scratch || !status || M < 1 || N < 1 || K < 1 || tr % 16 || tr < 16 || (tr > 64 && tr != 128)) {
+    afq_set_error("afq_test_gemm_digits: bad arguments");
+    return -1;
+  }
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  unsigned char* p = static_cast<unsigned char*>(scratch);
+  p += (256 - (reinterpret_cast<uintptr_t>(p) & 255)) & 255;
+  DigOp A, B;
+  A.d = p;
+  B.d = A.d + dig_bytes(M, K);
+  A.e = reinterpret_cast<int*>(B.d + dig_bytes(N, K, tr));
+  B.e = A.e + dig_exps(M) / sizeof(int);
+  A.rows = M;
+  B.rows = N;
+  A.K = B.K = K;
+  B.tr = tr;
+  cudaError_t e = cudaMemsetAsync(p, 0, afq_test_gemm_digits_bytes(M, N, K, tr) - 512, st);
+  if (e != cudaSuccess) {
+    afq_set_error("afq_test_gemm_digits: %s", cudaGetErrorString(e));
+    return (int)e;
+  }
+  if (int rc = dig_slice_real_rows(A, a, K, st)) return rc;
+  if (int rc = dig_slice_real_rows(B, b, K, st)) return rc;
+  return dig_gemm_r(K_PREP, A, B, M, N, d, N, status, st);
+}

@@ -1,0 +1,76 @@
+// FP64 contractions on the BF16 tensor cores, by exact digit slicing.
+//
+// Every FP64 operand row is scaled by a power of two 2^e >= max|row| and cut into eight
+// balanced digits, x 2^-e = sum_j d_j 2^(-7-7j) with |d_0| <= 128, |d_j| <= 64 and a remainder
+// of at most 2^-57 (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms
+// 59, 2012, with digits of a fixed weight). A digit times its weight is exact in BF16, a
+// product of two is exact in FP32, and the sum of all products with i + j = c over up to 512
+// terms of K is an integer below 2^24 in units of 2^(-14-7c) for c <= 5: the tensor core's FP32
+// accumulator never rounds it. One accumulator per c = 0..7 (36 of the 64 digit products;
+// the others are below 2^-70) is therefore exact, the eight are combined in 64-bit integer
+// arithmetic, and the only rounding of a dot product is the final one to FP64 (plus the
+// remainders, 2^-57 of the row's largest element each). A plain FP64 sum of K terms rounds K
+// times.
+//
+// Why: this part does FP64 at 1.04 TFLOP/s (DGEMM) and BF16 at 1.9 PFLOP/s, so 36 tensor-core
+// products cost about 2 % of the FP64 ones; integer instructions combine the accumulators
+// because FP64 adds and conversions (two per cycle and SM) would cost as much as the products.
+//
+// Layout of a sliced operand ("digit tiles"): rows in tiles of TR (128 for A; 16..128 for B),
+// K in blocks of 16. One (row tile, K block) is contiguous: two quads (digits 0-3, 4-7) of
+// [TR rows][128 bytes], a row's 128 bytes = 4 digits x 16 k in the 128-byte swizzle the
+// tensor core reads, so that a K block of an operand is one plain bulk copy (A 32 KB) and no
+// tensor map is needed. Padding rows and columns are zero.
+#pragma once
+#include "afq_kernels.cuh"
+
+namespace afq {
+
+constexpr int kDigTile = 128;     // A rows per tile
+constexpr int kDigSegBlocks = 32; // K blocks (of 16) an accumulator may sum exactly
+constexpr int kDigBad = 1 << 20;  // row exponent of a row with a NaN or an infinity
+
+inline size_t dig_bytes(long rows, long K, int tr = kDigTile) {
+  return (size_t)((rows + tr - 1) / tr) * ((K + 15) / 16) * tr * 256;
+}
+inline size_t dig_exps(long rows, int tr = kDigTile) { return (size_t)((rows + tr - 1) / tr) * tr * sizeof(int); }
+
+// One sliced operand: digit tiles and row exponents.
+struct DigOp {
+  unsigned char* d = nullptr;
+  int* e = nullptr;
+  int rows = 0, K = 0, tr = kDigTile;
+  int kb() const { return (K + 15) / 16; }
+};
+
+// ---- slicing --------------------------------------------------------------------------
+// complex [M][ld] (M walkers x K): rows 2m (real parts) and 2m + 1 (imaginary parts), times mul
+int dig_slice_cplx_rows(const DigOp& op, const double2* src, long ld, double mul, cudaStream_t st);
+// real [rows][ld]
+int dig_slice_real_rows(const DigOp& op, const double* src, long ld, cudaStream_t st);
+// real [K][ld], rows along the contiguous index
+int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_t st);
+
+// ---- contractions ---------------------------------------------------------------------
+// C[m][n] (complex, ldc) = i^rot 2^shift sum_k A[m][k] B[n][k]: A sliced by
+// dig_slice_cplx_rows, B real. part: split partials when the K range is cut (see
+// dig_gemm_plan); may be NULL when the plan has one split.
+struct DigPlan {
+  int splits, kps;  // K ranges computed independently, K blocks per range
+};
+// K ranges of a contraction with `tiles` output tiles on `sms` SMs
+DigPlan dig_plan(int tiles, int kb, int sms, int max_splits);
+// bytes of the partial results of dig_gemm_c
+size_t dig_partial_bytes(int M, int N, int splits);
+int dig_gemm_c(int cls, const DigOp& A, const DigOp& B, int M, int N, double2* C, long ldc, int rot, int shift,
+               const DigPlan& plan, double2* part, int* status, cudaStream_t st);
+// D[m][n] (real, ldd) = sum_k A[m][k] B[n][k], both real
+int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D, long ldd, int* status,
+               cudaStream_t st);
+int dig_sms();
+// B columns per tile for an output of 2 M x N with kb K blocks: 64 where the tiles (times up to
+// eight K ranges) reach half of the SMs, else 32, so that small problems still spread out; never
+// more than N needs.
+int dig_tr(int M, int N, int kb, int sms);
+
+}  // namespace afq

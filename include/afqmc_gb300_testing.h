@@ -2,13 +2,14 @@
  * afqmc_gb300_testing.h - test hooks of libafqmc_gb300.so.
  *
  * These entry points have no counterpart in the reference: they expose single kernels of
- * the mixed-precision path so that tests can compare each one with a PyTorch FP32
- * computation of the same operation. Same conventions as afqmc_gb300.h (device pointers,
+ * the library so that tests can compare each one with a plain computation of the same
+ * operation. Same conventions as afqmc_gb300.h (device pointers,
  * stream-ordered, 0 on success, afq_last_error() on failure).
  */
 #ifndef AFQMC_GB300_TESTING_H
 #define AFQMC_GB300_TESTING_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -38,6 +39,14 @@ int afq_test_gemm_split(const void* a_hi, const void* a_lo, const void* b_hi, co
  * included): enable = 1 CTA pairs (the default), 0 one CTA per tile, < 0 no change.
  * Returns the previous setting. Not thread-safe: for tests and timing comparisons. */
 int afq_test_split_pairs(int enable);
+
+/* D[M,N] (fp64, row-major) = A[M,K] B[N,K]^T (fp64, row-major) by exact digit slicing on the
+ * BF16 tensor cores, the FP64 path's contraction kernel. tr: output columns per tile
+ * (multiple of 16 up to 64, or 128). scratch: afq_test_gemm_digits_bytes bytes. *status as
+ * above. */
+size_t afq_test_gemm_digits_bytes(int M, int N, int K, int tr);
+int afq_test_gemm_digits(const double* a, const double* b, double* d, int M, int N, int K, int tr,
+                         void* scratch, int* status, void* stream);
 
 #ifdef __cplusplus
 }

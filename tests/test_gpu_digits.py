@@ -1,0 +1,103 @@
+"""The digit-sliced FP64 GEMM (afq_test_gemm_digits) against extended-precision products.
+
+Bound, from the slicing alone: with 2^e >= max|row|, each operand's remainder is at most
+2^-57 2^e per element (two of them: 2^-56), and the digit products left out (i + j >= 8) sum to
+at most 7 * 64 * 64 * 2^-70 (1 + 2^-6) < 2^-55 per term, so |error| <= K 2^(ea + eb) 2^-54 plus
+half an ulp of the result.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def run(a, b, tr):
+    import torch
+
+    from cs_afqmc_gb300 import _lib
+    from cs_afqmc_gb300._engine import stream_ptr
+
+    m, k = a.shape
+    n = b.shape[0]
+    ta, tb = (torch.as_tensor(np.ascontiguousarray(x), device="cuda") for x in (a, b))
+    d = torch.full((m, n), 7.0, dtype=torch.float64, device="cuda")
+    ws = torch.empty(_lib.load().afq_test_gemm_digits_bytes(m, n, k, tr), dtype=torch.uint8, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.call("afq_test_gemm_digits", ta.data_ptr(), tb.data_ptr(), d.data_ptr(), m, n, k, tr, ws.data_ptr(),
+              status.data_ptr(), stream_ptr())
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    return d.cpu().numpy()
+
+
+def longdouble_product(a, b):
+    out = np.zeros((a.shape[0], b.shape[0]), dtype=np.longdouble)
+    al, bl = a.astype(np.longdouble), b.astype(np.longdouble)
+    for k in range(a.shape[1]):
+        out += al[:, k][:, None] * bl[:, k][None, :]
+    return out
+
+
+def bound(a, b, ref):
+    def scale(x):
+        return np.exp2(np.frexp(np.abs(x).max(1))[1].astype(np.float64))
+
+    return a.shape[1] * np.outer(scale(a), scale(b)) * 2.0 ** -54 + np.abs(ref).astype(np.float64) * 2.0 ** -52
+
+
+@pytest.mark.parametrize("tr", [16, 32, 48, 64, 128])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (128, 128, 16), (129, 130, 17), (300, 257, 513), (64, 200, 1100)])
+def test_against_extended_precision(m, n, k, tr):
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((n, k))
+    a *= np.exp2(rng.integers(-40, 40, m))[:, None]          # rows of any size
+    b *= np.exp(-12.0 * np.arange(k) / k)[None, :]           # falling along K, as Cholesky vectors
+    ref = longdouble_product(a, b)
+    assert np.all(np.abs(run(a, b, tr) - ref) <= bound(a, b, ref))
+
+
+@pytest.mark.parametrize("tr", [32, 64, 128])
+def test_extreme_digits_are_exact(tr):
+    """Every digit at its largest with one sign: the accumulators reach their bound."""
+    k = 512
+    digits = np.float64(sum((128 if j == 0 else 63) * 2.0 ** (-7 - 7 * j) for j in range(7)) - 2.0 ** -40)
+    a, b = np.full((3, k), digits * 0.999), np.full((5, k), digits * 0.999)
+    ref = longdouble_product(a, b)
+    assert np.all(np.abs(run(a, b, tr) - ref) <= bound(a, b, ref))
+    ones = run(np.ones((3, k)), np.ones((5, k)), tr)
+    assert np.array_equal(ones, np.full((3, 5), float(k)))
+
+
+@pytest.mark.parametrize("tr", [64, 128])
+def test_zeros_tiny_huge_and_non_finite_rows(tr):
+    rng = np.random.default_rng(3)
+    a, b = rng.standard_normal((6, 40)), rng.standard_normal((7, 40))
+    a[1] = 0.0
+    a[2] *= 2.0 ** -1000
+    a[3] *= 1e300
+    a[4, 7] = np.nan
+    a[5, 3] = np.inf
+    b[2] *= 2.0 ** -1060  # denormals
+    b[3] = 0.0
+    d = run(a, b, tr)
+    ok = [0, 1, 2, 3]
+    ref = longdouble_product(a[ok], b)
+    lim = bound(a[ok], b, ref) + 5e-324
+    with np.errstate(over="ignore"):
+        assert np.all(np.abs(d[ok] - ref.astype(np.float64)) <= lim)
+    assert np.all(np.isnan(d[4:])) and not np.any(np.isnan(d[:4]))
+    assert np.all(d[1] == 0.0) and np.all(d[:4, 3] == 0.0)
+
+
+def test_error_against_a_plain_fp64_sum():
+    """Not further from the exact product than FP64 arithmetic, over the library's K range."""
+    for k in (40, 256, 600, 2400):
+        rng = np.random.default_rng(k)
+        a, b = rng.standard_normal((64, k)), rng.standard_normal((48, k))
+        ref = longdouble_product(a, b)
+        plain = np.zeros((64, 48))
+        for i in range(k):  # one FP64 accumulator per element, as a scalar loop
+            plain += a[:, i][:, None] * b[:, i][None, :]
+        err = lambda x: float(np.sqrt(np.mean((x - ref).astype(np.float64) ** 2)))  # noqa: E731
+        assert err(run(a, b, 128)) <= err(plain), k
