@@ -808,6 +808,10 @@ int a_launch_energy(const afq_ctx_dev& c, const AdjointBufs& a, const double2* g
     k_a_energy<<<c.nw, 256, smem, st>>>(c, green, a.ebar, a.gene);
   }
   if (int e = a_err("a_energy")) return e;
+  return a_launch_rot(c, a, green, st);
+}
+
+int a_launch_rot(const afq_ctx_dev& c, const AdjointBufs& a, const double2* green, cudaStream_t st) {
   {
     ProfScope _ps(K_ENERGY_FIN, st);
     k_a_rot<<<(c.ktot + 255) / 256, 256, 0, st>>>(c, green, a.ebar, a.grot[0], a.grot[1]);

@@ -39,6 +39,8 @@ int a_launch_end(int nblk, const double* be, const double* bw, const AdjointBufs
 int a_launch_block_stats(const afq_ctx_dev& c, const AdjointBufs& a, int blk, const double2* energy,
                          const double* weights, const double* scalars, const double* be, cudaStream_t st);
 int a_launch_energy(const afq_ctx_dev& c, const AdjointBufs& a, const double2* green, cudaStream_t st);
+// its rot_h1 cotangent alone
+int a_launch_rot(const afq_ctx_dev& c, const AdjointBufs& a, const double2* green, cudaStream_t st);
 // gt (may be NULL): the trial cotangents, accumulated (gtrial of AdjointBufs)
 int a_launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, const double2* ga, const double2* gb,
                    const double2* lbar, double2* wbu, double2* wbd, cudaStream_t st,

@@ -6,6 +6,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "afq_common.cuh"
@@ -33,7 +34,12 @@ struct DigCtx {
   afq::DigOp xa;    // [2 nw] x nchol
   afq::DigOp ga;    // [2 nw] x ktot
   afq::DigPlan fb;  // K ranges of the force bias
-  double2* fb_part;
+  // exchange energy: U per spin of G (rows (i, q), K = (k, p)); has_u 0: too few vectors for it
+  int has_u;
+  afq::DigOp u[2], ua[2], ub[2];  // ua, ub: rot_chol^T, at set-up only
+  afq::DigPlan uplan[2];
+  double2* z;     // [nw][ktot]
+  double2* part;  // partial results of split K ranges
   int* status;
 };
 
@@ -80,7 +86,9 @@ struct Layout {
 };
 
 struct Sizes {
-  size_t dg, dg_chol[2], dg_rc[2], dg_xa[2], dg_ga[2], dg_part, dg_status;  // digits: [tiles, row exponents]
+  // digits: [tiles, row exponents]
+  size_t dg, dg_chol[2], dg_rc[2], dg_xa[2], dg_ga[2], dg_u[2][2], dg_ua[2], dg_ub[2], dg_end, dg_status;
+  size_t dg_part, dg_z, dg_utmp;
   size_t green, fb, xt, shift, fbt, vhs, ovl_new, ene, epart, rccat, wcopy, sr_idx, cum, free_scr, tc, total;
 };
 
@@ -169,6 +177,18 @@ void dig_dims(const afq_ctx_dev& c, DigCtx* g) {
   op(g->ga, 2 * c.nw, c.ktot, afq::kDigTile);
   const int tiles = ((2 * c.nw + afq::kDigTile - 1) / afq::kDigTile) * ((c.nchol + g->rc.tr - 1) / g->rc.tr);
   g->fb = afq::dig_plan(tiles, g->rc.kb(), kPlanSms, 8);
+  // Z = U G costs 4 (nocc norb)^2 per walker on the tensor cores, about 1/28 of the time of the
+  // same flops on the FP64 units, where the sums over f_g cost 4 nchol norb nocc^2: even at
+  // norb = 28 nchol, and U takes memory, so a quarter of that.
+  g->has_u = c.norb <= 7 * c.nchol ? 1 : 0;
+  for (int s = 0; s < 2; ++s) {
+    const int on = g->has_u && s < c.nspin_g ? c.gocc[s] * c.norb : 0;
+    op(g->u[s], on, on, on ? afq::dig_tr(c.nw, on, 1, kPlanSms) : 16);
+    op(g->ua[s], on, c.nchol, afq::kDigTile);
+    op(g->ub[s], on, c.nchol, 64);
+    const int t = ((2 * c.nw + afq::kDigTile - 1) / afq::kDigTile) * ((on + g->u[s].tr - 1) / g->u[s].tr);
+    g->uplan[s] = afq::dig_plan(t, g->u[s].kb(), kPlanSms, 4);
+  }
 }
 
 Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chunks, size_t welem,
@@ -203,8 +223,17 @@ Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chu
     take(s.dg_rc, g.rc);
     take(s.dg_xa, g.xa);
     take(s.dg_ga, g.ga);
+    for (int i = 0; i < 2; ++i) take(s.dg_u[i], g.u[i]);
+    const int big = g.ua[1].rows > g.ua[0].rows ? 1 : 0;
+    take(s.dg_ua, g.ua[big]);
+    take(s.dg_ub, g.ub[big]);
     s.dg_status = L->take(256);
-    s.dg_part = L->take(afq::dig_partial_bytes(c.nw, c.nchol, g.fb.splits));
+    s.dg_end = L->off;
+    size_t part = afq::dig_partial_bytes(c.nw, c.nchol, g.fb.splits);
+    for (int i = 0; i < 2; ++i) part = std::max(part, afq::dig_partial_bytes(c.nw, g.u[i].rows, g.uplan[i].splits));
+    s.dg_part = L->take(part);
+    s.dg_z = L->take(g.has_u ? nw * c.ktot * C16 : 256);
+    s.dg_utmp = L->take(g.has_u ? (size_t)g.ua[big].rows * g.ua[big].rows * sizeof(double) : 256);
   }
   s.total = L->off;
   return s;
@@ -233,11 +262,26 @@ int green(afq_ctx* c, const void* wu, const void* wd, double2* g, double2* ovl, 
 }
 
 // out [nw][nchol] = alpha g . rc^T (FP64), alpha = 2 (RHF, one slab) or 1
-int fb_gemm(afq_ctx* c, const double2* g, const afq::DigOp& rc, double2* out, cudaStream_t st) {
+int fb_gemm(afq_ctx* c, const double2* g, const afq::DigOp& rc, double2* out, cudaStream_t st, bool coulomb = false) {
   const afq_ctx_dev& d = c->dev;
   CHECK(afq::dig_slice_cplx_rows(c->dg.ga, g, d.ktot, 1.0, st));
-  return afq::dig_gemm_c(afq::K_FB, c->dg.ga, rc, d.nw, d.nchol, out, d.nchol, 0, d.energy_mode == 0 ? 1 : 0, c->dg.fb,
-                         c->dg.fb_part, c->dg.status, st);
+  return afq::dig_gemm_c(coulomb ? afq::K_ENERGY : afq::K_FB, c->dg.ga, rc, d.nw, d.nchol, out, d.nchol, 0,
+                         d.energy_mode == 0 && !coulomb ? 1 : 0, c->dg.fb, c->dg.part, c->dg.status, st);
+}
+
+// The local energy's contractions of c->green: c->fb = Coulomb sums, dg.z = U G (FP64)
+int energy_gemms(afq_ctx* c, cudaStream_t st) {
+  const afq_ctx_dev& d = c->dev;
+  CHECK(fb_gemm(c, c->green, c->dg.rc, c->fb, st, true));
+  for (int s = 0, off = 0; s < d.nspin_g; ++s) {
+    afq::DigOp a = c->dg.ga;
+    a.K = c->dg.u[s].K;
+    if (d.nspin_g == 2) CHECK(afq::dig_slice_cplx_rows(a, c->green + off, d.ktot, 1.0, st));  // else as sliced above
+    CHECK(afq::dig_gemm_c(afq::K_ENERGY, a, c->dg.u[s], d.nw, a.K, c->dg.z + off, d.ktot, 0, 0, c->dg.uplan[s],
+                          c->dg.part, c->dg.status, st));
+    off += a.K;
+  }
+  return 0;
 }
 
 // vhs [nwc][norb^2] = i sqrt(dt) x . chol (FP64)
@@ -258,6 +302,10 @@ int force_bias_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
 
 int energy_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
   if (!is_fp64(c)) return afq::tc_energy(c->tc, c->dev, out, st);
+  if (c->dg.has_u) {
+    CHECK(energy_gemms(c, st));
+    return afq::dig_launch_energy(c->dev, c->green, c->dg.z, c->fb, out, st);
+  }
   return afq::launch_energy_f64(c->dev, c->e_chunks, c->e_gchunk, c->green, c->epart, out, st);
 }
 
@@ -663,8 +711,22 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
     at(c->dg.xa, sz.dg_xa);
     at(c->dg.ga, sz.dg_ga);
     c->dg.status = reinterpret_cast<int*>(ws + sz.dg_status);
-    c->dg.fb_part = reinterpret_cast<double2*>(ws + sz.dg_part);
-    int e = zero(ws + sz.dg, sz.dg_part - sz.dg, st);  // padding stays zero
+    c->dg.part = reinterpret_cast<double2*>(ws + sz.dg_part);
+    c->dg.z = reinterpret_cast<double2*>(ws + sz.dg_z);
+    int e = zero(ws + sz.dg, sz.dg_end - sz.dg, st);  // padding stays zero
+    for (int s = 0; s < dev.nspin_g && c->dg.has_u && !e; ++s) {
+      // U[(i,q),(k,p)] = (X X^T)[(i,p),(k,q)], X = rot_chol^T
+      at(c->dg.u[s], sz.dg_u[s]);
+      at(c->dg.ua[s], sz.dg_ua);
+      at(c->dg.ub[s], sz.dg_ub);
+      const int on = c->dg.u[s].rows;
+      double* tmp = reinterpret_cast<double*>(ws + sz.dg_utmp);
+      if (s == 1) e = zero(ws + sz.dg_ua[0], sz.dg_status - sz.dg_ua[0], st);  // the other spin's rows
+      if (!e) e = afq::dig_slice_real_cols(c->dg.ua[s], dev.rot_chol[s], on, st);
+      if (!e) e = afq::dig_slice_real_cols(c->dg.ub[s], dev.rot_chol[s], on, st);
+      if (!e) e = afq::dig_gemm_r(afq::K_PREP, c->dg.ua[s], c->dg.ub[s], on, on, tmp, on, dev.norb, c->dg.status, st);
+      if (!e) e = afq::dig_slice_real_rows(c->dg.u[s], tmp, on, st);
+    }
     if (!e) e = afq::dig_slice_real_cols(c->dg.chol, ham->chol, (long)dims->norb * dims->norb, st);
     if (!e) e = afq::dig_slice_real_rows(c->dg.rc, dev.nspin_g == 2 ? c->rccat : ham->rot_chol_up, dev.ktot, st);
     if (e) {
@@ -912,7 +974,13 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
       CHECK(afq::t_launch_qr(d, t, state->walkers_up, state->walkers_dn, st));
       CHECK(afq::t_launch_green(d, t, state->walkers_up, state->walkers_dn, ctx->green, t.dgreen, ovl, t.dlo, st));
       CHECK(energy_from_green(ctx, ctx->ene, st));
-      CHECK(afq::t_launch_energy(d, t, ctx->e_chunks, ctx->e_gchunk, ctx->green, st));
+      if (ctx->dg.has_u && !rot) {  // ctx->fb and dg.z are those of the energy just evaluated
+        CHECK(fb_gemm(ctx, t.dgreen, ctx->dg.rc, t.dfb, st, true));
+        CHECK(afq::dig_launch_energy_tangent(d, ctx->green, t.dgreen, ctx->dg.z, ctx->fb, t.dfb, t.drot[0], t.drot[1],
+                                             t.dene, st));
+      } else {
+        CHECK(afq::t_launch_energy(d, t, ctx->e_chunks, ctx->e_gchunk, ctx->green, st));
+      }
       CHECK(afq::launch_block_stats(d, ctx->ene, state->weights, state->scalars, block_energy + blk,
                                     block_weight + blk, st));
       CHECK(afq::t_launch_block_stats(d, t, ctx->ene, state->weights, state->scalars, block_energy + blk,
@@ -1119,7 +1187,16 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
     const int sq_i = b * (P + 2) + P + 1, sw_i = b * (P + 2) + P;
     CHECK(afq::a_launch_block_stats(d, a, b, tp.ene(b), tp.wt(sq_i), tp.sc(sq_i), block_energy, st));
     CHECK(afq::launch_green<double>(d, tp.w(sq_i, 0), tp.w(sq_i, 1), ctx->green, nullptr, true, st));
-    CHECK(afq::a_launch_energy(d, a, ctx->green, st));
+    if (ctx->dg.has_u) {
+      CHECK(energy_gemms(ctx, st));
+      CHECK(afq::dig_slice_cplx_rows(ctx->dg.xa, ctx->fb, d.nchol, 1.0, st));
+      CHECK(afq::dig_gemm_c(afq::K_ENERGY, ctx->dg.xa, ao.rt, d.nw, d.ktot, a.gene, d.ktot, 0, 0,
+                            afq::DigPlan{1, ctx->dg.xa.kb()}, nullptr, ctx->dg.status, st));
+      CHECK(afq::dig_launch_energy_adjoint(d, ctx->dg.z, a.ebar, a.gene, st));
+      CHECK(afq::a_launch_rot(d, a, ctx->green, st));
+    } else {
+      CHECK(afq::a_launch_energy(d, a, ctx->green, st));
+    }
     if (rot) CHECK(afq::a_launch_rc_energy(d, a, ctx->green, st));
     CHECK(afq::a_launch_green(d, tp.w(sq_i, 0), tp.w(sq_i, 1), a.gene, gp ? a.gpend : nullptr, a.lbar, a.wb[0],
                               a.wb[1], st, gt));

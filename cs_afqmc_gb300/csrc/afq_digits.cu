@@ -550,7 +550,7 @@ struct EpiDigR {
     double* d;
     int M, N, tr;
     long ldd;
-    int shift;
+    int shift, swap;
   };
   AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[8]) {
     const int m = w.m * kDigTile + r, n0 = w.n * p.tr + col0;
@@ -558,7 +558,12 @@ struct EpiDigR {
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (n0 + j < p.N) {
-        double* dst = p.d + (size_t)m * p.ldd + n0 + j;
+        int rr = m, cc = n0 + j;
+        if (p.swap) {
+          rr = m - m % p.swap + cc % p.swap;
+          cc = cc - cc % p.swap + m % p.swap;
+        }
+        double* dst = p.d + (size_t)rr * p.ldd + cc;
         *dst = w.add ? *dst + v[j] : v[j];
       }
   }
@@ -571,6 +576,97 @@ __global__ void k_dig_sum(long M, long N, int splits, long sst, const double2* _
     double2 a = part[i];
     for (int s = 1; s < splits; ++s) a = cadd(a, part[i + s * sst]);
     c[(i / N) * ldc + i % N] = a;
+  }
+}
+
+// ======================================================================================
+// Local energy (wavefunctions.py:529-561, 711-743) from Z = U G and the Coulomb sums
+//   exc = sum_g sum_ik f_g[i,k] f_g[k,i] = sum_(i,q) Z[i,q] G[i,q],
+//   U[(i,q),(k,p)] = sum_g rc_g[i,p] rc_g[k,q],   coul_g = tr f_g (both spins together),
+// which is 4 (nocc norb)^2 flops per walker instead of 4 nchol norb nocc^2, and a contraction
+// with one operand for all walkers. U is symmetric: d exc = 2 sum Z dG and d exc / dG = 2 Z.
+// ======================================================================================
+
+AFQ_D double2 block_sum2(double2 v, double* red) { return c2(block_sum(v.x, red), block_sum(v.y, red)); }
+
+__global__ void __launch_bounds__(128) k_dig_energy(const afq_ctx_dev c, const double2* __restrict__ green,
+                                                    const double2* __restrict__ z, const double2* __restrict__ coul,
+                                                    double2* __restrict__ energy) {
+  __shared__ double red[32];
+  const size_t w = blockIdx.x;
+  double2 e1 = c2(0, 0), ex = c2(0, 0), co = c2(0, 0);
+  for (int i = threadIdx.x; i < c.ktot; i += blockDim.x) {
+    const int s = (c.nspin_g == 2 && i >= c.gocc[0] * c.norb) ? 1 : 0;
+    const double2 g = green[w * c.ktot + i];
+    e1 = cadd(e1, cscale(g, c.rot_h1[s][i - s * c.gocc[0] * c.norb]));
+    ex = cadd(ex, cmul(z[w * c.ktot + i], g));
+  }
+  for (int g = threadIdx.x; g < c.nchol; g += blockDim.x) {
+    const double2 x = coul[w * c.nchol + g];
+    co = cadd(co, cmul(x, x));
+  }
+  e1 = block_sum2(e1, red);
+  ex = block_sum2(ex, red);
+  co = block_sum2(co, red);
+  if (threadIdx.x) return;
+  double2 e2;
+  if (c.energy_mode == 0) {  // RHF restricted
+    e1 = cscale(e1, 2.0);
+    e2 = csub(cscale(co, 2.0), ex);
+  } else if (c.energy_mode == 1) {  // RHF two-slab (G = G_up + G_dn)
+    e2 = csub(co, ex);
+  } else {  // UHF
+    e2 = cscale(csub(co, ex), 0.5);
+  }
+  energy[w] = cadd(cadd(e2, e1), c2(c.h0, 0.0));
+}
+
+__global__ void __launch_bounds__(128) k_dig_energy_tangent(const afq_ctx_dev c, const double2* __restrict__ green,
+                                                            const double2* __restrict__ dgreen,
+                                                            const double2* __restrict__ z,
+                                                            const double2* __restrict__ coul,
+                                                            const double2* __restrict__ dcoul, const double* drot_up,
+                                                            const double* drot_dn, double2* __restrict__ denergy) {
+  __shared__ double red[32];
+  const size_t w = blockIdx.x;
+  double2 e1 = c2(0, 0), ex = c2(0, 0), co = c2(0, 0);
+  for (int i = threadIdx.x; i < c.ktot; i += blockDim.x) {
+    const int s = (c.nspin_g == 2 && i >= c.gocc[0] * c.norb) ? 1 : 0, j = i - s * c.gocc[0] * c.norb;
+    const double2 g = green[w * c.ktot + i], dg = dgreen[w * c.ktot + i];
+    const double dr = (s == 0 ? drot_up : drot_dn)[j];
+    e1 = cadd(e1, cadd(cscale(dg, c.rot_h1[s][j]), cscale(g, dr)));
+    ex = cadd(ex, cmul(z[w * c.ktot + i], dg));
+  }
+  for (int g = threadIdx.x; g < c.nchol; g += blockDim.x)
+    co = cadd(co, cmul(coul[w * c.nchol + g], dcoul[w * c.nchol + g]));
+  e1 = block_sum2(e1, red);
+  ex = cscale(block_sum2(ex, red), 2.0);
+  co = cscale(block_sum2(co, red), 2.0);
+  if (threadIdx.x) return;
+  if (c.energy_mode == 0)
+    denergy[w] = cadd(csub(cscale(co, 2.0), ex), cscale(e1, 2.0));
+  else if (c.energy_mode == 1)
+    denergy[w] = cadd(csub(co, ex), e1);
+  else
+    denergy[w] = cadd(cscale(csub(co, ex), 0.5), e1);
+}
+
+// Convention of afq_adjoint.cu: G-bar = e-bar (kappa conj(Z) + gamma conj(sum_g c_g rc_g) + mult1
+// rot_h1); zero for a walker without an energy cotangent, whatever its G holds.
+__global__ void k_dig_energy_adjoint(const afq_ctx_dev c, const double2* __restrict__ z,
+                                     const double* __restrict__ ebar, double2* __restrict__ gene) {
+  const double kappa = c.energy_mode == 2 ? -1.0 : -2.0;
+  const double gamma = c.energy_mode == 0 ? 4.0 : (c.energy_mode == 1 ? 2.0 : 1.0);
+  const double mult1 = c.energy_mode == 0 ? 2.0 : 1.0;
+  const size_t w = blockIdx.x;
+  const double eb = ebar[w];
+  for (int i = threadIdx.x; i < c.ktot; i += blockDim.x) {
+    const int s = (c.nspin_g == 2 && i >= c.gocc[0] * c.norb) ? 1 : 0;
+    const double2 a = z[w * c.ktot + i], b = gene[w * c.ktot + i];
+    const double r = c.rot_h1[s][i - s * c.gocc[0] * c.norb];
+    gene[w * c.ktot + i] = eb == 0.0 ? c2(0, 0)
+                                     : c2(eb * (kappa * a.x + gamma * b.x + mult1 * r),
+                                          -eb * (kappa * a.y + gamma * b.y));
   }
 }
 
@@ -709,12 +805,40 @@ int dig_gemm_c(int cls, const DigOp& A, const DigOp& B, int M, int N, double2* C
   return dig_err("digit GEMM sum");
 }
 
-int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D, long ldd, int* status,
-               cudaStream_t st) {
+int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D, long ldd, int swap,
+               int* status, cudaStream_t st) {
   DigGemm g = dig_args(A, B);
-  EpiDigR::Params ep{D, M, N, B.tr, ldd, 0};
+  EpiDigR::Params ep{D, M, N, B.tr, ldd, 0, swap};
   return B.tr == 128 ? launch_digits<true, EpiDigR>(cls, g, ep, status, st)
                      : launch_digits<false, EpiDigR>(cls, g, ep, status, st);
+}
+
+int dig_launch_energy(const afq_ctx_dev& c, const double2* green, const double2* z, const double2* coul,
+                      double2* energy, cudaStream_t st) {
+  {
+    ProfScope _ps(K_ENERGY_FIN, st);
+    k_dig_energy<<<c.nw, 128, 0, st>>>(c, green, z, coul, energy);
+  }
+  return dig_err("energy");
+}
+
+int dig_launch_energy_tangent(const afq_ctx_dev& c, const double2* green, const double2* dgreen, const double2* z,
+                              const double2* coul, const double2* dcoul, const double* drot_up,
+                              const double* drot_dn, double2* denergy, cudaStream_t st) {
+  {
+    ProfScope _ps(K_ENERGY_FIN, st);
+    k_dig_energy_tangent<<<c.nw, 128, 0, st>>>(c, green, dgreen, z, coul, dcoul, drot_up, drot_dn, denergy);
+  }
+  return dig_err("energy tangent");
+}
+
+int dig_launch_energy_adjoint(const afq_ctx_dev& c, const double2* z, const double* ebar, double2* gene,
+                              cudaStream_t st) {
+  {
+    ProfScope _ps(K_ENERGY_FIN, st);
+    k_dig_energy_adjoint<<<c.nw, 128, 0, st>>>(c, z, ebar, gene);
+  }
+  return dig_err("energy adjoint");
 }
 
 }  // namespace afq
@@ -749,5 +873,5 @@ extern "C" int afq_test_gemm_digits(const double* a, const double* b, double* d,
   }
   if (int rc = dig_slice_real_rows(A, a, K, st)) return rc;
   if (int rc = dig_slice_real_rows(B, b, K, st)) return rc;
-  return dig_gemm_r(K_PREP, A, B, M, N, d, N, status, st);
+  return dig_gemm_r(K_PREP, A, B, M, N, d, N, 0, status, st);
 }

@@ -64,9 +64,22 @@ DigPlan dig_plan(int tiles, int kb, int sms, int max_splits);
 size_t dig_partial_bytes(int M, int N, int splits);
 int dig_gemm_c(int cls, const DigOp& A, const DigOp& B, int M, int N, double2* C, long ldc, int rot, int shift,
                const DigPlan& plan, double2* part, int* status, cudaStream_t st);
-// D[m][n] (real, ldd) = sum_k A[m][k] B[n][k], both real
-int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D, long ldd, int* status,
+// D[m][n] (real, ldd) = sum_k A[m][k] B[n][k], both real. swap > 0: rows m = (i, p) and columns
+// n = (k, q) with p, q < swap; the result goes to row (i, q), column (k, p)
+int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D, long ldd, int swap, int* status,
                cudaStream_t st);
+
+// ---- local energy from the sliced contractions -----------------------------------------
+// z [nw][ktot] = U G per spin, coul [nw][nchol] = rc . G; final sums per walker
+int dig_launch_energy(const afq_ctx_dev& c, const double2* green, const double2* z, const double2* coul,
+                      double2* energy, cudaStream_t st);
+// its tangent: dcoul [nw][nchol], the tangents of G and rot_h1
+int dig_launch_energy_tangent(const afq_ctx_dev& c, const double2* green, const double2* dgreen, const double2* z,
+                              const double2* coul, const double2* dcoul, const double* drot_up,
+                              const double* drot_dn, double2* denergy, cudaStream_t st);
+// its adjoint: gene [nw][ktot] holds sum_g c_g rc_g on entry and the G cotangent on return
+int dig_launch_energy_adjoint(const afq_ctx_dev& c, const double2* z, const double* ebar, double2* gene,
+                              cudaStream_t st);
 int dig_sms();
 // B columns per tile for an output of 2 M x N with kb K blocks: 64 where the tiles (times up to
 // eight K ranges) reach half of the SMs, else 32, so that small problems still spread out; never
