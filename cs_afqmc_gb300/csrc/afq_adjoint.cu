@@ -1007,6 +1007,17 @@ int a_launch_taylor(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc,
                                                       a.wb[1], a.tay, a.wb2[0], a.wb2[1]);
   }
   if (int e = a_err("a_taylor")) return e;
+  if (int e = a_launch_exp_grad(c, a, w0, nwc, wu, wd, st)) return e;
+  const int vt = (c.norb + 31) / 32;
+  {
+    ProfScope _ps(K_TAYLOR, st);
+    k_a_vbar<<<dim3(vt, vt, nwc), 256, 0, st>>>(c, a.tay, a.vbar);
+  }
+  return a_err("a_vbar");
+}
+
+int a_launch_exp_grad(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc, const void* wu, const void* wd,
+                      cudaStream_t st) {
   const size_t esmem = 4 * 16 * (size_t)c.kmax * sizeof(double2);
   cudaFuncSetAttribute(k_a_exp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem);
   const int tiles = (c.norb + 15) / 16;
@@ -1016,13 +1027,7 @@ int a_launch_taylor(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc,
                                                                   (const double2*)wu, (const double2*)wd, a.gexp[0],
                                                                   a.gexp[1]);
   }
-  if (int e = a_err("a_exp_grad")) return e;
-  const int vt = (c.norb + 31) / 32;
-  {
-    ProfScope _ps(K_TAYLOR, st);
-    k_a_vbar<<<dim3(vt, vt, nwc), 256, 0, st>>>(c, a.tay, a.vbar);
-  }
-  return a_err("a_vbar");
+  return a_err("a_exp_grad");
 }
 
 int a_launch_field(const afq_ctx_dev& c, const AdjointBufs& a, const double2* xt, cudaStream_t st) {

@@ -57,6 +57,9 @@ int a_launch_weights(const afq_ctx_dev& c, const AdjointBufs& a, const double2* 
                      const double* scalars, cudaStream_t st);
 int a_launch_taylor(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc, const double2* vhs,
                     const void* wu, const void* wd, cudaStream_t st);
+// exp_h1 cotangents of the chunk, from a.wb, a.tay (a_launch_taylor's layout) and the walkers
+int a_launch_exp_grad(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc, const void* wu, const void* wd,
+                      cudaStream_t st);
 int a_launch_field(const afq_ctx_dev& c, const AdjointBufs& a, const double2* xt, cudaStream_t st);
 int a_launch_sr(const afq_ctx_dev& c, const AdjointBufs& a, const int32_t* idx, cudaStream_t st);
 // chol-bar[g][pq] += sqrt(dt) Re(i sum_w xt[w][g] conj(vhs-bar[w][pq])) over a walker chunk

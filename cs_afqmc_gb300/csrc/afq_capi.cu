@@ -40,6 +40,9 @@ struct DigCtx {
   afq::DigPlan uplan[2];
   double2* z;     // [nw][ktot]
   double2* part;  // partial results of split K ranges
+  int use_walk;   // Taylor products on the digit GEMM (walk), else k_taylor_f64
+  afq::DigWalk walk;
+  double2 *walk_t, *walk_acc;  // [chunk][norb * (k0 + k1)]
   int* status;
 };
 
@@ -87,8 +90,9 @@ struct Layout {
 
 struct Sizes {
   // digits: [tiles, row exponents]
-  size_t dg, dg_chol[2], dg_rc[2], dg_xa[2], dg_ga[2], dg_u[2][2], dg_ua[2], dg_ub[2], dg_end, dg_status;
+  size_t dg, dg_chol[2], dg_rc[2], dg_xa[2], dg_ga[2], dg_u[2][2], dg_ua[2], dg_ub[2], dg_uend, dg_end, dg_status;
   size_t dg_part, dg_z, dg_utmp;
+  size_t dg_e[2][2], dg_v[2], dg_x[2], dg_wt, dg_wa;
   size_t green, fb, xt, shift, fbt, vhs, ovl_new, ene, epart, rccat, wcopy, sr_idx, cum, free_scr, tc, total;
 };
 
@@ -164,7 +168,8 @@ int derive(const afq_dims* d, afq_ctx_dev* c, int* nw_chunk, int* e_chunks, int*
 // Shapes of the sliced FP64 operands (no pointers). The plan assumes the full part's 152 SMs, so
 // that workspace sizes do not depend on where they are asked for.
 constexpr int kPlanSms = 152;
-void dig_dims(const afq_ctx_dev& c, DigCtx* g) {
+constexpr long kWalkMin = 1000000;
+void dig_dims(const afq_ctx_dev& c, int nw_chunk, DigCtx* g) {
   const int nn = c.norb * c.norb;
   auto op = [](afq::DigOp& o, int rows, int K, int tr) {
     o.rows = rows;
@@ -189,6 +194,8 @@ void dig_dims(const afq_ctx_dev& c, DigCtx* g) {
     const int t = ((2 * c.nw + afq::kDigTile - 1) / afq::kDigTile) * ((on + g->u[s].tr - 1) / g->u[s].tr);
     g->uplan[s] = afq::dig_plan(t, g->u[s].kb(), kPlanSms, 4);
   }
+  afq::dig_walk_dims(c.norb, c.kslab, c.nslab, nw_chunk, &g->walk);
+  g->use_walk = c.norb <= 256 && (long)nw_chunk * g->walk.ncol * nn >= kWalkMin;
 }
 
 Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chunks, size_t welem,
@@ -213,7 +220,7 @@ Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chu
                                                 : 256);
   if (d->precision == AFQ_PREC_FP64) {
     DigCtx g;
-    dig_dims(c, &g);
+    dig_dims(c, nw_chunk, &g);
     auto take = [&](size_t (&o)[2], const afq::DigOp& op) {
       o[0] = L->take(afq::dig_bytes(op.rows, op.K, op.tr));
       o[1] = L->take(afq::dig_exps(op.rows, op.tr));
@@ -227,8 +234,17 @@ Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chu
     const int big = g.ua[1].rows > g.ua[0].rows ? 1 : 0;
     take(s.dg_ua, g.ua[big]);
     take(s.dg_ub, g.ub[big]);
+    s.dg_uend = L->off;
+    for (int i = 0; i < c.nslab; ++i) take(s.dg_e[i], g.walk.e[i]);
+    s.dg_v[0] = L->take(g.use_walk ? afq::dig_walk_v_bytes(g.walk) : 256);
+    s.dg_v[1] = L->take(g.use_walk ? afq::dig_walk_ve_bytes(g.walk) : 256);
+    s.dg_x[0] = L->take(g.use_walk ? afq::dig_walk_x_bytes(g.walk) : 256);
+    s.dg_x[1] = L->take(g.use_walk ? afq::dig_walk_xe_bytes(g.walk) : 256);
     s.dg_status = L->take(256);
     s.dg_end = L->off;
+    const size_t wt = g.use_walk ? (size_t)g.walk.chunk * c.norb * g.walk.ncol * C16 : 256;
+    s.dg_wt = L->take(wt);
+    s.dg_wa = L->take(wt);
     size_t part = afq::dig_partial_bytes(c.nw, c.nchol, g.fb.splits);
     for (int i = 0; i < 2; ++i) part = std::max(part, afq::dig_partial_bytes(c.nw, g.u[i].rows, g.uplan[i].splits));
     s.dg_part = L->take(part);
@@ -322,6 +338,112 @@ int check_state(const afq_ctx* c, const afq_walker_state* s) {
   return 0;
 }
 
+// The walker slabs from walker w0 on, and a [walker][norb * (k0 + k1)] buffer.
+afq::WalkVec walk_slabs(const afq_ctx_dev& d, void* wu, void* wd, size_t w0) {
+  const size_t a = (size_t)d.norb * d.kslab[0], b = (size_t)d.norb * d.kslab[1];
+  return {{static_cast<double2*>(wu) + w0 * a, d.nslab == 2 ? static_cast<double2*>(wd) + w0 * b : nullptr}, a, b};
+}
+afq::WalkVec walk_buf(const afq_ctx_dev& d, double2* p, size_t nterm = 1) {
+  const size_t a = (size_t)d.norb * d.kslab[0], b = (size_t)d.norb * d.kslab[1];
+  return {{p, d.nslab == 2 ? p + a : nullptr}, nterm * (a + b), nterm * (a + b)};
+}
+
+// out = E_s y_s for every slab (y sliced); acc (optional) = out
+int walk_exp(const afq::DigWalk& w, const afq_ctx_dev& d, const afq::DigOp* E, const afq::WalkOut& o, int nw,
+             cudaStream_t st) {
+  for (int s = 0; s < d.nslab; ++s) CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w, s, E, o, nw, st));
+  return 0;
+}
+
+// W <- E exp(V) E W (propagation.py:67-92) of nwc walkers from w0 on, FP64
+int taylor_fp64(afq_ctx* c, int w0, int nwc, const double2* vhs, void* wu, void* wd, cudaStream_t st) {
+  const afq_ctx_dev& d = c->dev;
+  if (!c->dg.use_walk) return afq::launch_taylor_f64<double>(d, w0, nwc, vhs, wu, wd, st);
+  const afq::DigWalk& w = c->dg.walk;
+  const afq::WalkVec T = walk_buf(d, c->dg.walk_t), A = walk_buf(d, c->dg.walk_acc);
+  for (int k = 0; k < nwc; k += w.chunk) {
+    const int nw = std::min(w.chunk, nwc - k);
+    const afq::WalkVec W = walk_slabs(d, wu, wd, (size_t)w0 + k);
+    CHECK(afq::dig_walk_slice_v(w, vhs + (size_t)k * d.norb * d.norb, nw, false, st));
+    CHECK(afq::dig_walk_slice_y(w, W, nw, st));
+    afq::WalkOut o;
+    o.out = T;
+    o.acc = A;
+    o.init = 1;
+    CHECK(walk_exp(w, d, w.e, o, nw, st));
+    o.init = 0;
+    double fact = 1.0;
+    for (int m = 1; m < d.n_exp_terms; ++m) {
+      fact *= (double)m;
+      o.facc = 1.0 / fact;
+      CHECK(afq::dig_walk_slice_y(w, T, nw, st));
+      CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w, -1, nullptr, o, nw, st));
+    }
+    CHECK(afq::dig_walk_slice_y(w, A, nw, st));
+    afq::WalkOut last;
+    last.out = W;
+    CHECK(walk_exp(w, d, w.e, last, nw, st));
+  }
+  return 0;
+}
+
+// The same with tangents (t_launch_taylor's products): V and the walkers in w's digits, their
+// tangents in dw's.
+int taylor_jvp(afq_ctx* c, const afq::TangentBufs& t, const afq::DigWalk& dw, double2* dt_buf, double2* da_buf, int w0,
+               int nwc, const double2* vhs, void* wu, void* wd, cudaStream_t st) {
+  const afq_ctx_dev& d = c->dev;
+  const afq::DigWalk& w = c->dg.walk;
+  const afq::WalkVec T = walk_buf(d, c->dg.walk_t), A = walk_buf(d, c->dg.walk_acc), dT = walk_buf(d, dt_buf),
+                     dA = walk_buf(d, da_buf);
+  afq::DigWalk w_dy = w, dw_y = dw;  // V with the tangent columns, dV with the value columns
+  w_dy.xd = dw.xd;
+  w_dy.xe = dw.xe;
+  dw_y.xd = w.xd;
+  dw_y.xe = w.xe;
+  for (int k = 0; k < nwc; k += w.chunk) {
+    const int nw = std::min(w.chunk, nwc - k);
+    const size_t vo = (size_t)k * d.norb * d.norb;
+    const afq::WalkVec W = walk_slabs(d, wu, wd, (size_t)w0 + k), dW = walk_slabs(d, t.dw[0], t.dw[1], (size_t)w0 + k);
+    CHECK(afq::dig_walk_slice_v(w, vhs + vo, nw, false, st));
+    CHECK(afq::dig_walk_slice_v(dw, t.dvhs + vo, nw, false, st));
+    // (out, acc) = (r, acc + f r) of r = X y, and of its tangent X dy + dX y
+    auto both = [&](const afq::WalkVec& y, const afq::WalkVec& dy, int e, afq::WalkOut o, afq::WalkOut od) -> int {
+      CHECK(afq::dig_walk_slice_y(w, y, nw, st));
+      CHECK(afq::dig_walk_slice_y(dw, dy, nw, st));
+      afq::WalkOut part;
+      part.out = od.out;
+      od.in = od.out;
+      if (e < 0) {
+        CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w, -1, nullptr, o, nw, st));
+        CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w_dy, -1, nullptr, part, nw, st));
+        return afq::dig_walk_mul(afq::K_TAYLOR, dw_y, -1, nullptr, od, nw, st);
+      }
+      CHECK(walk_exp(w, d, w.e, o, nw, st));
+      CHECK(walk_exp(w_dy, d, w.e, part, nw, st));
+      return walk_exp(dw_y, d, dw.e, od, nw, st);
+    };
+    afq::WalkOut o, od;
+    o.out = T;
+    o.acc = A;
+    od.out = dT;
+    od.acc = dA;
+    o.init = od.init = 1;
+    CHECK(both(W, dW, 0, o, od));
+    o.init = od.init = 0;
+    double fact = 1.0;
+    for (int m = 1; m < d.n_exp_terms; ++m) {
+      fact *= (double)m;
+      o.facc = od.facc = 1.0 / fact;
+      CHECK(both(T, dT, -1, o, od));
+    }
+    afq::WalkOut last, dlast;
+    last.out = W;
+    dlast.out = dW;
+    CHECK(both(A, dA, 0, last, dlast));
+  }
+  return 0;
+}
+
 // chain: a step inside afq_propagate_phaseless, where the Green's-function work of the
 // previous overlap evaluation on the same walkers (c->gstate) is reused.
 // next_g (with chain): the next operation propagates the same walkers again, so the overlap
@@ -345,7 +467,7 @@ int propagate_impl(afq_ctx* c, afq_walker_state* s, const double* fields, cudaSt
   for (int b = 0; b < nb; ++b) {
     const int w0 = b * c->nw_chunk;
     CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
-    CHECK(afq::launch_taylor_f64<double>(d, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
+    CHECK(taylor_fp64(c, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
   }
   CHECK(green(c, s->walkers_up, s->walkers_dn, nullptr, c->ovl_new, false, st));
   return afq::launch_weights(d, c->shift, c->fbt, 1, c->ovl_new, reinterpret_cast<double2*>(s->overlaps),
@@ -384,7 +506,7 @@ int free_step(afq_ctx* c, afq_walker_state* s, const double* fields, double ene0
   for (int b = 0; b < nb; ++b) {
     const int w0 = b * c->nw_chunk;
     CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
-    CHECK(afq::launch_taylor_f64<double>(d, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
+    CHECK(taylor_fp64(c, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
   }
   CHECK(afq::launch_free_scale(d, consts, s->walkers_up, s->walkers_dn, st));
   CHECK(afq::launch_qr<double>(d, s->walkers_up, s->walkers_dn, st, rdiag));
@@ -413,6 +535,7 @@ int check_free(const afq_ctx* c) {
 struct TSizes {
   size_t dw[2], wold[2], dgreen, dfb, dxt, dshift, dfbt, dvhs, dlo, dlo_new, dweights, dscalars, dene, dpart,
       dsum, drccat, drc_d, drc_e, total;  // drc_*: sliced drccat
+  size_t wk, de[2][2], v[2], x[2], wt, wa;  // digits of the tangent Taylor products
 };
 
 TSizes tangent_sizes(const afq_ctx_dev& c, int nw_chunk, int e_chunks, Layout* L) {
@@ -437,17 +560,36 @@ TSizes tangent_sizes(const afq_ctx_dev& c, int nw_chunk, int e_chunks, Layout* L
   s.dsum = L->take(sizeof(double));
   s.drccat = L->take(c.nspin_g == 2 ? (size_t)c.nchol * c.ktot * sizeof(double) : 256);
   DigCtx g;
-  dig_dims(c, &g);
+  dig_dims(c, nw_chunk, &g);
   s.drc_d = L->take(afq::dig_bytes(g.rc.rows, g.rc.K, g.rc.tr));
   s.drc_e = L->take(afq::dig_exps(g.rc.rows, g.rc.tr));
+  s.wk = L->off;
+  if (g.use_walk) {
+    for (int i = 0; i < c.nslab; ++i) {
+      s.de[i][0] = L->take(afq::dig_bytes(c.norb, c.norb));
+      s.de[i][1] = L->take(afq::dig_exps(c.norb));
+    }
+    s.v[0] = L->take(afq::dig_walk_v_bytes(g.walk));
+    s.v[1] = L->take(afq::dig_walk_ve_bytes(g.walk));
+    s.x[0] = L->take(afq::dig_walk_x_bytes(g.walk));
+    s.x[1] = L->take(afq::dig_walk_xe_bytes(g.walk));
+    s.wt = L->take((size_t)g.walk.chunk * c.norb * g.walk.ncol * C16);
+    s.wa = L->take((size_t)g.walk.chunk * c.norb * g.walk.ncol * C16);
+  }
   s.total = L->off;
   return s;
 }
 
+// The Taylor products' tangent operands: dV, the tangent columns and d exp_h1; term and sum.
+struct JvpWalk {
+  afq::DigWalk w;
+  double2 *t, *a;
+};
+
 // One phaseless step with tangents (propagate_impl's FP64 branch, each stage followed by
 // its tangent).
 int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, const afq::DigOp& drc,
-                  const double* fields, cudaStream_t st) {
+                  const JvpWalk& jw, const double* fields, cudaStream_t st) {
   const afq_ctx_dev& d = c->dev;
   CHECK(afq::t_launch_green(d, t, s->walkers_up, s->walkers_dn, c->green, t.dgreen, c->ovl_new, t.dlo_new, st));
   CHECK(force_bias_from_green(c, c->fb, st));
@@ -462,7 +604,10 @@ int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, co
     const int w0 = b * c->nw_chunk;
     CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
     CHECK(vhs_gemm(c, t.dxt + (size_t)w0 * d.nchol, c->nw_chunk, t.dvhs, st));
-    CHECK(afq::t_launch_taylor(d, t, w0, c->nw_chunk, c->vhs, t.dvhs, s->walkers_up, s->walkers_dn, st));
+    if (c->dg.use_walk)
+      CHECK(taylor_jvp(c, t, jw.w, jw.t, jw.a, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
+    else
+      CHECK(afq::t_launch_taylor(d, t, w0, c->nw_chunk, c->vhs, t.dvhs, s->walkers_up, s->walkers_dn, st));
   }
   CHECK(afq::t_launch_green(d, t, s->walkers_up, s->walkers_dn, nullptr, nullptr, c->ovl_new, t.dlo_new, st));
   return afq::t_launch_weights(d, t, c->shift, c->fbt, c->ovl_new, reinterpret_cast<double2*>(s->overlaps),
@@ -482,6 +627,9 @@ struct AdjOps {
   afq::DigOp cn, rt, va;
   afq::DigPlan xtb;
 };
+// The Taylor adjoint on the digit GEMM (at least one V product)
+bool adj_walk(const afq_ctx_dev& c, const DigCtx& g) { return g.use_walk && c.n_exp_terms >= 2; }
+
 AdjOps adj_ops(const afq_ctx_dev& c, int nwc) {
   AdjOps o;
   const int nn = c.norb * c.norb, kb = (nn + 15) / 16;
@@ -505,7 +653,7 @@ AdjOps adj_ops(const afq_ctx_dev& c, int nwc) {
 struct AdjSizes {
   size_t snap_w, snap_wt, snap_ov, snap_sc, t_xt, t_sh, t_fbt, t_ene, t_idx;
   size_t wb, wb2, wbar, lbar, lbar2, gpend, gene, fbb, xtb, shb, fbtb, vbar, tay, ebar, scal, beb, bwb, total;
-  size_t dg_end, part;
+  size_t dg_end, part, et[2][2], vb_ad, vb_ae, vb_bd, vb_be;  // exp_h1^T; operands of the V cotangents
   size_t dg, cn_d, cn_e, rt_d, rt_e, va_d, va_e;  // digits: chol (rows g), rot_chol^T, V cotangents
   size_t wslab;  // walker elements of one snapshot, both slabs
   int nblk, nsteps, nsnap;
@@ -552,6 +700,20 @@ AdjSizes adjoint_sizes(const afq_ctx_dev& c, int nw_chunk, int n_prop, int n_ene
   s.rt_e = L->take(afq::dig_exps(o.rt.rows, o.rt.tr));
   s.va_d = L->take(afq::dig_bytes(o.va.rows, o.va.K));
   s.va_e = L->take(afq::dig_exps(o.va.rows));
+  DigCtx g;
+  dig_dims(c, nw_chunk, &g);
+  if (adj_walk(c, g)) {
+    afq::DigVbar v;
+    afq::dig_walk_vbar_dims(g.walk, c.n_exp_terms - 1, &v);
+    for (int i = 0; i < c.nslab; ++i) {
+      s.et[i][0] = L->take(afq::dig_bytes(c.norb, c.norb));
+      s.et[i][1] = L->take(afq::dig_exps(c.norb));
+    }
+    s.vb_ad = L->take(afq::dig_walk_vbar_a_bytes(g.walk, v));
+    s.vb_ae = L->take(afq::dig_walk_vbar_ae_bytes(g.walk, v));
+    s.vb_bd = L->take(afq::dig_walk_vbar_b_bytes(g.walk, v));
+    s.vb_be = L->take(afq::dig_walk_vbar_be_bytes(g.walk, v));
+  }
   s.dg_end = L->off;
   s.part = L->take(afq::dig_partial_bytes(nw_chunk, c.nchol, o.xtb.splits));
   s.total = L->off;
@@ -580,6 +742,62 @@ struct Tape {
   double2* ene(int blk) const { return reinterpret_cast<double2*>(base + s.t_ene) + (size_t)blk * d->nw; }
   int32_t* idx(int sr) const { return reinterpret_cast<int32_t*>(base + s.t_idx) + (size_t)sr * d->nw; }
 };
+
+// The Taylor adjoint (a_launch_taylor's chain and layout of a.tay) on the digit GEMM: products
+// with V, then with V^H, then the V cotangents; et: exp_h1^T per slab.
+int taylor_vjp(afq_ctx* c, const afq::AdjointBufs& a, const afq::DigOp* et, const afq::DigVbar& vb, int w0, int nwc,
+               const double2* vhs, double2* wu, double2* wd, cudaStream_t st) {
+  const afq_ctx_dev& d = c->dev;
+  const afq::DigWalk& w = c->dg.walk;
+  const int M = d.n_exp_terms - 1, T = 2 * M + 2;
+  const size_t nk = (size_t)d.norb * w.ncol, nn = (size_t)d.norb * d.norb;
+  const afq::WalkVec B = walk_buf(d, c->dg.walk_acc);  // W'-bar through exp_h1^T
+  for (int k = 0; k < nwc; k += w.chunk) {
+    const int nw = std::min(w.chunk, nwc - k);
+    double2* tay = a.tay + (size_t)k * T * nk;
+    auto term = [&](int i) { return walk_buf(d, tay + (size_t)i * nk, T); };
+    CHECK(afq::dig_walk_slice_v(w, vhs + k * nn, nw, false, st));
+    CHECK(afq::dig_walk_slice_y(w, walk_slabs(d, wu, wd, (size_t)w0 + k), nw, st));
+    afq::WalkOut f;
+    f.out = term(0);
+    f.acc = term(2 * M);
+    f.init = 1;
+    CHECK(walk_exp(w, d, w.e, f, nw, st));
+    f.init = 0;
+    double fact = 1.0;
+    for (int m = 1; m <= M; ++m) {
+      fact *= (double)m;
+      f.facc = 1.0 / fact;
+      f.out = m < M ? term(m) : afq::WalkVec{{nullptr, nullptr}, 0};
+      CHECK(afq::dig_walk_slice_y(w, term(m - 1), nw, st));
+      CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w, -1, nullptr, f, nw, st));
+    }
+    CHECK(afq::dig_walk_slice_v(w, vhs + k * nn, nw, true, st));
+    CHECK(afq::dig_walk_slice_y(w, walk_slabs(d, a.wb[0], a.wb[1], (size_t)w0 + k), nw, st));
+    afq::WalkOut top;
+    top.out = term(2 * M - 1);
+    top.fout = 1.0 / fact;
+    top.acc = B;
+    top.init = 1;
+    CHECK(walk_exp(w, d, et, top, nw, st));
+    double invf = 1.0 / fact;
+    for (int m = M - 1; m >= 0; --m) {
+      invf *= (double)(m + 1);  // 1 / m!
+      CHECK(afq::dig_walk_slice_y(w, term(M + m), nw, st));
+      afq::WalkOut o;
+      o.out = term(m >= 1 ? M + m - 1 : 2 * M + 1);
+      o.in = B;
+      o.fin = invf;
+      CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w, -1, nullptr, o, nw, st));
+    }
+    CHECK(afq::dig_walk_slice_y(w, term(2 * M + 1), nw, st));
+    afq::WalkOut out;
+    out.out = walk_slabs(d, a.wb2[0], a.wb2[1], (size_t)w0 + k);
+    CHECK(walk_exp(w, d, et, out, nw, st));
+    CHECK(afq::dig_walk_vbar(w, vb, tay, T, M, 0, M, a.vbar + k * nn, nw, st));
+  }
+  return afq::a_launch_exp_grad(d, a, w0, nwc, wu, wd, st);
+}
 
 int snapshot(const Tape& t, int i, const afq_walker_state* st_, cudaStream_t st) {
   const afq_ctx_dev& d = *t.d;
@@ -701,7 +919,7 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
     }
   }
   if (dims->precision == AFQ_PREC_FP64) {
-    dig_dims(c->dev, &c->dg);
+    dig_dims(c->dev, nwc, &c->dg);
     auto at = [&](afq::DigOp& o, const size_t (&off)[2]) {
       o.d = reinterpret_cast<unsigned char*>(ws + off[0]);
       o.e = reinterpret_cast<int*>(ws + off[1]);
@@ -714,6 +932,17 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
     c->dg.part = reinterpret_cast<double2*>(ws + sz.dg_part);
     c->dg.z = reinterpret_cast<double2*>(ws + sz.dg_z);
     int e = zero(ws + sz.dg, sz.dg_end - sz.dg, st);  // padding stays zero
+    c->dg.walk.vd = reinterpret_cast<unsigned char*>(ws + sz.dg_v[0]);
+    c->dg.walk.ve = reinterpret_cast<int*>(ws + sz.dg_v[1]);
+    c->dg.walk.xd = reinterpret_cast<unsigned char*>(ws + sz.dg_x[0]);
+    c->dg.walk.xe = reinterpret_cast<int*>(ws + sz.dg_x[1]);
+    c->dg.walk.status = c->dg.status;
+    c->dg.walk_t = reinterpret_cast<double2*>(ws + sz.dg_wt);
+    c->dg.walk_acc = reinterpret_cast<double2*>(ws + sz.dg_wa);
+    for (int s = 0; s < dev.nslab && !e; ++s) {
+      at(c->dg.walk.e[s], sz.dg_e[s]);
+      e = afq::dig_slice_real_rows(c->dg.walk.e[s], dev.exp_h1[s], dev.norb, st);
+    }
     for (int s = 0; s < dev.nspin_g && c->dg.has_u && !e; ++s) {
       // U[(i,q),(k,p)] = (X X^T)[(i,p),(k,q)], X = rot_chol^T
       at(c->dg.u[s], sz.dg_u[s]);
@@ -721,7 +950,7 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
       at(c->dg.ub[s], sz.dg_ub);
       const int on = c->dg.u[s].rows;
       double* tmp = reinterpret_cast<double*>(ws + sz.dg_utmp);
-      if (s == 1) e = zero(ws + sz.dg_ua[0], sz.dg_status - sz.dg_ua[0], st);  // the other spin's rows
+      if (s == 1) e = zero(ws + sz.dg_ua[0], sz.dg_uend - sz.dg_ua[0], st);  // the other spin's rows
       if (!e) e = afq::dig_slice_real_cols(c->dg.ua[s], dev.rot_chol[s], on, st);
       if (!e) e = afq::dig_slice_real_cols(c->dg.ub[s], dev.rot_chol[s], on, st);
       if (!e) e = afq::dig_gemm_r(afq::K_PREP, c->dg.ua[s], c->dg.ub[s], on, on, tmp, on, dev.norb, c->dg.status, st);
@@ -954,6 +1183,20 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
   drc.d = reinterpret_cast<unsigned char*>(tw + ts.drc_d);
   drc.e = reinterpret_cast<int*>(tw + ts.drc_e);
   if (t.drccat) CHECK(afq::dig_slice_real_rows(drc, t.drccat, d.ktot, st));
+  JvpWalk jw{ctx->dg.walk, nullptr, nullptr};
+  if (ctx->dg.use_walk) {  // (the workspace was cleared above: padding is zero)
+    jw.w.vd = reinterpret_cast<unsigned char*>(tw + ts.v[0]);
+    jw.w.ve = reinterpret_cast<int*>(tw + ts.v[1]);
+    jw.w.xd = reinterpret_cast<unsigned char*>(tw + ts.x[0]);
+    jw.w.xe = reinterpret_cast<int*>(tw + ts.x[1]);
+    jw.t = reinterpret_cast<double2*>(tw + ts.wt);
+    jw.a = reinterpret_cast<double2*>(tw + ts.wa);
+    for (int k = 0; k < d.nslab; ++k) {
+      jw.w.e[k].d = reinterpret_cast<unsigned char*>(tw + ts.de[k][0]);
+      jw.w.e[k].e = reinterpret_cast<int*>(tw + ts.de[k][1]);
+      CHECK(afq::dig_slice_real_rows(jw.w.e[k], t.dexp[k], d.norb, st));
+    }
+  }
   double2* ovl = reinterpret_cast<double2*>(state->overlaps);
   const size_t welems[2] = {(size_t)d.nw * d.norb * d.kslab[0], (size_t)d.nw * d.norb * d.kslab[1]};
   void* wslab[2] = {state->walkers_up, state->walkers_dn};
@@ -966,7 +1209,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
     for (int eb = 0; eb < n_ene_blocks; ++eb, ++blk) {
       for (int p = 0; p < n_prop_steps; ++p) {
         const double* f = fields + ((size_t)blk * n_prop_steps + p) * step_elems;
-        CHECK(propagate_jvp(ctx, state, t, drc, f, st));
+        CHECK(propagate_jvp(ctx, state, t, drc, jw, f, st));
       }
       for (int k = 0; k < d.nslab; ++k)
         CHECK(copy_d2d(t.wold[k], wslab[k], welems[k] * sizeof(double2), st, "walker copy before QR"));
@@ -1170,6 +1413,21 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
   CHECK(zero(base + as.dg, as.dg_end - as.dg, st));
   CHECK(afq::dig_slice_real_rows(ao.cn, ctx->h.chol, nn, st));
   CHECK(afq::dig_slice_real_cols(ao.rt, brc, d.ktot, st));
+  const bool walk = adj_walk(d, ctx->dg);
+  afq::DigOp et[2] = {ctx->dg.walk.e[0], ctx->dg.walk.e[1]};
+  afq::DigVbar vb;
+  if (walk) {
+    afq::dig_walk_vbar_dims(ctx->dg.walk, d.n_exp_terms - 1, &vb);
+    vb.ad = reinterpret_cast<unsigned char*>(base + as.vb_ad);
+    vb.ae = reinterpret_cast<int*>(base + as.vb_ae);
+    vb.bd = reinterpret_cast<unsigned char*>(base + as.vb_bd);
+    vb.be = reinterpret_cast<int*>(base + as.vb_be);
+    for (int k = 0; k < d.nslab; ++k) {
+      et[k].d = reinterpret_cast<unsigned char*>(base + as.et[k][0]);
+      et[k].e = reinterpret_cast<int*>(base + as.et[k][1]);
+      CHECK(afq::dig_slice_real_cols(et[k], d.exp_h1[k], d.norb, st));
+    }
+  }
   const double alpha = d.energy_mode == 0 ? 2.0 : 1.0;
   bool gp = false;  // a.gpend holds the pending G cotangent of the current point
   for (int b = blk - 1; b >= 0; --b) {
@@ -1214,7 +1472,10 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
       for (int k = 0; k < nb; ++k) {
         const int w0 = k * nwc;
         CHECK(vhs_gemm(ctx, tp.xt(step) + (size_t)w0 * d.nchol, nwc, ctx->vhs, st));
-        CHECK(afq::a_launch_taylor(d, a, w0, nwc, ctx->vhs, tp.w(start, 0), tp.w(start, 1), st));
+        if (walk)
+          CHECK(taylor_vjp(ctx, a, et, vb, w0, nwc, ctx->vhs, tp.w(start, 0), tp.w(start, 1), st));
+        else
+          CHECK(afq::a_launch_taylor(d, a, w0, nwc, ctx->vhs, tp.w(start, 0), tp.w(start, 1), st));
         if (cg) CHECK(afq::a_launch_chol_grad(d, a, nwc, tp.xt(step) + (size_t)w0 * d.nchol, st));
         CHECK(afq::dig_slice_cplx_rows(ao.va, a.vbar, nn, sqrt(d.dt), st));
         CHECK(afq::dig_gemm_c(afq::K_FB, ao.va, ao.cn, nwc, d.nchol, a.xtb + (size_t)w0 * d.nchol, d.nchol, 3, 0,

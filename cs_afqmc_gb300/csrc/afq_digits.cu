@@ -2,6 +2,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 #include "afq_common.cuh"
 #include "afq_digits.cuh"
 #include "afq_prof.cuh"
@@ -182,6 +184,189 @@ __global__ void __launch_bounds__(256) k_dig_real_cols(const double* __restrict_
   }
 }
 
+// y -> B digits of DigWalk. One CTA per walker; a work item is eight orbitals of one column.
+__global__ void __launch_bounds__(256) k_dig_walk_y(const double2* __restrict__ y0, const double2* __restrict__ y1,
+                                                    size_t ws0, size_t ws1, int o0, int ncol, int n, int np, int nt,
+                                                    int tr, unsigned char* __restrict__ d, int* __restrict__ e) {
+  __shared__ unsigned key[128];
+  const int w = blockIdx.x, kb = np >> 3, nchunk = np >> 3;
+  const int o1 = ncol - o0, items = ncol * nchunk;
+  for (int i = threadIdx.x; i < ncol; i += blockDim.x) key[i] = 0;
+  __syncthreads();
+  auto load = [&](int it, int& c, int& ch, double2 (&v)[8]) {
+    c = it % ncol;
+    ch = it / ncol;
+    const double2* src = c < o0 ? y0 + w * ws0 + c : y1 + w * ws1 + (c - o0);
+    const int o = c < o0 ? o0 : o1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int p = 8 * ch + i;
+      v[i] = p < n ? src[(size_t)p * o] : c2(0.0, 0.0);
+    }
+  };
+  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+    int c, ch;
+    double2 v[8];
+    load(it, c, ch, v);
+    unsigned k = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) k = max(k, max(dig_key(v[i].x), dig_key(v[i].y)));
+    atomicMax(&key[c], k);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ncol; i += blockDim.x) {
+    const int x = dig_row_exp(key[i]);
+    e[(size_t)w * nt * tr + 2 * i] = x;
+    e[(size_t)w * nt * tr + 2 * i + 1] = x;
+  }
+  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+    int c, ch;
+    double2 v[8];
+    load(it, c, ch, v);
+    const int x = dig_row_exp(key[c]), row = 2 * c, tile = row / tr, r = row % tr;
+    unsigned char* b = d + ((size_t)(w * nt + tile) * kb + (ch >> 1)) * ((size_t)tr * 256);
+    unsigned char* b2 = b + (size_t)(np >> 4) * ((size_t)tr * 256);
+    long long q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = dig_fixed(v[i].x, x);
+    dig_store(q, b, tr, r, ch & 1);
+    dig_store(q, b2, tr, r + 1, ch & 1);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = dig_fixed(v[i].y, x);
+    dig_store(q, b, tr, r + 1, ch & 1);
+    dig_store(q, b2, tr, r, ch & 1, 0x80008000u);
+  }
+}
+
+// V [w][n][n] -> A digits, rows p, K = [Re V[p][q] | Im V[p][q]]. LPR lanes per row, eight q each
+// (LPR * 8 >= np).
+template <int LPR>
+__global__ void __launch_bounds__(256) k_dig_walk_v(const double2* __restrict__ V, int nrows, int n, int np, int mt,
+                                                    unsigned char* __restrict__ d, int* __restrict__ e) {
+  const int g = (blockIdx.x * 256 + threadIdx.x) / LPR, ch = threadIdx.x % LPR, kb = np >> 3;
+  const bool in = g < nrows;
+  const int w = in ? g / n : 0, p = in ? g % n : 0;
+  const double2* src = V + ((size_t)w * n + p) * n;
+  double2 v[8];
+  unsigned k = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int q = 8 * ch + i;
+    v[i] = in && q < n ? src[q] : c2(0.0, 0.0);
+    k = max(k, max(dig_key(v[i].x), dig_key(v[i].y)));
+  }
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+  if (!in) return;
+  const int x = dig_row_exp(k);
+  if (ch == 0) e[(size_t)w * mt * kDigTile + p] = x;
+  if (8 * ch >= np) return;
+  unsigned char* b = dig_block(d + (size_t)w * mt * kb * (kDigTile * 256), p, ch >> 1, kb, kDigTile);
+  long long q8[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q8[i] = dig_fixed(v[i].x, x);
+  dig_store(q8, b, kDigTile, p & (kDigTile - 1), ch & 1);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q8[i] = dig_fixed(v[i].y, x);
+  dig_store(q8, b + (size_t)(np >> 4) * (kDigTile * 256), kDigTile, p & (kDigTile - 1), ch & 1);
+}
+
+// V^H: rows q, K = [Re V[p][q] | -Im V[p][q]] over p. CTA per (walker, 32 rows), lanes along q.
+__global__ void __launch_bounds__(256) k_dig_walk_vh(const double2* __restrict__ V, int n, int np, int mt,
+                                                     unsigned char* __restrict__ d, int* __restrict__ e) {
+  __shared__ unsigned red[8][32];
+  const int w = blockIdx.y, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = blockIdx.x * 32 + lane, kb = np >> 3;
+  const bool in = q < n;
+  const double2* src = V + (size_t)w * n * n + q;
+  unsigned k = 0;
+  if (in)
+    for (int p = wid; p < n; p += 8) {
+      const double2 v = src[(size_t)p * n];
+      k = max(k, max(dig_key(v.x), dig_key(v.y)));
+    }
+  red[wid][lane] = k;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) k = max(k, red[i][lane]);
+  const int x = dig_row_exp(k);
+  if (!in) return;
+  if (wid == 0) e[(size_t)w * mt * kDigTile + q] = x;
+  for (int t = wid; t < (np >> 3); t += 8) {
+    long long a[8], b8[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int p = 8 * t + i;
+      const double2 v = p < n ? src[(size_t)p * n] : c2(0.0, 0.0);
+      a[i] = dig_fixed(v.x, x);
+      b8[i] = dig_fixed(v.y, x);
+    }
+    unsigned char* b = dig_block(d + (size_t)w * mt * kb * (kDigTile * 256), q, t >> 1, kb, kDigTile);
+    dig_store(a, b, kDigTile, q & (kDigTile - 1), t & 1);
+    dig_store(b8, b + (size_t)(np >> 4) * (kDigTile * 256), kDigTile, q & (kDigTile - 1), t & 1, 0x80008000u);
+  }
+}
+
+// Operands of the V cotangents: rows r (an orbital) of a walker, K index m ncol + c over the terms
+// t0.. of tay. A (b = 0): rows p, [Re | Im]; B (b = 1): rows 2q = [Re | Im], 2q + 1 = [-Im | Re],
+// so that A B^T holds the parts of sum Q conj(P). CTA per walker.
+__global__ void __launch_bounds__(256) k_dig_vbar(const double2* __restrict__ tay, int terms, int t0, int M, int n,
+                                                  int o0, int ncol, int K, int b, int rt, int tr,
+                                                  unsigned char* __restrict__ d, int* __restrict__ e) {
+  __shared__ unsigned key[256];
+  const int w = blockIdx.x, kc = K >> 1, kb = K >> 4, nchunk = kc >> 3, items = n * nchunk, o1 = ncol - o0;
+  const size_t nk = (size_t)n * ncol;
+  const double2* src = tay + ((size_t)w * terms + t0) * nk;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) key[i] = 0;
+  __syncthreads();
+  auto load = [&](int it, int& r, int& ch, double2 (&v)[8]) {
+    ch = it % nchunk;
+    r = it / nchunk;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = 8 * ch + i, m = k / ncol, c = k % ncol;
+      v[i] = m < M ? src[(size_t)m * nk + (c < o0 ? (size_t)r * o0 + c : (size_t)n * o0 + (size_t)r * o1 + (c - o0))]
+                   : c2(0.0, 0.0);
+    }
+  };
+  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+    int r, ch;
+    double2 v[8];
+    load(it, r, ch, v);
+    unsigned k = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) k = max(k, max(dig_key(v[i].x), dig_key(v[i].y)));
+    atomicMax(&key[r], k);
+  }
+  __syncthreads();
+  const size_t erow = (size_t)w * rt * tr;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int x = dig_row_exp(key[i]);
+    if (b) {
+      e[erow + 2 * i] = x;
+      e[erow + 2 * i + 1] = x;
+    } else {
+      e[erow + i] = x;
+    }
+  }
+  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+    int r, ch;
+    double2 v[8];
+    load(it, r, ch, v);
+    const int x = dig_row_exp(key[r]), row = b ? 2 * r : r, tile = row / tr, rr = row % tr;
+    unsigned char* p = d + ((size_t)(w * rt + tile) * kb + (ch >> 1)) * ((size_t)tr * 256);
+    unsigned char* p2 = p + (size_t)(kc >> 4) * ((size_t)tr * 256);
+    long long q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = dig_fixed(v[i].x, x);
+    dig_store(q, p, tr, rr, ch & 1);
+    if (b) dig_store(q, p2, tr, rr + 1, ch & 1);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = dig_fixed(v[i].y, x);
+    dig_store(q, p2, tr, rr, ch & 1);
+    if (b) dig_store(q, p, tr, rr + 1, ch & 1, 0x80008000u);
+  }
+}
+
 // ======================================================================================
 // the digit GEMM
 // ======================================================================================
@@ -266,7 +451,8 @@ struct DigGemm {
 
 struct DigWhere {
   int batch, m, n, split;
-  bool add;  // a later K segment of the same range: add to what is there
+  bool add;   // a later K segment of the same range: add to what is there
+  bool more;  // not the last one
 };
 
 constexpr int kDigThreads = 320;
@@ -409,6 +595,14 @@ __global__ void __launch_bounds__(kDigThreads, 1)
               } else {
 #pragma unroll
                 for (int c = 0; c < 8; ++c) group(c, acc + (uint32_t)(c * acols));
+                if constexpr (Epi::kNine) {
+#pragma unroll
+                  for (int i = 1; i < 8; ++i) {
+                    const int j = 8 - i;
+                    ptx::mma_f16(acc + (uint32_t)(7 * acols), da + (i >> 2) * qa + (i & 3) * 2,
+                                 db + (j >> 2) * qb + (j & 3) * 2, g.idesc, 1u);
+                  }
+                }
               }
               ptx::mma_commit(&empty[s]);
             }
@@ -435,6 +629,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
       const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * tr;
       for (int k0 = ka; k0 < kz && ok; k0 += kDigSegBlocks) {
         w.add = k0 > ka;
+        w.more = k0 + kDigSegBlocks < kz;
         if constexpr (WIDE) {
           long long L[64];
           if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[0], run & 1))) {
@@ -520,6 +715,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
 // Complex results: rows 2m / 2m + 1 of D are the real and imaginary parts of row m of C.
 // Neighbouring lanes exchange halves so that each stores whole complex numbers.
 struct EpiDigC {
+  static constexpr bool kNine = false;
   struct Params {
     double2* c;
     int M, N, tr;
@@ -546,6 +742,7 @@ struct EpiDigC {
 };
 
 struct EpiDigR {
+  static constexpr bool kNine = false;
   struct Params {
     double* d;
     int M, N, tr;
@@ -566,6 +763,49 @@ struct EpiDigR {
         double* dst = p.d + (size_t)rr * p.ldd + cc;
         *dst = w.add ? *dst + v[j] : v[j];
       }
+  }
+};
+
+// Products of DigWalk: row p of tile m, columns 2c and 2c + 1 of one walker.
+// These also take the digit products with i + j = 8 (into the last accumulator, whose integer is
+// then rounded once): exp_h1 is nearly diagonal and a column of a walker has a few large
+// entries, so the scale of a dot product can be far above its value, and without them the
+// remainder (2^-55 of the scales) showed against FP64 (walkers 3.7e-15 instead of 2.6e-15 from
+// the 64-bit result after five steps at norb 120).
+struct EpiWalk {
+  static constexpr bool kNine = true;
+  struct Params {
+    WalkOut o;
+    int n, o0, ncol, tr, only;  // only: the slab to store (-1: both)
+    int shift;
+  };
+  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[8]) {
+    const int row = w.m * kDigTile + r;
+    if (row >= p.n) return;
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const int c = (w.n * p.tr + col0 + j) >> 1, s = c >= p.o0 ? 1 : 0;
+      if (c >= p.ncol || (p.only >= 0 && s != p.only)) continue;
+      const int k = s ? p.ncol - p.o0 : p.o0;
+      const size_t i = (size_t)row * k + (s ? c - p.o0 : c);
+      double2 x = c2(v[j], v[j + 1]);
+      if (w.add) x = cadd(x, p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i]);
+      const bool last = !w.more;
+      if (last && p.o.in.p[s]) {
+        const double2 y = p.o.in.p[s][(size_t)w.batch * p.o.in.stride(s) + i];
+        x = c2(fma(y.x, p.o.fin, x.x), fma(y.y, p.o.fin, x.y));
+      }
+      if (p.o.out.p[s]) p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i] = cscale(x, last ? p.o.fout : 1.0);
+      if (last && p.o.acc.p[s]) {
+        double2* a = p.o.acc.p[s] + (size_t)w.batch * p.o.acc.stride(s) + i;
+        if (p.o.init) {
+          *a = x;
+        } else {
+          const double2 y = *a;
+          *a = c2(fma(x.x, p.o.facc, y.x), fma(x.y, p.o.facc, y.y));
+        }
+      }
+    }
   }
 };
 
@@ -811,6 +1051,119 @@ int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D,
   EpiDigR::Params ep{D, M, N, B.tr, ldd, 0, swap};
   return B.tr == 128 ? launch_digits<true, EpiDigR>(cls, g, ep, status, st)
                      : launch_digits<false, EpiDigR>(cls, g, ep, status, st);
+}
+
+void dig_walk_dims(int norb, const int* k, int nslab, int nw, DigWalk* d) {
+  d->n = norb;
+  d->np = (norb + 15) / 16 * 16;
+  d->o[0] = k[0];
+  d->o[1] = nslab == 2 ? k[1] : 0;
+  d->ncol = d->o[0] + d->o[1];
+  d->mt = (norb + kDigTile - 1) / kDigTile;
+  d->nt = (2 * d->ncol + 63) / 64;
+  d->tr = ((2 * d->ncol + d->nt - 1) / d->nt + 15) / 16 * 16;
+  // V digits of a chunk: at most 160 MB, whole rounds of the 152 SMs where it is cut
+  const size_t per = (size_t)d->mt * kDigTile * d->np * 32;
+  const long most = std::max<long>((long)((160u << 20) / per) / 152 * 152, 152);
+  d->chunk = nw < most ? nw : (int)most;
+  for (int s = 0; s < 2; ++s) {
+    d->e[s].rows = norb;
+    d->e[s].K = norb;
+    d->e[s].tr = kDigTile;
+  }
+}
+size_t dig_walk_v_bytes(const DigWalk& d) { return (size_t)d.chunk * d.mt * kDigTile * d.np * 32; }
+size_t dig_walk_x_bytes(const DigWalk& d) { return (size_t)d.chunk * d.nt * d.tr * d.np * 32; }
+size_t dig_walk_ve_bytes(const DigWalk& d) { return (size_t)d.chunk * d.mt * kDigTile * sizeof(int); }
+size_t dig_walk_xe_bytes(const DigWalk& d) { return (size_t)d.chunk * d.nt * d.tr * sizeof(int); }
+
+int dig_walk_slice_v(const DigWalk& d, const double2* V, int nw, bool adjoint, cudaStream_t st) {
+  {
+    ProfScope _ps(K_TAYLOR, st);
+    const int rows = nw * d.n;
+    if (adjoint) {
+      k_dig_walk_vh<<<dim3((d.n + 31) / 32, nw), 256, 0, st>>>(V, d.n, d.np, d.mt, d.vd, d.ve);
+    } else if (d.np <= 64) {
+      k_dig_walk_v<8><<<(rows + 31) / 32, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.vd, d.ve);
+    } else if (d.np <= 128) {
+      k_dig_walk_v<16><<<(rows + 15) / 16, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.vd, d.ve);
+    } else {
+      k_dig_walk_v<32><<<(rows + 7) / 8, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.vd, d.ve);
+    }
+  }
+  return dig_err("slice V");
+}
+
+int dig_walk_slice_y(const DigWalk& d, const WalkVec& y, int nw, cudaStream_t st) {
+  {
+    ProfScope _ps(K_TAYLOR, st);
+    k_dig_walk_y<<<nw, 256, 0, st>>>(y.p[0], y.p[1], y.stride(0), y.stride(1), d.o[0], d.ncol, d.n, d.np, d.nt, d.tr,
+                                     d.xd, d.xe);
+  }
+  return dig_err("slice y");
+}
+
+int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut& o, int nw, cudaStream_t st) {
+  DigGemm g;
+  g.a = e < 0 ? d.vd : E[e].d;
+  g.ea = e < 0 ? d.ve : E[e].e;
+  g.b = d.xd;
+  g.eb = d.xe;
+  g.kbb = d.kbv();
+  g.kb = g.kba = e < 0 ? d.kbv() : d.np / 16;
+  g.mt = d.mt;
+  g.nt = d.nt;
+  g.nb = nw;
+  g.a_bt = e < 0 ? d.mt : 0;
+  g.b_bt = d.nt;
+  g.tr = d.tr;
+  g.splits = 1;
+  g.kps = g.kb;
+  EpiWalk::Params ep{o, d.n, d.o[0], d.ncol, d.tr, e < 0 || d.o[1] == 0 ? -1 : e, 0};
+  return launch_digits<false, EpiWalk>(cls, g, ep, d.status, st);
+}
+
+void dig_walk_vbar_dims(const DigWalk& d, int M, DigVbar* v) {
+  v->K = 2 * ((M * d.ncol + 15) / 16 * 16);
+  v->mt = d.mt;
+  v->nt = (2 * d.n + 63) / 64;
+  v->tr = ((2 * d.n + v->nt - 1) / v->nt + 15) / 16 * 16;
+}
+size_t dig_walk_vbar_a_bytes(const DigWalk& d, const DigVbar& v) {
+  return (size_t)d.chunk * v.mt * kDigTile * v.K * 16;
+}
+size_t dig_walk_vbar_b_bytes(const DigWalk& d, const DigVbar& v) { return (size_t)d.chunk * v.nt * v.tr * v.K * 16; }
+size_t dig_walk_vbar_ae_bytes(const DigWalk& d, const DigVbar& v) {
+  return (size_t)d.chunk * v.mt * kDigTile * sizeof(int);
+}
+size_t dig_walk_vbar_be_bytes(const DigWalk& d, const DigVbar& v) {
+  return (size_t)d.chunk * v.nt * v.tr * sizeof(int);
+}
+
+int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int terms, int qt, int pt, int M,
+                  double2* vbar, int nw, cudaStream_t st) {
+  {
+    ProfScope _ps(K_TAYLOR, st);
+    k_dig_vbar<<<nw, 256, 0, st>>>(tay, terms, qt, M, d.n, d.o[0], d.ncol, v.K, 0, v.mt, kDigTile, v.ad, v.ae);
+    k_dig_vbar<<<nw, 256, 0, st>>>(tay, terms, pt, M, d.n, d.o[0], d.ncol, v.K, 1, v.nt, v.tr, v.bd, v.be);
+  }
+  if (int e = dig_err("slice V cotangents")) return e;
+  DigGemm g;
+  g.a = v.ad;
+  g.ea = v.ae;
+  g.b = v.bd;
+  g.eb = v.be;
+  g.kba = g.kbb = g.kb = v.K / 16;
+  g.mt = g.a_bt = v.mt;
+  g.nt = g.b_bt = v.nt;
+  g.nb = nw;
+  g.tr = v.tr;
+  g.splits = 1;
+  g.kps = g.kb;
+  WalkOut o;  // [norb][norb] per walker: one slab of norb columns
+  o.out = WalkVec{{vbar, nullptr}, (size_t)d.n * d.n};
+  EpiWalk::Params ep{o, d.n, d.n, d.n, v.tr, -1, 0};
+  return launch_digits<false, EpiWalk>(K_TAYLOR, g, ep, d.status, st);
 }
 
 int dig_launch_energy(const afq_ctx_dev& c, const double2* green, const double2* z, const double2* coul,

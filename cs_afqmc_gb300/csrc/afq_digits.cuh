@@ -81,6 +81,61 @@ int dig_launch_energy_tangent(const afq_ctx_dev& c, const double2* green, const 
 int dig_launch_energy_adjoint(const afq_ctx_dev& c, const double2* z, const double* ebar, double2* gene,
                               cudaStream_t st);
 int dig_sms();
+
+// ---- products with one walker's matrices (Taylor series) -------------------------------
+// For every walker w of a chunk: out_w = X y_w, X = E (real, shared, per spin), V_w or V_w^H
+// (complex), y_w [norb][nocc_s] complex per slab. V is sliced as [Re | Im] along K, y as
+// columns 2c = [Re y_c | -Im y_c] and 2c + 1 = [Im y_c | Re y_c], so that one real contraction
+// over K = 2 np (np: norb padded to 16) gives both parts; E uses the first half of K.
+struct DigWalk {
+  int n, np, o[2], ncol;  // orbitals, padded; columns per slab and together
+  int mt, nt, tr;         // row tiles of V; column tiles per walker and columns (2 per c) per tile
+  int chunk;              // walkers sliced at a time
+  DigOp e[2];             // exp_h1 per slab
+  unsigned char *vd, *xd; // V digits, y digits
+  int *ve, *xe;
+  int* status;
+  int kbv() const { return np / 8; }
+};
+// complex [walker][norb][nocc_s] per slab, walker stride in elements
+struct WalkVec {
+  double2* p[2];
+  size_t ws;       // walker stride of slab 0 (and of slab 1 unless ws1 is set)
+  size_t ws1 = 0;
+  AFQ_HD size_t stride(int s) const { return s == 1 && ws1 ? ws1 : ws; }
+};
+void dig_walk_dims(int norb, const int* k, int nslab, int nw, DigWalk* d);
+size_t dig_walk_v_bytes(const DigWalk& d);  // digits, then row exponents
+size_t dig_walk_x_bytes(const DigWalk& d);
+size_t dig_walk_ve_bytes(const DigWalk& d);
+size_t dig_walk_xe_bytes(const DigWalk& d);
+// V [nw][norb][norb]; adjoint: V^H
+int dig_walk_slice_v(const DigWalk& d, const double2* V, int nw, bool adjoint, cudaStream_t st);
+int dig_walk_slice_y(const DigWalk& d, const WalkVec& y, int nw, cudaStream_t st);
+// What a product leaves: r = X y + fin in (in may be NULL), out = fout r, acc = r (init) or
+// acc + facc r (out, acc may be NULL; in, out and acc may be the same array).
+struct WalkOut {
+  WalkVec out{{nullptr, nullptr}, 0}, in{{nullptr, nullptr}, 0}, acc{{nullptr, nullptr}, 0};
+  double fin = 1.0, fout = 1.0, facc = 0.0;
+  int init = 0;
+};
+// V cotangents of the Taylor adjoint: vbar[w][p][q] = sum_{m=1..M} sum_c Q_m[p,c] conj(P_m[q,c])
+// over the columns of both slabs, Q_m = term qt + m - 1 and P_m = term pt + m - 1 of tay
+// [w][terms][norb (k0 + k1)]. ad / bd (+ exponents): digits, dig_walk_vbar_bytes each.
+struct DigVbar {
+  int K, mt, nt, tr;
+  unsigned char *ad, *bd;
+  int *ae, *be;
+};
+void dig_walk_vbar_dims(const DigWalk& d, int M, DigVbar* v);
+size_t dig_walk_vbar_a_bytes(const DigWalk& d, const DigVbar& v);
+size_t dig_walk_vbar_b_bytes(const DigWalk& d, const DigVbar& v);
+size_t dig_walk_vbar_ae_bytes(const DigWalk& d, const DigVbar& v);
+size_t dig_walk_vbar_be_bytes(const DigWalk& d, const DigVbar& v);
+int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int terms, int qt, int pt, int M,
+                  double2* vbar, int nw, cudaStream_t st);
+// X = the sliced V (e < 0) or e[slab] for that slab's columns
+int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut& o, int nw, cudaStream_t st);
 // B columns per tile for an output of 2 M x N with kb K blocks: 64 where the tiles (times up to
 // eight K ranges) reach half of the SMs, else 32, so that small problems still spread out; never
 // more than N needs.

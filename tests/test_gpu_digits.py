@@ -101,3 +101,90 @@ def test_error_against_a_plain_fp64_sum():
             plain += a[:, i][:, None] * b[:, i][None, :]
         err = lambda x: float(np.sqrt(np.mean((x - ref).astype(np.float64) ** 2)))  # noqa: E731
         assert err(run(a, b, 128)) <= err(plain), k
+
+
+# Sizes just above the line where the Taylor products go to the digit GEMM (nw * columns * norb^2 >=
+# 1e6); with the walkers in four chunks (n_batch) the same call stays on the FP64 units.
+ROUTES = [
+    dict(kind="rhf", restricted=True, norb=33, nelec=(6, 6), nchol=40, nw=160),     # one slab, ragged
+    dict(kind="uhf", restricted=False, norb=33, nelec=(6, 5), nchol=40, nw=88),     # two slabs, unequal
+    dict(kind="rhf", restricted=False, norb=64, nelec=(3, 3), nchol=50, nw=44),     # tile edge, few columns
+    dict(kind="rhf", restricted=True, norb=130, nelec=(33, 33), nchol=140, nw=4),   # two row and column tiles
+    dict(kind="uhf", restricted=False, norb=128, nelec=(20, 19), nchol=130, nw=4),
+]
+
+
+def route_case(cfg, n_batch):
+    from tests.helpers import Case
+
+    case = Case(precision="fp64", n_batch=n_batch, orthonormal=True, perturb=0.05, **cfg)
+    return case, case.gpu_prop_data()
+
+
+def draws(case, n_prop):
+    rng = np.random.default_rng(9)
+    return rng.standard_normal((1, 1, n_prop, case.nw, case.nchol)), rng.uniform(size=1)
+
+
+def close(x, y, tol=1e-11):
+    from tests.helpers import rel_err, to_np
+
+    if isinstance(x, (list, tuple)):
+        return all(close(a, b, tol) for a, b in zip(x, y))
+    return rel_err(to_np(x), to_np(y)) < tol
+
+
+def ids(c):
+    return f"{c['kind']}{'r' if c['restricted'] else 'u'}-n{c['norb']}"
+
+
+# Both routes round each product to FP64: relative differences are some 1e-15 per step, far
+# below 1e-11 after two of them.
+@pytest.mark.parametrize("cfg", ROUTES, ids=ids)
+def test_block_routes_agree(cfg):
+    from cs_afqmc_gb300 import sampling
+
+    out = []
+    for n_batch in (1, 4):
+        case, pd = route_case(cfg, n_batch)
+        f, z = draws(case, 2)
+        e, pd = sampling.sampler(2, 1, 1).propagate_phaseless(case.ham, case.ham_data, case.prop, pd, case.trial,
+                                                              case.wave_data, fields=f, zetas=z)
+        out.append((e, pd["walkers"], pd["weights"], pd["overlaps"]))
+    assert close(out[0], out[1])
+
+
+@pytest.mark.parametrize("mode", ["jvp", "vjp"])
+@pytest.mark.parametrize("cfg", ROUTES[:3], ids=ids)
+def test_derivative_routes_agree(cfg, mode):
+    from cs_afqmc_gb300 import sampling
+
+    out = []
+    for n_batch in (1, 4):
+        case, pd = route_case(cfg, n_batch)
+        f, z = draws(case, 2)
+        s = sampling.sampler(2, 1, 1)
+        args = (case.prop, pd, case.trial, case.wave_data)
+        if mode == "jvp":
+            op = np.random.default_rng(4).standard_normal((case.norb, case.norb))
+            e, d, pd = s.propagate_phaseless_ad_norot_jvp(case.ham, case.ham_data, op + op.T, *args, fields=f, zetas=z)
+        else:
+            e, d, pd = s.propagate_phaseless_ad_norot_vjp(case.ham, case.ham_data, *args, fields=f, zetas=z)
+        out.append((e, d, pd["walkers"], pd["weights"]))
+    assert close(out[0], out[1])
+
+
+@pytest.mark.parametrize("cfg", [
+    dict(kind="rhf", restricted=True, norb=17, nelec=(3, 3), nchol=3, nw=5),     # U form, ragged
+    dict(kind="rhf", restricted=False, norb=22, nelec=(5, 5), nchol=4, nw=70),
+    dict(kind="uhf", restricted=False, norb=21, nelec=(4, 1), nchol=3, nw=6),
+    dict(kind="uhf", restricted=False, norb=29, nelec=(4, 3), nchol=4, nw=6),    # too few vectors: sums over f_g
+], ids=["u-restricted", "u-two-slab", "u-uhf", "sums"])
+def test_energy_forms_against_the_oracle(cfg):
+    """Both forms of the local energy at the line between them (norb = 7 nchol)."""
+    from tests.helpers import rel_err, to_np
+
+    case, pd = route_case(cfg, 1)
+    e = to_np(case.trial.calc_energy(pd["walkers"], case.ham_data, case.wave_data))
+    w = [x.copy() for x in case.walkers0] if isinstance(case.walkers0, list) else case.walkers0
+    assert rel_err(e, case.o_trial.energy(w, case.o_ham, case.sys.mo_coeff)) < 1e-11
