@@ -371,12 +371,9 @@ __global__ void __launch_bounds__(256) k_dig_vbar(const double2* __restrict__ ta
 // the digit GEMM
 // ======================================================================================
 
-// i_c: the integer sums of the groups. Returns sum_c i_c 2^(-14-7c) 2^e rounded to FP64, from
-// H = i_0 2^21 + i_1 2^14 + i_2 2^7 + i_3 and L, the same of groups 4..7.
-AFQ_D double dig_combine(long long H, long long L, int e) {
-  const long long hi = H + (L >> 28);
-  const int sgn = (int)(hi >> 63);  // sign of the whole sum: the rest is non-negative
-  unsigned lo = (unsigned)L & 0xfffffffu;
+// The sum hi 2^28 + lo in units of 2^-63 (lo < 2^28), times 2^e, rounded to FP64.
+AFQ_D double dig_combine(long long hi, unsigned lo, int e) {
+  const int sgn = (int)(hi >> 63);  // sign of the whole sum: lo is non-negative
   unsigned long long a = (unsigned long long)(hi ^ sgn);  // |sum| = a 2^28 + lo, sum < 0: complement + 1
   lo = ((lo ^ (unsigned)sgn) & 0xfffffffu) - (unsigned)sgn;
   a += lo >> 28;
@@ -455,7 +452,8 @@ struct DigWhere {
   bool more;  // not the last one
 };
 
-constexpr int kDigThreads = 320;
+constexpr int kDigEpiWarps = 16;
+constexpr int kDigThreads = 64 + 32 * kDigEpiWarps;
 constexpr int kDigABlock = kDigTile * 256;  // bytes of an A K block
 constexpr int kDigRing = 196608;
 constexpr int kDigSmem = 1024 + kDigRing + 256;
@@ -469,17 +467,18 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 
 // Persistent over (K range, batch entry, column tile, row tile). Warp 0 loads K blocks
-// (A 32 KB + B) with bulk copies, warp 1 issues the MMAs, warps 2..9 combine and store: warp w
-// reads TMEM lanes 32 (w % 4).. and half of the columns.
+// (A 32 KB + B) with bulk copies, warp 1 issues the MMAs, warps 2..17 combine and store: warp w
+// reads TMEM lanes 32 (w % 4).. and a quarter of the columns.
 //
-// WIDE (128 columns): four accumulators of 128 columns fill the tensor memory, so a range is
-// contracted twice, first groups 4..7 (26 products), then 0..3 (10 products of the first four
-// digits only). A tcgen05.mma of M 128, N 128, K 16 takes 64 cycles and reads 8 KB of shared
-// memory, both at their limits; with N = 64 it is bound by the 6 KB it reads, so the wide form
-// needs about half the tensor time per flop. Narrow (tr <= 64 columns): all eight accumulators
-// at once, two sets when tr <= 32. Narrow tiles serve the batched products (tr = one walker's
-// columns) and problems with too few wide tiles for the SMs.
-template <bool WIDE, class Epi>
+// What bounds it: the tensor core. A tcgen05.mma of M 128, K 16 takes 58 cycles at N 16 and 32, 72
+// at N 64 and 130 at N 128 here (shared-memory operand reads), so tiles are up to 64 columns
+// wide and all eight accumulators fit the tensor memory (8 x 64 columns; two sets at 32). With one set
+// the MMAs of the next tile wait for the accumulators to be read: sixteen warps turn them into
+// the two 64-bit sums (14 integer instructions a group of four) and free them before the longer
+// part, the normalisation and the stores. 512 x 14400 x 512: 247 us, 31 TFLOP/s of FP64 products
+// (1.1 PFLOP/s of MMAs; 291 us with eight warps that stored before they freed the accumulators);
+// the FP64 units do 1.04 TFLOP/s.
+template <class Epi>
 __global__ void __launch_bounds__(kDigThreads, 1)
     k_gemm_digits(const DigGemm g, const __grid_constant__ typename Epi::Params ep, int* status) {
   extern __shared__ unsigned char smem_raw[];
@@ -493,9 +492,8 @@ __global__ void __launch_bounds__(kDigThreads, 1)
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tr = g.tr, bblock = tr * 256, unit = kDigABlock + bblock;
-  constexpr int PASSES = WIDE ? 2 : 1;
-  const int acols = WIDE ? 128 : tr <= 32 ? 32 : 64;  // columns between accumulators
-  const int nbuf = !WIDE && tr <= 32 ? 2 : 1;
+  const int acols = tr <= 32 ? 32 : 64;  // columns between accumulators
+  const int nbuf = tr <= 32 ? 2 : 1;
   const int mn = g.mt * g.nt * g.nb, ntiles = mn * g.splits;
   if (threadIdx.x == 0) {
     for (int s = 0; s < g.stages; ++s) {
@@ -504,7 +502,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&accfull[i], 1);
-      ptx::mbar_init(&accempty[i], 8);
+      ptx::mbar_init(&accempty[i], kDigEpiWarps);
     }
     ptx::mbar_init(done, 1);
     ptx::fence_mbar_init();
@@ -530,20 +528,16 @@ __global__ void __launch_bounds__(kDigThreads, 1)
         const unsigned char* pb = g.b + (size_t)(b * g.b_bt + n) * g.kbb * bblock;
         for (int k0 = ka; k0 < kz && ok; k0 += kDigSegBlocks) {
           const int k1 = min(kz, k0 + kDigSegBlocks);
-          for (int pass = 0; pass < PASSES && ok; ++pass) {
-            const uint32_t da = WIDE && pass == 1 ? kDigABlock / 2 : kDigABlock;
-            const uint32_t db = WIDE && pass == 1 ? bblock / 2 : bblock;
-            for (int k = k0; k < k1; ++k, ++it) {
-              const int s = it % g.stages, r = it / g.stages;
-              if (r > 0 && !ptx::mbar_wait(&empty[s], (r - 1) & 1)) {
-                ok = false;
-                break;
-              }
-              unsigned char* u = smem + s * unit;
-              ptx::mbar_expect_tx(&full[s], da + db);
-              bulk_load(u, pa + (size_t)k * kDigABlock, da, &full[s]);
-              bulk_load(u + kDigABlock, pb + (size_t)k * bblock, db, &full[s]);
+          for (int k = k0; k < k1; ++k, ++it) {
+            const int s = it % g.stages, r = it / g.stages;
+            if (r > 0 && !ptx::mbar_wait(&empty[s], (r - 1) & 1)) {
+              ok = false;
+              break;
             }
+            unsigned char* u = smem + s * unit;
+            ptx::mbar_expect_tx(&full[s], (uint32_t)unit);
+            bulk_load(u, pa + (size_t)k * kDigABlock, kDigABlock, &full[s]);
+            bulk_load(u + kDigABlock, pb + (size_t)k * bblock, (uint32_t)bblock, &full[s]);
           }
         }
       }
@@ -558,64 +552,48 @@ __global__ void __launch_bounds__(kDigThreads, 1)
         const int ka = (tile / mn) * g.kps, kz = min(g.kb, ka + g.kps);
         for (int k0 = ka; k0 < kz && ok; k0 += kDigSegBlocks) {
           const int k1 = min(kz, k0 + kDigSegBlocks);
-          for (int pass = 0; pass < PASSES && ok; ++pass, ++run) {
-            const int buf = run % nbuf, use = run / nbuf;
-            if (use > 0 && !ptx::mbar_wait(&accempty[buf], (use - 1) & 1)) {
+          const int buf = run % nbuf, use = run / nbuf;
+          ++run;
+          if (use > 0 && !ptx::mbar_wait(&accempty[buf], (use - 1) & 1)) {
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t acc = tmem + (uint32_t)(buf * 256);
+          for (int k = k0; k < k1; ++k, ++it) {
+            const int s = it % g.stages, r = it / g.stages;
+            if (!ptx::mbar_wait(&full[s], r & 1)) {
               ok = false;
               break;
             }
             ptx::tc_fence_after();
-            const uint32_t acc = tmem + (uint32_t)(buf * 256);
-            for (int k = k0; k < k1; ++k, ++it) {
-              const int s = it % g.stages, r = it / g.stages;
-              if (!ptx::mbar_wait(&full[s], r & 1)) {
-                ok = false;
-                break;
-              }
-              ptx::tc_fence_after();
-              const uint32_t ua = ptx::smem_u32(smem + s * unit), ub = ua + kDigABlock;
-              const uint64_t da = ptx::desc_kmajor_sw128(ua), db = ptx::desc_kmajor_sw128(ub);
-              const uint64_t qa = (kDigABlock / 2) >> 4, qb = (uint64_t)(bblock / 2) >> 4;
-              auto group = [&](int c, uint32_t d) {
+            const uint32_t ua = ptx::smem_u32(smem + s * unit), ub = ua + kDigABlock;
+            const uint64_t da = ptx::desc_kmajor_sw128(ua), db = ptx::desc_kmajor_sw128(ub);
+            const uint64_t qa = (kDigABlock / 2) >> 4, qb = (uint64_t)(bblock / 2) >> 4;
+            auto mma = [&](int c, int i, int j, uint32_t accumulate) {
+              ptx::mma_f16(acc + (uint32_t)(c * acols), da + (i >> 2) * qa + (i & 3) * 2,
+                           db + (j >> 2) * qb + (j & 3) * 2, g.idesc, accumulate);
+            };
 #pragma unroll
-                for (int i = 0; i <= c; ++i) {
-                  const int j = c - i;
-                  ptx::mma_f16(d, da + (i >> 2) * qa + (i & 3) * 2, db + (j >> 2) * qb + (j & 3) * 2, g.idesc,
-                               (k > k0 || i > 0) ? 1u : 0u);
-                }
-              };
-              if constexpr (WIDE) {
-                if (pass == 0) {
+            for (int c = 0; c < 8; ++c)
 #pragma unroll
-                  for (int c = 4; c < 8; ++c) group(c, acc + (uint32_t)((c - 4) * 128));
-                } else {
+              for (int i = 0; i <= c; ++i) mma(c, i, c - i, (k > k0 || i > 0) ? 1u : 0u);
+            if constexpr (Epi::kNine) {
 #pragma unroll
-                  for (int c = 0; c < 4; ++c) group(c, acc + (uint32_t)(c * 128));
-                }
-              } else {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) group(c, acc + (uint32_t)(c * acols));
-                if constexpr (Epi::kNine) {
-#pragma unroll
-                  for (int i = 1; i < 8; ++i) {
-                    const int j = 8 - i;
-                    ptx::mma_f16(acc + (uint32_t)(7 * acols), da + (i >> 2) * qa + (i & 3) * 2,
-                                 db + (j >> 2) * qb + (j & 3) * 2, g.idesc, 1u);
-                  }
-                }
-              }
-              ptx::mma_commit(&empty[s]);
+              for (int i = 1; i < 8; ++i) mma(7, i, 8 - i, 1u);
             }
-            ptx::mma_commit(&accfull[buf]);
+            ptx::mma_commit(&empty[s]);
           }
+          ptx::mma_commit(&accfull[buf]);
         }
       }
       ptx::mma_commit(done);
       if (!ptx::mbar_wait(done, 0)) ok = false;
     }
   } else {
-    const int q = warp & 3, half = (warp - 2) >> 2, r = q * 32 + lane;
-    const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+    const int q = warp & 3, r = q * 32 + lane;
+    const int nc = tr >> 2, col0 = ((warp - 2) >> 2) * nc;  // this warp's columns (4..16)
+    const uint32_t src0 = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)col0;
     int run = 0;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
       DigWhere w;
@@ -625,81 +603,46 @@ __global__ void __launch_bounds__(kDigThreads, 1)
       w.n = (x / g.mt) % g.nt;
       w.batch = x / (g.mt * g.nt);
       const int ka = w.split * g.kps, kz = min(g.kb, ka + g.kps);
-      const int er = g.ea[(size_t)(w.batch * g.a_bt + w.m) * kDigTile + r];
-      const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * tr;
-      for (int k0 = ka; k0 < kz && ok; k0 += kDigSegBlocks) {
+      const int er = g.ea[(size_t)(w.batch * g.a_bt + w.m) * kDigTile + r] + ep.shift;
+      const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * tr + col0;
+      for (int k0 = ka; k0 < kz; k0 += kDigSegBlocks, ++run) {
         w.add = k0 > ka;
         w.more = k0 + kDigSegBlocks < kz;
-        if constexpr (WIDE) {
-          long long L[64];
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[0], run & 1))) {
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          const uint32_t src = tmem + lane_off + (uint32_t)(half * 64);
-#pragma unroll
-          for (int c0 = 0; c0 < 64; c0 += 8) {
-            float v[4][8];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) ptx::tmem_ld8p(src + (uint32_t)(c * 128 + c0), v[c]);
-            ptx::tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 8; ++j) L[c0 + j] = dig_quad<4>(v[0][j], v[1][j], v[2][j], v[3][j]);
-          }
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&accempty[0]);
-          ++run;
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[0], run & 1))) {
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-#pragma unroll
-          for (int c0 = 0; c0 < 64; c0 += 8) {
-            float v[4][8];
-            double o[8];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) ptx::tmem_ld8p(src + (uint32_t)(c * 128 + c0), v[c]);
-            ptx::tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              o[j] = dig_combine(dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]), L[c0 + j],
-                                 er + eb[half * 64 + c0 + j] + ep.shift);
-            Epi::store(ep, w, r, half * 64 + c0, o);
-          }
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&accempty[0]);
-          ++run;
-        } else {
-          const int buf = run % nbuf, use = run / nbuf;
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[buf], use & 1))) {
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          const int hc = tr >> 1;
-          const uint32_t src = tmem + lane_off + (uint32_t)(buf * 256 + half * hc);
-          for (int c0 = 0; c0 < hc; c0 += 8) {
-            float v[8][8];
-            double o[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) ptx::tmem_ld8p(src + (uint32_t)(c * acols + c0), v[c]);
-            ptx::tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              o[j] = dig_combine(dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]),
-                                 dig_quad<4>(v[4][j], v[5][j], v[6][j], v[7][j]),
-                                 er + eb[half * hc + c0 + j] + ep.shift);
-            Epi::store(ep, w, r, half * hc + c0, o);
-          }
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
-          ++run;
+        const int buf = run % nbuf, use = run / nbuf;
+        // warp-uniform outcome: the TMEM loads below are .sync.aligned
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accfull[buf], use & 1))) {
+          ok = false;
+          break;
         }
+        ptx::tc_fence_after();
+        const uint32_t src = src0 + (uint32_t)(buf * 256);
+        long long hi[16];  // the sum in units of 2^-35 and its remainder in units of 2^-63
+        unsigned lo[16];
+#pragma unroll
+        for (int c0 = 0; c0 < 16; c0 += 4)
+          if (c0 < nc) {
+            float v[8][4];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) ptx::tmem_ld4p(src + (uint32_t)(c * acols + c0), v[c]);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const long long l = dig_quad<4>(v[4][j], v[5][j], v[6][j], v[7][j]);
+              hi[c0 + j] = dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]) + (l >> 28);
+              lo[c0 + j] = (unsigned)l & 0xfffffffu;
+            }
+          }
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
+#pragma unroll
+        for (int c0 = 0; c0 < 16; c0 += 4)
+          if (c0 < nc) {
+            double o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j] = dig_combine(hi[c0 + j], lo[c0 + j], er + eb[c0 + j]);
+            Epi::store(ep, w, r, col0 + c0, o);
+          }
       }
     }
   }
@@ -722,10 +665,10 @@ struct EpiDigC {
     long ldc, split_stride;
     int rot, shift;  // C = i^rot 2^shift D
   };
-  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[8]) {
+  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
     const int m = (w.m * kDigTile + r) >> 1, odd = r & 1, n0 = w.n * p.tr + col0;
 #pragma unroll
-    for (int j = 0; j < 8; j += 2) {
+    for (int j = 0; j < 4; j += 2) {
       const double x = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
       const double re = odd ? x : v[j], im = odd ? v[j + 1] : x;
       const int n = n0 + j + odd;
@@ -749,11 +692,11 @@ struct EpiDigR {
     long ldd;
     int shift, swap;
   };
-  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[8]) {
+  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
     const int m = w.m * kDigTile + r, n0 = w.n * p.tr + col0;
     if (m >= p.M) return;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 4; ++j)
       if (n0 + j < p.N) {
         int rr = m, cc = n0 + j;
         if (p.swap) {
@@ -768,10 +711,9 @@ struct EpiDigR {
 
 // Products of DigWalk: row p of tile m, columns 2c and 2c + 1 of one walker.
 // These also take the digit products with i + j = 8 (into the last accumulator, whose integer is
-// then rounded once): exp_h1 is nearly diagonal and a column of a walker has a few large
-// entries, so the scale of a dot product can be far above its value, and without them the
-// remainder (2^-55 of the scales) showed against FP64 (walkers 3.7e-15 instead of 2.6e-15 from
-// the 64-bit result after five steps at norb 120).
+// then rounded once): exp_h1 is nearly diagonal and a column of a walker has a few large entries,
+// so the scale of a dot product can be far above its value. Walkers after a step, against
+// extended precision: 1.7e-16 at norb 33, 2.1e-16 at norb 120; the FP64 units: 3.5e-16, 6.2e-16.
 struct EpiWalk {
   static constexpr bool kNine = true;
   struct Params {
@@ -779,11 +721,11 @@ struct EpiWalk {
     int n, o0, ncol, tr, only;  // only: the slab to store (-1: both)
     int shift;
   };
-  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[8]) {
+  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
     const int row = w.m * kDigTile + r;
     if (row >= p.n) return;
 #pragma unroll
-    for (int j = 0; j < 8; j += 2) {
+    for (int j = 0; j < 4; j += 2) {
       const int c = (w.n * p.tr + col0 + j) >> 1, s = c >= p.o0 ? 1 : 0;
       if (c >= p.ncol || (p.only >= 0 && s != p.only)) continue;
       const int k = s ? p.ncol - p.o0 : p.o0;
@@ -957,14 +899,14 @@ int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_
   return dig_err("slice columns");
 }
 
-template <bool WIDE, class Epi>
+template <class Epi>
 static int launch_digits(int cls, DigGemm g, const typename Epi::Params& ep, int* status, cudaStream_t st) {
   const int unit = kDigABlock + g.tr * 256;
   g.stages = kDigRing / unit < kDigMaxStages ? kDigRing / unit : kDigMaxStages;
   g.idesc = ptx::idesc_f16(128, g.tr, 1);
   const long tiles = (long)g.mt * g.nt * g.nb * g.splits;
   const int sms = dig_sms();
-  auto kfn = k_gemm_digits<WIDE, Epi>;
+  auto kfn = k_gemm_digits<Epi>;
   cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kDigSmem);
   if (e != cudaSuccess) {
     afq_set_error("digit GEMM: shared-memory attribute: %s", cudaGetErrorString(e));
@@ -1033,8 +975,7 @@ int dig_gemm_c(int cls, const DigOp& A, const DigOp& B, int M, int N, double2* C
   g.kps = plan.kps;
   const bool split = plan.splits > 1;
   EpiDigC::Params ep{split ? part : C, M, N, B.tr, split ? (long)N : ldc, (long)M * N, rot, shift};
-  int rc = B.tr == 128 ? launch_digits<true, EpiDigC>(cls, g, ep, status, st)
-                       : launch_digits<false, EpiDigC>(cls, g, ep, status, st);
+  int rc = launch_digits<EpiDigC>(cls, g, ep, status, st);
   if (rc || !split) return rc;
   {
     ProfScope _ps(cls, st);
@@ -1049,8 +990,7 @@ int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D,
                int* status, cudaStream_t st) {
   DigGemm g = dig_args(A, B);
   EpiDigR::Params ep{D, M, N, B.tr, ldd, 0, swap};
-  return B.tr == 128 ? launch_digits<true, EpiDigR>(cls, g, ep, status, st)
-                     : launch_digits<false, EpiDigR>(cls, g, ep, status, st);
+  return launch_digits<EpiDigR>(cls, g, ep, status, st);
 }
 
 void dig_walk_dims(int norb, const int* k, int nslab, int nw, DigWalk* d) {
@@ -1120,7 +1060,7 @@ int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut
   g.splits = 1;
   g.kps = g.kb;
   EpiWalk::Params ep{o, d.n, d.o[0], d.ncol, d.tr, e < 0 || d.o[1] == 0 ? -1 : e, 0};
-  return launch_digits<false, EpiWalk>(cls, g, ep, d.status, st);
+  return launch_digits<EpiWalk>(cls, g, ep, d.status, st);
 }
 
 void dig_walk_vbar_dims(const DigWalk& d, int M, DigVbar* v) {
@@ -1163,7 +1103,7 @@ int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int te
   WalkOut o;  // [norb][norb] per walker: one slab of norb columns
   o.out = WalkVec{{vbar, nullptr}, (size_t)d.n * d.n};
   EpiWalk::Params ep{o, d.n, d.n, d.n, v.tr, -1, 0};
-  return launch_digits<false, EpiWalk>(K_TAYLOR, g, ep, d.status, st);
+  return launch_digits<EpiWalk>(K_TAYLOR, g, ep, d.status, st);
 }
 
 int dig_launch_energy(const afq_ctx_dev& c, const double2* green, const double2* z, const double2* coul,
@@ -1203,7 +1143,7 @@ extern "C" size_t afq_test_gemm_digits_bytes(int M, int N, int K, int tr) {
 extern "C" int afq_test_gemm_digits(const double* a, const double* b, double* d, int M, int N, int K, int tr,
                                     void* scratch, int* status, void* stream) {
   using namespace afq;
-  if (!a || !b || !d || !scratch || !status || M < 1 || N < 1 || K < 1 || tr % 16 || tr < 16 || (tr > 64 && tr != 128)) {
+  if (!a || !b || !d || !scratch || !status || M < 1 || N < 1 || K < 1 || tr % 16 || tr < 16 || tr > 64) {
     afq_set_error("afq_test_gemm_digits: bad arguments");
     return -1;
   }

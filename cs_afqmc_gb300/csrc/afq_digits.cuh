@@ -16,7 +16,7 @@
 // products cost about 2 % of the FP64 ones; integer instructions combine the accumulators
 // because FP64 adds and conversions (two per cycle and SM) would cost as much as the products.
 //
-// Layout of a sliced operand ("digit tiles"): rows in tiles of TR (128 for A; 16..128 for B),
+// Layout of a sliced operand ("digit tiles"): rows in tiles of TR (128 for A; 16..64 for B),
 // K in blocks of 16. One (row tile, K block) is contiguous: two quads (digits 0-3, 4-7) of
 // [TR rows][128 bytes], a row's 128 bytes = 4 digits x 16 k in the 128-byte swizzle the
 // tensor core reads, so that a K block of an operand is one plain bulk copy (A 32 KB) and no

@@ -247,6 +247,16 @@ __device__ __forceinline__ void tmem_ld8p(uint32_t taddr, float* v) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
+// 32 lanes x 4 columns, no wait
+__device__ __forceinline__ void tmem_ld4p(uint32_t taddr, float* v) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
 // CW = 8 or 16 columns
 template <int CW>
 __device__ __forceinline__ void tmem_ldp(uint32_t taddr, float* v) {

@@ -42,7 +42,7 @@ int afq_test_split_pairs(int enable);
 
 /* D[M,N] (fp64, row-major) = A[M,K] B[N,K]^T (fp64, row-major) by exact digit slicing on the
  * BF16 tensor cores, the FP64 path's contraction kernel. tr: output columns per tile
- * (multiple of 16 up to 64, or 128). scratch: afq_test_gemm_digits_bytes bytes. *status as
+ * (multiple of 16, at most 64). scratch: afq_test_gemm_digits_bytes bytes. *status as
  * above. */
 size_t afq_test_gemm_digits_bytes(int M, int N, int K, int tr);
 int afq_test_gemm_digits(const double* a, const double* b, double* d, int M, int N, int K, int tr,

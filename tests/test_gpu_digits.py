@@ -46,7 +46,7 @@ def bound(a, b, ref):
     return a.shape[1] * np.outer(scale(a), scale(b)) * 2.0 ** -54 + np.abs(ref).astype(np.float64) * 2.0 ** -52
 
 
-@pytest.mark.parametrize("tr", [16, 32, 48, 64, 128])
+@pytest.mark.parametrize("tr", [16, 32, 48, 64])
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (128, 128, 16), (129, 130, 17), (300, 257, 513), (64, 200, 1100)])
 def test_against_extended_precision(m, n, k, tr):
     rng = np.random.default_rng(m + n + k)
@@ -57,7 +57,7 @@ def test_against_extended_precision(m, n, k, tr):
     assert np.all(np.abs(run(a, b, tr) - ref) <= bound(a, b, ref))
 
 
-@pytest.mark.parametrize("tr", [32, 64, 128])
+@pytest.mark.parametrize("tr", [16, 32, 64])
 def test_extreme_digits_are_exact(tr):
     """Every digit at its largest with one sign: the accumulators reach their bound."""
     k = 512
@@ -69,7 +69,7 @@ def test_extreme_digits_are_exact(tr):
     assert np.array_equal(ones, np.full((3, 5), float(k)))
 
 
-@pytest.mark.parametrize("tr", [64, 128])
+@pytest.mark.parametrize("tr", [48, 64])
 def test_zeros_tiny_huge_and_non_finite_rows(tr):
     rng = np.random.default_rng(3)
     a, b = rng.standard_normal((6, 40)), rng.standard_normal((7, 40))
@@ -100,7 +100,7 @@ def test_error_against_a_plain_fp64_sum():
         for i in range(k):  # one FP64 accumulator per element, as a scalar loop
             plain += a[:, i][:, None] * b[:, i][None, :]
         err = lambda x: float(np.sqrt(np.mean((x - ref).astype(np.float64) ** 2)))  # noqa: E731
-        assert err(run(a, b, 128)) <= err(plain), k
+        assert err(run(a, b, 64)) <= err(plain), k
 
 
 # Sizes just above the line where the Taylor products go to the digit GEMM (nw * columns * norb^2 >=
