@@ -4,6 +4,8 @@
 
 namespace afq {
 
+constexpr int kExpSplits = 16;
+
 struct AdjointBufs {
   double2* wb[2];      // walker cotangent at the current point of the backward sweep
   double2* wb2[2];     // second walker cotangent (outputs of the Taylor, QR and SR adjoints)
@@ -18,6 +20,7 @@ struct AdjointBufs {
   double2* fbtb;       // [nw]
   double2* vbar;       // vhs cotangent [nw_chunk][norb^2]
   double2* tay;        // Taylor scratch [nw_chunk][2 M + 2][norb * (k0 + k1)], M = n_exp_terms - 1
+  double* exp_part;    // partial exp_h1 cotangents [kExpSplits][slabs][norb^2]
   double* ebar;        // local-energy cotangent [nw]
   double* scal;        // [0]: cotangent of the population-control shift
   double* beb;         // block-energy cotangents [n blocks]

@@ -72,8 +72,8 @@ struct afq_ctx {
   double2* free_scr;  // free projection: spin constants and QR norm factors [4][nw]
   afq::TcState tc;  // tensor-core (mixed precision) operands and plans
   DigCtx dg;        // digit-sliced FP64 operands and plans
-  // Inside afq_propagate_phaseless only (mixed path): 1 when the operand buffers already
-  // hold G, its operands and the walker operand of the current walkers, else 0.
+  // Inside a block only: 1 when c->green (mixed path: the operand buffers, with G, its operands
+  // and the walker operand) already belongs to the current walkers, else 0.
   int gstate;
 };
 
@@ -267,12 +267,14 @@ bool is_fp64(const afq_ctx* c) { return c->d.precision == AFQ_PREC_FP64; }
 
 // Green's function + overlap. FP64: G into c->green. Mixed: the 16-bit operands of the
 // force-bias, energy and exp_h1 contractions (wg) and/or the overlap.
-// chain (mixed path, inside afq_propagate_phaseless): the walkers are propagated next, so
-// the same launch also forms G and the operands; c->gstate records that for the next step.
+// chain (inside a block): the walkers are propagated next, so the same launch also forms G (mixed
+// path: and the operands); c->gstate records that for the next step.
 int green(afq_ctx* c, const void* wu, const void* wd, double2* g, double2* ovl, bool wg, cudaStream_t st,
           bool chain = false) {
-  if (is_fp64(c)) return afq::launch_green<double>(c->dev, wu, wd, g, ovl, wg, st);
-  CHECK(afq::tc_green(c->tc, c->dev, wu, wd, ovl, wg, st, chain));
+  if (is_fp64(c))
+    CHECK(afq::launch_green<double>(c->dev, wu, wd, chain ? c->green : g, ovl, wg || chain, st));
+  else
+    CHECK(afq::tc_green(c->tc, c->dev, wu, wd, ovl, wg, st, chain));
   c->gstate = chain ? 1 : 0;
   return 0;
 }
@@ -460,7 +462,7 @@ int propagate_impl(afq_ctx* c, afq_walker_state* s, const double* fields, cudaSt
     return afq::tc_weights(c->tc, d, c->ovl_new, reinterpret_cast<double2*>(s->overlaps), s->weights,
                            s->scalars, st);
   }
-  CHECK(green(c, s->walkers_up, s->walkers_dn, c->green, nullptr, true, st));
+  if (!(chain && c->gstate == 1)) CHECK(green(c, s->walkers_up, s->walkers_dn, c->green, nullptr, true, st));
   CHECK(force_bias_from_green(c, c->fb, st));
   CHECK(afq::launch_field_shifts(d, fields, c->fb, c->xt, c->shift, c->fbt, st));
   const int nb = d.nw / c->nw_chunk;
@@ -469,7 +471,7 @@ int propagate_impl(afq_ctx* c, afq_walker_state* s, const double* fields, cudaSt
     CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
     CHECK(taylor_fp64(c, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
   }
-  CHECK(green(c, s->walkers_up, s->walkers_dn, nullptr, c->ovl_new, false, st));
+  CHECK(green(c, s->walkers_up, s->walkers_dn, nullptr, c->ovl_new, false, st, chain && next_g));
   return afq::launch_weights(d, c->shift, c->fbt, 1, c->ovl_new, reinterpret_cast<double2*>(s->overlaps),
                              s->weights, s->scalars, st, c->dg.status);
 }
@@ -587,11 +589,10 @@ struct JvpWalk {
 };
 
 // One phaseless step with tangents (propagate_impl's FP64 branch, each stage followed by
-// its tangent).
+// its tangent). c->green and t.dgreen belong to the walkers; next_g: also after the step.
 int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, const afq::DigOp& drc,
-                  const JvpWalk& jw, const double* fields, cudaStream_t st) {
+                  const JvpWalk& jw, const double* fields, cudaStream_t st, bool next_g) {
   const afq_ctx_dev& d = c->dev;
-  CHECK(afq::t_launch_green(d, t, s->walkers_up, s->walkers_dn, c->green, t.dgreen, c->ovl_new, t.dlo_new, st));
   CHECK(force_bias_from_green(c, c->fb, st));
   CHECK(fb_gemm(c, t.dgreen, c->dg.rc, t.dfb, st));
   if (t.drccat) {  // orbital rotation: + alpha G dRC^T (t.dxt as scratch, rewritten below)
@@ -609,7 +610,8 @@ int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, co
     else
       CHECK(afq::t_launch_taylor(d, t, w0, c->nw_chunk, c->vhs, t.dvhs, s->walkers_up, s->walkers_dn, st));
   }
-  CHECK(afq::t_launch_green(d, t, s->walkers_up, s->walkers_dn, nullptr, nullptr, c->ovl_new, t.dlo_new, st));
+  CHECK(afq::t_launch_green(d, t, s->walkers_up, s->walkers_dn, next_g ? c->green : nullptr,
+                            next_g ? t.dgreen : nullptr, c->ovl_new, t.dlo_new, st));
   return afq::t_launch_weights(d, t, c->shift, c->fbt, c->ovl_new, reinterpret_cast<double2*>(s->overlaps),
                                s->weights, s->scalars, st);
 }
@@ -652,7 +654,7 @@ AdjOps adj_ops(const afq_ctx_dev& c, int nwc) {
 // followed by the backward sweep's cotangents.
 struct AdjSizes {
   size_t snap_w, snap_wt, snap_ov, snap_sc, t_xt, t_sh, t_fbt, t_ene, t_idx;
-  size_t wb, wb2, wbar, lbar, lbar2, gpend, gene, fbb, xtb, shb, fbtb, vbar, tay, ebar, scal, beb, bwb, total;
+  size_t wb, wb2, wbar, lbar, lbar2, gpend, gene, fbb, xtb, shb, fbtb, vbar, tay, exp_part, ebar, scal, beb, bwb, total;
   size_t dg_end, part, et[2][2], vb_ad, vb_ae, vb_bd, vb_be;  // exp_h1^T; operands of the V cotangents
   size_t dg, cn_d, cn_e, rt_d, rt_e, va_d, va_e;  // digits: chol (rows g), rot_chol^T, V cotangents
   size_t wslab;  // walker elements of one snapshot, both slabs
@@ -688,6 +690,7 @@ AdjSizes adjoint_sizes(const afq_ctx_dev& c, int nw_chunk, int n_prop, int n_ene
   s.fbtb = L->take(nw * C16);
   s.vbar = L->take((size_t)nw_chunk * c.norb * c.norb * C16);
   s.tay = L->take((size_t)nw_chunk * (2 * (c.n_exp_terms - 1) + 2) * nk * C16);
+  s.exp_part = L->take((size_t)afq::kExpSplits * c.nslab * c.norb * c.norb * sizeof(double));
   s.ebar = L->take(nw * sizeof(double));
   s.scal = L->take(8 * sizeof(double));
   s.beb = L->take((size_t)s.nblk * sizeof(double));
@@ -1054,7 +1057,7 @@ int afq_propagate_phaseless(afq_ctx* ctx, afq_walker_state* state, const double*
     }
     ctx->gstate = 0;
     CHECK(sr_impl(ctx, state, zetas + sr, nullptr, st));
-    CHECK(green(ctx, state->walkers_up, state->walkers_dn, nullptr, ovl, false, st, true));
+    CHECK(green(ctx, state->walkers_up, state->walkers_dn, nullptr, ovl, false, st, sr + 1 < n_sr_blocks));
   }
   ctx->gstate = 0;
   return afq::launch_phaseless_end(blk, (double)n_sr_blocks * n_ene_blocks * d.nw, block_energy,
@@ -1201,7 +1204,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
   const size_t welems[2] = {(size_t)d.nw * d.norb * d.kslab[0], (size_t)d.nw * d.norb * d.kslab[1]};
   void* wslab[2] = {state->walkers_up, state->walkers_dn};
   ctx->gstate = 0;
-  CHECK(afq::t_launch_green(d, t, state->walkers_up, state->walkers_dn, nullptr, nullptr, ovl, t.dlo, st));
+  CHECK(afq::t_launch_green(d, t, state->walkers_up, state->walkers_dn, ctx->green, t.dgreen, ovl, t.dlo, st));
   CHECK(afq::launch_phaseless_begin(state->scalars, st));
   const size_t step_elems = (size_t)d.nw * d.nchol;
   int blk = 0;
@@ -1209,7 +1212,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
     for (int eb = 0; eb < n_ene_blocks; ++eb, ++blk) {
       for (int p = 0; p < n_prop_steps; ++p) {
         const double* f = fields + ((size_t)blk * n_prop_steps + p) * step_elems;
-        CHECK(propagate_jvp(ctx, state, t, drc, jw, f, st));
+        CHECK(propagate_jvp(ctx, state, t, drc, jw, f, st, p + 1 < n_prop_steps));
       }
       for (int k = 0; k < d.nslab; ++k)
         CHECK(copy_d2d(t.wold[k], wslab[k], welems[k] * sizeof(double2), st, "walker copy before QR"));
@@ -1233,7 +1236,9 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
     CHECK(afq::t_launch_sr_pre(d, t, st));
     CHECK(sr_impl(ctx, state, zetas + sr, nullptr, st));
     CHECK(afq::t_launch_sr_post(d, t, ctx->sr_idx, st));
-    CHECK(afq::t_launch_green(d, t, state->walkers_up, state->walkers_dn, nullptr, nullptr, ovl, t.dlo, st));
+    const bool more = sr + 1 < n_sr_blocks;
+    CHECK(afq::t_launch_green(d, t, state->walkers_up, state->walkers_dn, more ? ctx->green : nullptr,
+                              more ? t.dgreen : nullptr, ovl, t.dlo, st));
   }
   CHECK(afq::launch_phaseless_end(blk, (double)n_sr_blocks * n_ene_blocks * d.nw, block_energy, block_weight,
                                   state->scalars, energy, st));
@@ -1327,6 +1332,7 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
   a.fbtb = reinterpret_cast<double2*>(base + as.fbtb);
   a.vbar = reinterpret_cast<double2*>(base + as.vbar);
   a.tay = reinterpret_cast<double2*>(base + as.tay);
+  a.exp_part = reinterpret_cast<double*>(base + as.exp_part);
   a.ebar = reinterpret_cast<double*>(base + as.ebar);
   a.scal = reinterpret_cast<double*>(base + as.scal);
   a.beb = reinterpret_cast<double*>(base + as.beb);
@@ -1352,7 +1358,7 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
 
   // forward sweep: afq_propagate_phaseless's FP64 path, recording the state
   ctx->gstate = 0;
-  CHECK(green(ctx, state->walkers_up, state->walkers_dn, nullptr, ovl, false, st));
+  CHECK(green(ctx, state->walkers_up, state->walkers_dn, nullptr, ovl, false, st, true));
   CHECK(afq::launch_phaseless_begin(state->scalars, st));
   int blk = 0;
   for (int sr = 0; sr < n_sr_blocks; ++sr) {
@@ -1360,14 +1366,15 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
       for (int p = 0; p < P; ++p) {
         const int step = blk * P + p;
         CHECK(snapshot(tp, blk * (P + 2) + p, state, st));
-        CHECK(propagate_impl(ctx, state, fields + (size_t)step * step_elems, st));
+        CHECK(propagate_impl(ctx, state, fields + (size_t)step * step_elems, st, true, p + 1 < P));
         CHECK(copy_d2d(tp.xt(step), ctx->xt, step_elems * sizeof(double2), st, "shifted-field record"));
         CHECK(copy_d2d(tp.sh(step), ctx->shift, d.nw * sizeof(double2), st, "shift record"));
         CHECK(copy_d2d(tp.fbt(step), ctx->fbt, d.nw * sizeof(double2), st, "fbt record"));
       }
       CHECK(snapshot(tp, blk * (P + 2) + P, state, st));
+      ctx->gstate = 0;
       CHECK(qr_impl(ctx, state, st));
-      CHECK(green(ctx, state->walkers_up, state->walkers_dn, ctx->green, ovl, true, st));
+      CHECK(green(ctx, state->walkers_up, state->walkers_dn, ctx->green, ovl, true, st, true));
       CHECK(snapshot(tp, blk * (P + 2) + P + 1, state, st));
       CHECK(energy_from_green(ctx, ctx->ene, st));
       CHECK(copy_d2d(tp.ene(blk), ctx->ene, d.nw * sizeof(double2), st, "local-energy record"));
@@ -1375,9 +1382,11 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
                                     block_weight + blk, st));
     }
     if (!do_sr) continue;
+    ctx->gstate = 0;
     CHECK(sr_impl(ctx, state, zetas + sr, tp.idx(sr), st));
-    CHECK(green(ctx, state->walkers_up, state->walkers_dn, nullptr, ovl, false, st));
+    CHECK(green(ctx, state->walkers_up, state->walkers_dn, nullptr, ovl, false, st, sr + 1 < n_sr_blocks));
   }
+  ctx->gstate = 0;
   CHECK(afq::launch_phaseless_end(blk, (double)n_sr_blocks * NE * d.nw, block_energy, block_weight,
                                   state->scalars, energy, st));
 
