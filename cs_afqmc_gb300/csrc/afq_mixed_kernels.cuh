@@ -1,53 +1,10 @@
-// Device code of the mixed-precision path: 16-bit operand packing, the Green's function /
-// overlap kernel (FP32 Gauss-Jordan, FP64 log-determinant), GEMM epilogues (fused field
+// Device code of the mixed-precision path: GEMM epilogues (fused field
 // shifts, vhs scatter into the Taylor layout, exp_h1 products, exchange/Coulomb energy),
 // the per-walker tcgen05 Taylor kernel, and one-time operand preparation.
 #pragma once
-#include <cuda_fp16.h>
-
-#include "afq_tc.cuh"
+#include "afq_mixed_dev.cuh"
 
 namespace afq {
-
-// ---- 16-bit helpers -------------------------------------------------------------------
-
-__device__ __forceinline__ uint16_t f2h(float x, bool bf) {
-  return bf ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
-}
-__device__ __forceinline__ float h2f(uint16_t h, bool bf) {
-  return bf ? __bfloat162float(__ushort_as_bfloat16(h)) : __half2float(__ushort_as_half(h));
-}
-// x ~ hi + lo with both parts 16-bit
-__device__ __forceinline__ void split16(float x, bool bf, uint16_t& hi, uint16_t& lo) {
-  hi = f2h(x, bf);
-  lo = f2h(x - h2f(hi, bf), bf);
-}
-// byte offset of (row r, column k < 64) inside a [rows x 64] 16-bit tile, 128-byte swizzle
-__device__ __forceinline__ uint32_t sw128(int r, int k) {
-  return (uint32_t)(r * 128 + ((((k >> 3) ^ (r & 7)) << 4) | ((k & 7) << 1)));
-}
-// exact power of two 2^-e with 2^-e * amax in (0.5, 1]; 1 for amax == 0
-__device__ __forceinline__ float pow2_scale(float amax) {
-  if (!(amax > 0.0f) || !isfinite(amax)) return 1.0f;
-  int e;
-  frexpf(amax, &e);  // amax = m * 2^e, m in [0.5, 1)
-  return ldexpf(1.0f, -e);
-}
-
-// Plain-data view of the mixed state passed to kernels.
-struct MixedDev {
-  int n, nq, nk, ldfb, ldg, nw, nchol, nslab, nblk, kfb, restricted_square, energy_mode;
-  int o_slab[2], R[2], o_blk[2], ldkb[2];
-  int bf16;
-  double h0;
-  const float* trial32[2];
-  const float* rh1_32[2];
-  uint16_t* g_fb[2];
-  uint16_t* g_blk[2][2];  // per-block Green operand (two Green blocks only)
-  uint16_t* wt[2][2];
-  float* g_inv;
-  double2* ene1;
-};
 
 constexpr int kGreenMaxO = 40;  // occupied orbitals per slab (S is at most 40 x 40)
 
@@ -67,365 +24,6 @@ __device__ __forceinline__ void copy_batched(T* dst, const T* __restrict__ src, 
       const int e = base + u * NT;
       if (e < n) dst[map(e)] = v[u];
     }
-  }
-}
-
-// Row stride (complex elements) of the walker copy in k_green_fused: a multiple of 4 columns
-// rounded so that stride / 2 is odd (16-byte aligned rows; the row-per-thread reads of the
-// operand packing then hit each shared-memory bank at most twice per half warp).
-__host__ __device__ constexpr int green_s_ld(int o) {
-  return ((((o + 3) & ~3) >> 1) & 1) ? ((o + 3) & ~3) : ((o + 3) & ~3) + 2;
-}
-
-// ======================================================================================
-// Green's function, overlap and operands in one kernel, one CTA (NT = 128 or 256 threads)
-// per walker (wavefunctions.py:478-501 rhf, 658-692 uhf). Per slab: the walker and trial
-// copied to shared memory; S = C^T W (FP32, the orbital sum split over the NT / 128 thread
-// groups); Gauss-Jordan with partial pivoting on S, double-buffered in shared memory with one
-// barrier per pivot, thread (row group g = warp, column c = lane) updating rows g, g + NW, ..
-// of column c (NW warps); the determinant as the FP64 signed product of the pivots (squared
-// for restricted walkers); then, with kGreenG, G = (W S^-1)^T, its power-of-two scale, the
-// 16-bit operands and ene1 = sum G * rot_h1, with thread (p = tid % 128, h = tid / 128) on
-// orbital p and share h of the occupied columns.
-// kGreenWT also writes the walker operand of the exp_h1 products.
-// Pivoting is implicit, as in a row-per-lane register version: no rows move; the pivot of
-// step j is the unused row with the largest |re| + |im| in column j (ties to the lower row).
-// The working matrix ends as P^T S^-1 P^T for the pivot order P: its row r is row step(r)
-// of S^-1 and its column c is column piv(c); det(S) = sign(P) * prod(pivots).
-// ======================================================================================
-
-constexpr int kGreenWT = 1, kGreenG = 2;
-constexpr int kGfThreads = 128;  // threads per walker CTA (128 or 256; 128 measured faster)
-
-// G lives in its own region when two slabs contribute to it or norb > 128 (each thread then
-// owns two orbital rows); with one slab and norb <= 128 it overwrites the walker copy once
-// G's inputs are in registers
-__host__ __device__ constexpr size_t green_fused_smem(int n, int omax, int om, int gtot, bool g, int nslab) {
-  return (((size_t)n * green_s_ld(omax) * 8 + 15) & ~(size_t)15) +
-         (size_t)om * kGreenMaxO * 8 + ((g && (nslab == 2 || n > 128)) ? (size_t)gtot * n * 8 : 0);
-}
-
-// dst[(e / o) * ld + e % o] = src[e] for e < n * o, 8 loads in flight per thread, the row and
-// column advanced incrementally (no division per element)
-template <int NT>
-__device__ __forceinline__ void copy_rows(float2* dst, const float2* __restrict__ src, int n, int o, int ld) {
-  const int total = n * o, dq = NT / o, dr = NT - dq * o;
-  int p = threadIdx.x / o, k = threadIdx.x - p * o;
-  for (int base = threadIdx.x; base < total; base += 8 * NT) {
-    float2 v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = base + u * NT;
-      if (e < total) v[u] = src[e];
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = base + u * NT;
-      if (e < total) dst[p * ld + k] = v[u];
-      p += dq;
-      k += dr;
-      if (k >= o) {
-        k -= o;
-        ++p;
-      }
-    }
-  }
-}
-
-template <int OM, int NT>
-__global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : 512) / NT) k_green_fused(const MixedDev md, const float2* __restrict__ wu,
-                                                               const float2* __restrict__ wd,
-                                                               double2* __restrict__ ovl, int flags) {
-  extern __shared__ __align__(16) unsigned char sm[];
-  constexpr int NW = NT / 32, NH = NT / 128;  // warps; thread groups of 128 (orbital rows)
-  constexpr int RPT = (OM + NW - 1) / NW;     // rows of S per thread in the Gauss-Jordan phase
-  constexpr int CPL = (OM + 31) / 32;          // columns of S per lane (lane, lane + 32)
-  constexpr int RB = CPL == 1 ? 5 : 6;         // bits of the row index in the pivot-search key
-  const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = md.n;
-  const int p0 = tid & 127, h = tid >> 7;  // orbital rows p0, p0 + 128 (norb <= 256)
-  const bool overlay = md.nslab == 1 && n <= 128;  // G overwrites the walker copy
-  const int omax = md.o_slab[0] > md.o_slab[1] ? md.o_slab[0] : md.o_slab[1];
-  const int ldmax = green_s_ld(omax);
-  const bool do_g = (flags & kGreenG) != 0;
-  const int gtot = md.o_blk[0] + md.o_blk[1];
-  float2* Ws = reinterpret_cast<float2*>(sm);                    // [n][ld] (columns >= o zero)
-  float2* Si = reinterpret_cast<float2*>(sm + (((size_t)n * ldmax * 8 + 15) & ~(size_t)15));  // [OM][kGreenMaxO]
-  // [gtot][n]: after the walker copy's last use when it overlays it (ld >= o = gtot)
-  float2* Gs = overlay ? Ws : Si + OM * kGreenMaxO;
-  __shared__ float2 Ssh[2][OM][OM + 1];  // S (partials), then the double-buffered working matrix
-  __shared__ float2 pivv[OM];
-  __shared__ int piv_s[OM], step_s[OM];
-  __shared__ float2 e1w[NW], e1l[NW];
-  __shared__ float fred[NW];
-  const bool bf = md.bf16 != 0;
-  double2 det = c2(1.0, 0.0);  // thread 0
-  for (int s = 0; s < md.nslab; ++s) {
-    const int o = md.o_slab[s], o4 = (o + 3) & ~3, ld = green_s_ld(o);
-    const float2* W = (s == 0 ? wu : wd) + (size_t)w * n * o;
-    const float* __restrict__ Ct = md.trial32[s];  // [n][o] trial in FP32
-    if (o4 != o)
-      for (int pp = tid; pp < n; pp += NT)
-        for (int k = o; k < o4; ++k) Ws[pp * ld + k] = make_float2(0.f, 0.f);
-    copy_rows<NT>(Ws, W, n, o, ld);
-    __syncthreads();
-    for (int p = p0; (flags & kGreenWT) && p < n; p += 128) {  // walker operand of the exp_h1 products: row (w, 2k + c), column p
-      uint16_t* hi = md.wt[s][0] + (size_t)w * md.R[s] * md.nk + p;
-      uint16_t* lo = md.wt[s][1] + (size_t)w * md.R[s] * md.nk + p;
-      for (int k = h; k < o; k += NH) {
-        const float2 v = Ws[p * ld + k];
-        uint16_t hh, l;
-        split16(v.x, bf, hh, l);
-        hi[(size_t)(2 * k) * md.nk] = hh;
-        lo[(size_t)(2 * k) * md.nk] = l;
-        split16(v.y, bf, hh, l);
-        hi[(size_t)(2 * k + 1) * md.nk] = hh;
-        lo[(size_t)(2 * k + 1) * md.nk] = l;
-      }
-    }
-    // S[i][k..k+3] = sum_p C[p][i] W[p][k..k+3], orbitals split in two halves (partials in
-    // Ssh[0] and Ssh[1], then summed)
-    const int nk4 = o4 / 4, nh = (n + NH - 1) / NH;
-    for (int e = tid; e < NH * o * nk4; e += NT) {
-      const int hh = e / (o * nk4), e2 = e - hh * o * nk4;
-      const int i = e2 / nk4, k0 = (e2 - i * nk4) * 4;
-      float2 a0 = make_float2(0.f, 0.f), a1 = a0, a2 = a0, a3 = a0;
-      const int p1 = hh + 1 == NH ? n : (hh + 1) * nh;
-#pragma unroll 4
-      for (int pp = hh * nh; pp < p1; ++pp) {
-        const float cv = __ldg(&Ct[pp * o + i]);  // the trial: the same for every walker (L1)
-        const float4 x = *reinterpret_cast<const float4*>(&Ws[pp * ld + k0]);
-        const float4 y = *reinterpret_cast<const float4*>(&Ws[pp * ld + k0 + 2]);
-        a0.x = fmaf(cv, x.x, a0.x); a0.y = fmaf(cv, x.y, a0.y);
-        a1.x = fmaf(cv, x.z, a1.x); a1.y = fmaf(cv, x.w, a1.y);
-        a2.x = fmaf(cv, y.x, a2.x); a2.y = fmaf(cv, y.y, a2.y);
-        a3.x = fmaf(cv, y.z, a3.x); a3.y = fmaf(cv, y.w, a3.y);
-      }
-      float2* Sr = &Ssh[hh][i][k0];
-      Sr[0] = a0;
-      if (k0 + 1 < o) Sr[1] = a1;
-      if (k0 + 2 < o) Sr[2] = a2;
-      if (k0 + 3 < o) Sr[3] = a3;
-    }
-    __syncthreads();
-    if (NH == 2) {
-#pragma unroll
-      for (int cc = 0; cc < CPL; ++cc) {
-        const int col = lane + 32 * cc;
-        if (col < o) {
-#pragma unroll
-          for (int m = 0; m < RPT; ++m) {
-            const int r = warp + NW * m;
-            if (r < o) Ssh[0][r][col] = cadd(Ssh[0][r][col], Ssh[1][r][col]);
-          }
-        }
-      }
-      __syncthreads();
-    }
-    // Gauss-Jordan, double-buffered in shared memory: step j reads Ssh[j & 1] and writes
-    // Ssh[(j & 1) ^ 1], so one barrier per pivot; thread (warp, lane) updates rows
-    // warp, warp + 8, .. of columns lane (and lane + 32 for more than 32 electrons).
-    bool used[CPL];  // row lane + 32 cc already pivoted (the same in every warp)
-#pragma unroll
-    for (int cc = 0; cc < CPL; ++cc) used[cc] = lane + 32 * cc >= o;
-#pragma unroll 1
-    for (int j = 0; j < o; ++j) {
-      const int b = j & 1;
-      // loads that do not depend on the pivot first: column j (search), own elements, and
-      // the column-j factors of the own rows
-      float2 own[RPT][CPL], fj[RPT];
-#pragma unroll
-      for (int m = 0; m < RPT; ++m) {
-        const int r = warp + NW * m;
-#pragma unroll
-        for (int cc = 0; cc < CPL; ++cc)
-          own[m][cc] = (r < o && lane + 32 * cc < o) ? Ssh[b][r][lane + 32 * cc] : make_float2(0.f, 0.f);
-        fj[m] = r < o ? Ssh[b][r][j] : make_float2(0.f, 0.f);
-      }
-      unsigned key = 0u;  // |re| + |im| of the candidate rows with the row index in the low bits
-#pragma unroll
-      for (int cc = 0; cc < CPL; ++cc) {
-        const int row = lane + 32 * cc;
-        const float2 v = row < o ? Ssh[b][row][j] : make_float2(0.f, 0.f);
-        const float mag = fabsf(v.x) + fabsf(v.y);
-        const unsigned kc = used[cc] ? 0u
-                                     : ((__float_as_uint(mag) & ~((1u << RB) - 1u)) |
-                                        (unsigned)((1 << RB) - 1 - row));
-        key = kc > key ? kc : key;
-      }
-      const int pr = (1 << RB) - 1 - (int)(__reduce_max_sync(0xffffffffu, key) & ((1u << RB) - 1u));
-#pragma unroll
-      for (int cc = 0; cc < CPL; ++cc)
-        if (lane + 32 * cc == pr) used[cc] = true;
-      const float2 pv = Ssh[b][pr][j];
-      // 1 / pv = conj(pv) / |pv|^2 with pv scaled by a power of two first (no overflow)
-      int ex;
-      frexpf(fmaxf(fabsf(pv.x), fabsf(pv.y)), &ex);
-      const float px = ldexpf(pv.x, -ex), py = ldexpf(pv.y, -ex);
-      const float dd = ldexpf(__frcp_rn(fmaf(px, px, py * py)), -ex);
-      const float2 inv = make_float2(px * dd, -py * dd);
-#pragma unroll
-      for (int cc = 0; cc < CPL; ++cc) {
-        const int col = lane + 32 * cc;
-        if (col < o) {
-          const float2 ap = Ssh[b][pr][col];
-          const float2 sp = (col == j) ? inv : cmul(ap, inv);
-#pragma unroll
-          for (int m = 0; m < RPT; ++m) {
-            const int r = warp + NW * m;
-            if (r < o)
-              Ssh[b ^ 1][r][col] =
-                  (r == pr) ? sp : csub((col == j) ? make_float2(0.f, 0.f) : own[m][cc], cmul(fj[m], sp));
-          }
-        }
-      }
-      if (tid == 0) {
-        pivv[j] = pv;
-        piv_s[j] = pr;
-        step_s[pr] = j;
-      }
-      __syncthreads();
-    }
-    const int fbuf = o & 1;  // buffer holding the final working matrix
-    if (warp == 0) {  // det: FP64 product of the pivots (a shuffle tree), sign of the pivot order
-      int cnt = 0;
-      double2 pd = c2(1.0, 0.0);
-#pragma unroll
-      for (int cc = 0; cc < CPL; ++cc) {
-        const int x = lane + 32 * cc;
-        if (x < o) {
-          for (int y = x + 1; y < o; ++y) cnt += piv_s[x] > piv_s[y] ? 1 : 0;
-          pd = cmul(pd, c2((double)pivv[x].x, (double)pivv[x].y));
-        }
-      }
-      cnt = __reduce_add_sync(0xffffffffu, cnt);
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-        pd = cmul(pd, c2(__shfl_xor_sync(0xffffffffu, pd.x, off), __shfl_xor_sync(0xffffffffu, pd.y, off)));
-      if (lane == 0) det = cmul(det, (cnt & 1) ? c2(-pd.x, -pd.y) : pd);
-    }
-    if (!do_g) {
-      __syncthreads();  // the next slab rewrites Ws and Ssh
-      continue;
-    }
-#pragma unroll
-    for (int cc = 0; cc < CPL; ++cc) {
-      const int col = lane + 32 * cc;
-      if (col < o) {
-#pragma unroll
-        for (int m = 0; m < RPT; ++m) {
-          const int r = warp + NW * m;
-          if (r < o) Si[step_s[r] * kGreenMaxO + piv_s[col]] = Ssh[fbuf][r][col];
-        }
-      }
-    }
-    __syncthreads();
-    // overlay: one row per thread and one pass, every thread reaching the barrier; otherwise
-    // rows p0 and p0 + 128, G in its own region
-    for (int p = p0; p < (overlay ? 128 : n); p += 128) {
-      const bool prow_ok = p < n;
-      float2 wr[OM];
-#pragma unroll
-      for (int k = 0; k < OM; ++k) wr[k] = (prow_ok && k < o) ? Ws[p * ld + k] : make_float2(0.f, 0.f);
-      if (overlay) __syncthreads();  // G overwrites the walker copy
-      if (!prow_ok) continue;
-      const int b = md.nblk == 2 ? s : 0;
-      float2* Gb = Gs + (size_t)(b == 0 ? 0 : md.o_blk[0]) * n;
-      // four columns i at a time (this half's groups): independent accumulation chains,
-      // 16-byte reads of S^-1
-      for (int i0 = 4 * h; i0 < o; i0 += 4 * NH) {
-        float2 a0 = make_float2(0.f, 0.f), a1 = a0, a2 = a0, a3 = a0;
-#pragma unroll
-        for (int k = 0; k < OM; ++k) {
-          if (k < o) {
-            const float4 s01 = *reinterpret_cast<const float4*>(&Si[k * kGreenMaxO + i0]);
-            const float4 s23 = *reinterpret_cast<const float4*>(&Si[k * kGreenMaxO + i0 + 2]);
-            a0 = cadd(a0, cmul(wr[k], make_float2(s01.x, s01.y)));
-            a1 = cadd(a1, cmul(wr[k], make_float2(s01.z, s01.w)));
-            a2 = cadd(a2, cmul(wr[k], make_float2(s23.x, s23.y)));
-            a3 = cadd(a3, cmul(wr[k], make_float2(s23.z, s23.w)));
-          }
-        }
-        const float2 av[4] = {a0, a1, a2, a3};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i0 + u;
-          if (i < o) {
-            float2 acc = av[u];
-            if (md.nblk == 1 && s == 1) acc = cadd(acc, Gb[(size_t)i * n + p]);  // RHF two slabs
-            Gb[(size_t)i * n + p] = acc;
-          }
-        }
-      }
-    }
-    __syncthreads();  // Ws, Ssh and Si are rewritten by the next slab
-  }
-  if (tid == 0 && ovl) ovl[w] = md.restricted_square ? cmul(det, det) : det;
-  if (!do_g) return;
-  float mx = 0.f;
-  for (int p = p0; p < n; p += 128)
-    for (int i = h; i < gtot; i += NH) {
-      const float2 g = Gs[(size_t)i * n + p];
-      mx = fmaxf(mx, fmaxf(fabsf(g.x), fabsf(g.y)));
-    }
-  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  if (lane == 0) fred[warp] = mx;
-  __syncthreads();
-  float mall = fred[0];
-#pragma unroll
-  for (int q = 1; q < NW; ++q) mall = fmaxf(mall, fred[q]);
-  const float scl = pow2_scale(mall);
-  if (tid == 0) md.g_inv[w] = 1.0f / scl;
-  float e1x = 0.f, e1y = 0.f;  // per-thread partials of <= 64 terms; FP64 across warps
-  for (int p = p0; p < n; p += 128) {
-    for (int i = h; i < gtot; i += NH) {
-      const float2 g = Gs[(size_t)i * n + p];
-      const int e = i * n + p;
-      uint16_t hh, l;
-      split16(g.x * scl, bf, hh, l);
-      md.g_fb[0][(size_t)(2 * w) * md.ldfb + e] = hh;
-      md.g_fb[1][(size_t)(2 * w) * md.ldfb + e] = l;
-      split16(g.y * scl, bf, hh, l);
-      md.g_fb[0][(size_t)(2 * w + 1) * md.ldfb + e] = hh;
-      md.g_fb[1][(size_t)(2 * w + 1) * md.ldfb + e] = l;
-      const int b = (md.nblk == 2 && i >= md.o_blk[0]) ? 1 : 0;
-      const int eb = e - b * md.o_blk[0] * n;
-      if (md.nblk == 2) {  // per-block operand (exchange / Coulomb of each spin separately)
-        split16(g.x * scl, bf, hh, l);
-        md.g_blk[b][0][(size_t)(2 * w) * md.ldkb[b] + eb] = hh;
-        md.g_blk[b][1][(size_t)(2 * w) * md.ldkb[b] + eb] = l;
-        split16(g.y * scl, bf, hh, l);
-        md.g_blk[b][0][(size_t)(2 * w + 1) * md.ldkb[b] + eb] = hh;
-        md.g_blk[b][1][(size_t)(2 * w + 1) * md.ldkb[b] + eb] = l;
-      }
-      const float r1 = md.rh1_32[b][eb];
-      e1x = fmaf(g.x, r1, e1x);
-      e1y = fmaf(g.y, r1, e1y);
-    }
-  }
-  // warp sums as unevaluated float pairs (hi + lo, Knuth's TwoSum at every level)
-  float lx = 0.f, ly = 0.f;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const float ox = __shfl_xor_sync(0xffffffffu, e1x, off), oy = __shfl_xor_sync(0xffffffffu, e1y, off);
-    const float olx = __shfl_xor_sync(0xffffffffu, lx, off), oly = __shfl_xor_sync(0xffffffffu, ly, off);
-    float sx = e1x + ox, bx = sx - e1x;
-    lx += olx + ((e1x - (sx - bx)) + (ox - bx));
-    e1x = sx;
-    float sy = e1y + oy, by = sy - e1y;
-    ly += oly + ((e1y - (sy - by)) + (oy - by));
-    e1y = sy;
-  }
-  if (lane == 0) {
-    e1w[warp] = make_float2(e1x, e1y);
-    e1l[warp] = make_float2(lx, ly);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double2 t = c2(0.0, 0.0);
-#pragma unroll
-    for (int q = 0; q < NW; ++q)
-      t = c2(t.x + ((double)e1w[q].x + (double)e1l[q].x), t.y + ((double)e1w[q].y + (double)e1l[q].y));
-    md.ene1[w] = t;
   }
 }
 

@@ -415,6 +415,13 @@ __global__ void k_to_f32(const double* __restrict__ src, float* __restrict__ dst
     dst[i] = (float)src[i];
 }
 
+// rows of `cols` padded to `ld` (the padding is zero already)
+__global__ void k_to_f32_rows(const double* __restrict__ src, float* __restrict__ dst, int rows, int cols, int ld) {
+  const long n = (long)rows * cols;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    dst[i / cols * ld + i % cols] = (float)src[i];
+}
+
 // 2^-e_g with 2^e_g max|src[g][:]| in (0.5, 1]
 __global__ void k_row_scale(const double* __restrict__ src, int len, float* __restrict__ inv) {
   __shared__ float mx_sh[32];
@@ -1050,7 +1057,8 @@ int tc_init(TcState* out, const afq_ctx_dev& c, const afq_hamiltonian& h, const 
   ProfScope _ps(K_PREP, st);
   if (t.cfg & kDiagChol) k_prep_diag<<<c.nchol, 256, 0, st>>>(h.chol, t.n, t.dchol, t.status);
   for (int s = 0; s < t.nslab; ++s) {
-    k_to_f32<<<64, 256, 0, st>>>(c.trial[s], const_cast<float*>(t.trial32[s]), (long)t.n * t.o_slab[s]);
+    k_to_f32_rows<<<64, 256, 0, st>>>(c.trial[s], const_cast<float*>(t.trial32[s]), t.n, t.o_slab[s],
+                                      (t.o_slab[s] + 3) & ~3);
     k_prep_eop<<<64, 256, 0, st>>>(c.exp_h1[s], t.n, t.nk, bf, t.eop[s][0], t.eop[s][1]);
   }
   for (int b = 0; b < t.nblk; ++b) {
@@ -1216,14 +1224,6 @@ int tc_init(TcState* out, const afq_ctx_dev& c, const afq_hamiltonian& h, const 
   return 0;
 }
 
-template <int OM>
-static void launch_green_fused(const MixedDev& md, size_t smem, const float2* w0, const float2* w1, double2* ovl,
-                               int flags, cudaStream_t st) {
-  // a refused attribute surfaces as the launch error checked by the caller
-  cudaFuncSetAttribute(k_green_fused<OM, kGfThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_green_fused<OM, kGfThreads><<<md.nw, kGfThreads, smem, st>>>(md, w0, w1, ovl, flags);
-}
-
 int tc_green(TcState& t, const afq_ctx_dev& c, const void* wu, const void* wd, double2* ovl, bool write_ops,
              cudaStream_t st, bool for_propagation) {
   MixedDev md = mixed_dev(t, c);
@@ -1236,21 +1236,8 @@ int tc_green(TcState& t, const afq_ctx_dev& c, const void* wu, const void* wd, d
   const float2* w1 = static_cast<const float2*>(wd);
   // the walker operand of the exp_h1 GEMMs is needed only when they run as separate launches
   const int flags = (write_ops || for_propagation) ? ((t.fused || t.wide ? 0 : kGreenWT) | kGreenG) : 0;
-  const int om = omax <= 8 ? 8 : omax <= 16 ? 16 : omax <= 24 ? 24 : omax <= 32 ? 32 : 40;
-  const size_t smem =
-      green_fused_smem(t.n, omax, om, md.o_blk[0] + md.o_blk[1], (flags & kGreenG) != 0, md.nslab);
-  if (int rc = check_smem_optin(smem + sizeof(float2) * 2 * om * (om + 1) + 1024,
-                                "mixed Green's-function kernel (norb x electrons too large for one CTA)"))
-    return rc;
-  {
-    ProfScope _ps(K_GREEN, st);
-    if (om == 8) launch_green_fused<8>(md, smem, w0, w1, ovl, flags, st);
-    else if (om == 16) launch_green_fused<16>(md, smem, w0, w1, ovl, flags, st);
-    else if (om == 24) launch_green_fused<24>(md, smem, w0, w1, ovl, flags, st);
-    else if (om == 32) launch_green_fused<32>(md, smem, w0, w1, ovl, flags, st);
-    else launch_green_fused<40>(md, smem, w0, w1, ovl, flags, st);
-  }
-  return launch_check("green_fused");
+  TC_CHECK(launch_green_mixed(md, w0, w1, ovl, flags, st));
+  return launch_check("green");
 }
 
 // energy (with maps == nullptr): the Coulomb contraction of the local energy on the split

@@ -101,7 +101,7 @@ struct TcState {
   double2* part_fbt;        // [nw][fb_ntiles]
   double2* c_out;           // [nblk][nw][nchol]
   double2* exc_part;        // [nblk][nw][mt_z]
-  const float* trial32[2];  // [norb][o_s] trial in FP32
+  const float* trial32[2];  // [norb][o_s padded to 4] trial in FP32
   const float* rh1_32[2];   // [o_b][norb] rot_h1 in FP32
   int* status;              // device word: nonzero after a pipeline timeout (2, 1) or a
                             // non-diagonal Cholesky vector under kDiagChol (4)
