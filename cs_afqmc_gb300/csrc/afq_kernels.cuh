@@ -33,6 +33,9 @@ int check_smem_optin(size_t smem, const char* what);
 template <typename WT>
 int launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, double2* green,
                  double2* ovl, bool write_green, cudaStream_t st);
+// the same for up to 32 electrons per spin, FP64 walkers (afq_green64.cu); errors by cudaGetLastError
+int launch_green_f64(const afq_ctx_dev& c, const void* wu, const void* wd, double2* green, double2* ovl,
+                     bool write_green, cudaStream_t st);
 int launch_gemm_cr(int M, int N, int K, const double2* A, long lda, const double* B,
                    long ldb, double2* C, long ldc, double2 alpha, cudaStream_t st);
 int launch_field_shifts(const afq_ctx_dev& c, const double* fields, const double2* fb,

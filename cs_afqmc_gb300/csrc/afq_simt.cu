@@ -14,7 +14,7 @@ namespace afq {
 
 // ======================================================================================
 // Green's function and overlap.
-// One CTA per walker. For each stored slab s: S = C_s^T W_s (C real), Gauss-Jordan with
+// Above 32 electrons per spin (up to there: afq_green64.cu). One CTA per walker. For each stored slab s: S = C_s^T W_s (C real), Gauss-Jordan with
 // partial pivoting on [S | I] gives det(S) and S^-1, then G_s = (W_s S^-1)^T.
 // wavefunctions.py:478-501 (rhf), 658-692 (uhf).
 // ======================================================================================
@@ -868,6 +868,10 @@ int check_smem_optin(size_t smem, const char* what) {
 template <typename WT>
 int launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, double2* green,
                  double2* ovl, bool write_green, cudaStream_t st) {
+  if (c.kmax <= 32) {
+    launch_green_f64(c, wu, wd, green, ovl, write_green, st);
+    return launch_err("green_f64");
+  }
   const size_t smem = green_f64_smem(c.norb, c.kmax);
   if (int rc = check_smem_optin(smem, "green_overlap (norb x occupied orbitals too large)")) return rc;
   auto kfn = k_green_overlap<WT>;
@@ -1062,7 +1066,6 @@ int launch_fill_uniform(double* out, int64_t n, uint64_t seed, uint64_t offset, 
 }
 
 template int launch_green<double>(const afq_ctx_dev&, const void*, const void*, double2*, double2*, bool, cudaStream_t);
-template int launch_green<float>(const afq_ctx_dev&, const void*, const void*, double2*, double2*, bool, cudaStream_t);
 template int launch_taylor_f64<double>(const afq_ctx_dev&, int, int, const double2*, void*, void*, cudaStream_t);
 template int launch_taylor_f64<float>(const afq_ctx_dev&, int, int, const double2*, void*, void*, cudaStream_t);
 template int launch_qr<double>(const afq_ctx_dev&, void*, void*, cudaStream_t, double2*);
