@@ -477,7 +477,7 @@ int propagate_impl(afq_ctx* c, afq_walker_state* s, const double* fields, cudaSt
 }
 
 int qr_impl(afq_ctx* c, afq_walker_state* s, cudaStream_t st) {
-  if (is_fp64(c)) return afq::launch_qr<double>(c->dev, s->walkers_up, s->walkers_dn, st);
+  if (is_fp64(c)) return afq::launch_qr_f64(c->dev, s->walkers_up, s->walkers_dn, st);
   return afq::tc_orthonormalize(c->tc, c->dev, s->walkers_up, s->walkers_dn, st);
 }
 
@@ -511,7 +511,7 @@ int free_step(afq_ctx* c, afq_walker_state* s, const double* fields, double ene0
     CHECK(taylor_fp64(c, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
   }
   CHECK(afq::launch_free_scale(d, consts, s->walkers_up, s->walkers_dn, st));
-  CHECK(afq::launch_qr<double>(d, s->walkers_up, s->walkers_dn, st, rdiag));
+  CHECK(afq::launch_qr_f64(d, s->walkers_up, s->walkers_dn, st, rdiag));
   CHECK(green(c, s->walkers_up, s->walkers_dn, nullptr, ovl, false, st));
   CHECK(afq::launch_free_finish(d.nw, rdiag, norms, ovl, st));
   // normed overlaps: the walkers through the QR once more, on a copy
@@ -521,7 +521,7 @@ int free_step(afq_ctx* c, afq_walker_state* s, const double* fields, double ene0
   cudaError_t e = cudaMemcpyAsync(cu, s->walkers_up, e0 * sizeof(double2), cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(cd, s->walkers_dn, e1 * sizeof(double2), cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) { afq_set_error("walker copy: %s", cudaGetErrorString(e)); return (int)e; }
-  CHECK(afq::launch_qr<double>(d, cu, cd, st));
+  CHECK(afq::launch_qr_f64(d, cu, cd, st));
   return green(c, cu, cd, nullptr, normed, false, st);
 }
 

@@ -218,15 +218,15 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
 #pragma unroll
     for (int rr = 0; rr < RR; ++rr) {
       const int row = lane + 32 * rr;
-      used[rr] = row >= OM;
+      used[rr] = row >= o;
       step[rr] = 0;
 #pragma unroll
       for (int k = 0; k < OM; ++k) a[rr][k] = row < OM ? Sm[s][row * (OM + 1) + k] : make_float2(0.f, 0.f);
     }
-    unsigned long long open = (1ull << OM) - 1ull;  // rows without a pivot
+    unsigned long long open = (1ull << o) - 1ull;  // rows without a pivot
     int odd = 0;
 #pragma unroll 1
-    for (int j = 0; j < OM; ++j) {
+    for (int j = 0; j < o; ++j) {  // column c ends in register OM - o + c
       float2* pw = prow[s][j & 1];
       unsigned key = 0u;
 #pragma unroll
@@ -299,7 +299,10 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
       for (int rr = 0; rr < RR; ++rr)
         if (lane + 32 * rr < OM) {
 #pragma unroll
-          for (int k = 0; k < OM; ++k) Sm[s][step[rr] * OM + piv_s[s][k]] = a[rr][k];
+          for (int k = 0; k < OM; ++k) {
+            if (lane + 32 * rr >= o) Sm[s][(lane + 32 * rr) * OM + k] = make_float2(0.f, 0.f);
+            else if (k >= OM - o) Sm[s][step[rr] * OM + piv_s[s][k - (OM - o)]] = a[rr][k];
+          }
         }
     }
   }

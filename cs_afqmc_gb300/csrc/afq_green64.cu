@@ -9,12 +9,12 @@ namespace afq {
 
 constexpr int kG64Threads = 128;
 
-// 1 / d for d in [0.5, 16): the FP32 reciprocal and three Newton steps r <- r + r (1 - d r), the
+// 1 / d for d in [0.5, 16): the FP32 reciprocal and two Newton steps r <- r + r (1 - d r), the
 // relative error squared by each (2^-23, 2^-46, then rounding)
 AFQ_D double rcp_scaled(double d) {
   double r = (double)__frcp_rn((float)d);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) r = fma(r, fma(-d, r, 1.0), r);
+  for (int i = 0; i < 2; ++i) r = fma(r, fma(-d, r, 1.0), r);
   return r;
 }
 
@@ -86,15 +86,17 @@ __global__ void __launch_bounds__(kG64Threads, OM <= 20 ? 3 : 2)
   if (warp < (one_warp ? 1 : c.nslab)) {
     const int s = one_warp ? lane >> 4 : warp, row = one_warp ? lane & 15 : lane;
     const unsigned mask = one_warp ? (lane < 16 ? 0xffffu : 0xffff0000u) : 0xffffffffu;
+    // pivots: the electrons (with two slabs in the warp, the larger count; the identity fills up)
+    const int steps = one_warp ? max(c.nocc_slab[0], c.nocc_slab[1]) : c.nocc_slab[s];
     double2 a[OM];
-    bool used = row >= OM;
+    bool used = row >= steps;
     int step = 0;
 #pragma unroll
     for (int k = 0; k < OM; ++k) a[k] = row < OM ? Sm[s][row * (OM + 1) + k] : c2(0.0, 0.0);
-    unsigned open = OM == 32 ? 0xffffffffu : (1u << OM) - 1u;  // rows without a pivot
+    unsigned open = steps == 32 ? 0xffffffffu : (1u << steps) - 1u;  // rows without a pivot
     int odd = 0;
 #pragma unroll 1
-    for (int j = 0; j < OM; ++j) {
+    for (int j = 0; j < steps; ++j) {  // column c ends in register OM - steps + c
       double2* pw = prow[s][j & 1];
       // |re| + |im| of the candidates by the high word, the row index in its low bits
       const unsigned mag = (unsigned)__double2hiint(fabs(a[0].x) + fabs(a[0].y));
@@ -135,7 +137,10 @@ __global__ void __launch_bounds__(kG64Threads, OM <= 20 ? 3 : 2)
     if (row == 0) odd_s[s] = odd;
     if (write_green && row < OM) {
 #pragma unroll
-      for (int k = 0; k < OM; ++k) Sm[s][step * OM + piv_s[s][k]] = a[k];
+      for (int k = 0; k < OM; ++k) {
+        if (row >= steps) Sm[s][row * OM + k] = c2(0.0, 0.0);
+        else if (k >= OM - steps) Sm[s][step * OM + piv_s[s][k - (OM - steps)]] = a[k];
+      }
     }
   }
   __syncthreads();

@@ -51,8 +51,8 @@ int launch_weights(const afq_ctx_dev& c, const double2* shift, const double2* fb
 int launch_energy_f64(const afq_ctx_dev& c, int nchunks, int gchunk, const double2* green,
                       double2* epart, double2* energy, cudaStream_t st);
 // rdiag (optional, [nslab][nw] complex): prod(diag R) per walker slab
-template <typename WT>
-int launch_qr(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, double2* rdiag = nullptr);
+int launch_qr_f64(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, double2* rdiag = nullptr);
+int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st);
 template <typename WT>
 int launch_sr(const afq_ctx_dev& c, const double* zeta, double* weights, double* cum, int32_t* idx,
               void* wu, void* wd, void* wcopy, cudaStream_t st);

@@ -6,6 +6,9 @@
 // float -> complex64 slabs); arithmetic is FP64 throughout this file.
 
 #include <math.h>
+
+#include <algorithm>
+
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
 #include "afq_prof.cuh"
@@ -311,6 +314,82 @@ __global__ void __launch_bounds__(256) k_taylor_f64(const afq_ctx_dev c, int w0,
   }
 }
 
+// The same for small slabs (norb * k <= 512): four lanes per element, each a quarter of the sum
+// over q, so that a product of a few hundred elements is a few dependent FMAs long instead of norb
+// (norb 20, 5 electrons, 50 walkers: 44 us with an element per thread).
+constexpr int kTaylorSmall = 512;
+
+__global__ void __launch_bounds__(256) k_taylor_small(const afq_ctx_dev c, int w0, const double2* __restrict__ vhs,
+                                                      double2* __restrict__ w_up, double2* __restrict__ w_dn) {
+  __shared__ double2 Ta[kTaylorSmall], Tb[kTaylorSmall], Acc[kTaylorSmall];
+  const int wl = blockIdx.x, s = blockIdx.y, norb = c.norb, ks = c.kslab[s], n = norb * ks, tid = threadIdx.x;
+  const int part = tid & 3;
+  const double* __restrict__ E = c.exp_h1[s];
+  const double2* __restrict__ V = vhs + (size_t)wl * norb * norb;
+  double2* W = (s == 0 ? w_up : w_dn) + (size_t)(w0 + wl) * n;
+  for (int i = tid; i < n; i += 256) Ta[i] = W[i];
+  __syncthreads();
+  // dot products over q by four lanes, summed by two shuffles; every lane gets the sum
+  auto sum4 = [&](double2 a) {
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1)
+      a = cadd(a, c2(__shfl_xor_sync(0xffffffffu, a.x, off), __shfl_xor_sync(0xffffffffu, a.y, off)));
+    return a;
+  };
+  auto exp_row = [&](const double2* src, int i) {
+    double2 a = c2(0, 0);
+    if (i < n) {
+      const int p = i / ks, col = i - p * ks;
+#pragma unroll 4
+      for (int q = part; q < norb; q += 4) {
+        const double e = __ldg(E + (size_t)p * norb + q);
+        const double2 t = src[q * ks + col];
+        a = c2(fma(e, t.x, a.x), fma(e, t.y, a.y));
+      }
+    }
+    return sum4(a);
+  };
+  for (int i0 = 0; i0 < n; i0 += 64) {
+    const int i = i0 + (tid >> 2);
+    const double2 a = exp_row(Ta, i);
+    if (i < n && part == 0) Tb[i] = Acc[i] = a;
+  }
+  __syncthreads();
+  double fact = 1.0;
+  double2 *src = Tb, *dst = Ta;
+  for (int m = 1; m < c.n_exp_terms; ++m) {
+    fact *= (double)m;
+    const double invf = 1.0 / fact;
+    for (int i0 = 0; i0 < n; i0 += 64) {
+      const int i = i0 + (tid >> 2);
+      double2 a = c2(0, 0), b = c2(0, 0);  // real and imaginary factors of V apart: shorter chains
+      if (i < n) {
+        const int p = i / ks, col = i - p * ks;
+#pragma unroll 4
+        for (int q = part; q < norb; q += 4) {
+          const double2 v = __ldg(V + (size_t)p * norb + q), t = src[q * ks + col];
+          a = c2(fma(v.x, t.x, a.x), fma(v.x, t.y, a.y));
+          b = c2(fma(-v.y, t.y, b.x), fma(v.y, t.x, b.y));
+        }
+      }
+      a = sum4(cadd(a, b));
+      if (i < n && part == 0) {
+        dst[i] = a;
+        Acc[i] = c2(fma(a.x, invf, Acc[i].x), fma(a.y, invf, Acc[i].y));
+      }
+    }
+    __syncthreads();
+    double2* t = src;
+    src = dst;
+    dst = t;
+  }
+  for (int i0 = 0; i0 < n; i0 += 64) {
+    const int i = i0 + (tid >> 2);
+    const double2 a = exp_row(Acc, i);
+    if (i < n && part == 0) W[i] = a;
+  }
+}
+
 // ======================================================================================
 // Phaseless importance function and weights (propagation.py:133-164). One CTA.
 // ======================================================================================
@@ -471,50 +550,150 @@ __global__ void k_energy_final(const afq_ctx_dev c, int nchunks, const double2* 
 }
 
 // ======================================================================================
-// Householder QR, LAPACK zgeqr2 + zung2r conventions (R has a real diagonal,
-// beta = -sign(Re alpha) * |(alpha, x)|). One CTA per (walker, slab). Q overwrites W.
-// Arithmetic in the walker's precision (FP64 for complex128 walkers, FP32 for complex64).
-// linalg_utils.py:51-65 (jnp.linalg.qr, reduced mode).
+// Householder QR of FP64 walkers, LAPACK zgeqr2 + zung2r conventions (R has a real diagonal,
+// beta = -sign(Re alpha) * |(alpha, x)|), linalg_utils.py:51-65 (jnp.linalg.qr, reduced mode). One
+// warp per (walker, slab) with the slab in shared memory (odd row stride: conflict-free column
+// walks), Q over W. 8 m k^2 FP64 FMAs: a single warp keeps the FP64 units of its SM near busy (18
+// cycles an instruction), and a warp needs no barriers; with 256 threads per slab and seven barriers a
+// column norb 120 / 20 electrons / 256 walkers took 691 us.
+// Column sums are owned by lanes per column, the rank-1 updates by lane = row.
+// rdiag (optional, [nslab][nw]): prod(diag R) per walker slab (linalg_utils.py:51-65 returns
+// it as the norm factor; the free-projection step multiplies its norms by it)
 // ======================================================================================
 
-template <typename CT> struct QrT;
-template <> struct QrT<double2> {
-  using R = double;
-  AFQ_D static double2 mk(double a, double b) { return make_double2(a, b); }
-};
-template <> struct QrT<float2> {
-  using R = float;
-  AFQ_D static float2 mk(float a, float b) { return make_float2(a, b); }
-};
+// y[c] = sum_{r >= j} conj(A[r][j]) A[r][c] for c in (j, k): lpc lanes (a power of two) per column
+AFQ_D void qr64_colsum(const double2* A, int ld, int m, int k, int j, int lane, double2* y) {
+  const int nc = k - j - 1;
+  if (nc <= 0) return;
+  int lpc = 1;
+  while (lpc * 2 * nc <= 32) lpc *= 2;
+  for (int c0 = 0; c0 < nc; c0 += 32 / lpc) {
+    const int c = c0 + lane / lpc, part = lane % lpc;
+    double2 a = c2(0, 0), b = c2(0, 0);
+    if (c < nc) {
+      int r = j + part;
+      for (; r + lpc < m; r += 2 * lpc) {
+        const double2 x = A[r * ld + j + 1 + c], v = A[r * ld + j];
+        const double2 x2 = A[(r + lpc) * ld + j + 1 + c], v2 = A[(r + lpc) * ld + j];
+        a = c2(fma(x.x, v.x, fma(x.y, v.y, a.x)), fma(x.y, v.x, fma(-x.x, v.y, a.y)));
+        b = c2(fma(x2.x, v2.x, fma(x2.y, v2.y, b.x)), fma(x2.y, v2.x, fma(-x2.x, v2.y, b.y)));
+      }
+      if (r < m) {
+        const double2 x = A[r * ld + j + 1 + c], v = A[r * ld + j];
+        a = c2(fma(x.x, v.x, fma(x.y, v.y, a.x)), fma(x.y, v.x, fma(-x.x, v.y, a.y)));
+      }
+      a = cadd(a, b);
+    }
+    for (int off = 1; off < lpc; off <<= 1)
+      a = cadd(a, c2(__shfl_xor_sync(0xffffffffu, a.x, off), __shfl_xor_sync(0xffffffffu, a.y, off)));
+    if (c < nc && part == 0) y[j + 1 + c] = a;
+  }
+}
+
+// A[r][c] -= t v[r] y[c] for r >= j, c > j, v in column j
+AFQ_D void qr64_update(double2* A, int ld, int m, int k, int j, int lane, double2 t, const double2* y) {
+  for (int r = j + lane; r < m; r += 32) {
+    const double2 tv = cmul(t, A[r * ld + j]);
+#pragma unroll 4
+    for (int c = j + 1; c < k; ++c) {
+      const double2 yc = y[c], a = A[r * ld + c];
+      A[r * ld + c] = c2(fma(-tv.x, yc.x, fma(tv.y, yc.y, a.x)), fma(-tv.x, yc.y, fma(-tv.y, yc.x, a.y)));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(32) k_qr_f64(const afq_ctx_dev c, double2* __restrict__ w_up,
+                                               double2* __restrict__ w_dn, double2* __restrict__ rdiag) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int wlk = blockIdx.x, s = blockIdx.y, lane = threadIdx.x;
+  const int m = c.norb, k = c.kslab[s], ld = k | 1;
+  double2* A = reinterpret_cast<double2*>(smem_raw);  // [m][ld]
+  double2* y = A + (size_t)m * ld;                    // [k]
+  double2* tau = y + k;                               // [k]
+  double2* W = (s == 0 ? w_up : w_dn) + (size_t)wlk * m * k;
+  for (int i = lane; i < m * k; i += 32) {
+    const int r = i / k;
+    A[r * ld + (i - r * k)] = W[i];
+  }
+  double2 rprod = c2(1.0, 0.0);
+  __syncwarp();
+  for (int j = 0; j < k; ++j) {
+    double xn = 0.0;
+    for (int r = j + 1 + lane; r < m; r += 32) xn += cabs2(A[r * ld + j]);
+    xn = warp_sum(xn);
+    const double2 alpha = A[j * ld + j];
+    double2 t, scl, beta;
+    if (xn == 0.0 && alpha.y == 0.0) {
+      t = c2(0, 0);
+      beta = alpha;
+      scl = c2(1, 0);
+    } else {
+      const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
+      const double b = alpha.x >= 0.0 ? -nrm : nrm;
+      t = c2((b - alpha.x) / b, -alpha.y / b);
+      scl = cdiv(c2(1, 0), csub(alpha, c2(b, 0)));
+      beta = c2(b, 0);
+    }
+    rprod = cmul(rprod, beta);
+    __syncwarp();
+    for (int r = j + 1 + lane; r < m; r += 32) A[r * ld + j] = cmul(A[r * ld + j], scl);
+    if (lane == 0) {
+      A[j * ld + j] = c2(1, 0);
+      tau[j] = t;
+    }
+    __syncwarp();
+    qr64_colsum(A, ld, m, k, j, lane, y);
+    __syncwarp();
+    qr64_update(A, ld, m, k, j, lane, cconj(t), y);
+    __syncwarp();
+  }
+  if (lane == 0 && rdiag) rdiag[(size_t)s * c.nw + wlk] = rprod;
+  // form Q (zung2r): columns from last to first (the diagonal of column j still holds the reflector's 1)
+  for (int j = k - 1; j >= 0; --j) {
+    const double2 t = tau[j];
+    if (j < k - 1) {
+      qr64_colsum(A, ld, m, k, j, lane, y);
+      __syncwarp();
+      qr64_update(A, ld, m, k, j, lane, t, y);
+      __syncwarp();
+    }
+    const double2 mt = c2(-t.x, -t.y);
+    for (int r = j + 1 + lane; r < m; r += 32) A[r * ld + j] = cmul(mt, A[r * ld + j]);
+    if (lane == 0) A[j * ld + j] = c2(1.0 - t.x, -t.y);
+    for (int r = lane; r < j; r += 32) A[r * ld + j] = c2(0, 0);
+    __syncwarp();
+  }
+  for (int i = lane; i < m * k; i += 32) {
+    const int r = i / k;
+    W[i] = A[r * ld + (i - r * k)];
+  }
+}
+
+// ======================================================================================
+// The same for FP32 walkers whose slabs are too large for the mixed path's warp kernel: one CTA per
+// (walker, slab). Q overwrites W.
+// ======================================================================================
 
 AFQ_D float warp_sumf(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-AFQ_D double warp_sum_t(double v) { return warp_sum(v); }
-AFQ_D float warp_sum_t(float v) { return warp_sumf(v); }
 
-// rdiag (optional, [nslab][nw]): prod(diag R) per walker slab (linalg_utils.py:51-65 returns
-// it as the norm factor; the free-projection step multiplies its norms by it)
-template <typename WT>
-__global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, WT* __restrict__ w_up,
-                                                        WT* __restrict__ w_dn, double2* __restrict__ rdiag) {
-  using CT = typename CplxOf<WT>::type;  // compute in the storage precision
-  using R = typename QrT<CT>::R;
+__global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, float2* __restrict__ w_up,
+                                                        float2* __restrict__ w_dn) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int wlk = blockIdx.x, s = blockIdx.y;
   const int m = c.norb, k = c.kslab[s];
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5,
             nwarp = nt >> 5;
-  CT* A = reinterpret_cast<CT*>(smem_raw);  // [m][k]
-  CT* y = A + (size_t)m * k;                // [k]
-  CT* tau = y + k;                          // [k]
+  float2* A = reinterpret_cast<float2*>(smem_raw);  // [m][k]
+  float2* y = A + (size_t)m * k;                // [k]
+  float2* tau = y + k;                          // [k]
   __shared__ double red[32];
-  __shared__ CT sc_sh, beta_sh;
-  CT* W = reinterpret_cast<CT*>(s == 0 ? w_up : w_dn) + (size_t)wlk * m * k;
+  __shared__ float2 sc_sh, beta_sh;
+  float2* W = (s == 0 ? w_up : w_dn) + (size_t)wlk * m * k;
   for (int i = tid; i < m * k; i += nt) A[i] = W[i];
-  double2 rprod = c2(1.0, 0.0);  // thread 0
   __syncthreads();
   // ---- factorisation
   for (int j = 0; j < k; ++j) {
@@ -522,39 +701,39 @@ __global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, WT*
     for (int r = j + 1 + tid; r < m; r += nt) xnd += (double)cabs2(A[r * k + j]);
     xnd = block_sum(xnd, red);
     if (tid == 0) {
-      const CT alpha = A[j * k + j];
-      const R xn = (R)xnd;
-      if (xn == (R)0 && alpha.y == (R)0) {
-        tau[j] = QrT<CT>::mk(0, 0);
+      const float2 alpha = A[j * k + j];
+      const float xn = (float)xnd;
+      if (xn == (float)0 && alpha.y == (float)0) {
+        tau[j] = make_float2(0, 0);
         beta_sh = alpha;
-        sc_sh = QrT<CT>::mk(1, 0);
+        sc_sh = make_float2(1, 0);
       } else {
-        const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
-        const R beta = (alpha.x >= (R)0) ? -nrm : nrm;
-        tau[j] = QrT<CT>::mk((beta - alpha.x) / beta, -alpha.y / beta);
-        sc_sh = cdiv(QrT<CT>::mk(1, 0), csub(alpha, QrT<CT>::mk(beta, 0)));
-        beta_sh = QrT<CT>::mk(beta, 0);
+        const float nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
+        const float beta = (alpha.x >= (float)0) ? -nrm : nrm;
+        tau[j] = make_float2((beta - alpha.x) / beta, -alpha.y / beta);
+        sc_sh = cdiv(make_float2(1, 0), csub(alpha, make_float2(beta, 0)));
+        beta_sh = make_float2(beta, 0);
       }
     }
     __syncthreads();
-    const CT scl = sc_sh;
+    const float2 scl = sc_sh;
     for (int r = j + 1 + tid; r < m; r += nt) A[r * k + j] = cmul(A[r * k + j], scl);
-    if (tid == 0) A[j * k + j] = QrT<CT>::mk(1, 0);
+    if (tid == 0) A[j * k + j] = make_float2(1, 0);
     __syncthreads();
     // y[col] = sum_r conj(v[r]) A[r][col], col > j ; then A -= conj(tau) v y
     for (int col = j + 1 + wid; col < k; col += nwarp) {
-      R yx = 0, yy = 0;
+      float yx = 0, yy = 0;
       for (int r = j + lane; r < m; r += 32) {
-        const CT pr = cmulc(A[r * k + col], A[r * k + j]);
+        const float2 pr = cmulc(A[r * k + col], A[r * k + j]);
         yx += pr.x;
         yy += pr.y;
       }
-      yx = warp_sum_t(yx);
-      yy = warp_sum_t(yy);
-      if (lane == 0) y[col] = QrT<CT>::mk(yx, yy);
+      yx = warp_sumf(yx);
+      yy = warp_sumf(yy);
+      if (lane == 0) y[col] = make_float2(yx, yy);
     }
     __syncthreads();
-    const CT ct = cconj(tau[j]);
+    const float2 ct = cconj(tau[j]);
     const int ncol = k - j - 1;
     if (ncol > 0) {
       for (int e = tid; e < (m - j) * ncol; e += nt) {
@@ -563,31 +742,27 @@ __global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, WT*
       }
     }
     __syncthreads();
-    if (tid == 0) {
-      A[j * k + j] = beta_sh;
-      rprod = cmul(rprod, c2((double)beta_sh.x, (double)beta_sh.y));
-    }
+    if (tid == 0) A[j * k + j] = beta_sh;
     __syncthreads();
   }
-  if (tid == 0 && rdiag) rdiag[(size_t)s * c.nw + wlk] = rprod;
   // ---- form Q (zung2r): columns from last to first
   for (int j = k - 1; j >= 0; --j) {
     if (j < k - 1) {
-      if (tid == 0) A[j * k + j] = QrT<CT>::mk(1, 0);
+      if (tid == 0) A[j * k + j] = make_float2(1, 0);
       __syncthreads();
       for (int col = j + 1 + wid; col < k; col += nwarp) {
-        R yx = 0, yy = 0;
+        float yx = 0, yy = 0;
         for (int r = j + lane; r < m; r += 32) {
-          const CT pr = cmulc(A[r * k + col], A[r * k + j]);
+          const float2 pr = cmulc(A[r * k + col], A[r * k + j]);
           yx += pr.x;
           yy += pr.y;
         }
-        yx = warp_sum_t(yx);
-        yy = warp_sum_t(yy);
-        if (lane == 0) y[col] = QrT<CT>::mk(yx, yy);
+        yx = warp_sumf(yx);
+        yy = warp_sumf(yy);
+        if (lane == 0) y[col] = make_float2(yx, yy);
       }
       __syncthreads();
-      const CT t = tau[j];
+      const float2 t = tau[j];
       const int ncol = k - j - 1;
       for (int e = tid; e < (m - j) * ncol; e += nt) {
         const int r = j + e / ncol, col = j + 1 + e % ncol;
@@ -595,11 +770,11 @@ __global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, WT*
       }
       __syncthreads();
     }
-    const CT t = tau[j];
-    const CT mt = QrT<CT>::mk(-t.x, -t.y);
+    const float2 t = tau[j];
+    const float2 mt = make_float2(-t.x, -t.y);
     for (int r = j + 1 + tid; r < m; r += nt) A[r * k + j] = cmul(mt, A[r * k + j]);
-    if (tid == 0) A[j * k + j] = QrT<CT>::mk(1 - t.x, -t.y);
-    for (int r = tid; r < j; r += nt) A[r * k + j] = QrT<CT>::mk(0, 0);
+    if (tid == 0) A[j * k + j] = make_float2(1 - t.x, -t.y);
+    for (int r = tid; r < j; r += nt) A[r * k + j] = make_float2(0, 0);
     __syncthreads();
   }
   for (int i = tid; i < m * k; i += nt) W[i] = A[i];
@@ -619,9 +794,19 @@ __global__ void k_sr_indices(int nw, const double* __restrict__ zeta, double* __
   if (in_smem) {
     for (int i = threadIdx.x; i < nw; i += blockDim.x) cum_s[i] = fabs(weights[i]);
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0) {  // sixteen loads ahead of the chain of adds (its latency is all that is left)
       double a = 0.0;
-      for (int i = 0; i < nw; ++i) {
+      int i = 0;
+      for (; i + 16 <= nw; i += 16) {
+        double v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = cum_s[i + u];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = a = a + v[u];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) cum_s[i + u] = v[u];
+      }
+      for (; i < nw; ++i) {
         a += cum_s[i];
         cum_s[i] = a;
       }
@@ -907,6 +1092,13 @@ int launch_field_shifts(const afq_ctx_dev& c, const double* fields, const double
 template <typename WT>
 int launch_taylor_f64(const afq_ctx_dev& c, int w0, int nwc, const double2* vhs, void* wu, void* wd,
                       cudaStream_t st) {
+  if (c.norb * c.kmax <= kTaylorSmall) {
+    {
+      ProfScope _ps(K_TAYLOR, st);
+      k_taylor_small<<<dim3(nwc, c.nslab), 256, 0, st>>>(c, w0, vhs, (double2*)wu, (double2*)wd);
+    }
+    return launch_err("taylor_small");
+  }
   size_t smem = 2 * (size_t)c.norb * c.kmax * sizeof(double2);
   auto kfn = k_taylor_f64<WT>;
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -950,14 +1142,24 @@ int launch_energy_f64(const afq_ctx_dev& c, int nchunks, int gchunk, const doubl
   return launch_err("energy_final");
 }
 
-template <typename WT>
-int launch_qr(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, double2* rdiag) {
-  size_t smem = ((size_t)c.norb * c.kmax + 2 * c.kmax) * sizeof(typename CplxOf<WT>::type);
-  auto kfn = k_qr_householder<WT>;
-  cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+int launch_qr_f64(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, double2* rdiag) {
+  size_t smem = 0;
+  for (int s = 0; s < c.nslab; ++s)
+    smem = std::max(smem, ((size_t)c.norb * (c.kslab[s] | 1) + 2 * c.kslab[s]) * sizeof(double2));
+  cudaFuncSetAttribute(k_qr_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   {
     ProfScope _ps(K_QR, st);
-    kfn<<<dim3(c.nw, c.nslab), 256, smem, st>>>(c, (WT*)wu, (WT*)wd, rdiag);
+    k_qr_f64<<<dim3(c.nw, c.nslab), 32, smem, st>>>(c, (double2*)wu, (double2*)wd, rdiag);
+  }
+  return launch_err("qr_f64");
+}
+
+int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
+  size_t smem = ((size_t)c.norb * c.kmax + 2 * c.kmax) * sizeof(float2);
+  cudaFuncSetAttribute(k_qr_householder, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  {
+    ProfScope _ps(K_QR, st);
+    k_qr_householder<<<dim3(c.nw, c.nslab), 256, smem, st>>>(c, (float2*)wu, (float2*)wd);
   }
   return launch_err("qr_householder");
 }
@@ -1067,9 +1269,6 @@ int launch_fill_uniform(double* out, int64_t n, uint64_t seed, uint64_t offset, 
 
 template int launch_green<double>(const afq_ctx_dev&, const void*, const void*, double2*, double2*, bool, cudaStream_t);
 template int launch_taylor_f64<double>(const afq_ctx_dev&, int, int, const double2*, void*, void*, cudaStream_t);
-template int launch_taylor_f64<float>(const afq_ctx_dev&, int, int, const double2*, void*, void*, cudaStream_t);
-template int launch_qr<double>(const afq_ctx_dev&, void*, void*, cudaStream_t, double2*);
-template int launch_qr<float>(const afq_ctx_dev&, void*, void*, cudaStream_t, double2*);
 template int launch_sr<double>(const afq_ctx_dev&, const double*, double*, double*, int32_t*, void*, void*, void*, cudaStream_t);
 template int launch_sr<float>(const afq_ctx_dev&, const double*, double*, double*, int32_t*, void*, void*, void*, cudaStream_t);
 

@@ -1597,7 +1597,7 @@ int tc_orthonormalize(TcState& t, const afq_ctx_dev& c, void* wu, void* wd, cuda
     const size_t smem = (size_t)kQrWarps * ((size_t)c.norb * qr_ld(k) + 64) * sizeof(float2);
     // the warp kernel holds kQrWarps slabs in shared memory; wider or longer slabs take the
     // one-CTA-per-slab Householder kernel
-    if (k > 32 || smem > 227 * 1024) return launch_qr<float>(c, wu, wd, st);
+    if (k > 32 || smem > 227 * 1024) return launch_qr_f32(c, wu, wd, st);
     cudaFuncSetAttribute(k_qr_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     {
       ProfScope _ps(K_QR, st);
