@@ -235,7 +235,7 @@ Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chu
     take(s.dg_ua, g.ua[big]);
     take(s.dg_ub, g.ub[big]);
     s.dg_uend = L->off;
-    for (int i = 0; i < c.nslab; ++i) take(s.dg_e[i], g.walk.e[i]);
+    for (int i = 0; i < g.walk.n_e(c.nslab); ++i) take(s.dg_e[i], g.walk.e[i]);
     s.dg_v[0] = L->take(g.use_walk ? afq::dig_walk_v_bytes(g.walk) : 256);
     s.dg_v[1] = L->take(g.use_walk ? afq::dig_walk_ve_bytes(g.walk) : 256);
     s.dg_x[0] = L->take(g.use_walk ? afq::dig_walk_x_bytes(g.walk) : 256);
@@ -353,7 +353,7 @@ afq::WalkVec walk_buf(const afq_ctx_dev& d, double2* p, size_t nterm = 1) {
 // out = E_s y_s for every slab (y sliced); acc (optional) = out
 int walk_exp(const afq::DigWalk& w, const afq_ctx_dev& d, const afq::DigOp* E, const afq::WalkOut& o, int nw,
              cudaStream_t st) {
-  for (int s = 0; s < d.nslab; ++s) CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w, s, E, o, nw, st));
+  for (int s = 0; s < w.n_e(d.nslab); ++s) CHECK(afq::dig_walk_mul(afq::K_TAYLOR, w, s, E, o, nw, st));
   return 0;
 }
 
@@ -567,9 +567,9 @@ TSizes tangent_sizes(const afq_ctx_dev& c, int nw_chunk, int e_chunks, Layout* L
   s.drc_e = L->take(afq::dig_exps(g.rc.rows, g.rc.tr));
   s.wk = L->off;
   if (g.use_walk) {
-    for (int i = 0; i < c.nslab; ++i) {
-      s.de[i][0] = L->take(afq::dig_bytes(c.norb, c.norb));
-      s.de[i][1] = L->take(afq::dig_exps(c.norb));
+    for (int i = 0; i < g.walk.n_e(c.nslab); ++i) {
+      s.de[i][0] = L->take(afq::dig_bytes(g.walk.e[i].rows, c.norb));
+      s.de[i][1] = L->take(afq::dig_exps(g.walk.e[i].rows));
     }
     s.v[0] = L->take(afq::dig_walk_v_bytes(g.walk));
     s.v[1] = L->take(afq::dig_walk_ve_bytes(g.walk));
@@ -708,9 +708,9 @@ AdjSizes adjoint_sizes(const afq_ctx_dev& c, int nw_chunk, int n_prop, int n_ene
   if (adj_walk(c, g)) {
     afq::DigVbar v;
     afq::dig_walk_vbar_dims(g.walk, c.n_exp_terms - 1, &v);
-    for (int i = 0; i < c.nslab; ++i) {
-      s.et[i][0] = L->take(afq::dig_bytes(c.norb, c.norb));
-      s.et[i][1] = L->take(afq::dig_exps(c.norb));
+    for (int i = 0; i < g.walk.n_e(c.nslab); ++i) {
+      s.et[i][0] = L->take(afq::dig_bytes(g.walk.e[i].rows, c.norb));
+      s.et[i][1] = L->take(afq::dig_exps(g.walk.e[i].rows));
     }
     s.vb_ad = L->take(afq::dig_walk_vbar_a_bytes(g.walk, v));
     s.vb_ae = L->take(afq::dig_walk_vbar_ae_bytes(g.walk, v));
@@ -942,10 +942,8 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
     c->dg.walk.status = c->dg.status;
     c->dg.walk_t = reinterpret_cast<double2*>(ws + sz.dg_wt);
     c->dg.walk_acc = reinterpret_cast<double2*>(ws + sz.dg_wa);
-    for (int s = 0; s < dev.nslab && !e; ++s) {
-      at(c->dg.walk.e[s], sz.dg_e[s]);
-      e = afq::dig_slice_real_rows(c->dg.walk.e[s], dev.exp_h1[s], dev.norb, st);
-    }
+    for (int s = 0; s < c->dg.walk.n_e(dev.nslab); ++s) at(c->dg.walk.e[s], sz.dg_e[s]);
+    if (!e) e = afq::dig_walk_slice_e(c->dg.walk, c->dg.walk.e, dev.exp_h1, dev.nslab, false, st);
     for (int s = 0; s < dev.nspin_g && c->dg.has_u && !e; ++s) {
       // U[(i,q),(k,p)] = (X X^T)[(i,p),(k,q)], X = rot_chol^T
       at(c->dg.u[s], sz.dg_u[s]);
@@ -1194,11 +1192,11 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
     jw.w.xe = reinterpret_cast<int*>(tw + ts.x[1]);
     jw.t = reinterpret_cast<double2*>(tw + ts.wt);
     jw.a = reinterpret_cast<double2*>(tw + ts.wa);
-    for (int k = 0; k < d.nslab; ++k) {
+    for (int k = 0; k < jw.w.n_e(d.nslab); ++k) {
       jw.w.e[k].d = reinterpret_cast<unsigned char*>(tw + ts.de[k][0]);
       jw.w.e[k].e = reinterpret_cast<int*>(tw + ts.de[k][1]);
-      CHECK(afq::dig_slice_real_rows(jw.w.e[k], t.dexp[k], d.norb, st));
     }
+    CHECK(afq::dig_walk_slice_e(jw.w, jw.w.e, t.dexp, d.nslab, false, st));
   }
   double2* ovl = reinterpret_cast<double2*>(state->overlaps);
   const size_t welems[2] = {(size_t)d.nw * d.norb * d.kslab[0], (size_t)d.nw * d.norb * d.kslab[1]};
@@ -1431,11 +1429,11 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
     vb.ae = reinterpret_cast<int*>(base + as.vb_ae);
     vb.bd = reinterpret_cast<unsigned char*>(base + as.vb_bd);
     vb.be = reinterpret_cast<int*>(base + as.vb_be);
-    for (int k = 0; k < d.nslab; ++k) {
+    for (int k = 0; k < ctx->dg.walk.n_e(d.nslab); ++k) {
       et[k].d = reinterpret_cast<unsigned char*>(base + as.et[k][0]);
       et[k].e = reinterpret_cast<int*>(base + as.et[k][1]);
-      CHECK(afq::dig_slice_real_cols(et[k], d.exp_h1[k], d.norb, st));
     }
+    CHECK(afq::dig_walk_slice_e(ctx->dg.walk, et, d.exp_h1, d.nslab, true, st));
   }
   const double alpha = d.energy_mode == 0 ? 2.0 : 1.0;
   bool gp = false;  // a.gpend holds the pending G cotangent of the current point

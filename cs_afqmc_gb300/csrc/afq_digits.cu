@@ -137,10 +137,11 @@ __global__ void __launch_bounds__(128) k_dig_cplx_rows(const double2* __restrict
 }
 
 __global__ void __launch_bounds__(128) k_dig_real_rows(const double* __restrict__ src, long ld, int K, int kb, int tr,
-                                                       unsigned char* __restrict__ d, int* __restrict__ e) {
+                                                       int row0, unsigned char* __restrict__ d,
+                                                       int* __restrict__ e) {
   __shared__ unsigned red[4];
-  const int m = blockIdx.x;
-  const double* s = src + (size_t)m * ld;
+  const int m = row0 + blockIdx.x;
+  const double* s = src + (size_t)blockIdx.x * ld;
   unsigned er = 0;
   for (int k = threadIdx.x; k < K; k += blockDim.x) er = max(er, dig_key(s[k]));
   const int xr = dig_row_exp(block_max_u(er, red));
@@ -158,14 +159,14 @@ __global__ void __launch_bounds__(128) k_dig_real_rows(const double* __restrict_
 
 // src [K][ld]: lanes along the rows (contiguous), the eight warps split K.
 __global__ void __launch_bounds__(256) k_dig_real_cols(const double* __restrict__ src, long ld, int rows, int K,
-                                                       int kb, int tr, unsigned char* __restrict__ d,
+                                                       int kb, int tr, int row0, unsigned char* __restrict__ d,
                                                        int* __restrict__ e) {
   __shared__ unsigned red[8][32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
-  const bool in = row < rows;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, col = blockIdx.x * 32 + lane, row = row0 + col;
+  const bool in = col < rows;
   unsigned er = 0;
   if (in)
-    for (int k = wid; k < K; k += 8) er = max(er, dig_key(src[(size_t)k * ld + row]));
+    for (int k = wid; k < K; k += 8) er = max(er, dig_key(src[(size_t)k * ld + col]));
   red[wid][lane] = er;
   __syncthreads();
 #pragma unroll
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(256) k_dig_real_cols(const double* __restrict_
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int k = 8 * t + i;
-      q[i] = dig_fixed(k < K ? src[(size_t)k * ld + row] : 0.0, x);
+      q[i] = dig_fixed(k < K ? src[(size_t)k * ld + col] : 0.0, x);
     }
     dig_store(q, dig_block(d, row, t >> 1, kb, tr), tr, row % tr, t & 1);
   }
@@ -187,9 +188,10 @@ __global__ void __launch_bounds__(256) k_dig_real_cols(const double* __restrict_
 // y -> B digits of DigWalk. One CTA per walker; a work item is eight orbitals of one column.
 __global__ void __launch_bounds__(256) k_dig_walk_y(const double2* __restrict__ y0, const double2* __restrict__ y1,
                                                     size_t ws0, size_t ws1, int o0, int ncol, int n, int np, int nt,
-                                                    int tr, unsigned char* __restrict__ d, int* __restrict__ e) {
+                                                    int tr, int stack, unsigned char* __restrict__ d,
+                                                    int* __restrict__ e) {
   __shared__ unsigned key[128];
-  const int w = blockIdx.x, kb = np >> 3, nchunk = np >> 3;
+  const int w = blockIdx.x, kb = stack ? np >> 4 : np >> 3, nchunk = np >> 3;
   const int o1 = ncol - o0, items = ncol * nchunk;
   for (int i = threadIdx.x; i < ncol; i += blockDim.x) key[i] = 0;
   __syncthreads();
@@ -230,20 +232,22 @@ __global__ void __launch_bounds__(256) k_dig_walk_y(const double2* __restrict__ 
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] = dig_fixed(v[i].x, x);
     dig_store(q, b, tr, r, ch & 1);
-    dig_store(q, b2, tr, r + 1, ch & 1);
+    if (!stack) dig_store(q, b2, tr, r + 1, ch & 1);
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] = dig_fixed(v[i].y, x);
     dig_store(q, b, tr, r + 1, ch & 1);
-    dig_store(q, b2, tr, r, ch & 1, 0x80008000u);
+    if (!stack) dig_store(q, b2, tr, r, ch & 1, 0x80008000u);
   }
 }
 
-// V [w][n][n] -> A digits, rows p, K = [Re V[p][q] | Im V[p][q]]. LPR lanes per row, eight q each
+// V [w][n][n] -> A digits, rows p, K = [Re V[p][q] | Im V[p][q]], or stacked, rows p = Re V[p][q] and
+// 64 + p = Im V[p][q]. LPR lanes per row, eight q each
 // (LPR * 8 >= np).
 template <int LPR>
 __global__ void __launch_bounds__(256) k_dig_walk_v(const double2* __restrict__ V, int nrows, int n, int np, int mt,
-                                                    unsigned char* __restrict__ d, int* __restrict__ e) {
-  const int g = (blockIdx.x * 256 + threadIdx.x) / LPR, ch = threadIdx.x % LPR, kb = np >> 3;
+                                                    int stack, unsigned char* __restrict__ d,
+                                                    int* __restrict__ e) {
+  const int g = (blockIdx.x * 256 + threadIdx.x) / LPR, ch = threadIdx.x % LPR, kb = stack ? np >> 4 : np >> 3;
   const bool in = g < nrows;
   const int w = in ? g / n : 0, p = in ? g % n : 0;
   const double2* src = V + ((size_t)w * n + p) * n;
@@ -259,7 +263,10 @@ __global__ void __launch_bounds__(256) k_dig_walk_v(const double2* __restrict__ 
   for (int o = LPR / 2; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
   if (!in) return;
   const int x = dig_row_exp(k);
-  if (ch == 0) e[(size_t)w * mt * kDigTile + p] = x;
+  if (ch == 0) {
+    e[(size_t)w * mt * kDigTile + p] = x;
+    if (stack) e[(size_t)w * mt * kDigTile + 64 + p] = x;
+  }
   if (8 * ch >= np) return;
   unsigned char* b = dig_block(d + (size_t)w * mt * kb * (kDigTile * 256), p, ch >> 1, kb, kDigTile);
   long long q8[8];
@@ -268,14 +275,16 @@ __global__ void __launch_bounds__(256) k_dig_walk_v(const double2* __restrict__ 
   dig_store(q8, b, kDigTile, p & (kDigTile - 1), ch & 1);
 #pragma unroll
   for (int i = 0; i < 8; ++i) q8[i] = dig_fixed(v[i].y, x);
-  dig_store(q8, b + (size_t)(np >> 4) * (kDigTile * 256), kDigTile, p & (kDigTile - 1), ch & 1);
+  if (stack) dig_store(q8, b, kDigTile, 64 + p, ch & 1);
+  else dig_store(q8, b + (size_t)(np >> 4) * (kDigTile * 256), kDigTile, p & (kDigTile - 1), ch & 1);
 }
 
-// V^H: rows q, K = [Re V[p][q] | -Im V[p][q]] over p. CTA per (walker, 32 rows), lanes along q.
-__global__ void __launch_bounds__(256) k_dig_walk_vh(const double2* __restrict__ V, int n, int np, int mt,
+// V^H: rows q, K = [Re V[p][q] | -Im V[p][q]] over p, or stacked the same way. CTA per (walker, 32 rows), lanes along q.
+__global__ void __launch_bounds__(256) k_dig_walk_vh(const double2* __restrict__ V, int n, int np, int mt, int stack,
                                                      unsigned char* __restrict__ d, int* __restrict__ e) {
   __shared__ unsigned red[8][32];
-  const int w = blockIdx.y, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = blockIdx.x * 32 + lane, kb = np >> 3;
+  const int w = blockIdx.y, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = blockIdx.x * 32 + lane,
+            kb = stack ? np >> 4 : np >> 3;
   const bool in = q < n;
   const double2* src = V + (size_t)w * n * n + q;
   unsigned k = 0;
@@ -290,7 +299,10 @@ __global__ void __launch_bounds__(256) k_dig_walk_vh(const double2* __restrict__
   for (int i = 0; i < 8; ++i) k = max(k, red[i][lane]);
   const int x = dig_row_exp(k);
   if (!in) return;
-  if (wid == 0) e[(size_t)w * mt * kDigTile + q] = x;
+  if (wid == 0) {
+    e[(size_t)w * mt * kDigTile + q] = x;
+    if (stack) e[(size_t)w * mt * kDigTile + 64 + q] = x;
+  }
   for (int t = wid; t < (np >> 3); t += 8) {
     long long a[8], b8[8];
 #pragma unroll
@@ -302,7 +314,8 @@ __global__ void __launch_bounds__(256) k_dig_walk_vh(const double2* __restrict__
     }
     unsigned char* b = dig_block(d + (size_t)w * mt * kb * (kDigTile * 256), q, t >> 1, kb, kDigTile);
     dig_store(a, b, kDigTile, q & (kDigTile - 1), t & 1);
-    dig_store(b8, b + (size_t)(np >> 4) * (kDigTile * 256), kDigTile, q & (kDigTile - 1), t & 1, 0x80008000u);
+    if (stack) dig_store(b8, b, kDigTile, 64 + q, t & 1, 0x80008000u);
+    else dig_store(b8, b + (size_t)(np >> 4) * (kDigTile * 256), kDigTile, q & (kDigTile - 1), t & 1, 0x80008000u);
   }
 }
 
@@ -457,6 +470,11 @@ constexpr int kDigThreads = 64 + 32 * kDigEpiWarps;
 constexpr int kDigABlock = kDigTile * 256;  // bytes of an A K block
 constexpr int kDigRing = 196608;
 constexpr int kDigSmem = 1024 + kDigRing + 256;
+// stacked products: a shorter ring and the exchange of half of each warp's sums (8-byte and 4-byte
+// words, up to 8 per thread)
+constexpr int kDigRingS = 3 * (kDigTile * 256 + 64 * 256);
+constexpr int kDigXchg = 32 * kDigEpiWarps * 8 * 12;
+constexpr int kDigSmemS = 1024 + kDigRingS + 256 + kDigXchg;
 constexpr int kDigMaxStages = 5;
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -484,12 +502,13 @@ __global__ void __launch_bounds__(kDigThreads, 1)
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kDigRing);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (Epi::kStack ? kDigRingS : kDigRing));
   uint64_t* empty = full + kDigMaxStages;
   uint64_t* accfull = empty + kDigMaxStages;  // [2]
   uint64_t* accempty = accfull + 2;           // [2]
   uint64_t* done = accempty + 2;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
+  uint64_t* xbar = done + 1;  // [8] stacked: the two warps that exchange sums
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(xbar + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tr = g.tr, bblock = tr * 256, unit = kDigABlock + bblock;
   const int acols = tr <= 32 ? 32 : 64;  // columns between accumulators
@@ -505,6 +524,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
       ptx::mbar_init(&accempty[i], kDigEpiWarps);
     }
     ptx::mbar_init(done, 1);
+    for (int i = 0; i < 8; ++i) ptx::mbar_init(&xbar[i], 2);
     ptx::fence_mbar_init();
   }
   if (warp == 1) {
@@ -594,7 +614,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
     const int q = warp & 3, r = q * 32 + lane;
     const int nc = tr >> 2, col0 = ((warp - 2) >> 2) * nc;  // this warp's columns (4..16)
     const uint32_t src0 = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)col0;
-    int run = 0;
+    int run = 0, meets = 0;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
       DigWhere w;
       w.split = tile / mn;
@@ -635,6 +655,64 @@ __global__ void __launch_bounds__(kDigThreads, 1)
         ptx::tc_fence_before();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
+        if constexpr (Epi::kStack) {
+          // Row p of Re V (lanes quarters 0, 1) and of Im V (2, 3): the first takes the lower half of this
+          // warp's column pairs, the second the upper half, and each gets the other's sums for them.
+          if (ep.pair) {
+            long long* xh = reinterpret_cast<long long*>(smem + kDigRingS + 256);
+            unsigned* xl = reinterpret_cast<unsigned*>(xh + 32 * kDigEpiWarps * 8);
+            // warps q and q ^ 2 of a column quarter are two apart in the CTA (q = 2, 3 come first)
+            const int up = q >> 1, me = threadIdx.x - 64, peer = up ? me + 64 : me - 64;
+            uint64_t* bar = &xbar[((warp - 2) >> 2) * 2 + (q & 1)];
+            auto meet = [&]() {  // bounded, as every wait here
+              __syncwarp();
+              if (lane == 0) ptx::mbar_arrive(bar);
+              const bool got = ptx::mbar_wait(bar, meets & 1);
+              ++meets;
+              return __all_sync(0xffffffffu, got) != 0;
+            };
+            const int hc = nc >> 1;  // columns kept; the other hc go to the peer
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (j < nc && (j < hc) == (up != 0)) {
+                const int t = up ? j : j - hc;
+                xh[t * (32 * kDigEpiWarps) + me] = hi[j];
+                xl[t * (32 * kDigEpiWarps) + me] = lo[j];
+              }
+            if (!meet()) {
+              ok = false;
+              break;
+            }
+#pragma unroll
+            for (int j = 0; j < 16; j += 2)
+              if (j < nc && (j < hc) != (up != 0)) {
+                const int t = up ? j - hc : j;
+                const long long h0 = xh[t * (32 * kDigEpiWarps) + peer], h1 = xh[(t + 1) * (32 * kDigEpiWarps) + peer];
+                const unsigned l0 = xl[t * (32 * kDigEpiWarps) + peer], l1 = xl[(t + 1) * (32 * kDigEpiWarps) + peer];
+                // Re = Re V Re y - Im V Im y, Im = Re V Im y + Im V Re y: own a, b, peer's l0, l1 (or swapped)
+                const long long rh = up ? h0 : hi[j], ih = up ? hi[j + 1] : h1;
+                const int dl = (int)(up ? l0 : lo[j]) - (int)(up ? lo[j + 1] : l1);
+                const long long sh = up ? h1 + hi[j] : hi[j + 1] + h0;
+                const unsigned sl = up ? l1 + lo[j] : lo[j + 1] + l0;
+                const int e = er + eb[j];
+                const double2 z = c2(dig_combine(rh - ih + (dl >> 28), (unsigned)dl & 0xfffffffu, e),
+                                     dig_combine(sh + (sl >> 28), sl & 0xfffffffu, e));
+                Epi::store_c(ep, w, r & 63, (w.n * tr + col0 + j) >> 1, z);
+              }
+            if (!meet()) {  // read before the next tile's sums go there
+              ok = false;
+              break;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; j += 2)
+              if (j < nc) {
+                const int c = (w.n * tr + col0 + j) >> 1, e = er + eb[j];
+                if ((c >= ep.o0) == (r >= 64))
+                  Epi::store_c(ep, w, r & 63, c, c2(dig_combine(hi[j], lo[j], e), dig_combine(hi[j + 1], lo[j + 1], e)));
+              }
+          }
+        } else {
 #pragma unroll
         for (int c0 = 0; c0 < 16; c0 += 4)
           if (c0 < nc) {
@@ -643,6 +721,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
             for (int j = 0; j < 4; ++j) o[j] = dig_combine(hi[c0 + j], lo[c0 + j], er + eb[c0 + j]);
             Epi::store(ep, w, r, col0 + c0, o);
           }
+        }
       }
     }
   }
@@ -658,7 +737,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
 // Complex results: rows 2m / 2m + 1 of D are the real and imaginary parts of row m of C.
 // Neighbouring lanes exchange halves so that each stores whole complex numbers.
 struct EpiDigC {
-  static constexpr bool kNine = false;
+  static constexpr bool kNine = false, kStack = false;
   struct Params {
     double2* c;
     int M, N, tr;
@@ -685,7 +764,7 @@ struct EpiDigC {
 };
 
 struct EpiDigR {
-  static constexpr bool kNine = false;
+  static constexpr bool kNine = false, kStack = false;
   struct Params {
     double* d;
     int M, N, tr;
@@ -714,41 +793,49 @@ struct EpiDigR {
 // then rounded once): exp_h1 is nearly diagonal and a column of a walker has a few large entries,
 // so the scale of a dot product can be far above its value. Walkers after a step, against
 // extended precision: 1.7e-16 at norb 33, 2.1e-16 at norb 120; the FP64 units: 3.5e-16, 6.2e-16.
-struct EpiWalk {
-  static constexpr bool kNine = true;
-  struct Params {
-    WalkOut o;
-    int n, o0, ncol, tr, only;  // only: the slab to store (-1: both)
-    int shift;
-  };
-  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
-    const int row = w.m * kDigTile + r;
-    if (row >= p.n) return;
-#pragma unroll
-    for (int j = 0; j < 4; j += 2) {
-      const int c = (w.n * p.tr + col0 + j) >> 1, s = c >= p.o0 ? 1 : 0;
-      if (c >= p.ncol || (p.only >= 0 && s != p.only)) continue;
-      const int k = s ? p.ncol - p.o0 : p.o0;
-      const size_t i = (size_t)row * k + (s ? c - p.o0 : c);
-      double2 x = c2(v[j], v[j + 1]);
-      if (w.add) x = cadd(x, p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i]);
-      const bool last = !w.more;
-      if (last && p.o.in.p[s]) {
-        const double2 y = p.o.in.p[s][(size_t)w.batch * p.o.in.stride(s) + i];
-        x = c2(fma(y.x, p.o.fin, x.x), fma(y.y, p.o.fin, x.y));
-      }
-      if (p.o.out.p[s]) p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i] = cscale(x, last ? p.o.fout : 1.0);
-      if (last && p.o.acc.p[s]) {
-        double2* a = p.o.acc.p[s] + (size_t)w.batch * p.o.acc.stride(s) + i;
-        if (p.o.init) {
-          *a = x;
-        } else {
-          const double2 y = *a;
-          *a = c2(fma(x.x, p.o.facc, y.x), fma(x.y, p.o.facc, y.y));
-        }
-      }
+struct WalkParams {
+  WalkOut o;
+  int n, o0, ncol, tr, only;  // only: the slab to store (-1: both)
+  int pair;                   // stacked: V (two row halves make one result) or E (a slab each)
+  int shift;
+};
+
+AFQ_D void walk_store(const WalkParams& p, const DigWhere& w, int row, int c, double2 x) {
+  const int s = c >= p.o0 ? 1 : 0;
+  if (row >= p.n || c >= p.ncol || (p.only >= 0 && s != p.only)) return;
+  const int k = s ? p.ncol - p.o0 : p.o0;
+  const size_t i = (size_t)row * k + (s ? c - p.o0 : c);
+  if (w.add) x = cadd(x, p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i]);
+  const bool last = !w.more;
+  if (last && p.o.in.p[s]) {
+    const double2 y = p.o.in.p[s][(size_t)w.batch * p.o.in.stride(s) + i];
+    x = c2(fma(y.x, p.o.fin, x.x), fma(y.y, p.o.fin, x.y));
+  }
+  if (p.o.out.p[s]) p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i] = last && p.o.fout != 1.0 ? cscale(x, p.o.fout) : x;
+  if (last && p.o.acc.p[s]) {
+    double2* a = p.o.acc.p[s] + (size_t)w.batch * p.o.acc.stride(s) + i;
+    if (p.o.init) {
+      *a = x;
+    } else {
+      const double2 y = *a;
+      *a = c2(fma(x.x, p.o.facc, y.x), fma(x.y, p.o.facc, y.y));
     }
   }
+}
+
+struct EpiWalk {
+  static constexpr bool kNine = true, kStack = false;
+  using Params = WalkParams;
+  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; j += 2)
+      walk_store(p, w, w.m * kDigTile + r, (w.n * p.tr + col0 + j) >> 1, c2(v[j], v[j + 1]));
+  }
+};
+struct EpiWalkStack {
+  static constexpr bool kNine = true, kStack = true;
+  using Params = WalkParams;
+  AFQ_D static void store_c(const Params& p, const DigWhere& w, int row, int c, double2 z) { walk_store(p, w, row, c, z); }
 };
 
 // C = sum of the partial results of a split contraction
@@ -883,38 +970,40 @@ int dig_slice_cplx_rows(const DigOp& op, const double2* src, long ld, double mul
   return dig_err("slice rows");
 }
 
-int dig_slice_real_rows(const DigOp& op, const double* src, long ld, cudaStream_t st) {
+int dig_slice_real_rows(const DigOp& op, const double* src, long ld, cudaStream_t st, int rows, int row0) {
   {
     ProfScope _ps(K_PREP, st);
-    k_dig_real_rows<<<op.rows, 128, 0, st>>>(src, ld, op.K, op.kb(), op.tr, op.d, op.e);
+    k_dig_real_rows<<<rows < 0 ? op.rows : rows, 128, 0, st>>>(src, ld, op.K, op.kb(), op.tr, row0, op.d, op.e);
   }
   return dig_err("slice rows");
 }
 
-int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_t st) {
+int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_t st, int rows, int row0) {
   {
     ProfScope _ps(K_PREP, st);
-    k_dig_real_cols<<<(op.rows + 31) / 32, 256, 0, st>>>(src, ld, op.rows, op.K, op.kb(), op.tr, op.d, op.e);
+    const int r = rows < 0 ? op.rows : rows;
+    k_dig_real_cols<<<(r + 31) / 32, 256, 0, st>>>(src, ld, r, op.K, op.kb(), op.tr, row0, op.d, op.e);
   }
   return dig_err("slice columns");
 }
 
 template <class Epi>
 static int launch_digits(int cls, DigGemm g, const typename Epi::Params& ep, int* status, cudaStream_t st) {
-  const int unit = kDigABlock + g.tr * 256;
-  g.stages = kDigRing / unit < kDigMaxStages ? kDigRing / unit : kDigMaxStages;
+  const int unit = kDigABlock + g.tr * 256, ring = Epi::kStack ? kDigRingS : kDigRing;
+  const int smem = Epi::kStack ? kDigSmemS : kDigSmem;
+  g.stages = ring / unit < kDigMaxStages ? ring / unit : kDigMaxStages;
   g.idesc = ptx::idesc_f16(128, g.tr, 1);
   const long tiles = (long)g.mt * g.nt * g.nb * g.splits;
   const int sms = dig_sms();
   auto kfn = k_gemm_digits<Epi>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kDigSmem);
+  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) {
     afq_set_error("digit GEMM: shared-memory attribute: %s", cudaGetErrorString(e));
     return (int)e;
   }
   {
     ProfScope _ps(cls, st);
-    kfn<<<(unsigned)(tiles < sms ? tiles : sms), kDigThreads, kDigSmem, st>>>(g, ep, status);
+    kfn<<<(unsigned)(tiles < sms ? tiles : sms), kDigThreads, smem, st>>>(g, ep, status);
   }
   return dig_err("digit GEMM");
 }
@@ -994,6 +1083,7 @@ int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D,
 }
 
 void dig_walk_dims(int norb, const int* k, int nslab, int nw, DigWalk* d) {
+  d->stack = norb <= 64 ? 1 : 0;
   d->n = norb;
   d->np = (norb + 15) / 16 * 16;
   d->o[0] = k[0];
@@ -1003,17 +1093,17 @@ void dig_walk_dims(int norb, const int* k, int nslab, int nw, DigWalk* d) {
   d->nt = (2 * d->ncol + 63) / 64;
   d->tr = ((2 * d->ncol + d->nt - 1) / d->nt + 15) / 16 * 16;
   // V digits of a chunk: at most 160 MB, whole rounds of the 152 SMs where it is cut
-  const size_t per = (size_t)d->mt * kDigTile * d->np * 32;
+  const size_t per = (size_t)d->mt * kDigTile * d->kbv() * 256;
   const long most = std::max<long>((long)((160u << 20) / per) / 152 * 152, 152);
   d->chunk = nw < most ? nw : (int)most;
   for (int s = 0; s < 2; ++s) {
-    d->e[s].rows = norb;
+    d->e[s].rows = d->stack ? kDigTile : norb;
     d->e[s].K = norb;
     d->e[s].tr = kDigTile;
   }
 }
-size_t dig_walk_v_bytes(const DigWalk& d) { return (size_t)d.chunk * d.mt * kDigTile * d.np * 32; }
-size_t dig_walk_x_bytes(const DigWalk& d) { return (size_t)d.chunk * d.nt * d.tr * d.np * 32; }
+size_t dig_walk_v_bytes(const DigWalk& d) { return (size_t)d.chunk * d.mt * kDigTile * d.kbv() * 256; }
+size_t dig_walk_x_bytes(const DigWalk& d) { return (size_t)d.chunk * d.nt * d.tr * d.kbv() * 256; }
 size_t dig_walk_ve_bytes(const DigWalk& d) { return (size_t)d.chunk * d.mt * kDigTile * sizeof(int); }
 size_t dig_walk_xe_bytes(const DigWalk& d) { return (size_t)d.chunk * d.nt * d.tr * sizeof(int); }
 
@@ -1022,13 +1112,13 @@ int dig_walk_slice_v(const DigWalk& d, const double2* V, int nw, bool adjoint, c
     ProfScope _ps(K_TAYLOR, st);
     const int rows = nw * d.n;
     if (adjoint) {
-      k_dig_walk_vh<<<dim3((d.n + 31) / 32, nw), 256, 0, st>>>(V, d.n, d.np, d.mt, d.vd, d.ve);
+      k_dig_walk_vh<<<dim3((d.n + 31) / 32, nw), 256, 0, st>>>(V, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     } else if (d.np <= 64) {
-      k_dig_walk_v<8><<<(rows + 31) / 32, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.vd, d.ve);
+      k_dig_walk_v<8><<<(rows + 31) / 32, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     } else if (d.np <= 128) {
-      k_dig_walk_v<16><<<(rows + 15) / 16, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.vd, d.ve);
+      k_dig_walk_v<16><<<(rows + 15) / 16, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     } else {
-      k_dig_walk_v<32><<<(rows + 7) / 8, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.vd, d.ve);
+      k_dig_walk_v<32><<<(rows + 7) / 8, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     }
   }
   return dig_err("slice V");
@@ -1038,7 +1128,7 @@ int dig_walk_slice_y(const DigWalk& d, const WalkVec& y, int nw, cudaStream_t st
   {
     ProfScope _ps(K_TAYLOR, st);
     k_dig_walk_y<<<nw, 256, 0, st>>>(y.p[0], y.p[1], y.stride(0), y.stride(1), d.o[0], d.ncol, d.n, d.np, d.nt, d.tr,
-                                     d.xd, d.xe);
+                                     d.stack, d.xd, d.xe);
   }
   return dig_err("slice y");
 }
@@ -1059,8 +1149,21 @@ int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut
   g.tr = d.tr;
   g.splits = 1;
   g.kps = g.kb;
-  EpiWalk::Params ep{o, d.n, d.o[0], d.ncol, d.tr, e < 0 || d.o[1] == 0 ? -1 : e, 0};
-  return launch_digits<EpiWalk>(cls, g, ep, d.status, st);
+  WalkParams ep{o, d.n, d.o[0], d.ncol, d.tr, d.stack || e < 0 || d.o[1] == 0 ? -1 : e, e < 0 ? 1 : 0, 0};
+  return d.stack ? launch_digits<EpiWalkStack>(cls, g, ep, d.status, st)
+                 : launch_digits<EpiWalk>(cls, g, ep, d.status, st);
+}
+
+int dig_walk_slice_e(const DigWalk& d, const DigOp* e, const double* const* exp_h1, int nslab, bool transpose,
+                     cudaStream_t st) {
+  for (int s = 0; s < nslab; ++s) {
+    const DigOp& op = d.stack ? e[0] : e[s];
+    const int row0 = d.stack ? 64 * s : 0;
+    if (int rc = transpose ? dig_slice_real_cols(op, exp_h1[s], d.n, st, d.n, row0)
+                           : dig_slice_real_rows(op, exp_h1[s], d.n, st, d.n, row0))
+      return rc;
+  }
+  return 0;
 }
 
 void dig_walk_vbar_dims(const DigWalk& d, int M, DigVbar* v) {
@@ -1102,7 +1205,7 @@ int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int te
   g.kps = g.kb;
   WalkOut o;  // [norb][norb] per walker: one slab of norb columns
   o.out = WalkVec{{vbar, nullptr}, (size_t)d.n * d.n};
-  EpiWalk::Params ep{o, d.n, d.n, d.n, v.tr, -1, 0};
+  WalkParams ep{o, d.n, d.n, d.n, v.tr, -1, 0, 0};
   return launch_digits<EpiWalk>(K_TAYLOR, g, ep, d.status, st);
 }
 

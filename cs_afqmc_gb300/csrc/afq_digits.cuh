@@ -46,10 +46,10 @@ struct DigOp {
 // ---- slicing --------------------------------------------------------------------------
 // complex [M][ld] (M walkers x K): rows 2m (real parts) and 2m + 1 (imaginary parts), times mul
 int dig_slice_cplx_rows(const DigOp& op, const double2* src, long ld, double mul, cudaStream_t st);
-// real [rows][ld]
-int dig_slice_real_rows(const DigOp& op, const double* src, long ld, cudaStream_t st);
+// real [rows][ld] (to rows row0.. of the operand)
+int dig_slice_real_rows(const DigOp& op, const double* src, long ld, cudaStream_t st, int rows = -1, int row0 = 0);
 // real [K][ld], rows along the contiguous index
-int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_t st);
+int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_t st, int rows = -1, int row0 = 0);
 
 // ---- contractions ---------------------------------------------------------------------
 // C[m][n] (complex, ldc) = i^rot 2^shift sum_k A[m][k] B[n][k]: A sliced by
@@ -87,15 +87,21 @@ int dig_sms();
 // (complex), y_w [norb][nocc_s] complex per slab. V is sliced as [Re | Im] along K, y as
 // columns 2c = [Re y_c | -Im y_c] and 2c + 1 = [Im y_c | Re y_c], so that one real contraction
 // over K = 2 np (np: norb padded to 16) gives both parts; E uses the first half of K.
+// Up to 64 orbitals (stack) Re V has rows 0..63 of the 128-row tile and Im V rows 64..127, the
+// columns are plain [Re y_c], [Im y_c] and K = np: half the products, half the digits, and the four
+// partial sums of an element are added in the epilogue. E has up in rows 0..63 and down in
+// 64..127, so that both slabs are one product.
 struct DigWalk {
+  int stack;
   int n, np, o[2], ncol;  // orbitals, padded; columns per slab and together
   int mt, nt, tr;         // row tiles of V; column tiles per walker and columns (2 per c) per tile
   int chunk;              // walkers sliced at a time
-  DigOp e[2];             // exp_h1 per slab
+  DigOp e[2];             // exp_h1 per slab (stack: both in e[0])
   unsigned char *vd, *xd; // V digits, y digits
   int *ve, *xe;
   int* status;
-  int kbv() const { return np / 8; }
+  int kbv() const { return stack ? np / 16 : np / 8; }
+  int n_e(int nslab) const { return stack ? 1 : nslab; }  // operands in e
 };
 // complex [walker][norb][nocc_s] per slab, walker stride in elements
 struct WalkVec {
@@ -134,7 +140,10 @@ size_t dig_walk_vbar_ae_bytes(const DigWalk& d, const DigVbar& v);
 size_t dig_walk_vbar_be_bytes(const DigWalk& d, const DigVbar& v);
 int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int terms, int qt, int pt, int M,
                   double2* vbar, int nw, cudaStream_t st);
-// X = the sliced V (e < 0) or e[slab] for that slab's columns
+// E (or its transpose) of both slabs into the operands e
+int dig_walk_slice_e(const DigWalk& d, const DigOp* e, const double* const* exp_h1, int nslab, bool transpose,
+                     cudaStream_t st);
+// X = the sliced V (e < 0) or E[e]: that slab's columns (stack: e = 0, every column)
 int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut& o, int nw, cudaStream_t st);
 // B columns per tile for an output of 2 M x N with kb K blocks: 64 where the tiles (times up to
 // eight K ranges) reach half of the SMs, else 32, so that small problems still spread out; never

@@ -109,6 +109,9 @@ ROUTES = [
     dict(kind="rhf", restricted=True, norb=33, nelec=(6, 6), nchol=40, nw=160),     # one slab, ragged
     dict(kind="uhf", restricted=False, norb=33, nelec=(6, 5), nchol=40, nw=88),     # two slabs, unequal
     dict(kind="rhf", restricted=False, norb=64, nelec=(3, 3), nchol=50, nw=44),     # tile edge, few columns
+    dict(kind="uhf", restricted=False, norb=65, nelec=(9, 2), nchol=60, nw=24),     # past the stacked form
+    dict(kind="rhf", restricted=True, norb=48, nelec=(24, 24), nchol=60, nw=20),    # a 48-column tile
+    dict(kind="uhf", restricted=False, norb=50, nelec=(24, 20), nchol=60, nw=16),   # two column tiles
     dict(kind="rhf", restricted=True, norb=130, nelec=(33, 33), nchol=140, nw=4),   # two row and column tiles
     dict(kind="uhf", restricted=False, norb=128, nelec=(20, 19), nchol=130, nw=4),
 ]
@@ -155,7 +158,7 @@ def test_block_routes_agree(cfg):
 
 
 @pytest.mark.parametrize("mode", ["jvp", "vjp"])
-@pytest.mark.parametrize("cfg", ROUTES[:3], ids=ids)
+@pytest.mark.parametrize("cfg", ROUTES[:6], ids=ids)
 def test_derivative_routes_agree(cfg, mode):
     from cs_afqmc_gb300 import sampling
 
