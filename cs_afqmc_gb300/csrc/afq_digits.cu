@@ -455,7 +455,7 @@ struct DigGemm {
   int a_bt, b_bt;  // row tiles per batch entry (0: one operand for all entries)
   int tr;          // B rows per tile
   int splits, kps; // K ranges, K blocks per range
-  int stages;
+  int stages, ring;  // operand K blocks in flight and the bytes they take
   uint32_t idesc;
 };
 
@@ -468,13 +468,11 @@ struct DigWhere {
 constexpr int kDigEpiWarps = 16;
 constexpr int kDigThreads = 64 + 32 * kDigEpiWarps;
 constexpr int kDigABlock = kDigTile * 256;  // bytes of an A K block
-constexpr int kDigRing = 196608;
-constexpr int kDigSmem = 1024 + kDigRing + 256;
-// stacked products: a shorter ring and the exchange of half of each warp's sums (8-byte and 4-byte
-// words, up to 8 per thread)
-constexpr int kDigRingS = 3 * (kDigTile * 256 + 64 * 256);
-constexpr int kDigXchg = 32 * kDigEpiWarps * 8 * 12;
-constexpr int kDigSmemS = 1024 + kDigRingS + 256 + kDigXchg;
+// Walker products stage a tile's sums in shared memory: per column 128 rows (+ 1: conflict-free
+// reads along the columns) of the 8-byte and the 4-byte part.
+constexpr int kDigStageRows = kDigTile + 1;
+constexpr int kDigStageCol = kDigStageRows * 12;
+constexpr int kDigSmemMax = 227 * 1024;
 constexpr int kDigMaxStages = 5;
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -502,13 +500,13 @@ __global__ void __launch_bounds__(kDigThreads, 1)
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (Epi::kStack ? kDigRingS : kDigRing));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + g.ring);
   uint64_t* empty = full + kDigMaxStages;
   uint64_t* accfull = empty + kDigMaxStages;  // [2]
   uint64_t* accempty = accfull + 2;           // [2]
   uint64_t* done = accempty + 2;
-  uint64_t* xbar = done + 1;  // [8] stacked: the two warps that exchange sums
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(xbar + 8);
+  uint64_t* staged = done + 1;  // walker products: the epilogue warps meet
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(staged + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tr = g.tr, bblock = tr * 256, unit = kDigABlock + bblock;
   const int acols = tr <= 32 ? 32 : 64;  // columns between accumulators
@@ -524,7 +522,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
       ptx::mbar_init(&accempty[i], kDigEpiWarps);
     }
     ptx::mbar_init(done, 1);
-    for (int i = 0; i < 8; ++i) ptx::mbar_init(&xbar[i], 2);
+    ptx::mbar_init(staged, kDigEpiWarps);
     ptx::fence_mbar_init();
   }
   if (warp == 1) {
@@ -623,8 +621,6 @@ __global__ void __launch_bounds__(kDigThreads, 1)
       w.n = (x / g.mt) % g.nt;
       w.batch = x / (g.mt * g.nt);
       const int ka = w.split * g.kps, kz = min(g.kb, ka + g.kps);
-      const int er = g.ea[(size_t)(w.batch * g.a_bt + w.m) * kDigTile + r] + ep.shift;
-      const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * tr + col0;
       for (int k0 = ka; k0 < kz; k0 += kDigSegBlocks, ++run) {
         w.add = k0 > ka;
         w.more = k0 + kDigSegBlocks < kz;
@@ -636,11 +632,13 @@ __global__ void __launch_bounds__(kDigThreads, 1)
         }
         ptx::tc_fence_after();
         const uint32_t src = src0 + (uint32_t)(buf * 256);
-        long long hi[16];  // the sum in units of 2^-35 and its remainder in units of 2^-63
-        unsigned lo[16];
-#pragma unroll
-        for (int c0 = 0; c0 < 16; c0 += 4)
-          if (c0 < nc) {
+        if constexpr (Epi::kWalk) {
+          // The sums of the tile to shared memory (free the accumulators), then one element of the result
+          // per thread and turn, neighbours along the columns.
+          long long* sh = reinterpret_cast<long long*>(smem + g.ring + 256);
+          unsigned* sl = reinterpret_cast<unsigned*>(sh + tr * kDigStageRows);
+#pragma unroll 1
+          for (int c0 = 0; c0 < nc; c0 += 4) {
             float v[8][4];
 #pragma unroll
             for (int c = 0; c < 8; ++c) ptx::tmem_ld4p(src + (uint32_t)(c * acols + c0), v[c]);
@@ -648,79 +646,61 @@ __global__ void __launch_bounds__(kDigThreads, 1)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const long long l = dig_quad<4>(v[4][j], v[5][j], v[6][j], v[7][j]);
-              hi[c0 + j] = dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]) + (l >> 28);
-              lo[c0 + j] = (unsigned)l & 0xfffffffu;
+              // column 2c goes to plane c, column 2c + 1 to plane tr / 2 + c
+              const int at = (((col0 + c0 + j) >> 1) + (j & 1) * (tr >> 1)) * kDigStageRows + r;
+              sh[at] = dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]) + (l >> 28);
+              sl[at] = (unsigned)l & 0xfffffffu;
             }
           }
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
-        if constexpr (Epi::kStack) {
-          // Row p of Re V (lanes quarters 0, 1) and of Im V (2, 3): the first takes the lower half of this
-          // warp's column pairs, the second the upper half, and each gets the other's sums for them.
-          if (ep.pair) {
-            long long* xh = reinterpret_cast<long long*>(smem + kDigRingS + 256);
-            unsigned* xl = reinterpret_cast<unsigned*>(xh + 32 * kDigEpiWarps * 8);
-            // warps q and q ^ 2 of a column quarter are two apart in the CTA (q = 2, 3 come first)
-            const int up = q >> 1, me = threadIdx.x - 64, peer = up ? me + 64 : me - 64;
-            uint64_t* bar = &xbar[((warp - 2) >> 2) * 2 + (q & 1)];
-            auto meet = [&]() {  // bounded, as every wait here
-              __syncwarp();
-              if (lane == 0) ptx::mbar_arrive(bar);
-              const bool got = ptx::mbar_wait(bar, meets & 1);
-              ++meets;
-              return __all_sync(0xffffffffu, got) != 0;
-            };
-            const int hc = nc >> 1;  // columns kept; the other hc go to the peer
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (j < nc && (j < hc) == (up != 0)) {
-                const int t = up ? j : j - hc;
-                xh[t * (32 * kDigEpiWarps) + me] = hi[j];
-                xl[t * (32 * kDigEpiWarps) + me] = lo[j];
-              }
-            if (!meet()) {
-              ok = false;
-              break;
-            }
-#pragma unroll
-            for (int j = 0; j < 16; j += 2)
-              if (j < nc && (j < hc) != (up != 0)) {
-                const int t = up ? j - hc : j;
-                const long long h0 = xh[t * (32 * kDigEpiWarps) + peer], h1 = xh[(t + 1) * (32 * kDigEpiWarps) + peer];
-                const unsigned l0 = xl[t * (32 * kDigEpiWarps) + peer], l1 = xl[(t + 1) * (32 * kDigEpiWarps) + peer];
-                // Re = Re V Re y - Im V Im y, Im = Re V Im y + Im V Re y: own a, b, peer's l0, l1 (or swapped)
-                const long long rh = up ? h0 : hi[j], ih = up ? hi[j + 1] : h1;
-                const int dl = (int)(up ? l0 : lo[j]) - (int)(up ? lo[j + 1] : l1);
-                const long long sh = up ? h1 + hi[j] : hi[j + 1] + h0;
-                const unsigned sl = up ? l1 + lo[j] : lo[j + 1] + l0;
-                const int e = er + eb[j];
-                const double2 z = c2(dig_combine(rh - ih + (dl >> 28), (unsigned)dl & 0xfffffffu, e),
-                                     dig_combine(sh + (sl >> 28), sl & 0xfffffffu, e));
-                Epi::store_c(ep, w, r & 63, (w.n * tr + col0 + j) >> 1, z);
-              }
-            if (!meet()) {  // read before the next tile's sums go there
-              ok = false;
-              break;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; j += 2)
-              if (j < nc) {
-                const int c = (w.n * tr + col0 + j) >> 1, e = er + eb[j];
-                if ((c >= ep.o0) == (r >= 64))
-                  Epi::store_c(ep, w, r & 63, c, c2(dig_combine(hi[j], lo[j], e), dig_combine(hi[j + 1], lo[j + 1], e)));
-              }
+          ptx::tc_fence_before();
+          auto meet = [&]() {  // bounded, as every wait here
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(staged);
+            const bool got = ptx::mbar_wait(staged, meets & 1);
+            ++meets;
+            return __all_sync(0xffffffffu, got) != 0;
+          };
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
+          if (!meet()) {
+            ok = false;
+            break;
+          }
+          Epi::finish(ep, g, w, sh, sl, threadIdx.x - 64);
+          if (!meet()) {  // read before the next tile's sums go there
+            ok = false;
+            break;
           }
         } else {
+          long long hi[16];  // the sum in units of 2^-35 and its remainder in units of 2^-63
+          unsigned lo[16];
 #pragma unroll
-        for (int c0 = 0; c0 < 16; c0 += 4)
-          if (c0 < nc) {
-            double o[4];
+          for (int c0 = 0; c0 < 16; c0 += 4)
+            if (c0 < nc) {
+              float v[8][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) o[j] = dig_combine(hi[c0 + j], lo[c0 + j], er + eb[c0 + j]);
-            Epi::store(ep, w, r, col0 + c0, o);
-          }
+              for (int c = 0; c < 8; ++c) ptx::tmem_ld4p(src + (uint32_t)(c * acols + c0), v[c]);
+              ptx::tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const long long l = dig_quad<4>(v[4][j], v[5][j], v[6][j], v[7][j]);
+                hi[c0 + j] = dig_quad<0>(v[0][j], v[1][j], v[2][j], v[3][j]) + (l >> 28);
+                lo[c0 + j] = (unsigned)l & 0xfffffffu;
+              }
+            }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
+          const int er = g.ea[(size_t)(w.batch * g.a_bt + w.m) * kDigTile + r] + ep.shift;
+          const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * tr + col0;
+#pragma unroll
+          for (int c0 = 0; c0 < 16; c0 += 4)
+            if (c0 < nc) {
+              double o[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) o[j] = dig_combine(hi[c0 + j], lo[c0 + j], er + eb[c0 + j]);
+              Epi::store(ep, w, r, col0 + c0, o);
+            }
         }
       }
     }
@@ -737,7 +717,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
 // Complex results: rows 2m / 2m + 1 of D are the real and imaginary parts of row m of C.
 // Neighbouring lanes exchange halves so that each stores whole complex numbers.
 struct EpiDigC {
-  static constexpr bool kNine = false, kStack = false;
+  static constexpr bool kNine = false, kWalk = false;
   struct Params {
     double2* c;
     int M, N, tr;
@@ -764,7 +744,7 @@ struct EpiDigC {
 };
 
 struct EpiDigR {
-  static constexpr bool kNine = false, kStack = false;
+  static constexpr bool kNine = false, kWalk = false;
   struct Params {
     double* d;
     int M, N, tr;
@@ -796,46 +776,72 @@ struct EpiDigR {
 struct WalkParams {
   WalkOut o;
   int n, o0, ncol, tr, only;  // only: the slab to store (-1: both)
-  int pair;                   // stacked: V (two row halves make one result) or E (a slab each)
+  int stack, pair;            // stacked rows; V (the two row halves make one result) or E (a slab each)
   int shift;
 };
 
-AFQ_D void walk_store(const WalkParams& p, const DigWhere& w, int row, int c, double2 x) {
-  const int s = c >= p.o0 ? 1 : 0;
-  if (row >= p.n || c >= p.ncol || (p.only >= 0 && s != p.only)) return;
-  const int k = s ? p.ncol - p.o0 : p.o0;
-  const size_t i = (size_t)row * k + (s ? c - p.o0 : c);
-  if (w.add) x = cadd(x, p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i]);
-  const bool last = !w.more;
-  if (last && p.o.in.p[s]) {
-    const double2 y = p.o.in.p[s][(size_t)w.batch * p.o.in.stride(s) + i];
-    x = c2(fma(y.x, p.o.fin, x.x), fma(y.y, p.o.fin, x.y));
-  }
-  if (p.o.out.p[s]) p.o.out.p[s][(size_t)w.batch * p.o.out.stride(s) + i] = last && p.o.fout != 1.0 ? cscale(x, p.o.fout) : x;
-  if (last && p.o.acc.p[s]) {
-    double2* a = p.o.acc.p[s] + (size_t)w.batch * p.o.acc.stride(s) + i;
-    if (p.o.init) {
-      *a = x;
-    } else {
-      const double2 y = *a;
-      *a = c2(fma(x.x, p.o.facc, y.x), fma(x.y, p.o.facc, y.y));
+struct EpiWalk {
+  static constexpr bool kNine = true, kWalk = true;
+  using Params = WalkParams;
+  AFQ_D static void finish(const Params& p, const DigGemm& g, const DigWhere& w, const long long* sh, const unsigned* sl,
+                           int t) {
+    constexpr int NT = 32 * kDigEpiWarps, U = 2;  // results in flight per thread (their loads are from L2)
+    const int half = p.tr >> 1, c_lo = w.n * half, cc = min(half, p.ncol - c_lo), rows = min(p.n - w.m * kDigTile, kDigTile);
+    const int* ea = g.ea + (size_t)(w.batch * g.a_bt + w.m) * kDigTile;
+    const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * p.tr;
+    const int dp = NT / cc, dc = NT - dp * cc, items = rows * cc;
+    int pr = t / cc, c = t - pr * cc;
+    const bool last = !w.more;
+    for (int it = t; it < items; it += U * NT) {
+      double2 z[U], in[U], ac[U];
+      size_t at[U];
+      int sl_[U];
+      bool on[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int s = c_lo + c >= p.o0 ? 1 : 0;
+        on[u] = it + u * NT < items && (p.only < 0 || s == p.only);
+        sl_[u] = s;
+        const int k = s ? p.ncol - p.o0 : p.o0;
+        at[u] = (size_t)(w.m * kDigTile + pr) * k + (c_lo + c - (s ? p.o0 : 0));
+        if (on[u]) {
+          if (last && p.o.in.p[s]) in[u] = p.o.in.p[s][(size_t)w.batch * p.o.in.stride(s) + at[u]];
+          if (last && p.o.acc.p[s] && !p.o.init) ac[u] = p.o.acc.p[s][(size_t)w.batch * p.o.acc.stride(s) + at[u]];
+          const int row = p.stack && !p.pair ? pr + 64 * s : pr, e = ea[row] + eb[2 * c];
+          const int a = c * kDigStageRows + row, b = a + half * kDigStageRows;
+          long long rh = sh[a], ih = sh[b];
+          int rl = (int)sl[a], il = (int)sl[b];
+          if (p.pair) {  // Re = Re V Re y - Im V Im y, Im = Re V Im y + Im V Re y
+            rh -= sh[b + 64];
+            rl -= (int)sl[b + 64];
+            ih += sh[a + 64];
+            il += (int)sl[a + 64];
+          }
+          z[u] = c2(dig_combine(rh + (rl >> 28), (unsigned)rl & 0xfffffffu, e),
+                    dig_combine(ih + (il >> 28), (unsigned)il & 0xfffffffu, e));
+        }
+        pr += dp;
+        c += dc;
+        if (c >= cc) {
+          c -= cc;
+          ++pr;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (on[u]) {
+          const int s = sl_[u];
+          double2* out = p.o.out.p[s] ? p.o.out.p[s] + (size_t)w.batch * p.o.out.stride(s) + at[u] : nullptr;
+          double2 x = z[u];
+          if (w.add) x = cadd(x, *out);
+          if (last && p.o.in.p[s]) x = c2(fma(in[u].x, p.o.fin, x.x), fma(in[u].y, p.o.fin, x.y));
+          if (out) *out = last && p.o.fout != 1.0 ? cscale(x, p.o.fout) : x;
+          if (last && p.o.acc.p[s])
+            p.o.acc.p[s][(size_t)w.batch * p.o.acc.stride(s) + at[u]] =
+                p.o.init ? x : c2(fma(x.x, p.o.facc, ac[u].x), fma(x.y, p.o.facc, ac[u].y));
+        }
     }
   }
-}
-
-struct EpiWalk {
-  static constexpr bool kNine = true, kStack = false;
-  using Params = WalkParams;
-  AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
-#pragma unroll
-    for (int j = 0; j < 4; j += 2)
-      walk_store(p, w, w.m * kDigTile + r, (w.n * p.tr + col0 + j) >> 1, c2(v[j], v[j + 1]));
-  }
-};
-struct EpiWalkStack {
-  static constexpr bool kNine = true, kStack = true;
-  using Params = WalkParams;
-  AFQ_D static void store_c(const Params& p, const DigWhere& w, int row, int c, double2 z) { walk_store(p, w, row, c, z); }
 };
 
 // C = sum of the partial results of a split contraction
@@ -989,9 +995,10 @@ int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_
 
 template <class Epi>
 static int launch_digits(int cls, DigGemm g, const typename Epi::Params& ep, int* status, cudaStream_t st) {
-  const int unit = kDigABlock + g.tr * 256, ring = Epi::kStack ? kDigRingS : kDigRing;
-  const int smem = Epi::kStack ? kDigSmemS : kDigSmem;
-  g.stages = ring / unit < kDigMaxStages ? ring / unit : kDigMaxStages;
+  const int unit = kDigABlock + g.tr * 256, stage = Epi::kWalk ? g.tr * kDigStageCol : 0;
+  g.stages = std::min((kDigSmemMax - 1024 - 256 - stage) / unit, kDigMaxStages);
+  g.ring = g.stages * unit;
+  const int smem = 1024 + g.ring + 256 + stage;
   g.idesc = ptx::idesc_f16(128, g.tr, 1);
   const long tiles = (long)g.mt * g.nt * g.nb * g.splits;
   const int sms = dig_sms();
@@ -1149,9 +1156,8 @@ int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut
   g.tr = d.tr;
   g.splits = 1;
   g.kps = g.kb;
-  WalkParams ep{o, d.n, d.o[0], d.ncol, d.tr, d.stack || e < 0 || d.o[1] == 0 ? -1 : e, e < 0 ? 1 : 0, 0};
-  return d.stack ? launch_digits<EpiWalkStack>(cls, g, ep, d.status, st)
-                 : launch_digits<EpiWalk>(cls, g, ep, d.status, st);
+  WalkParams ep{o, d.n, d.o[0], d.ncol, d.tr, d.stack || e < 0 || d.o[1] == 0 ? -1 : e, d.stack, d.stack && e < 0, 0};
+  return launch_digits<EpiWalk>(cls, g, ep, d.status, st);
 }
 
 int dig_walk_slice_e(const DigWalk& d, const DigOp* e, const double* const* exp_h1, int nslab, bool transpose,
@@ -1205,7 +1211,7 @@ int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int te
   g.kps = g.kb;
   WalkOut o;  // [norb][norb] per walker: one slab of norb columns
   o.out = WalkVec{{vbar, nullptr}, (size_t)d.n * d.n};
-  WalkParams ep{o, d.n, d.n, d.n, v.tr, -1, 0, 0};
+  WalkParams ep{o, d.n, d.n, d.n, v.tr, -1, 0, 0, 0};
   return launch_digits<EpiWalk>(K_TAYLOR, g, ep, d.status, st);
 }
 
