@@ -6,6 +6,7 @@
 
 #include "afq_common.cuh"
 #include "afq_digits.cuh"
+#include "afq_launch.cuh"
 #include "afq_prof.cuh"
 #include "afq_ptx.cuh"
 
@@ -106,6 +107,7 @@ AFQ_D unsigned block_max_u(unsigned v, unsigned* red) {
 __global__ void __launch_bounds__(128) k_dig_cplx_rows(const double2* __restrict__ src, long ld, int K, int kb,
                                                        double mul, unsigned char* __restrict__ d,
                                                        int* __restrict__ e) {
+  pdl_enter();
   __shared__ unsigned red[2][4];
   const int m = blockIdx.x;
   const double2* s = src + (size_t)m * ld;
@@ -190,6 +192,7 @@ __global__ void __launch_bounds__(256) k_dig_walk_y(const double2* __restrict__ 
                                                     size_t ws0, size_t ws1, int o0, int ncol, int n, int np, int nt,
                                                     int tr, int stack, unsigned char* __restrict__ d,
                                                     int* __restrict__ e) {
+  pdl_enter();
   __shared__ unsigned key[128];
   const int w = blockIdx.x, kb = stack ? np >> 4 : np >> 3, nchunk = np >> 3;
   const int o1 = ncol - o0, items = ncol * nchunk;
@@ -247,6 +250,7 @@ template <int LPR>
 __global__ void __launch_bounds__(256) k_dig_walk_v(const double2* __restrict__ V, int nrows, int n, int np, int mt,
                                                     int stack, unsigned char* __restrict__ d,
                                                     int* __restrict__ e) {
+  pdl_enter();
   const int g = (blockIdx.x * 256 + threadIdx.x) / LPR, ch = threadIdx.x % LPR, kb = stack ? np >> 4 : np >> 3;
   const bool in = g < nrows;
   const int w = in ? g / n : 0, p = in ? g % n : 0;
@@ -282,6 +286,7 @@ __global__ void __launch_bounds__(256) k_dig_walk_v(const double2* __restrict__ 
 // V^H: rows q, K = [Re V[p][q] | -Im V[p][q]] over p, or stacked the same way. CTA per (walker, 32 rows), lanes along q.
 __global__ void __launch_bounds__(256) k_dig_walk_vh(const double2* __restrict__ V, int n, int np, int mt, int stack,
                                                      unsigned char* __restrict__ d, int* __restrict__ e) {
+  pdl_enter();
   __shared__ unsigned red[8][32];
   const int w = blockIdx.y, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = blockIdx.x * 32 + lane,
             kb = stack ? np >> 4 : np >> 3;
@@ -325,6 +330,7 @@ __global__ void __launch_bounds__(256) k_dig_walk_vh(const double2* __restrict__
 __global__ void __launch_bounds__(256) k_dig_vbar(const double2* __restrict__ tay, int terms, int t0, int M, int n,
                                                   int o0, int ncol, int K, int b, int rt, int tr,
                                                   unsigned char* __restrict__ d, int* __restrict__ e) {
+  pdl_enter();
   __shared__ unsigned key[256];
   const int w = blockIdx.x, kc = K >> 1, kb = K >> 4, nchunk = kc >> 3, items = n * nchunk, o1 = ncol - o0;
   const size_t nk = (size_t)n * ncol;
@@ -533,6 +539,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  pdl_enter();
   bool ok = true;
 
   if (warp == 0) {
@@ -847,6 +854,7 @@ struct EpiWalk {
 // C = sum of the partial results of a split contraction
 __global__ void k_dig_sum(long M, long N, int splits, long sst, const double2* __restrict__ part,
                           double2* __restrict__ c, long ldc) {
+  pdl_enter();
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < M * N; i += (long)gridDim.x * blockDim.x) {
     double2 a = part[i];
     for (int s = 1; s < splits; ++s) a = cadd(a, part[i + s * sst]);
@@ -867,6 +875,7 @@ AFQ_D double2 block_sum2(double2 v, double* red) { return c2(block_sum(v.x, red)
 __global__ void __launch_bounds__(128) k_dig_energy(const afq_ctx_dev c, const double2* __restrict__ green,
                                                     const double2* __restrict__ z, const double2* __restrict__ coul,
                                                     double2* __restrict__ energy) {
+  pdl_enter();
   __shared__ double red[32];
   const size_t w = blockIdx.x;
   double2 e1 = c2(0, 0), ex = c2(0, 0), co = c2(0, 0);
@@ -902,6 +911,7 @@ __global__ void __launch_bounds__(128) k_dig_energy_tangent(const afq_ctx_dev c,
                                                             const double2* __restrict__ coul,
                                                             const double2* __restrict__ dcoul, const double* drot_up,
                                                             const double* drot_dn, double2* __restrict__ denergy) {
+  pdl_enter();
   __shared__ double red[32];
   const size_t w = blockIdx.x;
   double2 e1 = c2(0, 0), ex = c2(0, 0), co = c2(0, 0);
@@ -930,6 +940,7 @@ __global__ void __launch_bounds__(128) k_dig_energy_tangent(const afq_ctx_dev c,
 // rot_h1); zero for a walker without an energy cotangent, whatever its G holds.
 __global__ void k_dig_energy_adjoint(const afq_ctx_dev c, const double2* __restrict__ z,
                                      const double* __restrict__ ebar, double2* __restrict__ gene) {
+  pdl_enter();
   const double kappa = c.energy_mode == 2 ? -1.0 : -2.0;
   const double gamma = c.energy_mode == 0 ? 4.0 : (c.energy_mode == 1 ? 2.0 : 1.0);
   const double mult1 = c.energy_mode == 0 ? 2.0 : 1.0;
@@ -971,7 +982,7 @@ int dig_sms() {
 int dig_slice_cplx_rows(const DigOp& op, const double2* src, long ld, double mul, cudaStream_t st) {
   {
     ProfScope _ps(K_PREP, st);
-    k_dig_cplx_rows<<<op.rows / 2, 128, 0, st>>>(src, ld, op.K, op.kb(), mul, op.d, op.e);
+    launch_pdl(k_dig_cplx_rows, op.rows / 2, 128, 0, st, src, ld, op.K, op.kb(), mul, op.d, op.e);
   }
   return dig_err("slice rows");
 }
@@ -1010,7 +1021,7 @@ static int launch_digits(int cls, DigGemm g, const typename Epi::Params& ep, int
   }
   {
     ProfScope _ps(cls, st);
-    kfn<<<(unsigned)(tiles < sms ? tiles : sms), kDigThreads, smem, st>>>(g, ep, status);
+    launch_pdl(kfn, (unsigned)(tiles < sms ? tiles : sms), kDigThreads, smem, st, g, ep, status);
   }
   return dig_err("digit GEMM");
 }
@@ -1076,7 +1087,7 @@ int dig_gemm_c(int cls, const DigOp& A, const DigOp& B, int M, int N, double2* C
   {
     ProfScope _ps(cls, st);
     const long n = (long)M * N;
-    k_dig_sum<<<(unsigned)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096), 256, 0, st>>>(M, N, plan.splits, n, part,
+    launch_pdl(k_dig_sum, (unsigned)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096), 256, 0, st, M, N, plan.splits, n, part,
                                                                                           C, ldc);
   }
   return dig_err("digit GEMM sum");
@@ -1119,13 +1130,13 @@ int dig_walk_slice_v(const DigWalk& d, const double2* V, int nw, bool adjoint, c
     ProfScope _ps(K_TAYLOR, st);
     const int rows = nw * d.n;
     if (adjoint) {
-      k_dig_walk_vh<<<dim3((d.n + 31) / 32, nw), 256, 0, st>>>(V, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
+      launch_pdl(k_dig_walk_vh, dim3((d.n + 31) / 32, nw), 256, 0, st, V, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     } else if (d.np <= 64) {
-      k_dig_walk_v<8><<<(rows + 31) / 32, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
+      launch_pdl(k_dig_walk_v<8>, (rows + 31) / 32, 256, 0, st, V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     } else if (d.np <= 128) {
-      k_dig_walk_v<16><<<(rows + 15) / 16, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
+      launch_pdl(k_dig_walk_v<16>, (rows + 15) / 16, 256, 0, st, V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     } else {
-      k_dig_walk_v<32><<<(rows + 7) / 8, 256, 0, st>>>(V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
+      launch_pdl(k_dig_walk_v<32>, (rows + 7) / 8, 256, 0, st, V, rows, d.n, d.np, d.mt, d.stack, d.vd, d.ve);
     }
   }
   return dig_err("slice V");
@@ -1134,7 +1145,7 @@ int dig_walk_slice_v(const DigWalk& d, const double2* V, int nw, bool adjoint, c
 int dig_walk_slice_y(const DigWalk& d, const WalkVec& y, int nw, cudaStream_t st) {
   {
     ProfScope _ps(K_TAYLOR, st);
-    k_dig_walk_y<<<nw, 256, 0, st>>>(y.p[0], y.p[1], y.stride(0), y.stride(1), d.o[0], d.ncol, d.n, d.np, d.nt, d.tr,
+    launch_pdl(k_dig_walk_y, nw, 256, 0, st, y.p[0], y.p[1], y.stride(0), y.stride(1), d.o[0], d.ncol, d.n, d.np, d.nt, d.tr,
                                      d.stack, d.xd, d.xe);
   }
   return dig_err("slice y");
@@ -1193,8 +1204,8 @@ int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int te
                   double2* vbar, int nw, cudaStream_t st) {
   {
     ProfScope _ps(K_TAYLOR, st);
-    k_dig_vbar<<<nw, 256, 0, st>>>(tay, terms, qt, M, d.n, d.o[0], d.ncol, v.K, 0, v.mt, kDigTile, v.ad, v.ae);
-    k_dig_vbar<<<nw, 256, 0, st>>>(tay, terms, pt, M, d.n, d.o[0], d.ncol, v.K, 1, v.nt, v.tr, v.bd, v.be);
+    launch_pdl(k_dig_vbar, nw, 256, 0, st, tay, terms, qt, M, d.n, d.o[0], d.ncol, v.K, 0, v.mt, kDigTile, v.ad, v.ae);
+    launch_pdl(k_dig_vbar, nw, 256, 0, st, tay, terms, pt, M, d.n, d.o[0], d.ncol, v.K, 1, v.nt, v.tr, v.bd, v.be);
   }
   if (int e = dig_err("slice V cotangents")) return e;
   DigGemm g;
@@ -1219,7 +1230,7 @@ int dig_launch_energy(const afq_ctx_dev& c, const double2* green, const double2*
                       double2* energy, cudaStream_t st) {
   {
     ProfScope _ps(K_ENERGY_FIN, st);
-    k_dig_energy<<<c.nw, 128, 0, st>>>(c, green, z, coul, energy);
+    launch_pdl(k_dig_energy, c.nw, 128, 0, st, c, green, z, coul, energy);
   }
   return dig_err("energy");
 }
@@ -1229,7 +1240,7 @@ int dig_launch_energy_tangent(const afq_ctx_dev& c, const double2* green, const 
                               const double* drot_dn, double2* denergy, cudaStream_t st) {
   {
     ProfScope _ps(K_ENERGY_FIN, st);
-    k_dig_energy_tangent<<<c.nw, 128, 0, st>>>(c, green, dgreen, z, coul, dcoul, drot_up, drot_dn, denergy);
+    launch_pdl(k_dig_energy_tangent, c.nw, 128, 0, st, c, green, dgreen, z, coul, dcoul, drot_up, drot_dn, denergy);
   }
   return dig_err("energy tangent");
 }
@@ -1238,7 +1249,7 @@ int dig_launch_energy_adjoint(const afq_ctx_dev& c, const double2* z, const doub
                               cudaStream_t st) {
   {
     ProfScope _ps(K_ENERGY_FIN, st);
-    k_dig_energy_adjoint<<<c.nw, 128, 0, st>>>(c, z, ebar, gene);
+    launch_pdl(k_dig_energy_adjoint, c.nw, 128, 0, st, c, z, ebar, gene);
   }
   return dig_err("energy adjoint");
 }

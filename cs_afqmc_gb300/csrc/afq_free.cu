@@ -8,6 +8,7 @@
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
+#include "afq_launch.cuh"
 #include "afq_prof.cuh"
 
 namespace afq {
@@ -27,6 +28,7 @@ static int free_err(const char* what) {
 __global__ void k_free_prep(int nw, int nchol, double sqdt, double dt, double h0p, int n0, int n1,
                             const double* __restrict__ fields, const double2* __restrict__ mf,
                             double2* __restrict__ xt, double2* __restrict__ consts) {
+  pdl_enter();
   __shared__ double red[32];
   const int w = blockIdx.x;
   double sx = 0.0, sy = 0.0;
@@ -48,6 +50,7 @@ __global__ void k_free_prep(int nw, int nchol, double sqdt, double dt, double h0
 // each walker slab times its spin's constant (propagation.py:455-457)
 __global__ void k_free_scale(const afq_ctx_dev c, const double2* __restrict__ consts, double2* __restrict__ wu,
                              double2* __restrict__ wd) {
+  pdl_enter();
   const int w = blockIdx.x, s = blockIdx.y;
   const size_t n = (size_t)c.norb * c.kslab[s];
   double2* W = (s == 0 ? wu : wd) + (size_t)w * n;
@@ -58,6 +61,7 @@ __global__ void k_free_scale(const afq_ctx_dev c, const double2* __restrict__ co
 // norms *= prod(diag R_up) prod(diag R_dn); overlaps *= norms (propagation.py:458-461)
 __global__ void k_free_finish(int nw, const double2* __restrict__ rdiag, double2* __restrict__ norms,
                               double2* __restrict__ ovl) {
+  pdl_enter();
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nw) return;
   const double2 nrm = cmul(norms[w], cmul(rdiag[w], rdiag[nw + w]));
@@ -68,6 +72,7 @@ __global__ void k_free_finish(int nw, const double2* __restrict__ rdiag, double2
 // block_energy = sum_w E_w O_w / sum_w O_w, block_weight = sum_w O_w (sampling.py:118-123)
 __global__ void k_free_block_stats(int nw, const double2* __restrict__ energy, const double2* __restrict__ ovl,
                                    double2* __restrict__ be, double2* __restrict__ bw) {
+  pdl_enter();
   __shared__ double red[32];
   double ax = 0, ay = 0, ox = 0, oy = 0;
   for (int w = threadIdx.x; w < nw; w += blockDim.x) {
@@ -91,8 +96,8 @@ int launch_free_prep(const afq_ctx_dev& c, const double* fields, double ene0, do
                      cudaStream_t st) {
   {
     ProfScope _ps(K_FIELD, st);
-    k_free_prep<<<c.nw, 256, 0, st>>>(c.nw, c.nchol, sqrt(c.dt), c.dt, c.h0_prop_re + ene0, c.nocc_slab[0],
-                                      c.nocc_slab[1], fields, c.mf, xt, consts);
+    launch_pdl(k_free_prep, c.nw, 256, 0, st, c.nw, c.nchol, sqrt(c.dt), c.dt, c.h0_prop_re + ene0, c.nocc_slab[0],
+               c.nocc_slab[1], fields, c.mf, xt, consts);
   }
   return free_err("free_prep");
 }
@@ -100,7 +105,7 @@ int launch_free_prep(const afq_ctx_dev& c, const double* fields, double ene0, do
 int launch_free_scale(const afq_ctx_dev& c, const double2* consts, void* wu, void* wd, cudaStream_t st) {
   {
     ProfScope _ps(K_WEIGHTS, st);
-    k_free_scale<<<dim3(c.nw, 2), 256, 0, st>>>(c, consts, static_cast<double2*>(wu), static_cast<double2*>(wd));
+    launch_pdl(k_free_scale, dim3(c.nw, 2), 256, 0, st, c, consts, static_cast<double2*>(wu), static_cast<double2*>(wd));
   }
   return free_err("free_scale");
 }
@@ -108,7 +113,7 @@ int launch_free_scale(const afq_ctx_dev& c, const double2* consts, void* wu, voi
 int launch_free_finish(int nw, const double2* rdiag, double2* norms, double2* ovl, cudaStream_t st) {
   {
     ProfScope _ps(K_WEIGHTS, st);
-    k_free_finish<<<(nw + 127) / 128, 128, 0, st>>>(nw, rdiag, norms, ovl);
+    launch_pdl(k_free_finish, (nw + 127) / 128, 128, 0, st, nw, rdiag, norms, ovl);
   }
   return free_err("free_finish");
 }
@@ -117,7 +122,7 @@ int launch_free_block_stats(int nw, const double2* energy, const double2* ovl, d
                             cudaStream_t st) {
   {
     ProfScope _ps(K_STATS, st);
-    k_free_block_stats<<<1, 1024, 0, st>>>(nw, energy, ovl, be, bw);
+    launch_pdl(k_free_block_stats, 1, 1024, 0, st, nw, energy, ovl, be, bw);
   }
   return free_err("free_block_stats");
 }

@@ -19,6 +19,7 @@
 // accumulator into a third TMEM region with round-to-nearest FP32 adds while the tensor
 // core fills the other one. Every truncated run then spans 4 d MMAs only.
 #pragma once
+#include "afq_launch.cuh"
 #include "afq_ptx.cuh"
 
 namespace afq {
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  pdl_enter();
   bool ok = true;
 
   if (warp == 0) {

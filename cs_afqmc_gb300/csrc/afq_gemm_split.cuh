@@ -33,6 +33,7 @@
 // the even CTA's `accempty` barriers. Each CTA drains and stores its own 128 accumulator rows
 // from its own TMEM.
 #pragma once
+#include "afq_launch.cuh"
 #include "afq_ptx.cuh"
 
 namespace afq {
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  pdl_enter();
   bool ok = true;
 
   if (warp == 0) {

@@ -3,6 +3,7 @@
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
+#include "afq_launch.cuh"
 #include "afq_mixed_dev.cuh"
 #include "afq_prof.cuh"
 
@@ -103,6 +104,7 @@ template <int OM, int NT>
 __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / NT)
     k_green_mixed(const MixedDev md, const float2* __restrict__ wu, const float2* __restrict__ wd,
                   double2* __restrict__ ovl, int flags) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int NW = NT / 32, RR = OM > 32 ? 2 : 1;
   const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = md.n;
@@ -476,7 +478,7 @@ static int green_launch(const MixedDev& md, const float2* wu, const float2* wd, 
   auto kfn = k_green_mixed<OM, NT>;
   // a refused attribute surfaces as the launch error checked by the caller
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kfn<<<md.nw, NT, smem, st>>>(md, wu, wd, ovl, flags);
+  launch_pdl(kfn, md.nw, NT, smem, st, md, wu, wd, ovl, flags);
   return 0;
 }
 

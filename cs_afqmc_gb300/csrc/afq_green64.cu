@@ -3,6 +3,7 @@
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
+#include "afq_launch.cuh"
 #include "afq_prof.cuh"
 
 namespace afq {
@@ -31,6 +32,7 @@ template <int OM>
 __global__ void __launch_bounds__(kG64Threads, OM <= 20 ? 3 : 2)
     k_green_f64(const afq_ctx_dev c, const double2* __restrict__ w_up, const double2* __restrict__ w_dn,
                 double2* __restrict__ green, double2* __restrict__ overlap, int write_green) {
+  pdl_enter();
   constexpr int NT = kG64Threads, NW = NT / 32;
   constexpr bool HALF = OM <= 16;
   __shared__ double2 Pt[4 * NT];
@@ -190,14 +192,14 @@ int launch_green_f64(const afq_ctx_dev& c, const void* wu, const void* wd, doubl
   const double2 *u = (const double2*)wu, *d = (const double2*)wd;
   const int wg = write_green ? 1 : 0;
   switch ((c.kmax + 3) / 4) {
-    case 1: k_green_f64<4><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
-    case 2: k_green_f64<8><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
-    case 3: k_green_f64<12><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
-    case 4: k_green_f64<16><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
-    case 5: k_green_f64<20><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
-    case 6: k_green_f64<24><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
-    case 7: k_green_f64<28><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
-    default: k_green_f64<32><<<c.nw, kG64Threads, 0, st>>>(c, u, d, green, ovl, wg); break;
+    case 1: launch_pdl(k_green_f64<4>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
+    case 2: launch_pdl(k_green_f64<8>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
+    case 3: launch_pdl(k_green_f64<12>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
+    case 4: launch_pdl(k_green_f64<16>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
+    case 5: launch_pdl(k_green_f64<20>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
+    case 6: launch_pdl(k_green_f64<24>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
+    case 7: launch_pdl(k_green_f64<28>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
+    default: launch_pdl(k_green_f64<32>, c.nw, kG64Threads, 0, st, c, u, d, green, ovl, wg); break;
   }
   return 0;
 }

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_fp16.h>
 
+#include "afq_launch.cuh"
 #include "afq_tc.cuh"
 
 namespace afq {

@@ -118,6 +118,7 @@ struct FbReduce {
 
 __global__ void __launch_bounds__(256, 3) k_fb_reduce(const FbReduce r) {
   __shared__ double red[32];
+  pdl_enter();
   const int w = blockIdx.x;
   const float gi = r.g_inv[w];
   const bool bf = r.bf16 != 0;
@@ -394,6 +395,7 @@ __device__ __forceinline__ void qr_colsum(const float2* A, int ld, int m, int k,
 }
 
 __global__ void __launch_bounds__(32 * kQrWarps) k_qr_warp(int nw, int m, int k, float2* __restrict__ wbase) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char qsm_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wlk = blockIdx.x * kQrWarps + warp;

@@ -38,6 +38,7 @@
 // Every wait is bounded (ptx::kWaitLimit polls): on a timeout the CTA sets bit 2 of
 // *status, stops, waits (bounded) for its own copies and MMAs in flight and frees TMEM.
 #pragma once
+#include "afq_launch.cuh"
 #include "afq_mixed_kernels.cuh"
 
 namespace afq {
@@ -121,6 +122,7 @@ __global__ void __launch_bounds__(128 * NP + 160, 1)
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  pdl_enter();
   const uint32_t c_eh = 0, c_el = kw, c_vh = 2 * kw, c_vl = 4 * kw, c_d = 6 * kw;
   bool ok = true;
 

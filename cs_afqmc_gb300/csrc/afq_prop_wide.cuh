@@ -16,6 +16,7 @@
 // one FP32 accumulator over K = 256. Every wait is bounded; on a timeout the CTA sets bit 2
 // of *status, stops, waits (bounded) for its copies and MMAs in flight and frees TMEM.
 #pragma once
+#include "afq_launch.cuh"
 #include "afq_prop_fused.cuh"
 
 namespace afq {
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(128 * NP + 64, 1)
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  pdl_enter();
   bool ok = true;
 
   if (warp == kProd) {

@@ -11,6 +11,7 @@
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
+#include "afq_launch.cuh"
 #include "afq_prof.cuh"
 
 namespace afq {
@@ -198,6 +199,7 @@ __global__ void k_field_shifts(int nchol, double sqdt, const double* __restrict_
                                const double2* __restrict__ fb, const double2* __restrict__ mf,
                                double2* __restrict__ xt, double2* __restrict__ shift,
                                double2* __restrict__ fbt) {
+  pdl_enter();
   __shared__ double red[32];
   const int w = blockIdx.x;
   double sx = 0, sy = 0, fx = 0, fy = 0;
@@ -238,6 +240,7 @@ template <typename WT>
 __global__ void __launch_bounds__(256) k_taylor_f64(const afq_ctx_dev c, int w0,
                                                     const double2* __restrict__ vhs,
                                                     WT* __restrict__ w_up, WT* __restrict__ w_dn) {
+  pdl_enter();
   using CT = typename CplxOf<WT>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int wl = blockIdx.x, s = blockIdx.y;
@@ -321,6 +324,7 @@ constexpr int kTaylorSmall = 512;
 
 __global__ void __launch_bounds__(256) k_taylor_small(const afq_ctx_dev c, int w0, const double2* __restrict__ vhs,
                                                       double2* __restrict__ w_up, double2* __restrict__ w_dn) {
+  pdl_enter();
   __shared__ double2 Ta[kTaylorSmall], Tb[kTaylorSmall], Acc[kTaylorSmall];
   const int wl = blockIdx.x, s = blockIdx.y, norb = c.norb, ks = c.kslab[s], n = norb * ks, tid = threadIdx.x;
   const int part = tid & 3;
@@ -398,6 +402,7 @@ __global__ void k_weights(int nw, double dt, double2 h0_prop, const double2* __r
                           const double2* __restrict__ fbt, int ntiles,
                           const double2* __restrict__ ovl_new, double2* __restrict__ ovl,
                           double* __restrict__ weights, const double* __restrict__ scalars) {
+  pdl_enter();
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nw) return;
   const double sqdt = sqrt(dt);
@@ -430,6 +435,7 @@ __global__ void k_weights(int nw, double dt, double2 h0_prop, const double2* __r
 // scalars[AFQ_S_STATUS] so that callers see a timeout or a bad operand in the state
 __global__ void k_pop_control(int nw, double dt, const double* __restrict__ weights,
                               double* __restrict__ scalars, const int* __restrict__ status) {
+  pdl_enter();
   __shared__ double red[32];
   double sum = 0.0;
   for (int w = threadIdx.x; w < nw; w += blockDim.x) sum += weights[w];
@@ -604,6 +610,7 @@ AFQ_D void qr64_update(double2* A, int ld, int m, int k, int j, int lane, double
 
 __global__ void __launch_bounds__(32) k_qr_f64(const afq_ctx_dev c, double2* __restrict__ w_up,
                                                double2* __restrict__ w_dn, double2* __restrict__ rdiag) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int wlk = blockIdx.x, s = blockIdx.y, lane = threadIdx.x;
   const int m = c.norb, k = c.kslab[s], ld = k | 1;
@@ -682,6 +689,7 @@ AFQ_D float warp_sumf(float v) {
 
 __global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, float2* __restrict__ w_up,
                                                         float2* __restrict__ w_dn) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int wlk = blockIdx.x, s = blockIdx.y;
   const int m = c.norb, k = c.kslab[s];
@@ -789,6 +797,7 @@ __global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, flo
 // thread in index order (the summation order of numpy/jnp.cumsum) and searched there.
 __global__ void k_sr_indices(int nw, const double* __restrict__ zeta, double* __restrict__ weights,
                              double* __restrict__ cum_g, int32_t* __restrict__ idx, int in_smem) {
+  pdl_enter();
   extern __shared__ double cum_s[];
   double* cum = in_smem ? cum_s : cum_g;
   if (in_smem) {
@@ -837,6 +846,7 @@ __global__ void k_sr_indices(int nw, const double* __restrict__ zeta, double* __
 template <typename WT>
 __global__ void k_gather_slab(int slab_elems, const int32_t* __restrict__ idx,
                               const WT* __restrict__ src, WT* __restrict__ dst) {
+  pdl_enter();
   using CT = typename CplxOf<WT>::type;
   const int w = blockIdx.x;
   const CT* s = reinterpret_cast<const CT*>(src) + (size_t)idx[w] * slab_elems;
@@ -851,6 +861,7 @@ __global__ void k_gather_slab(int slab_elems, const int32_t* __restrict__ idx,
 __global__ void k_block_stats(int nw, double dt, const double2* __restrict__ energy,
                               const double* __restrict__ weights, double* __restrict__ scalars,
                               double* __restrict__ be_out, double* __restrict__ bw_out) {
+  pdl_enter();
   __shared__ double red[32];
   const double e_est = scalars[AFQ_S_E_ESTIMATE];
   const double lim = sqrt(2.0 / dt);
@@ -880,6 +891,7 @@ __global__ void k_block_stats(int nw, double dt, const double2* __restrict__ ene
 // en_samples (corr_sample.py:482-491): Re(E) clamped to e_estimate beyond sqrt(2/dt)
 __global__ void k_clamped_energies(int nw, double dt, const double2* __restrict__ energy,
                                    const double* __restrict__ scalars, double* __restrict__ out) {
+  pdl_enter();
   const double e_est = scalars[AFQ_S_E_ESTIMATE];
   const double lim = sqrt(2.0 / dt);
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += gridDim.x * blockDim.x) {
@@ -894,6 +906,7 @@ __global__ void k_clamped_energies(int nw, double dt, const double2* __restrict_
 __global__ void k_cs_outlier(int nw, double z_thresh, double* __restrict__ w1, double* __restrict__ w2,
                              const double* __restrict__ e1, const double* __restrict__ e2,
                              double* __restrict__ sums) {
+  pdl_enter();
   __shared__ double red[32];
   double s1 = 0, s2 = 0;
   for (int i = threadIdx.x; i < nw; i += blockDim.x) {
@@ -936,6 +949,7 @@ __global__ void k_cs_outlier(int nw, double z_thresh, double* __restrict__ w1, d
 }
 
 __global__ void k_phaseless_begin(double* scalars) {
+  pdl_enter();
   scalars[AFQ_S_N_KILLED] = 0.0;
   scalars[AFQ_S_POP_CONTROL_SHIFT] = scalars[AFQ_S_E_ESTIMATE];
 }
@@ -943,6 +957,7 @@ __global__ void k_phaseless_begin(double* scalars) {
 __global__ void k_phaseless_end(int nblk, double denom, const double* __restrict__ be,
                                 const double* __restrict__ bw, double* __restrict__ scalars,
                                 double* __restrict__ energy) {
+  pdl_enter();
   if (threadIdx.x == 0) {
     double a = 0, b = 0;
     for (int i = 0; i < nblk; ++i) {
@@ -958,6 +973,7 @@ __global__ void k_phaseless_end(int nblk, double denom, const double* __restrict
 __global__ void k_driver_update(int nw, const double* __restrict__ weights,
                                 const double* __restrict__ energy, double* __restrict__ scalars,
                                 double* __restrict__ wsum) {
+  pdl_enter();
   __shared__ double red[32];
   double s = 0.0;
   for (int w = threadIdx.x; w < nw; w += blockDim.x) s += weights[w];
@@ -1084,7 +1100,7 @@ int launch_field_shifts(const afq_ctx_dev& c, const double* fields, const double
                         double2* xt, double2* shift, double2* fbt, cudaStream_t st) {
   {
     ProfScope _ps(K_FIELD, st);
-    k_field_shifts<<<c.nw, 256, 0, st>>>(c.nchol, sqrt(c.dt), fields, fb, c.mf, xt, shift, fbt);
+    launch_pdl(k_field_shifts, c.nw, 256, 0, st, c.nchol, sqrt(c.dt), fields, fb, c.mf, xt, shift, fbt);
   }
   return launch_err("field_shifts");
 }
@@ -1095,7 +1111,7 @@ int launch_taylor_f64(const afq_ctx_dev& c, int w0, int nwc, const double2* vhs,
   if (c.norb * c.kmax <= kTaylorSmall) {
     {
       ProfScope _ps(K_TAYLOR, st);
-      k_taylor_small<<<dim3(nwc, c.nslab), 256, 0, st>>>(c, w0, vhs, (double2*)wu, (double2*)wd);
+      launch_pdl(k_taylor_small, dim3(nwc, c.nslab), 256, 0, st, c, w0, vhs, (double2*)wu, (double2*)wd);
     }
     return launch_err("taylor_small");
   }
@@ -1115,12 +1131,12 @@ int launch_weights(const afq_ctx_dev& c, const double2* shift, const double2* fb
   {
     ProfScope _ps(K_WEIGHTS, st);
     // FP64 transcendentals per walker: 8 walkers per CTA spread them over the SMs' FP64 units
-    k_weights<<<(c.nw + 7) / 8, 8, 0, st>>>(c.nw, c.dt, c2(c.h0_prop_re, c.h0_prop_im), shift, fbt, ntiles,
+    launch_pdl(k_weights, (c.nw + 7) / 8, 8, 0, st, c.nw, c.dt, c2(c.h0_prop_re, c.h0_prop_im), shift, fbt, ntiles,
                                             ovl_new, ovl, weights, scalars);
   }
   {
     ProfScope _ps(K_WEIGHTS, st);
-    k_pop_control<<<1, 1024, 0, st>>>(c.nw, c.dt, weights, scalars, status);
+    launch_pdl(k_pop_control, 1, 1024, 0, st, c.nw, c.dt, weights, scalars, status);
   }
   return launch_err("weights");
 }
@@ -1149,7 +1165,7 @@ int launch_qr_f64(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, dou
   cudaFuncSetAttribute(k_qr_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   {
     ProfScope _ps(K_QR, st);
-    k_qr_f64<<<dim3(c.nw, c.nslab), 32, smem, st>>>(c, (double2*)wu, (double2*)wd, rdiag);
+    launch_pdl(k_qr_f64, dim3(c.nw, c.nslab), 32, smem, st, c, (double2*)wu, (double2*)wd, rdiag);
   }
   return launch_err("qr_f64");
 }
@@ -1159,7 +1175,7 @@ int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
   cudaFuncSetAttribute(k_qr_householder, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   {
     ProfScope _ps(K_QR, st);
-    k_qr_householder<<<dim3(c.nw, c.nslab), 256, smem, st>>>(c, (float2*)wu, (float2*)wd);
+    launch_pdl(k_qr_householder, dim3(c.nw, c.nslab), 256, smem, st, c, (float2*)wu, (float2*)wd);
   }
   return launch_err("qr_householder");
 }
@@ -1170,7 +1186,7 @@ int launch_sr(const afq_ctx_dev& c, const double* zeta, double* weights, double*
   {
     ProfScope _ps(K_SR, st);
     const int in_smem = c.nw * 8 <= 48 * 1024 ? 1 : 0;
-    k_sr_indices<<<1, 1024, in_smem ? c.nw * 8 : 0, st>>>(c.nw, zeta, weights, cum, idx, in_smem);
+    launch_pdl(k_sr_indices, 1, 1024, in_smem ? c.nw * 8 : 0, st, c.nw, zeta, weights, cum, idx, in_smem);
   }
   int e = launch_err("sr_indices");
   if (e) return e;
@@ -1184,7 +1200,7 @@ int launch_sr(const afq_ctx_dev& c, const double* zeta, double* weights, double*
     cudaMemcpyAsync(cp, w, bytes, cudaMemcpyDeviceToDevice, st);
     {
       ProfScope _ps(K_SR, st);
-      k_gather_slab<WT><<<c.nw, 256, 0, st>>>((int)elems, idx, (const WT*)cp, (WT*)w);
+      launch_pdl(k_gather_slab<WT>, c.nw, 256, 0, st, (int)elems, idx, (const WT*)cp, (WT*)w);
     }
     off += bytes;
   }
@@ -1195,7 +1211,7 @@ int launch_block_stats(const afq_ctx_dev& c, const double2* energy, const double
                        double* scalars, double* be, double* bw, cudaStream_t st) {
   {
     ProfScope _ps(K_STATS, st);
-    k_block_stats<<<1, 1024, 0, st>>>(c.nw, c.dt, energy, weights, scalars, be, bw);
+    launch_pdl(k_block_stats, 1, 1024, 0, st, c.nw, c.dt, energy, weights, scalars, be, bw);
   }
   return launch_err("block_stats");
 }
@@ -1204,7 +1220,7 @@ int launch_clamped_energies(const afq_ctx_dev& c, const double2* energy, const d
                             double* out, cudaStream_t st) {
   {
     ProfScope _ps(K_STATS, st);
-    k_clamped_energies<<<(c.nw + 255) / 256, 256, 0, st>>>(c.nw, c.dt, energy, scalars, out);
+    launch_pdl(k_clamped_energies, (c.nw + 255) / 256, 256, 0, st, c.nw, c.dt, energy, scalars, out);
   }
   return launch_err("clamped_energies");
 }
@@ -1213,7 +1229,7 @@ int launch_cs_outlier(double* w1, double* w2, const double* e1, const double* e2
                       double z_thresh, double* sums, cudaStream_t st) {
   {
     ProfScope _ps(K_STATS, st);
-    k_cs_outlier<<<1, 1024, 0, st>>>(nw, z_thresh, w1, w2, e1, e2, sums);
+    launch_pdl(k_cs_outlier, 1, 1024, 0, st, nw, z_thresh, w1, w2, e1, e2, sums);
   }
   return launch_err("cs_outlier");
 }
@@ -1221,7 +1237,7 @@ int launch_cs_outlier(double* w1, double* w2, const double* e1, const double* e2
 int launch_phaseless_begin(double* scalars, cudaStream_t st) {
   {
     ProfScope _ps(K_STATS, st);
-    k_phaseless_begin<<<1, 1, 0, st>>>(scalars);
+    launch_pdl(k_phaseless_begin, 1, 1, 0, st, scalars);
   }
   return launch_err("phaseless_begin");
 }
@@ -1230,7 +1246,7 @@ int launch_phaseless_end(int nblk, double denom, const double* be, const double*
                          double* scalars, double* energy, cudaStream_t st) {
   {
     ProfScope _ps(K_STATS, st);
-    k_phaseless_end<<<1, 32, 0, st>>>(nblk, denom, be, bw, scalars, energy);
+    launch_pdl(k_phaseless_end, 1, 32, 0, st, nblk, denom, be, bw, scalars, energy);
   }
   return launch_err("phaseless_end");
 }
@@ -1239,7 +1255,7 @@ int launch_driver_update(const afq_ctx_dev& c, const double* weights, const doub
                          double* scalars, double* wsum, cudaStream_t st) {
   {
     ProfScope _ps(K_STATS, st);
-    k_driver_update<<<1, 1024, 0, st>>>(c.nw, weights, energy, scalars, wsum);
+    launch_pdl(k_driver_update, 1, 1024, 0, st, c.nw, weights, energy, scalars, wsum);
   }
   return launch_err("driver_update");
 }

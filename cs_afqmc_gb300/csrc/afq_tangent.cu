@@ -15,6 +15,7 @@
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
+#include "afq_launch.cuh"
 #include "afq_prof.cuh"
 #include "afq_tangent.cuh"
 
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256) k_t_green(const afq_ctx_dev c, const doub
                                                  double2* __restrict__ ovl, double2* __restrict__ dlog_ovl,
                                                  const double* __restrict__ dc_up,
                                                  const double* __restrict__ dc_dn) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int wlk = blockIdx.x, norb = c.norb, tid = threadIdx.x, nt = blockDim.x;
   const int km = c.kmax;
@@ -215,6 +217,7 @@ __global__ void k_t_field_shifts(int nchol, double sqdt, const double* __restric
                                  double2* __restrict__ dxt, double2* __restrict__ shift,
                                  double2* __restrict__ dshift, double2* __restrict__ fbt,
                                  double2* __restrict__ dfbt) {
+  pdl_enter();
   __shared__ double red[32];
   const int w = blockIdx.x;
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -366,6 +369,7 @@ __global__ void k_t_weights(int nw, double dt, double2 h0_prop, const double2* _
                             double2* __restrict__ dlo, double* __restrict__ weights,
                             double* __restrict__ dweights, const double* __restrict__ scalars,
                             const double* __restrict__ dscalars) {
+  pdl_enter();
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nw) return;
   const double sqdt = sqrt(dt);
@@ -403,6 +407,7 @@ __global__ void k_t_weights(int nw, double dt, double2 h0_prop, const double2* _
 __global__ void k_t_pop_control(int nw, double dt, const double* __restrict__ weights,
                                 const double* __restrict__ dweights, double* __restrict__ scalars,
                                 double* __restrict__ dscalars) {
+  pdl_enter();
   __shared__ double red[32];
   double s = 0.0, ds = 0.0;
   for (int w = threadIdx.x; w < nw; w += blockDim.x) {
@@ -698,7 +703,7 @@ int t_launch_green(const afq_ctx_dev& c, const TangentBufs& t, const void* wu, c
   cudaFuncSetAttribute(k_t_green, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   {
     ProfScope _ps(K_GREEN, st);
-    k_t_green<<<c.nw, 256, smem, st>>>(c, (const double2*)wu, (const double2*)wd, t.dw[0], t.dw[1], green, dgreen,
+    launch_pdl(k_t_green, c.nw, 256, smem, st, c, (const double2*)wu, (const double2*)wd, t.dw[0], t.dw[1], green, dgreen,
                                        ovl, dlog, t.dtrial[0], c.nslab == 2 ? t.dtrial[1] : nullptr);
   }
   return t_err("t_green");
@@ -709,7 +714,7 @@ int t_launch_field_shifts(const afq_ctx_dev& c, const double* fields, const doub
                           cudaStream_t st) {
   {
     ProfScope _ps(K_FIELD, st);
-    k_t_field_shifts<<<c.nw, 256, 0, st>>>(c.nchol, sqrt(c.dt), fields, fb, dfb, c.mf, xt, dxt, shift, dshift, fbt,
+    launch_pdl(k_t_field_shifts, c.nw, 256, 0, st, c.nchol, sqrt(c.dt), fields, fb, dfb, c.mf, xt, dxt, shift, dshift, fbt,
                                            dfbt);
   }
   return t_err("t_field_shifts");
@@ -737,10 +742,10 @@ int t_launch_weights(const afq_ctx_dev& c, const TangentBufs& t, const double2* 
                      const double2* ovl_new, double2* ovl, double* weights, double* scalars, cudaStream_t st) {
   {
     ProfScope _ps(K_WEIGHTS, st);
-    k_t_weights<<<(c.nw + 127) / 128, 128, 0, st>>>(c.nw, c.dt, c2(c.h0_prop_re, c.h0_prop_im), shift, t.dshift, fbt,
+    launch_pdl(k_t_weights, (c.nw + 127) / 128, 128, 0, st, c.nw, c.dt, c2(c.h0_prop_re, c.h0_prop_im), shift, t.dshift, fbt,
                                                     t.dfbt, ovl_new, t.dlo_new, ovl, t.dlo, weights, t.dweights,
                                                     scalars, t.dscalars);
-    k_t_pop_control<<<1, 1024, 0, st>>>(c.nw, c.dt, weights, t.dweights, scalars, t.dscalars);
+    launch_pdl(k_t_pop_control, 1, 1024, 0, st, c.nw, c.dt, weights, t.dweights, scalars, t.dscalars);
   }
   return t_err("t_weights");
 }

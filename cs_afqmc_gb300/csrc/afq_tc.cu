@@ -3,6 +3,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include "afq_launch.cuh"
 #include "afq_mixed_kernels.cuh"
 #include "afq_prof.cuh"
 #include "afq_prop_fused.cuh"
@@ -87,7 +88,7 @@ static int launch_gemm(int cls, const GemmMaps& maps, int nterms, int k_tiles, i
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   {
     ProfScope _ps(cls, st);
-    kfn<<<dim3(n_tiles, m_tiles), kGemmThreads, smem, st>>>(
+    launch_pdl(kfn, dim3(n_tiles, m_tiles), kGemmThreads, smem, st,
         maps, nterms, k_tiles, bn, a_row0, drain, ptx::idesc_f16(128, bn, bf16 ? 1 : 0), ep, status);
   }
   return launch_check("gemm_tc");
@@ -113,11 +114,13 @@ static int launch_split(int cls, const SplitMaps& maps, SplitArgs g, int num_sms
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
     g.idesc = ptx::idesc_f16(256, kSplitBN, bf16 ? 1 : 0);
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_pdl
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.blockDim = dim3(kSplitThreads);
     cfg.dynamicSmemBytes = kSplitSmem;
     cfg.stream = st;
@@ -135,6 +138,7 @@ static int launch_split(int cls, const SplitMaps& maps, SplitArgs g, int num_sms
     cudaError_t e;
     {
       ProfScope _ps(cls, st);
+      cfg.numAttrs = 2;
       e = cudaLaunchKernelEx(&cfg, kfn, maps, g, ep, status);
     }
     if (e != cudaSuccess) {
@@ -148,7 +152,7 @@ static int launch_split(int cls, const SplitMaps& maps, SplitArgs g, int num_sms
   const int grid = ntiles < num_sms ? ntiles : num_sms;
   {
     ProfScope _ps(cls, st);
-    kfn<<<grid, kSplitThreads, kSplitSmem, st>>>(maps, g, ep, status);
+    launch_pdl(kfn, grid, kSplitThreads, kSplitSmem, st, maps, g, ep, status);
   }
   return launch_check("gemm_split");
 }
@@ -627,6 +631,7 @@ struct TaylorDiag {
 constexpr int kDiagSplit = 8;  // partial sums over g per orbital (256 threads: 8 x 32 orbitals)
 
 __global__ void __launch_bounds__(256) k_taylor_diag(const TaylorDiag td) {
+  pdl_enter();
   __shared__ float2 poly[128];
   __shared__ float2 part[kDiagSplit][128];
   const int w = blockIdx.x, s = blockIdx.y, n = td.n, tid = threadIdx.x;
@@ -735,6 +740,7 @@ __global__ void k_prep_eop(const double* __restrict__ e, int n, int nk, int bf16
 __global__ void k_energy_final_mixed(int nw, int nchol, int nblk, int mt0, int mt1, int mode, double h0,
                                      const double2* __restrict__ c_out, const double2* __restrict__ exc,
                                      const double2* __restrict__ ene1, double2* __restrict__ out) {
+  pdl_enter();
   __shared__ double red[32];
   const int w = blockIdx.x;
   double a[5][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};
@@ -1303,7 +1309,7 @@ static int fb_gemm(TcState& t, const afq_ctx_dev& c, const double* fields, doubl
     r.fb_out = fb_out;
     {
       ProfScope _ps(cls, st);
-      k_fb_reduce<<<t.nw, 256, 0, st>>>(r);
+      launch_pdl(k_fb_reduce, t.nw, 256, 0, st, r);
     }
     return launch_check("fb_reduce");
   }
@@ -1358,7 +1364,7 @@ static int launch_prop_fused(const TcState& t, int s, const PropDev& pd, cudaStr
   }
   {
     ProfScope _ps(K_PROP, st);
-    kfn<<<pd.nwc < t.num_sms ? pd.nwc : t.num_sms, 128 * NP + 160, smem, st>>>(
+    launch_pdl(kfn, pd.nwc < t.num_sms ? pd.nwc : t.num_sms, 128 * NP + 160, smem, st,
         t.m_vt[s][0], t.m_vt[s][1], t.eop[s][0], t.eop[s][1], t.nk, pd, t.status);
   }
   return launch_check("prop_fused");
@@ -1375,7 +1381,7 @@ static int launch_prop_wide(const TcState& t, int s, const PropDev& pd, cudaStre
   }
   {
     ProfScope _ps(K_PROP, st);
-    kfn<<<pd.nwc < t.num_sms ? pd.nwc : t.num_sms, 128 * NP + 64, smem, st>>>(
+    launch_pdl(kfn, pd.nwc < t.num_sms ? pd.nwc : t.num_sms, 128 * NP + 64, smem, st,
         t.m_vt[s][0], t.m_vt[s][1], t.m_ew[s][0], t.m_ew[s][1], pd, t.status);
   }
   return launch_check("prop_wide");
@@ -1474,7 +1480,7 @@ int tc_propagate_walkers(TcState& t, const afq_ctx_dev& c, void* wu, void* wd, c
     td.sqdt = (float)sqrt(c.dt);
     {
       ProfScope _ps(K_TAYLOR, st);
-      k_taylor_diag<<<dim3(t.nw, t.nslab), 256, 0, st>>>(td);
+      launch_pdl(k_taylor_diag, dim3(t.nw, t.nslab), 256, 0, st, td);
     }
     TC_CHECK(launch_check("taylor_diag"));
     for (int s = 0; s < t.nslab; ++s) TC_CHECK(exp_gemm(t, c, s, true, W[s], st));
@@ -1585,7 +1591,7 @@ int tc_energy(TcState& t, const afq_ctx_dev& c, double2* out, cudaStream_t st) {
   }
   {
     ProfScope _ps(K_ENERGY_FIN, st);
-    k_energy_final_mixed<<<t.nw, 256, 0, st>>>(t.nw, c.nchol, t.nblk, t.mt_z[0], t.nblk == 2 ? t.mt_z[1] : 0,
+    launch_pdl(k_energy_final_mixed, t.nw, 256, 0, st, t.nw, c.nchol, t.nblk, t.mt_z[0], t.nblk == 2 ? t.mt_z[1] : 0,
                                                c.energy_mode, c.h0, t.c_out, t.exc_part, t.ene1, out);
   }
   return launch_check("energy_final_mixed");
@@ -1601,8 +1607,7 @@ int tc_orthonormalize(TcState& t, const afq_ctx_dev& c, void* wu, void* wd, cuda
     cudaFuncSetAttribute(k_qr_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     {
       ProfScope _ps(K_QR, st);
-      k_qr_warp<<<(c.nw + kQrWarps - 1) / kQrWarps, 32 * kQrWarps, smem, st>>>(
-          c.nw, c.norb, k, static_cast<float2*>(s == 0 ? wu : wd));
+      launch_pdl(k_qr_warp, (c.nw + kQrWarps - 1) / kQrWarps, 32 * kQrWarps, smem, st, c.nw, c.norb, k, static_cast<float2*>(s == 0 ? wu : wd));
     }
     TC_CHECK(launch_check("qr_warp"));
   }
