@@ -478,7 +478,7 @@ int propagate_impl(afq_ctx* c, afq_walker_state* s, const double* fields, cudaSt
 
 int qr_impl(afq_ctx* c, afq_walker_state* s, cudaStream_t st) {
   if (is_fp64(c)) return afq::launch_qr_f64(c->dev, s->walkers_up, s->walkers_dn, st);
-  return afq::tc_orthonormalize(c->tc, c->dev, s->walkers_up, s->walkers_dn, st);
+  return afq::launch_qr_f32(c->dev, s->walkers_up, s->walkers_dn, st);
 }
 
 int sr_impl(afq_ctx* c, afq_walker_state* s, const double* zeta, int32_t* indices, cudaStream_t st) {

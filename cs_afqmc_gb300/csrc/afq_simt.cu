@@ -677,118 +677,6 @@ __global__ void __launch_bounds__(32) k_qr_f64(const afq_ctx_dev c, double2* __r
 }
 
 // ======================================================================================
-// The same for FP32 walkers whose slabs are too large for the mixed path's warp kernel: one CTA per
-// (walker, slab). Q overwrites W.
-// ======================================================================================
-
-AFQ_D float warp_sumf(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-__global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, float2* __restrict__ w_up,
-                                                        float2* __restrict__ w_dn) {
-  pdl_enter();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int wlk = blockIdx.x, s = blockIdx.y;
-  const int m = c.norb, k = c.kslab[s];
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5,
-            nwarp = nt >> 5;
-  float2* A = reinterpret_cast<float2*>(smem_raw);  // [m][k]
-  float2* y = A + (size_t)m * k;                // [k]
-  float2* tau = y + k;                          // [k]
-  __shared__ double red[32];
-  __shared__ float2 sc_sh, beta_sh;
-  float2* W = (s == 0 ? w_up : w_dn) + (size_t)wlk * m * k;
-  for (int i = tid; i < m * k; i += nt) A[i] = W[i];
-  __syncthreads();
-  // ---- factorisation
-  for (int j = 0; j < k; ++j) {
-    double xnd = 0.0;
-    for (int r = j + 1 + tid; r < m; r += nt) xnd += (double)cabs2(A[r * k + j]);
-    xnd = block_sum(xnd, red);
-    if (tid == 0) {
-      const float2 alpha = A[j * k + j];
-      const float xn = (float)xnd;
-      if (xn == (float)0 && alpha.y == (float)0) {
-        tau[j] = make_float2(0, 0);
-        beta_sh = alpha;
-        sc_sh = make_float2(1, 0);
-      } else {
-        const float nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
-        const float beta = (alpha.x >= (float)0) ? -nrm : nrm;
-        tau[j] = make_float2((beta - alpha.x) / beta, -alpha.y / beta);
-        sc_sh = cdiv(make_float2(1, 0), csub(alpha, make_float2(beta, 0)));
-        beta_sh = make_float2(beta, 0);
-      }
-    }
-    __syncthreads();
-    const float2 scl = sc_sh;
-    for (int r = j + 1 + tid; r < m; r += nt) A[r * k + j] = cmul(A[r * k + j], scl);
-    if (tid == 0) A[j * k + j] = make_float2(1, 0);
-    __syncthreads();
-    // y[col] = sum_r conj(v[r]) A[r][col], col > j ; then A -= conj(tau) v y
-    for (int col = j + 1 + wid; col < k; col += nwarp) {
-      float yx = 0, yy = 0;
-      for (int r = j + lane; r < m; r += 32) {
-        const float2 pr = cmulc(A[r * k + col], A[r * k + j]);
-        yx += pr.x;
-        yy += pr.y;
-      }
-      yx = warp_sumf(yx);
-      yy = warp_sumf(yy);
-      if (lane == 0) y[col] = make_float2(yx, yy);
-    }
-    __syncthreads();
-    const float2 ct = cconj(tau[j]);
-    const int ncol = k - j - 1;
-    if (ncol > 0) {
-      for (int e = tid; e < (m - j) * ncol; e += nt) {
-        const int r = j + e / ncol, col = j + 1 + e % ncol;
-        A[r * k + col] = csub(A[r * k + col], cmul(ct, cmul(A[r * k + j], y[col])));
-      }
-    }
-    __syncthreads();
-    if (tid == 0) A[j * k + j] = beta_sh;
-    __syncthreads();
-  }
-  // ---- form Q (zung2r): columns from last to first
-  for (int j = k - 1; j >= 0; --j) {
-    if (j < k - 1) {
-      if (tid == 0) A[j * k + j] = make_float2(1, 0);
-      __syncthreads();
-      for (int col = j + 1 + wid; col < k; col += nwarp) {
-        float yx = 0, yy = 0;
-        for (int r = j + lane; r < m; r += 32) {
-          const float2 pr = cmulc(A[r * k + col], A[r * k + j]);
-          yx += pr.x;
-          yy += pr.y;
-        }
-        yx = warp_sumf(yx);
-        yy = warp_sumf(yy);
-        if (lane == 0) y[col] = make_float2(yx, yy);
-      }
-      __syncthreads();
-      const float2 t = tau[j];
-      const int ncol = k - j - 1;
-      for (int e = tid; e < (m - j) * ncol; e += nt) {
-        const int r = j + e / ncol, col = j + 1 + e % ncol;
-        A[r * k + col] = csub(A[r * k + col], cmul(t, cmul(A[r * k + j], y[col])));
-      }
-      __syncthreads();
-    }
-    const float2 t = tau[j];
-    const float2 mt = make_float2(-t.x, -t.y);
-    for (int r = j + 1 + tid; r < m; r += nt) A[r * k + j] = cmul(mt, A[r * k + j]);
-    if (tid == 0) A[j * k + j] = make_float2(1 - t.x, -t.y);
-    for (int r = tid; r < j; r += nt) A[r * k + j] = make_float2(0, 0);
-    __syncthreads();
-  }
-  for (int i = tid; i < m * k; i += nt) W[i] = A[i];
-}
-
-// ======================================================================================
 // Comb stochastic reconfiguration (sr.py:24-47). One CTA computes the indices with a
 // sequential cumulative sum (same summation order as numpy/jnp.cumsum), then a gather.
 // ======================================================================================
@@ -1168,16 +1056,6 @@ int launch_qr_f64(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, dou
     launch_pdl(k_qr_f64, dim3(c.nw, c.nslab), 32, smem, st, c, (double2*)wu, (double2*)wd, rdiag);
   }
   return launch_err("qr_f64");
-}
-
-int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
-  size_t smem = ((size_t)c.norb * c.kmax + 2 * c.kmax) * sizeof(float2);
-  cudaFuncSetAttribute(k_qr_householder, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  {
-    ProfScope _ps(K_QR, st);
-    launch_pdl(k_qr_householder, dim3(c.nw, c.nslab), 256, smem, st, c, (float2*)wu, (float2*)wd);
-  }
-  return launch_err("qr_householder");
 }
 
 template <typename WT>

@@ -1597,23 +1597,6 @@ int tc_energy(TcState& t, const afq_ctx_dev& c, double2* out, cudaStream_t st) {
   return launch_check("energy_final_mixed");
 }
 
-int tc_orthonormalize(TcState& t, const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
-  for (int s = 0; s < c.nslab; ++s) {
-    const int k = c.kslab[s];
-    const size_t smem = (size_t)kQrWarps * ((size_t)c.norb * qr_ld(k) + 64) * sizeof(float2);
-    // the warp kernel holds kQrWarps slabs in shared memory; wider or longer slabs take the
-    // one-CTA-per-slab Householder kernel
-    if (k > 32 || smem > 227 * 1024) return launch_qr_f32(c, wu, wd, st);
-    cudaFuncSetAttribute(k_qr_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    {
-      ProfScope _ps(K_QR, st);
-      launch_pdl(k_qr_warp, (c.nw + kQrWarps - 1) / kQrWarps, 32 * kQrWarps, smem, st, c.nw, c.norb, k, static_cast<float2*>(s == 0 ? wu : wd));
-    }
-    TC_CHECK(launch_check("qr_warp"));
-  }
-  return 0;
-}
-
 }  // namespace afq
 
 // ---- test hooks (include/afqmc_gb300_testing.h) ---------------------------------------

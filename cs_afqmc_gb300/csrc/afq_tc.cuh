@@ -136,6 +136,5 @@ int tc_field_shifts(TcState& t, const afq_ctx_dev& c, const double* fields, cuda
 int tc_propagate_walkers(TcState& t, const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st);
 int tc_weights(TcState& t, const afq_ctx_dev& c, const double2* ovl_new, double2* ovl,
                double* weights, double* scalars, cudaStream_t st);
-int tc_orthonormalize(TcState& t, const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st);
 
 }  // namespace afq
