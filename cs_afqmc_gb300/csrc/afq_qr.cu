@@ -27,9 +27,10 @@ namespace afq {
 // slabs 305 -> 131 us; 120 x 20, 1024 slabs 159 -> 114 us; 198 x 33, 256 slabs 219 -> 161 us; 60 x 10 and
 // 60 x 8, 512 walkers 45 us for one spin -> 16 us for both; 53 x 8, 64 slabs 26 -> 10 us.
 //
-// FP64 walkers keep a warp per slab in shared memory (k_qr_f64): their units take some 18 cycles for a warp
+// FP64 walkers keep the slab in shared memory (k_qr_f64): their units take some 18 cycles for a warp
 // instruction whatever its lanes do, and with eight lanes along the rows instead of 32 there are more of
-// them. Measured in this form at 256 walkers of two slabs: 100 x 20 electrons 559 -> 919 us, 60 x 36 959 -> 1835 us.
+// them. Measured in this form at 256 walkers of two slabs, against a warp per slab in shared memory: 100 x 20 electrons
+// 559 -> 919 us, 60 x 36 959 -> 1835 us.
 constexpr int kQrRows = 8;   // rows per lane: 64 a warp
 constexpr int kQrWarps = 8;  // warps per CTA at most: 255 registers a thread
 

@@ -557,41 +557,47 @@ __global__ void k_energy_final(const afq_ctx_dev c, int nchunks, const double2* 
 
 // ======================================================================================
 // Householder QR of FP64 walkers, LAPACK zgeqr2 + zung2r conventions (R has a real diagonal,
-// beta = -sign(Re alpha) * |(alpha, x)|), linalg_utils.py:51-65 (jnp.linalg.qr, reduced mode). One
-// warp per (walker, slab) with the slab in shared memory (odd row stride: conflict-free column
-// walks), Q over W. 8 m k^2 FP64 FMAs: a single warp keeps the FP64 units of its SM near busy (18
-// cycles an instruction), and a warp needs no barriers; with 256 threads per slab and seven barriers a
-// column norb 120 / 20 electrons / 256 walkers took 691 us.
-// Column sums are owned by lanes per column, the rank-1 updates by lane = row.
+// beta = -sign(Re alpha) * |(alpha, x)|), linalg_utils.py:51-65 (jnp.linalg.qr, reduced mode). One CTA
+// per (walker, slab) with the slab in shared memory (odd row stride: conflict-free column walks), a thread
+// per row up to eight warps, Q over W.
+//
+// What bounds it: latency in FP64 chains, then the FP64 units (a warp instruction takes some 18 cycles
+// whatever its lanes do; 10 m k^2 of them, with 32 elements each). So a column is one reduction, a few scalar
+// steps by one warp and one update: the squares of column j are one more of the sums over its raw elements,
+// v^H a_c = a_jc + conj(scale) sum, the divisions are lanes of one instruction, tau goes into the sums.
+// Row j right of the diagonal (R) is never read again and is left alone.
+// Against a warp per slab with a pass for the norm: 40 x 7 and 40 x 6 electrons, 200 walkers 71 -> 52 us; 60 x 10 and
+// 60 x 8, 512 walkers 186 -> 193 us; a block of five steps with one QR, 120 x 20, 256 walkers 7.82 -> 7.45 ms.
 // rdiag (optional, [nslab][nw]): prod(diag R) per walker slab (linalg_utils.py:51-65 returns
 // it as the norm factor; the free-projection step multiplies its norms by it)
 // ======================================================================================
 
-// y[c] = sum_{r >= j} conj(A[r][j]) A[r][c] for c in (j, k): lpc lanes (a power of two) per column.
+// y[c] = mul sum_{r > j} conj(A[r][j]) A[r][c] for c in [c_lo, k): lpc lanes (a power of two) per column.
 // Two chains of eight rows at a time: with two over all rows of a lane, and the update below as an FMA chain, Q
 // was further off than with a sum over 32 lanes (against extended precision, walkers of 120 x 20: 4.45e-16
-// instead of 3.12e-16, now 3.33e-16; 180 x 30: 5.51e-16, 3.46e-16, 3.59e-16).
-AFQ_D void qr64_colsum(const double2* A, int ld, int m, int k, int j, int lane, double2* y) {
-  const int nc = k - j - 1;
-  if (nc <= 0) return;
-  int lpc = 1;
-  while (lpc * 2 * nc <= 32) lpc *= 2;
-  for (int c0 = 0; c0 < nc; c0 += 32 / lpc) {
-    const int c = c0 + lane / lpc, part = lane % lpc;
+// instead of 3.12e-16, now 3.31e-16; 180 x 30: 5.51e-16, 3.46e-16, 3.44e-16).
+AFQ_D void qr64_sums(const double2* A, int ld, int m, int k, int j, int c_lo, double2 mul, double2* y) {
+  const int nc = k - c_lo, tid = threadIdx.x, nt = blockDim.x;
+  int sh = 0;
+  while (sh < 5 && (nc << (sh + 1)) <= nt) ++sh;
+  const int lpc = 1 << sh, part = tid & (lpc - 1);
+  for (int c0 = 0; c0 < nc; c0 += nt >> sh) {
+    const int c = c_lo + c0 + (tid >> sh);
     double2 sum = c2(0, 0);
-    if (c < nc) {
-      for (int r0 = j + part; r0 < m; r0 += 16 * lpc) {
+    if (c < k) {
+      for (int r0 = j + 1 + part; r0 < m; r0 += 16 * lpc) {
         const int r1 = min(m, r0 + 16 * lpc);
         double2 a = c2(0, 0), b = c2(0, 0);
         int r = r0;
+#pragma unroll 4
         for (; r + lpc < r1; r += 2 * lpc) {
-          const double2 x = A[r * ld + j + 1 + c], v = A[r * ld + j];
-          const double2 x2 = A[(r + lpc) * ld + j + 1 + c], v2 = A[(r + lpc) * ld + j];
+          const double2 x = A[r * ld + c], v = A[r * ld + j];
+          const double2 x2 = A[(r + lpc) * ld + c], v2 = A[(r + lpc) * ld + j];
           a = c2(fma(x.x, v.x, fma(x.y, v.y, a.x)), fma(x.y, v.x, fma(-x.x, v.y, a.y)));
           b = c2(fma(x2.x, v2.x, fma(x2.y, v2.y, b.x)), fma(x2.y, v2.x, fma(-x2.x, v2.y, b.y)));
         }
         if (r < r1) {
-          const double2 x = A[r * ld + j + 1 + c], v = A[r * ld + j];
+          const double2 x = A[r * ld + c], v = A[r * ld + j];
           a = c2(fma(x.x, v.x, fma(x.y, v.y, a.x)), fma(x.y, v.x, fma(-x.x, v.y, a.y)));
         }
         sum = cadd(sum, cadd(a, b));
@@ -599,86 +605,94 @@ AFQ_D void qr64_colsum(const double2* A, int ld, int m, int k, int j, int lane, 
     }
     for (int off = 1; off < lpc; off <<= 1)
       sum = cadd(sum, c2(__shfl_xor_sync(0xffffffffu, sum.x, off), __shfl_xor_sync(0xffffffffu, sum.y, off)));
-    if (c < nc && part == 0) y[j + 1 + c] = sum;
+    if (c < k && part == 0) y[c] = cmul(mul, sum);
   }
 }
 
-// A[r][c] -= t v[r] y[c] for r >= j, c > j, v in column j. The product is rounded before it meets the
-// element (an FMA chain onto the element rounds twice at its size).
-AFQ_D void qr64_update(double2* A, int ld, int m, int k, int j, int lane, double2 t, const double2* y) {
-  for (int r = j + lane; r < m; r += 32) {
-    const double2 tv = cmul(t, A[r * ld + j]);
+// row[c] -= v z[c] for c > j. The product is rounded before it meets the element (an FMA chain onto the
+// element rounds twice at its size).
+AFQ_D void qr64_row(double2* row, int k, int j, double2 v, const double2* z) {
 #pragma unroll 4
-    for (int c = j + 1; c < k; ++c) {
-      const double2 yc = y[c], a = A[r * ld + c];
-      A[r * ld + c] = c2(a.x - fma(tv.x, yc.x, -tv.y * yc.y), a.y - fma(tv.x, yc.y, tv.y * yc.x));
-    }
+  for (int c = j + 1; c < k; ++c) {
+    const double2 x = z[c], a = row[c];
+    row[c] = c2(a.x - fma(v.x, x.x, -v.y * x.y), a.y - fma(v.x, x.y, v.y * x.x));
   }
 }
 
-__global__ void __launch_bounds__(32) k_qr_f64(const afq_ctx_dev c, double2* __restrict__ w_up,
-                                               double2* __restrict__ w_dn, double2* __restrict__ rdiag) {
+__global__ void __launch_bounds__(256) k_qr_f64(const afq_ctx_dev c, double2* __restrict__ w_up,
+                                                double2* __restrict__ w_dn, double2* __restrict__ rdiag) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int wlk = blockIdx.x, s = blockIdx.y, lane = threadIdx.x;
+  __shared__ double2 scale;
+  const int wlk = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
   const int m = c.norb, k = c.kslab[s], ld = k | 1;
   double2* A = reinterpret_cast<double2*>(smem_raw);  // [m][ld]
   double2* y = A + (size_t)m * ld;                    // [k]
   double2* tau = y + k;                               // [k]
   double2* W = (s == 0 ? w_up : w_dn) + (size_t)wlk * m * k;
-  for (int i = lane; i < m * k; i += 32) {
+  for (int i = tid; i < m * k; i += nt) {
     const int r = i / k;
     A[r * ld + (i - r * k)] = W[i];
   }
-  double2 rprod = c2(1.0, 0.0);
-  __syncwarp();
+  double2 rprod = c2(1.0, 0.0);  // warp 0
+  __syncthreads();
   for (int j = 0; j < k; ++j) {
-    double xn = 0.0;
-    for (int r = j + 1 + lane; r < m; r += 32) xn += cabs2(A[r * ld + j]);
-    xn = warp_sum(xn);
-    const double2 alpha = A[j * ld + j];
-    double2 t, scl, beta;
-    if (xn == 0.0 && alpha.y == 0.0) {
-      t = c2(0, 0);
-      beta = alpha;
-      scl = c2(1, 0);
-    } else {
-      const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
-      const double b = alpha.x >= 0.0 ? -nrm : nrm;
-      t = c2((b - alpha.x) / b, -alpha.y / b);
-      scl = cdiv(c2(1, 0), csub(alpha, c2(b, 0)));
-      beta = c2(b, 0);
+    qr64_sums(A, ld, m, k, j, j, c2(1.0, 0.0), y);
+    __syncthreads();
+    if (tid < 32) {
+      const double2 alpha = A[j * ld + j];
+      const double xn = y[j].x;
+      double2 t = c2(0, 0), scl = c2(1, 0), beta = alpha;
+      if (!(xn == 0.0 && alpha.y == 0.0)) {
+        const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
+        const double b = alpha.x >= 0.0 ? -nrm : nrm, dx = alpha.x - b, d2 = dx * dx + alpha.y * alpha.y;
+        // tau = (b - alpha) / b and scale = 1 / (alpha - b), a quotient per lane
+        const double num = tid == 0 ? -dx : tid == 1 ? -alpha.y : tid == 2 ? dx : -alpha.y;
+        const double q = num / (tid < 2 ? b : d2);
+        t = c2(__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1));
+        scl = c2(__shfl_sync(0xffffffffu, q, 2), __shfl_sync(0xffffffffu, q, 3));
+        beta = c2(b, 0);
+      }
+      for (int i = j + 1 + tid; i < k; i += 32)
+        y[i] = cmul(cconj(t), cadd(A[j * ld + i], cmul(cconj(scl), y[i])));
+      if (tid == 0) {
+        rprod = cmul(rprod, beta);
+        tau[j] = t;
+        scale = scl;
+      }
     }
-    rprod = cmul(rprod, beta);
-    __syncwarp();
-    for (int r = j + 1 + lane; r < m; r += 32) A[r * ld + j] = cmul(A[r * ld + j], scl);
-    if (lane == 0) {
-      A[j * ld + j] = c2(1, 0);
-      tau[j] = t;
+    __syncthreads();
+    const double2 scl = scale;
+    for (int r = j + 1 + tid; r < m; r += nt) {
+      double2* row = A + r * ld;
+      const double2 v = cmul(row[j], scl);
+      row[j] = v;
+      qr64_row(row, k, j, v, y);
     }
-    __syncwarp();
-    qr64_colsum(A, ld, m, k, j, lane, y);
-    __syncwarp();
-    qr64_update(A, ld, m, k, j, lane, cconj(t), y);
-    __syncwarp();
+    __syncthreads();
   }
-  if (lane == 0 && rdiag) rdiag[(size_t)s * c.nw + wlk] = rprod;
-  // form Q (zung2r): columns from last to first (the diagonal of column j still holds the reflector's 1)
+  if (tid == 0 && rdiag) rdiag[(size_t)s * c.nw + wlk] = rprod;
+  // form Q (zung2r): columns from last to first; row j of the columns behind j is still zero
   for (int j = k - 1; j >= 0; --j) {
     const double2 t = tau[j];
-    if (j < k - 1) {
-      qr64_colsum(A, ld, m, k, j, lane, y);
-      __syncwarp();
-      qr64_update(A, ld, m, k, j, lane, t, y);
-      __syncwarp();
+    qr64_sums(A, ld, m, k, j, j + 1, t, y);
+    __syncthreads();
+    for (int r = tid; r < m; r += nt) {
+      double2* row = A + r * ld;
+      if (r < j) {
+        row[j] = c2(0, 0);
+      } else if (r == j) {
+        row[j] = c2(1.0 - t.x, -t.y);
+        for (int i = j + 1; i < k; ++i) row[i] = c2(-y[i].x, -y[i].y);
+      } else {
+        const double2 v = row[j];
+        qr64_row(row, k, j, v, y);
+        row[j] = cmul(c2(-t.x, -t.y), v);
+      }
     }
-    const double2 mt = c2(-t.x, -t.y);
-    for (int r = j + 1 + lane; r < m; r += 32) A[r * ld + j] = cmul(mt, A[r * ld + j]);
-    if (lane == 0) A[j * ld + j] = c2(1.0 - t.x, -t.y);
-    for (int r = lane; r < j; r += 32) A[r * ld + j] = c2(0, 0);
-    __syncwarp();
+    __syncthreads();
   }
-  for (int i = lane; i < m * k; i += 32) {
+  for (int i = tid; i < m * k; i += nt) {
     const int r = i / k;
     W[i] = A[r * ld + (i - r * k)];
   }
@@ -1061,7 +1075,7 @@ int launch_qr_f64(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, dou
   cudaFuncSetAttribute(k_qr_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   {
     ProfScope _ps(K_QR, st);
-    launch_pdl(k_qr_f64, dim3(c.nw, c.nslab), 32, smem, st, c, (double2*)wu, (double2*)wd, rdiag);
+    launch_pdl(k_qr_f64, dim3(c.nw, c.nslab), 32 * std::min(8, (c.norb + 31) / 32), smem, st, c, (double2*)wu, (double2*)wd, rdiag);
   }
   return launch_err("qr_f64");
 }
