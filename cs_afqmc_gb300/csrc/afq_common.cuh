@@ -61,6 +61,18 @@ AFQ_HD float2 cdiv(float2 a, float2 b) {
   }
 }
 
+// The same with every rounding spelled out, for sums whose bits are part of the results: how the
+// compiler contracts a * b + c * d changes with the code around it.
+AFQ_D float2 mul_rn(float2 a, float2 b) {
+  return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+AFQ_D float2 mulc_rn(float2 a, float2 b) {
+  return make_float2(fmaf(a.x, b.x, __fmul_rn(a.y, b.y)), fmaf(a.y, b.x, -__fmul_rn(a.x, b.y)));
+}
+AFQ_D float2 add_rn(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
+AFQ_D float2 sub_rn(float2 a, float2 b) { return make_float2(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y)); }
+AFQ_D float abs2_rn(float2 a) { return fmaf(a.x, a.x, __fmul_rn(a.y, a.y)); }
+
 // walker storage <-> double2
 AFQ_D double2 ld_c(const double2* p) { return *p; }
 AFQ_D double2 ld_c(const float2* p) {

@@ -54,13 +54,12 @@ __device__ __forceinline__ void copy_rows(float2* dst, const float2* __restrict_
   }
 }
 
-// Shared memory: walker slabs [n][ld] (G overwrites them row by row), the partial sums of S
-// (16 complex per thread), then per slab S / S^-1 [OM][OM + 1].
+// Shared memory: per slab the walker [n][ld] (G overwrites it row by row) and S / S^-1 [OM][OM + 1].
 __host__ __device__ constexpr size_t green_slab_bytes(int n, int o) {
   return ((size_t)n * green_s_ld(o) * 8 + 15) & ~(size_t)15;
 }
-static size_t green_smem(const MixedDev& md, int om, int nt) {
-  size_t b = (size_t)nt * 128;
+static size_t green_smem(const MixedDev& md, int om) {
+  size_t b = 0;
   for (int s = 0; s < md.nslab; ++s) b += green_slab_bytes(md.n, md.o_slab[s]) + (size_t)om * (om + 1) * 8 + 16;
   return b;
 }
@@ -82,24 +81,32 @@ __device__ __forceinline__ void split16_pair(float x, float y, bool bf, uint32_t
   }
 }
 
+// The order of every sum below is part of the mixed path's results: resampling compares sums of weights
+// with the comb's teeth, and a weight that moves by one FP32 rounding exchanges a whole walker wherever a tooth
+// lies that close to a boundary. (With the orbitals of S dealt to several threads, populations of 2048 walkers on 64 sites
+// came out with another walker on one of twelve inputs.) So an element of S sums the orbitals in their order, the
+// elimination divides the pivot row before the other rows take their multiples of it, and a thread sums
+// the one-body energy of an orbital; the roundings are spelled out (mul_rn).
+//
 // What bounds it: instruction issue and latency, not arithmetic (0.35 M FP32 FMAs per walker at
 // norb 120, 20 electrons, are 2.8 k of an SM's cycles). The phases:
-//  * S = C^T W by 4 x 4 register blocks (two 16-byte shared loads and one cached 16-byte load of
-//    the trial per 32 FMAs), the orbitals dealt to NT / blocks threads each, partial sums added
-//    afterwards;
+//  * S = C^T W in register blocks of RI x CK elements, sized so that one pass takes most of the threads;
 //  * Gauss-Jordan by one warp per slab with a matrix row per lane (two rows above 32) in
 //    registers. Partial pivoting is implicit: no rows move, the pivot of step j is the unused
 //    row with the largest |re| + |im| in column j (ties to the lower row; its index rides in the
 //    low bits of the key). The columns rotate by one register each step, so that the pivot
 //    column is always register 0 and one step's code serves all; the pivot lane publishes its
-//    row through shared memory. S is padded to OM with an identity block. The working matrix
-//    ends as P^T S^-1 P^T for the pivot order P: row r is row step(r) of S^-1, column c its
-//    column piv(c); det(S) = sign(P) prod(pivots), the product in FP64.
+//    row through shared memory, where a lane per element multiplies it by 1 / pivot. S is padded to OM with an
+//    identity block. The working matrix ends as P^T S^-1 P^T for the pivot order P: row r is row step(r) of S^-1,
+//    column c its column piv(c); det(S) = sign(P) prod(pivots), the product in FP64.
 //    (A thread block per matrix with a barrier per pivot took 1200 cycles a step where five
 //    walkers shared an SM.)
 //  * G = (W S^-1)^T: a walker row per thread in registers, G written over it;
 //  * the power-of-two scale of G, its 16-bit operands (two orbitals per store) and
 //    ene1 = sum G * rot_h1.
+// Against the kernel with a block-wide elimination, the same bits: 64 x 28 electrons, 2048 walkers 190 -> 130 us;
+// 198 x 33, 256 walkers 208 -> 70 us; 60 x 10 and 60 x 8, 512 walkers 27 -> 18 us; 120 x 20, 1024 walkers
+// 76 -> 61 us. (Sums in any order: 111, 64, 18, 48 us.)
 template <int OM, int NT>
 __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / NT)
     k_green_mixed(const MixedDev md, const float2* __restrict__ wu, const float2* __restrict__ wd,
@@ -107,10 +114,10 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
   pdl_enter();
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int NW = NT / 32, RR = OM > 32 ? 2 : 1;
+  constexpr unsigned RM = RR == 1 ? 31u : 63u;  // row index in the low bits of the pivot key
   const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = md.n;
   const bool do_g = (flags & kGreenG) != 0, bf = md.bf16 != 0;
-  float2* Pt = reinterpret_cast<float2*>(sm);
-  unsigned char* at = sm + (size_t)NT * 128;
+  unsigned char* at = sm;
   float2* Wsl[2];
   float2* Sm[2];
 #pragma unroll
@@ -153,64 +160,80 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
         }
     }
   }
+  // S: blocks of RI trial columns x CK walker columns, an element's sum over the orbitals in their order
+  constexpr int CK = OM <= 8 ? 1 : OM <= 20 ? 2 : 4, RI = OM <= 16 ? 1 : OM <= 32 ? 2 : 4;
   for (int s = 0; s < md.nslab; ++s) {
-    const int o = md.o_slab[s], o4 = (o + 3) & ~3, ld = green_s_ld(o), nb = o4 >> 2, nbb = nb * nb, ps_n = NT / nbb;
-    const int ps = tid / nbb, b = tid - ps * nbb, bi = b / nb, bk = b - bi * nb, stride = ps_n * nbb;
-    if (ps < ps_n) {
-      float2 acc[4][4];
+    const int o = md.o_slab[s], o4 = (o + 3) & ~3, ld = green_s_ld(o), nk = (o + CK - 1) / CK, ni = (o + RI - 1) / RI;
+    for (int e = tid; e < ni * nk; e += NT) {
+      const int bi = e / nk, i0 = bi * RI, k0 = (e - bi * nk) * CK;
+      const float* __restrict__ C = md.trial32[s] + i0;  // [n][o4], the same for every walker (L1); columns o.. are zero
+      auto load = [&](float (&c)[RI], const float* src) {
+        if constexpr (RI == 1) {
+          c[0] = __ldg(src);
+        } else if constexpr (RI == 2) {
+          const float2 v = __ldg(reinterpret_cast<const float2*>(src));
+          c[0] = v.x;
+          c[1] = v.y;
+        } else {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+          c[0] = v.x;
+          c[1] = v.y;
+          c[2] = v.z;
+          c[3] = v.w;
+        }
+      };
+      const float2* W = Wsl[s] + k0;
+      float2 acc[RI][CK];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < RI; ++i)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) acc[i][k] = make_float2(0.f, 0.f);
-      const float* __restrict__ C = md.trial32[s] + 4 * bi;  // [n][o4], the same for every walker (L1)
-      const float2* W = Wsl[s] + 4 * bk;
-      // the trial rows of a batch in flight together
-      constexpr int U = 6;
-      const int cs = ps_n * o4, wst = ps_n * ld;
-      C += ps * o4;
-      W += ps * ld;
-      int left = (n - ps + ps_n - 1) / ps_n;  // this thread's orbitals
-      auto row = [&](const float4 c, const float2* wp) {
-        const float4 x = *reinterpret_cast<const float4*>(wp), y = *reinterpret_cast<const float4*>(wp + 2);
-        const float cv[4] = {c.x, c.y, c.z, c.w};
-        const float2 wv[4] = {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y),
-                              make_float2(y.z, y.w)};
+        for (int k = 0; k < CK; ++k) acc[i][k] = make_float2(0.f, 0.f);
+      auto row = [&](const float (&c)[RI], const float2* wp) {
+        float2 wv[CK];
+        if constexpr (CK >= 2) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+          for (int k = 0; k < CK; k += 2) {
+            const float4 x = *reinterpret_cast<const float4*>(wp + k);
+            wv[k] = make_float2(x.x, x.y);
+            wv[k + 1] = make_float2(x.z, x.w);
+          }
+        } else {
+          wv[0] = wp[0];
+        }
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            acc[i][k].x = fmaf(cv[i], wv[k].x, acc[i][k].x);
-            acc[i][k].y = fmaf(cv[i], wv[k].y, acc[i][k].y);
+        for (int i = 0; i < RI; ++i)
+#pragma unroll
+          for (int k = 0; k < CK; ++k) {
+            acc[i][k].x = fmaf(c[i], wv[k].x, acc[i][k].x);
+            acc[i][k].y = fmaf(c[i], wv[k].y, acc[i][k].y);
           }
       };
-      for (; left >= U; left -= U) {
-        float4 c[U];
+      constexpr int U = 8;  // the trial rows of a batch in flight together
+      int p = 0;
+      for (; p + U <= n; p += U) {
+        float c[U][RI];
 #pragma unroll
-        for (int u = 0; u < U; ++u) c[u] = __ldg(reinterpret_cast<const float4*>(C + u * cs));
+        for (int u = 0; u < U; ++u) load(c[u], C + (p + u) * o4);
 #pragma unroll
-        for (int u = 0; u < U; ++u) row(c[u], W + u * wst);
-        C += U * cs;
-        W += U * wst;
+        for (int u = 0; u < U; ++u) row(c[u], W + (p + u) * ld);
       }
-      for (; left > 0; --left, C += cs, W += wst) row(__ldg(reinterpret_cast<const float4*>(C)), W);
+      for (; p < n; ++p) {
+        float c[RI];
+        load(c, C + p * o4);
+        row(c, W + p * ld);
+      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < RI; ++i)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) Pt[(4 * i + k) * stride + tid] = acc[i][k];
+        for (int k = 0; k < CK; ++k)
+          if (i0 + i < o && k0 + k < o) Sm[s][(i0 + i) * (OM + 1) + k0 + k] = acc[i][k];
     }
-    __syncthreads();
-    for (int e = tid; e < OM * OM; e += NT) {
+    for (int e = tid; e < OM * OM; e += NT) {  // identity beyond the electrons
       const int i = e / OM, k = e - i * OM;
-      float2 v = make_float2(i == k ? 1.f : 0.f, 0.f);
-      if (i < o && k < o) {
-        const float2* src = Pt + (4 * (i & 3) + (k & 3)) * stride + (i >> 2) * nb + (k >> 2);
-        v = src[0];
-        for (int q = 1; q < ps_n; ++q) v = cadd(v, src[q * nbb]);
-      }
-      Sm[s][i * (OM + 1) + k] = v;
+      if (i >= o || k >= o) Sm[s][i * (OM + 1) + k] = make_float2(i == k ? 1.f : 0.f, 0.f);
     }
-    __syncthreads();
   }
+  __syncthreads();
 
   if (warp < md.nslab) {
     const int s = warp, o = md.o_slab[s];
@@ -234,10 +257,10 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
 #pragma unroll
       for (int rr = 0; rr < RR; ++rr) {
         const float mag = fabsf(a[rr][0].x) + fabsf(a[rr][0].y);
-        const unsigned kc = used[rr] ? 0u : ((__float_as_uint(mag) & ~63u) | (unsigned)(63 - (lane + 32 * rr)));
+        const unsigned kc = used[rr] ? 0u : ((__float_as_uint(mag) & ~RM) | (RM - (unsigned)(lane + 32 * rr)));
         key = max(key, kc);
       }
-      const int pr = 63 - (int)(__reduce_max_sync(0xffffffffu, key) & 63u);
+      const int pr = (int)(RM - (__reduce_max_sync(0xffffffffu, key) & RM));
       // every row's own 1 / a0 while the reduction runs: conj(a0) / |a0|^2, scaled by a power of
       // two near 1 / |a0| (no overflow)
       float2 rin[RR];
@@ -247,7 +270,7 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
         const int ef = min(max((int)(__float_as_uint(m) >> 23), 1), 253);
         const float sc = __uint_as_float((unsigned)(254 - ef) << 23);
         const float px = a[rr][0].x * sc, py = a[rr][0].y * sc;
-        const float dd = __frcp_rn(fmaf(px, px, py * py)) * sc;
+        const float dd = __frcp_rn(fmaf(px, px, __fmul_rn(py, py))) * sc;
         rin[rr] = make_float2(px * dd, -py * dd);
       }
       bool own[RR];
@@ -259,38 +282,41 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
           step[rr] = j;
           pivv[s][j] = a[rr][0];
           piv_s[s][j] = pr;
-          *reinterpret_cast<float4*>(pw) = make_float4(rin[rr].x, rin[rr].y, a[rr][1].x, a[rr][1].y);
+          pw[0] = rin[rr];
+          pw[1] = a[rr][1];
 #pragma unroll
           for (int k = 2; k < OM; k += 2)
             *reinterpret_cast<float4*>(pw + k) = make_float4(a[rr][k].x, a[rr][k].y, a[rr][k + 1].x, a[rr][k + 1].y);
+          a[rr][0] = make_float2(-1.f, 0.f);  // 0 - (-1) (row / pv) is the pivot row's new value
 #pragma unroll
           for (int k = 1; k < OM; ++k) a[rr][k] = make_float2(0.f, 0.f);
         }
       }
       __syncwarp();
-      const float4 p01 = *reinterpret_cast<const float4*>(pw);  // 1 / pivot, element 1 of its row
-      const float2 inv = make_float2(p01.x, p01.y);
-      float2 f[RR];  // minus the row's factor: row - (a0 / pv) pivot row; the pivot row itself becomes row / pv
+      const float2 inv = pw[0];
+      float2 sp[RR];  // the pivot row over the pivot, an element per lane
 #pragma unroll
-      for (int rr = 0; rr < RR; ++rr) {
-        const float2 t = cmul(a[rr][0], inv);
-        f[rr] = own[rr] ? inv : make_float2(-t.x, -t.y);
-      }
+      for (int rr = 0; rr < RR; ++rr)
+        if (lane + 32 * rr < OM) sp[rr] = mul_rn(pw[lane + 32 * rr], inv);
+      __syncwarp();
+#pragma unroll
+      for (int rr = 0; rr < RR; ++rr)
+        if (lane + 32 * rr < OM && lane + 32 * rr > 0) pw[lane + 32 * rr] = sp[rr];
+      __syncwarp();
+      float2 f[RR];
+#pragma unroll
+      for (int rr = 0; rr < RR; ++rr) f[rr] = a[rr][0];
 #pragma unroll
       for (int k = 0; k < OM; k += 2) {
-        const float4 v = k == 0 ? p01 : *reinterpret_cast<const float4*>(pw + k);
+        const float4 v = *reinterpret_cast<const float4*>(pw + k);
 #pragma unroll
         for (int rr = 0; rr < RR; ++rr) {
-          if (k > 0) {
-            a[rr][k - 1].x = fmaf(f[rr].x, v.x, fmaf(-f[rr].y, v.y, a[rr][k].x));
-            a[rr][k - 1].y = fmaf(f[rr].x, v.y, fmaf(f[rr].y, v.x, a[rr][k].y));
-          }
-          a[rr][k].x = fmaf(f[rr].x, v.z, fmaf(-f[rr].y, v.w, a[rr][k + 1].x));
-          a[rr][k].y = fmaf(f[rr].x, v.w, fmaf(f[rr].y, v.z, a[rr][k + 1].y));
+          if (k > 0) a[rr][k - 1] = sub_rn(a[rr][k], mul_rn(f[rr], make_float2(v.x, v.y)));
+          a[rr][k] = sub_rn(a[rr][k + 1], mul_rn(f[rr], make_float2(v.z, v.w)));
         }
       }
 #pragma unroll
-      for (int rr = 0; rr < RR; ++rr) a[rr][OM - 1] = f[rr];
+      for (int rr = 0; rr < RR; ++rr) a[rr][OM - 1] = sub_rn(make_float2(0.f, 0.f), mul_rn(f[rr], inv));
       odd += __popcll(open & ((1ull << pr) - 1ull));  // later pivots in lower rows
       open &= ~(1ull << pr);
     }
@@ -349,16 +375,16 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
         for (int k = 0; k < OM; ++k) {
           const float4 s01 = *reinterpret_cast<const float4*>(&Sm[s][k * OM + i0]);
           const float4 s23 = *reinterpret_cast<const float4*>(&Sm[s][k * OM + i0 + 2]);
-          g[0] = cadd(g[0], cmul(wr[k], make_float2(s01.x, s01.y)));
-          g[1] = cadd(g[1], cmul(wr[k], make_float2(s01.z, s01.w)));
-          g[2] = cadd(g[2], cmul(wr[k], make_float2(s23.x, s23.y)));
-          g[3] = cadd(g[3], cmul(wr[k], make_float2(s23.z, s23.w)));
+          g[0] = add_rn(g[0], mul_rn(wr[k], make_float2(s01.x, s01.y)));
+          g[1] = add_rn(g[1], mul_rn(wr[k], make_float2(s01.z, s01.w)));
+          g[2] = add_rn(g[2], mul_rn(wr[k], make_float2(s23.x, s23.y)));
+          g[3] = add_rn(g[3], mul_rn(wr[k], make_float2(s23.z, s23.w)));
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           if (i0 + u < o) {
             float2* dst = (sum ? Wsl[0] + p * ld : row) + i0 + u;
-            if (sum) g[u] = cadd(g[u], *dst);
+            if (sum) g[u] = add_rn(g[u], *dst);
             *dst = g[u];
             if (md.nblk == 2 || s + 1 == md.nslab) mx = fmaxf(mx, fmaxf(fabsf(g[u].x), fabsf(g[u].y)));
           }
@@ -375,26 +401,37 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
   const float scl = pow2_scale(mall);
   if (tid == 0) md.g_inv[w] = 1.0f / scl;
 
-  float e1x = 0.f, e1y = 0.f;  // per-thread partials of some 20 terms; FP64 across warps
   const int gtot = md.o_blk[0] + md.o_blk[1];
+  float e1x = 0.f, e1y = 0.f;  // per-thread partials of <= 64 terms, an orbital a thread; FP64 across warps
+  for (int p = tid; p < n; p += NT)
+    for (int b = 0; b < md.nblk; ++b) {
+      const int o = md.o_blk[b];
+      const float2* G = Wsl[b] + p * green_s_ld(md.o_slab[b]);
+      const float* __restrict__ rh = md.rh1_32[b] + p;
+#pragma unroll 4
+      for (int i = 0; i < o; ++i) {
+        const float2 g = G[i];
+        const float r1 = __ldg(rh + (size_t)i * n);
+        e1x = fmaf(g.x, r1, e1x);
+        e1y = fmaf(g.y, r1, e1y);
+      }
+    }
   const bool even = (n & 1) == 0;
   for (int ii = warp; ii < gtot; ii += NW) {
     const int b = (md.nblk == 2 && ii >= md.o_blk[0]) ? 1 : 0, i = ii - b * md.o_blk[0];
     const int ld = green_s_ld(md.o_slab[b]);
     const float2* G = Wsl[b] + i;
-    const float* rh = md.rh1_32[b] + (size_t)i * n;
     uint16_t* fh[2] = {md.g_fb[0] + (size_t)(2 * w) * md.ldfb + (size_t)ii * n,
                        md.g_fb[1] + (size_t)(2 * w) * md.ldfb + (size_t)ii * n};
     uint16_t* kh[2] = {nullptr, nullptr};  // per-block operand (exchange / Coulomb of each spin separately)
     if (md.nblk == 2)
       for (int q = 0; q < 2; ++q) kh[q] = md.g_blk[b][q] + (size_t)(2 * w) * md.ldkb[b] + (size_t)i * n;
     if (even) {
-      float2 r1[4], g0[4], g1[4];  // n <= 256
+      float2 g0[4], g1[4];  // n <= 256
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int p = 2 * lane + 64 * u;
         if (p < n) {
-          r1[u] = __ldg(reinterpret_cast<const float2*>(rh + p));
           g0[u] = G[p * ld];
           g1[u] = G[(p + 1) * ld];
         }
@@ -416,8 +453,6 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
           *reinterpret_cast<uint32_t*>(kh[0] + md.ldkb[b] + p) = ihi;
           *reinterpret_cast<uint32_t*>(kh[1] + md.ldkb[b] + p) = ilo;
         }
-        e1x = fmaf(g1[u].x, r1[u].y, fmaf(g0[u].x, r1[u].x, e1x));
-        e1y = fmaf(g1[u].y, r1[u].y, fmaf(g0[u].y, r1[u].x, e1y));
       }
     } else {  // rows of the operands start at odd elements
       for (int p = lane; p < n; p += 32) {
@@ -435,8 +470,6 @@ __global__ void __launch_bounds__(NT, (OM <= 24 ? 640 : OM <= 32 ? 512 : 256) / 
           kh[0][md.ldkb[b] + p] = hi;
           kh[1][md.ldkb[b] + p] = li;
         }
-        e1x = fmaf(g.x, rh[p], e1x);
-        e1y = fmaf(g.y, rh[p], e1y);
       }
     }
   }
@@ -471,7 +504,7 @@ template <int OM>
 static int green_launch(const MixedDev& md, const float2* wu, const float2* wd, double2* ovl, int flags,
                         cudaStream_t st) {
   constexpr int NT = kGreenThreads;
-  const size_t smem = green_smem(md, OM, NT);
+  const size_t smem = green_smem(md, OM);
   if (int rc = check_smem_optin(smem + sizeof(float2) * 6 * OM + 1024,
                                 "mixed Green's-function kernel (norb x electrons too large for one CTA)"))
     return rc;

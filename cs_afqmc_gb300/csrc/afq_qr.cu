@@ -1,8 +1,5 @@
-// QR of FP32 walker slabs with the slab in registers (propagation.py:251-253 -> linalg_utils.py:51-65):
-// the LAPACK Householder factorisation (zgeqr2) and explicit Q (zung2r), up to 40 electrons per slab.
-
-#include <type_traits>
-#include <utility>
+// QR of FP32 walker slabs (propagation.py:251-253 -> linalg_utils.py:51-65): the LAPACK Householder
+// factorisation (zgeqr2) and explicit Q (zung2r). Q overwrites W.
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
@@ -11,280 +8,273 @@
 
 namespace afq {
 
-// A warp's lanes are eight row groups by four column groups: lane (g, cg) holds rows base + 8 r + g and
-// columns 4 i + cg of the slab. Step j broadcasts column j from its column group with shuffles, sums its
-// norm over the row groups, scales it into the reflector v, forms v^H a_c for every trailing column in
-// the same way and updates. Slabs of more than 64 rows are split between the warps of the CTA, which
-// exchange their sums through shared memory with two barriers a step. Nothing else leaves the
-// registers: the reflectors stay in place as in zgeqr2, and zung2r runs backwards over them.
-//
-// What bounds it: the chain of a step (norm, square root, divisions, shuffles: some 2000 cycles) over the
-// two to four slabs that an SM's scheduler has registers for. Fewer registers, more slabs: lost to the
-// spills (28 columns: 125 us at 184 registers and 160 at 144, 118 without a limit, in a form that fused the
-// update into two roundings an element; the product is rounded first now, which keeps the error of Q at
-// what it was: 7.1e-7 at 120 x 20, 1.04e-6 at 198 x 33 against quadruple precision, and costs 8%).
-// Measured against a slab per warp, or per CTA above 32 columns, in shared memory: 64 x 28 electrons, 2048
-// slabs 305 -> 131 us; 120 x 20, 1024 slabs 159 -> 114 us; 198 x 33, 256 slabs 219 -> 161 us; 60 x 10 and
-// 60 x 8, 512 walkers 45 us for one spin -> 16 us for both; 53 x 8, 64 slabs 26 -> 10 us.
-//
-// FP64 walkers keep the slab in shared memory (k_qr_f64): their units take some 18 cycles for a warp
-// instruction whatever its lanes do, and with eight lanes along the rows instead of 32 there are more of
-// them. Measured in this form at 256 walkers of two slabs, against a warp per slab in shared memory: 100 x 20 electrons
-// 559 -> 919 us, 60 x 36 959 -> 1835 us.
-constexpr int kQrRows = 8;   // rows per lane: 64 a warp
-constexpr int kQrWarps = 8;  // warps per CTA at most: 255 registers a thread
+// The order of every sum below is part of the mixed path's results: resampling compares sums of weights
+// with the comb's teeth, and a weight that moves by one FP32 rounding exchanges a whole walker wherever a
+// tooth lies that close (64 sites, 2048 walkers: with the slab in registers and its column sums split over
+// eight row groups, one of twelve populations came out with another walker). So a
+// column is summed as it always was, which costs 64 x 28 electrons, 2048 slabs 131 -> 254 us; 120 x 20, 1024 slabs
+// 114 -> 131; 198 x 33, 256 slabs 161 -> 215; 60 x 10 and 60 x 8, 512 walkers 16 -> 30.
 
-struct QrArgs {
-  float2* w[2];
-  int k[2];
-  int m;
-};
+// v y of a rank-1 update and -tau v of a column of Q (the compiler's contractions of the first version)
+AFQ_D float2 qr_vy(float2 v, float2 y) {
+  return make_float2(fmaf(v.x, y.x, -__fmul_rn(v.y, y.y)), fmaf(v.y, y.x, __fmul_rn(v.x, y.y)));
+}
+AFQ_D float2 qr_mtau(float2 t, float2 v) {
+  return make_float2(fmaf(t.y, v.y, -__fmul_rn(t.x, v.x)), fmaf(-t.y, v.x, -__fmul_rn(t.x, v.y)));
+}
+// a - f (v y)
+AFQ_D float2 qr_update(float2 a, float2 f, float2 v, float2 y) { return sub_rn(a, mul_rn(f, qr_vy(v, y))); }
 
-// sum of squares as an unevaluated pair (TwoSum per term): FP64-class accuracy without the FP64 units
-struct QrNorm {
-  float h = 0.f, l = 0.f;
-  __device__ __forceinline__ void add(float o, float ol) {
-    const float s = h + o, b = s - h;
-    l += ol + ((h - (s - b)) + (o - b));
-    h = s;
+// tau, the scale of the reflector and the new diagonal element of a column with the element alpha on the
+// diagonal and the squares xn below it (|alpha - b| >= |Im alpha|). FUSED: the divisor in one rounding
+template <bool FUSED>
+AFQ_D void qr_reflector(float2 alpha, float xn, float2& tau, float2& scl, float2& beta) {
+  if (xn == 0.f && alpha.y == 0.f) {
+    tau = make_float2(0.f, 0.f);
+    scl = make_float2(1.f, 0.f);
+    beta = alpha;
+    return;
   }
-};
-
-__device__ __forceinline__ float qr_shfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-
-template <class F, class G, int... I>
-__device__ __forceinline__ void qr_blocks(F& factor, G& form, std::integer_sequence<int, I...>) {
-  (factor(std::integral_constant<int, I>{}), ...);
-  (form(std::integral_constant<int, (int)sizeof...(I) - 1 - I>{}), ...);
+  const float nrm = sqrtf(__fadd_rn(abs2_rn(alpha), xn)), b = alpha.x >= 0.f ? -nrm : nrm;
+  tau = make_float2((b - alpha.x) / b, -alpha.y / b);
+  const float dx = alpha.x - b, r = alpha.y / dx;
+  const float den = FUSED ? fmaf(alpha.y, r, dx) : __fadd_rn(dx, __fmul_rn(alpha.y, r));
+  scl = make_float2(1.f / den, -r / den);
+  beta = make_float2(b, 0.f);
 }
 
-template <int NCL, bool MULTI>
-__global__ void __launch_bounds__(MULTI ? 32 * kQrWarps : 32) k_qr_regs(const QrArgs q) {
-  constexpr int RL = kQrRows, NW = MULTI ? kQrWarps : 1;
-  __shared__ float2 part[2][NW][MULTI ? 4 * NCL : 1];  // column sums of each warp
-  __shared__ float4 pnorm[NW];                         // its share of the norm, and the diagonal element
-  pdl_enter();
-  const int s = blockIdx.y, m = q.m, k = q.k[s], lane = threadIdx.x & 31, warp = MULTI ? threadIdx.x >> 5 : 0;
-  const int g = lane >> 2, cg = lane & 3, row0 = warp * 8 * RL + g, nwarp = MULTI ? blockDim.x >> 5 : 1;
-  float2* W = q.w[s] + (size_t)blockIdx.x * m * k;
-  float ax[RL][NCL], ay[RL][NCL], tx[NCL], ty[NCL];
-#pragma unroll
-  for (int r = 0; r < RL; ++r)
-#pragma unroll
-    for (int c = 0; c < NCL; ++c) {
-      const int row = row0 + 8 * r, col = 4 * c + cg;
-      const float2 v = row < m && col < k ? W[(size_t)row * k + col] : make_float2(0.f, 0.f);
-      ax[r][c] = v.x;
-      ay[r][c] = v.y;
-    }
-  int par = 0;
+// One warp per slab with the slab in shared memory (row stride k | 1: conflict-free column walks) and only
+// warp-level synchronisation. Column sums (the reflector applied to the trailing columns) are owned by
+// lanes per column (qr_colsum); the rank-1 updates by lane = row. The squared norm below the diagonal
+// is accumulated as a float pair.
+constexpr int kQrWarps = 4;
 
-  // sums over all rows of y[c], c >= B
-  auto reduce = [&](auto bc, float* yx, float* yy) {
-    constexpr int B = decltype(bc)::value;
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1)
-#pragma unroll
-      for (int c = B; c < NCL; ++c) {
-        yx[c] += __shfl_xor_sync(0xffffffffu, yx[c], o);
-        yy[c] += __shfl_xor_sync(0xffffffffu, yy[c], o);
+__host__ __device__ constexpr int qr_ld(int k) { return k | 1; }
+
+// y[c] = sum_{r >= j} conj(A[r][c]) A[r][j] for c in (j, k) by one warp: lpc = the largest
+// power of two with lpc * (k - j - 1) <= 32 lanes per column, each summing every lpc-th row,
+// combined by shuffles (the rows of a column are the serial part otherwise).
+__device__ __forceinline__ void qr_colsum(const float2* A, int ld, int m, int k, int j, int lane, float2* y) {
+  const int nc = k - j - 1;
+  if (nc <= 0) return;
+  int lpc = 1;
+  while (lpc * 2 * nc <= 32) lpc *= 2;
+  const int col = j + 1 + lane / lpc, part = lane % lpc;
+  const bool active = lane < lpc * nc;
+  float yx = 0.f, yy = 0.f;
+  if (active) {
+#pragma unroll 4
+    for (int r = j + part; r < m; r += lpc) {
+      const float2 pr = mulc_rn(A[r * ld + col], A[r * ld + j]);
+      yx = __fadd_rn(yx, pr.x);
+      yy = __fadd_rn(yy, pr.y);
+    }
+  }
+  for (int off = 1; off < lpc; off <<= 1) {  // lpc is warp-uniform
+    yx += __shfl_xor_sync(0xffffffffu, yx, off);
+    yy += __shfl_xor_sync(0xffffffffu, yy, off);
+  }
+  if (active && part == 0) y[col] = make_float2(yx, yy);
+}
+
+__global__ void __launch_bounds__(32 * kQrWarps) k_qr_warp(const afq_ctx_dev c, int s0, float2* __restrict__ w_up,
+                                                          float2* __restrict__ w_dn) {
+  pdl_enter();
+  extern __shared__ __align__(16) unsigned char qsm_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wlk = blockIdx.x * kQrWarps + warp, s = s0 + blockIdx.y, m = c.norb, k = c.kslab[s];
+  if (wlk >= c.nw) return;  // warp-level work only: no block barrier below
+  const int ld = qr_ld(k);
+  float2* A = reinterpret_cast<float2*>(qsm_raw) + (size_t)warp * ((size_t)m * ld + 64);
+  float2* y = A + (size_t)m * ld;
+  float2* tau = y + 32;
+  float2* W = (s == 0 ? w_up : w_dn) + (size_t)wlk * m * k;
+  for (int i = lane; i < m * k; i += 32) {
+    const int r = i / k;
+    A[r * ld + (i - r * k)] = W[i];
+  }
+  __syncwarp();
+  // ---- factorisation
+  for (int j = 0; j < k; ++j) {
+    // squared norm below the diagonal as an unevaluated float pair (TwoSum per term and per
+    // shuffle level): FP64-class accuracy without the FP64 pipe
+    float xh = 0.f, xl = 0.f;
+    for (int r = j + 1 + lane; r < m; r += 32) {
+      const float a2 = abs2_rn(A[r * ld + j]), sum = xh + a2, bb = sum - xh;
+      xl += (xh - (sum - bb)) + (a2 - bb);
+      xh = sum;
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+      const float o = __shfl_xor_sync(0xffffffffu, xh, off), ol = __shfl_xor_sync(0xffffffffu, xl, off);
+      const float sum = xh + o, bb = sum - xh;
+      xl += ol + ((xh - (sum - bb)) + (o - bb));
+      xh = sum;
+    }
+    const float2 alpha = A[j * ld + j];
+    const float xn = xh + xl;
+    float2 t, scl, beta;
+    qr_reflector<true>(alpha, xn, t, scl, beta);
+    __syncwarp();
+    for (int r = j + 1 + lane; r < m; r += 32) A[r * ld + j] = mul_rn(A[r * ld + j], scl);
+    if (lane == 0) {
+      A[j * ld + j] = make_float2(1.f, 0.f);
+      tau[j] = t;
+    }
+    __syncwarp();
+    qr_colsum(A, ld, m, k, j, lane, y);
+    __syncwarp();
+    const float2 ct = make_float2(t.x, -t.y);
+    for (int r = j + lane; r < m; r += 32) {
+      const float2 v = A[r * ld + j];
+#pragma unroll 4
+      for (int cc = j + 1; cc < k; ++cc)
+        A[r * ld + cc] = qr_update(A[r * ld + cc], ct, v, y[cc]);
+    }
+    __syncwarp();
+    if (lane == 0) A[j * ld + j] = beta;
+    __syncwarp();
+  }
+  // ---- form Q (zung2r): columns from last to first
+  for (int j = k - 1; j >= 0; --j) {
+    const float2 t = tau[j];
+    if (j < k - 1) {
+      if (lane == 0) A[j * ld + j] = make_float2(1.f, 0.f);
+      __syncwarp();
+      qr_colsum(A, ld, m, k, j, lane, y);
+      __syncwarp();
+      for (int r = j + lane; r < m; r += 32) {
+        const float2 v = A[r * ld + j];
+#pragma unroll 4
+        for (int cc = j + 1; cc < k; ++cc)
+          A[r * ld + cc] = qr_update(A[r * ld + cc], t, v, y[cc]);
       }
-    if constexpr (MULTI) {
-      if (g == 0) {
+      __syncwarp();
+    }
+    for (int r = j + 1 + lane; r < m; r += 32) A[r * ld + j] = qr_mtau(t, A[r * ld + j]);
+    if (lane == 0) A[j * ld + j] = make_float2(1.f - t.x, -t.y);
+    for (int r = lane; r < j; r += 32) A[r * ld + j] = make_float2(0.f, 0.f);
+    __syncwarp();
+  }
+  for (int i = lane; i < m * k; i += 32) {
+    const int r = i / k;
+    W[i] = A[r * ld + (i - r * k)];
+  }
+}
+
+// Slabs of more than 32 columns, or too long for four to share a CTA: one CTA per (walker, slab).
+AFQ_D float warp_sumf(float v) {
 #pragma unroll
-        for (int c = B; c < NCL; ++c) part[par][warp][4 * c + cg] = make_float2(yx[c], yy[c]);
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+__global__ void __launch_bounds__(256) k_qr_householder(const afq_ctx_dev c, int s0, float2* __restrict__ w_up,
+                                                        float2* __restrict__ w_dn) {
+  pdl_enter();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int wlk = blockIdx.x, s = s0;
+  const int m = c.norb, k = c.kslab[s];
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5,
+            nwarp = nt >> 5;
+  float2* A = reinterpret_cast<float2*>(smem_raw);  // [m][k]
+  float2* y = A + (size_t)m * k;                // [k]
+  float2* tau = y + k;                          // [k]
+  __shared__ double red[32];
+  __shared__ float2 sc_sh, beta_sh;
+  float2* W = (s == 0 ? w_up : w_dn) + (size_t)wlk * m * k;
+  for (int i = tid; i < m * k; i += nt) A[i] = W[i];
+  __syncthreads();
+  // ---- factorisation
+  for (int j = 0; j < k; ++j) {
+    double xnd = 0.0;
+    for (int r = j + 1 + tid; r < m; r += nt) xnd += (double)abs2_rn(A[r * k + j]);
+    xnd = block_sum(xnd, red);
+    if (tid == 0) {
+      const float2 alpha = A[j * k + j];
+      qr_reflector<false>(alpha, (float)xnd, tau[j], sc_sh, beta_sh);
+    }
+    __syncthreads();
+    const float2 scl = sc_sh;
+    for (int r = j + 1 + tid; r < m; r += nt) A[r * k + j] = mul_rn(A[r * k + j], scl);
+    if (tid == 0) A[j * k + j] = make_float2(1, 0);
+    __syncthreads();
+    // y[col] = sum_r conj(v[r]) A[r][col], col > j ; then A -= conj(tau) v y
+    for (int col = j + 1 + wid; col < k; col += nwarp) {
+      float yx = 0, yy = 0;
+      for (int r = j + lane; r < m; r += 32) {
+        const float2 pr = mulc_rn(A[r * k + col], A[r * k + j]);
+        yx = __fadd_rn(yx, pr.x);
+        yy = __fadd_rn(yy, pr.y);
+      }
+      yx = warp_sumf(yx);
+      yy = warp_sumf(yy);
+      if (lane == 0) y[col] = make_float2(yx, yy);
+    }
+    __syncthreads();
+    const float2 ct = cconj(tau[j]);
+    const int ncol = k - j - 1;
+    if (ncol > 0) {
+      for (int e = tid; e < (m - j) * ncol; e += nt) {
+        const int r = j + e / ncol, col = j + 1 + e % ncol;
+        A[r * k + col] = qr_update(A[r * k + col], ct, A[r * k + j], y[col]);
+      }
+    }
+    __syncthreads();
+    if (tid == 0) A[j * k + j] = beta_sh;
+    __syncthreads();
+  }
+  // ---- form Q (zung2r): columns from last to first
+  for (int j = k - 1; j >= 0; --j) {
+    if (j < k - 1) {
+      if (tid == 0) A[j * k + j] = make_float2(1, 0);
+      __syncthreads();
+      for (int col = j + 1 + wid; col < k; col += nwarp) {
+        float yx = 0, yy = 0;
+        for (int r = j + lane; r < m; r += 32) {
+          const float2 pr = mulc_rn(A[r * k + col], A[r * k + j]);
+          yx = __fadd_rn(yx, pr.x);
+          yy = __fadd_rn(yy, pr.y);
+        }
+        yx = warp_sumf(yx);
+        yy = warp_sumf(yy);
+        if (lane == 0) y[col] = make_float2(yx, yy);
       }
       __syncthreads();
-#pragma unroll
-      for (int c = B; c < NCL; ++c) yx[c] = yy[c] = 0.f;
-      for (int w = 0; w < nwarp; ++w)
-#pragma unroll
-        for (int c = B; c < NCL; ++c) {
-          const float2 p = part[par][w][4 * c + cg];
-          yx[c] += p.x;
-          yy[c] += p.y;
-        }
-      par ^= 1;  // a warp that is still reading is at most one reduction behind
+      const float2 t = tau[j];
+      const int ncol = k - j - 1;
+      for (int e = tid; e < (m - j) * ncol; e += nt) {
+        const int r = j + e / ncol, col = j + 1 + e % ncol;
+        A[r * k + col] = qr_update(A[r * k + col], t, A[r * k + j], y[col]);
+      }
+      __syncthreads();
     }
-  };
-
-  // ---- factorisation: steps j = 4 b + ii
-  auto factor = [&](auto bc) {
-    constexpr int B = decltype(bc)::value, WJ = (B / 2) / RL, RJ = (B / 2) % RL, R0 = MULTI ? 0 : RJ;
-#pragma unroll 1
-    for (int ii = 0; ii < 4; ++ii) {
-      const int j = 4 * B + ii;
-      if (j >= k) break;
-      const int src = (lane & ~3) | ii, gj = (4 * B) % 8 + ii;
-      float vx[RL], vy[RL], yx[NCL], yy[NCL];
-      QrNorm nrm;
-      float2 al = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int r = R0; r < RL; ++r) {
-        const float bx = qr_shfl(ax[r][B], src), by = qr_shfl(ay[r][B], src);
-        if (r == RJ) al = make_float2(qr_shfl(bx, 4 * gj), qr_shfl(by, 4 * gj));
-        const bool below = row0 + 8 * r > j;
-        vx[r] = below ? bx : 0.f;
-        vy[r] = below ? by : 0.f;
-        nrm.add(vx[r] * vx[r] + vy[r] * vy[r], 0.f);
-      }
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1)
-        nrm.add(__shfl_xor_sync(0xffffffffu, nrm.h, o), __shfl_xor_sync(0xffffffffu, nrm.l, o));
-      if constexpr (MULTI) {
-        // the column sums' barrier below stands between these reads and the next step's writes
-        if (lane == 0) pnorm[warp] = make_float4(nrm.h, nrm.l, al.x, al.y);
-        __syncthreads();
-        al = make_float2(pnorm[WJ].z, pnorm[WJ].w);
-        nrm.h = nrm.l = 0.f;
-        for (int w = 0; w < nwarp; ++w) nrm.add(pnorm[w].x, pnorm[w].y);
-      }
-      const float xn = nrm.h + nrm.l;
-      float2 t = make_float2(0.f, 0.f), scl = make_float2(1.f, 0.f);
-      if (!(xn == 0.f && al.y == 0.f)) {
-        const float n2 = sqrtf(al.x * al.x + al.y * al.y + xn), b = al.x >= 0.f ? -n2 : n2;
-        t = make_float2((b - al.x) / b, -al.y / b);
-        scl = cdiv(make_float2(1.f, 0.f), make_float2(al.x - b, al.y));
-      }
-      if (cg == ii) {
-        tx[B] = t.x;
-        ty[B] = t.y;
-      }
-#pragma unroll
-      for (int c = B; c < NCL; ++c) yx[c] = yy[c] = 0.f;
-#pragma unroll
-      for (int r = R0; r < RL; ++r) {
-        const float2 v = row0 + 8 * r == j ? make_float2(1.f, 0.f) : cmul(make_float2(vx[r], vy[r]), scl);
-        vx[r] = v.x;
-        vy[r] = v.y;
-#pragma unroll
-        for (int c = B; c < NCL; ++c) {
-          yx[c] = fmaf(v.x, ax[r][c], fmaf(v.y, ay[r][c], yx[c]));
-          yy[c] = fmaf(v.x, ay[r][c], fmaf(-v.y, ax[r][c], yy[c]));
-        }
-      }
-      reduce(bc, yx, yy);
-      // a_c -= conj(tau) v (v^H a_c), columns behind j only
-#pragma unroll
-      for (int c = B; c < NCL; ++c) {
-        const float2 p = cmul(make_float2(t.x, -t.y), make_float2(yx[c], yy[c]));
-        yx[c] = p.x;
-        yy[c] = p.y;
-      }
-#pragma unroll
-      for (int r = R0; r < RL; ++r) {
-        if (cg == ii && row0 + 8 * r > j) {
-          ax[r][B] = vx[r];
-          ay[r][B] = vy[r];
-        }
-        if (cg > ii) {
-          ax[r][B] -= fmaf(vx[r], yx[B], -vy[r] * yy[B]);
-          ay[r][B] -= fmaf(vx[r], yy[B], vy[r] * yx[B]);
-        }
-#pragma unroll
-        for (int c = B + 1; c < NCL; ++c) {
-          ax[r][c] -= fmaf(vx[r], yx[c], -vy[r] * yy[c]);
-          ay[r][c] -= fmaf(vx[r], yy[c], vy[r] * yx[c]);
-        }
-      }
-    }
-  };
-
-  // ---- Q = H_0 .. H_{k-1} I: column j becomes e_j - tau v, after H_j acts on the columns behind it
-  auto form = [&](auto bc) {
-    constexpr int B = decltype(bc)::value, RJ = (B / 2) % RL, R0 = MULTI ? 0 : RJ;
-#pragma unroll 1
-    for (int ii = 3; ii >= 0; --ii) {
-      const int j = 4 * B + ii;
-      if (j >= k) continue;
-      const int src = (lane & ~3) | ii;
-      float vx[RL], vy[RL], yx[NCL], yy[NCL];
-#pragma unroll
-      for (int c = B; c < NCL; ++c) yx[c] = yy[c] = 0.f;
-#pragma unroll
-      for (int r = R0; r < RL; ++r) {
-        const float bx = qr_shfl(ax[r][B], src), by = qr_shfl(ay[r][B], src);
-        const int row = row0 + 8 * r;
-        vx[r] = row > j ? bx : row == j ? 1.f : 0.f;
-        vy[r] = row > j ? by : 0.f;
-#pragma unroll
-        for (int c = B; c < NCL; ++c) {
-          yx[c] = fmaf(vx[r], ax[r][c], fmaf(vy[r], ay[r][c], yx[c]));
-          yy[c] = fmaf(vx[r], ay[r][c], fmaf(-vy[r], ax[r][c], yy[c]));
-        }
-      }
-      reduce(bc, yx, yy);
-      const float2 t = make_float2(qr_shfl(tx[B], ii), qr_shfl(ty[B], ii));
-#pragma unroll
-      for (int c = B; c < NCL; ++c) {
-        const float2 p = cmul(t, make_float2(yx[c], yy[c]));
-        yx[c] = p.x;
-        yy[c] = p.y;
-      }
-#pragma unroll
-      for (int r = 0; r < RL; ++r) {
-        if (r < R0) {
-          if (cg == ii) ax[r][B] = ay[r][B] = 0.f;
-          continue;
-        }
-        if (cg == ii) {
-          const float2 p = cmul(t, make_float2(vx[r], vy[r]));
-          ax[r][B] = (row0 + 8 * r == j ? 1.f : 0.f) - p.x;
-          ay[r][B] = -p.y;
-        }
-        if (cg > ii) {
-          ax[r][B] -= fmaf(vx[r], yx[B], -vy[r] * yy[B]);
-          ay[r][B] -= fmaf(vx[r], yy[B], vy[r] * yx[B]);
-        }
-#pragma unroll
-        for (int c = B + 1; c < NCL; ++c) {
-          ax[r][c] -= fmaf(vx[r], yx[c], -vy[r] * yy[c]);
-          ay[r][c] -= fmaf(vx[r], yy[c], vy[r] * yx[c]);
-        }
-      }
-    }
-  };
-
-  qr_blocks(factor, form, std::make_integer_sequence<int, NCL>{});
-
-#pragma unroll
-  for (int r = 0; r < RL; ++r)
-#pragma unroll
-    for (int c = 0; c < NCL; ++c) {
-      const int row = row0 + 8 * r, col = 4 * c + cg;
-      if (row < m && col < k) W[(size_t)row * k + col] = make_float2(ax[r][c], ay[r][c]);
-    }
-}
-
-template <int NCL>
-static void launch_regs(const QrArgs& q, int nw, int nslab, cudaStream_t st) {
-  const int nwarp = (q.m + 8 * kQrRows - 1) / (8 * kQrRows);
-  ProfScope _ps(K_QR, st);
-  if (nwarp == 1)
-    launch_pdl(k_qr_regs<NCL, false>, dim3(nw, nslab), 32, 0, st, q);
-  else
-    launch_pdl(k_qr_regs<NCL, true>, dim3(nw, nslab), 32 * nwarp, 0, st, q);
+    const float2 t = tau[j];
+    for (int r = j + 1 + tid; r < m; r += nt) A[r * k + j] = qr_mtau(t, A[r * k + j]);
+    if (tid == 0) A[j * k + j] = make_float2(1 - t.x, -t.y);
+    for (int r = tid; r < j; r += nt) A[r * k + j] = make_float2(0, 0);
+    __syncthreads();
+  }
+  for (int i = tid; i < m * k; i += nt) W[i] = A[i];
 }
 
 int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
-  const QrArgs q = {{static_cast<float2*>(wu), static_cast<float2*>(wd)}, {c.kslab[0], c.nslab > 1 ? c.kslab[1] : 0}, c.norb};
-  const int ncl = ((q.k[0] > q.k[1] ? q.k[0] : q.k[1]) + 3) / 4;
-  if (q.m > 8 * kQrRows * kQrWarps || ncl > 10) {
-    afq_set_error("FP32 QR: at most %d orbitals and 40 electrons per spin", 8 * kQrRows * kQrWarps);
-    return -1;
-  }
-  switch (ncl) {
-    case 0:
-    case 1: launch_regs<1>(q, c.nw, c.nslab, st); break;
-    case 2: launch_regs<2>(q, c.nw, c.nslab, st); break;
-    case 3: launch_regs<3>(q, c.nw, c.nslab, st); break;
-    case 4: launch_regs<4>(q, c.nw, c.nslab, st); break;
-    case 5: launch_regs<5>(q, c.nw, c.nslab, st); break;
-    case 6: launch_regs<6>(q, c.nw, c.nslab, st); break;
-    case 7: launch_regs<7>(q, c.nw, c.nslab, st); break;
-    case 8: launch_regs<8>(q, c.nw, c.nslab, st); break;
-    case 9: launch_regs<9>(q, c.nw, c.nslab, st); break;
-    default: launch_regs<10>(q, c.nw, c.nslab, st); break;
+  float2 *u = static_cast<float2*>(wu), *d = static_cast<float2*>(wd);
+  auto warp_smem = [&](int s) {
+    return kQrWarps * ((size_t)c.norb * qr_ld(c.kslab[s]) + 64) * sizeof(float2);
+  };
+  auto by_warp = [&](int s) { return c.kslab[s] <= 32 && warp_smem(s) <= 227 * 1024; };
+  const bool both = c.nslab == 2 && by_warp(0) && by_warp(1);  // one launch for both slabs
+  ProfScope _ps(K_QR, st);
+  for (int s = 0; s < (both ? 1 : c.nslab); ++s) {
+    if (by_warp(s)) {
+      const size_t smem = both && warp_smem(1) > warp_smem(0) ? warp_smem(1) : warp_smem(s);
+      cudaFuncSetAttribute(k_qr_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      launch_pdl(k_qr_warp, dim3((c.nw + kQrWarps - 1) / kQrWarps, both ? 2 : 1), 32 * kQrWarps, smem, st, c, s, u, d);
+    } else {
+      const size_t smem = ((size_t)c.norb + 2) * c.kslab[s] * sizeof(float2);
+      cudaFuncSetAttribute(k_qr_householder, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      launch_pdl(k_qr_householder, c.nw, 256, smem, st, c, s, u, d);
+    }
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

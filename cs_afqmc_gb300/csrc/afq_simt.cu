@@ -463,25 +463,24 @@ __global__ void k_pop_control(const WeightArgs g) {
 // FP64 units, and their sums meet in the first CTA's shared memory. Against two launches: 512 walkers
 // 10.9 -> 9.1 us, 1024 11.9 -> 10.7, and a launch less in the chain of a step (ten steps of 64 walkers 787 -> 774 us).
 // Above 1024 walkers an SM would run more than four warps of FP64 exponentials, 1.8 us each.
+// The weights are summed as the two launches do, a warp of 32 consecutive walkers and then the 32 warps.
 constexpr int kWeightsCluster = 1024, kWeightsCtas = 8;
 
-__global__ void __cluster_dims__(kWeightsCtas, 1, 1) __launch_bounds__(128) k_weights_pop(const WeightArgs g, int per) {
+__global__ void __cluster_dims__(kWeightsCtas, 1, 1) __launch_bounds__(128) k_weights_pop(const WeightArgs g) {
   namespace cg = cooperative_groups;
-  __shared__ double part[kWeightsCtas], red[32];
+  __shared__ double part[32];
   const cg::cluster_group cl = cg::this_cluster();
+  if (threadIdx.x < 32) part[threadIdx.x] = 0.0;
   cl.sync();  // every CTA runs: its shared memory may be written from here on
   pdl_enter();
-  const int rank = (int)cl.block_rank(), w = rank * per + threadIdx.x;
+  const int w = (int)cl.block_rank() * blockDim.x + threadIdx.x;
   const double pcs = g.scalars[AFQ_S_POP_CONTROL_SHIFT];
-  double v = 0.0;
-  if ((int)threadIdx.x < per && w < g.nw) v = weight_step(g, w, pcs);
-  v = blockDim.x == 32 ? warp_sum(v) : block_sum(v, red);
-  if (threadIdx.x == 0) *cl.map_shared_rank(&part[rank], 0) = v;
+  const double v = warp_sum(w < g.nw ? weight_step(g, w, pcs) : 0.0);
+  if ((threadIdx.x & 31) == 0) *cl.map_shared_rank(&part[w >> 5], 0) = v;
   cl.sync();  // all have read the old shift, too
-  if (rank == 0 && threadIdx.x == 0) {
-    double sum = part[0];
-    for (int i = 1; i < kWeightsCtas; ++i) sum += part[i];
-    pop_control(g, sum);
+  if (cl.block_rank() == 0 && threadIdx.x < 32) {
+    const double sum = warp_sum(part[threadIdx.x]);
+    if (threadIdx.x == 0) pop_control(g, sum);
   }
 }
 
@@ -1163,7 +1162,7 @@ int launch_weights(const afq_ctx_dev& c, const double2* shift, const double2* fb
   if (c.nw <= kWeightsCluster) {
     ProfScope _ps(K_WEIGHTS, st);
     const int per = (c.nw + kWeightsCtas - 1) / kWeightsCtas;
-    launch_pdl(k_weights_pop, kWeightsCtas, (per + 31) / 32 * 32, 0, st, g, per);
+    launch_pdl(k_weights_pop, kWeightsCtas, (per + 31) / 32 * 32, 0, st, g);
     return launch_err("weights_pop");
   }
   {
