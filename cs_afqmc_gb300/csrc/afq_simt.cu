@@ -601,18 +601,20 @@ __global__ void k_energy_final(const afq_ctx_dev c, int nchunks, const double2* 
 // What bounds it: latency in FP64 chains, then the FP64 units (a warp instruction takes some 18 cycles
 // whatever its lanes do; 10 m k^2 of them, with 32 elements each). So a column is one reduction, a few scalar
 // steps by one warp and one update: the squares of column j are one more of the sums over its raw elements,
-// v^H a_c = a_jc + conj(scale) sum, the divisions are lanes of one instruction, tau goes into the sums.
+// v^H a_c = a_jc + conj(scale) sum, the divisions are lanes of one instruction, tau goes into the sums
+// (conj(tau) conj(scale) = -1 / b).
 // Row j right of the diagonal (R) is never read again and is left alone.
-// Against a warp per slab with a pass for the norm: 40 x 7 and 40 x 6 electrons, 200 walkers 71 -> 52 us; 60 x 10 and
-// 60 x 8, 512 walkers 186 -> 193 us; a block of five steps with one QR, 120 x 20, 256 walkers 7.82 -> 7.45 ms.
+// Against a warp per slab with a pass for the norm: 40 x 7 and 40 x 6 electrons, 200 walkers 71 -> 57 us; 60 x 10 and
+// 60 x 8, 512 walkers 186 -> 207 us; a block of five steps with one QR, 120 x 20, 256 walkers 7.82 -> 7.46 ms.
 // rdiag (optional, [nslab][nw]): prod(diag R) per walker slab (linalg_utils.py:51-65 returns
 // it as the norm factor; the free-projection step multiplies its norms by it)
 // ======================================================================================
 
 // y[c] = mul sum_{r > j} conj(A[r][j]) A[r][c] for c in [c_lo, k): lpc lanes (a power of two) per column.
-// Two chains of eight rows at a time: with two over all rows of a lane, and the update below as an FMA chain, Q
-// was further off than with a sum over 32 lanes (against extended precision, walkers of 120 x 20: 4.45e-16
-// instead of 3.12e-16, now 3.31e-16; 180 x 30: 5.51e-16, 3.46e-16, 3.44e-16).
+// Short chains, the four products of a complex one in their own: two chains of eight rows at a time. Q
+// against extended precision, walkers of 120 x 20 and 60 x 28: 3.10e-16 and 3.74e-16 with a sum over 32 lanes, 4.45e-16
+// at 120 x 20 with chains over all rows of a lane and the update below as an FMA chain, 3.26e-16 and 3.97e-16 with
+// two products a chain, now (with the reflector's scale to one rounding) 2.98e-16 and 3.65e-16.
 AFQ_D void qr64_sums(const double2* A, int ld, int m, int k, int j, int c_lo, double2 mul, double2* y) {
   const int nc = k - c_lo, tid = threadIdx.x, nt = blockDim.x;
   int sh = 0;
@@ -624,20 +626,26 @@ AFQ_D void qr64_sums(const double2* A, int ld, int m, int k, int j, int c_lo, do
     if (c < k) {
       for (int r0 = j + 1 + part; r0 < m; r0 += 16 * lpc) {
         const int r1 = min(m, r0 + 16 * lpc);
-        double2 a = c2(0, 0), b = c2(0, 0);
+        // sums of x.x v.x and x.y v.x (a, b), of x.y v.y and x.x v.y (e, f)
+        double2 a = c2(0, 0), b = a, e = a, f = a;
         int r = r0;
 #pragma unroll 4
         for (; r + lpc < r1; r += 2 * lpc) {
           const double2 x = A[r * ld + c], v = A[r * ld + j];
           const double2 x2 = A[(r + lpc) * ld + c], v2 = A[(r + lpc) * ld + j];
-          a = c2(fma(x.x, v.x, fma(x.y, v.y, a.x)), fma(x.y, v.x, fma(-x.x, v.y, a.y)));
-          b = c2(fma(x2.x, v2.x, fma(x2.y, v2.y, b.x)), fma(x2.y, v2.x, fma(-x2.x, v2.y, b.y)));
+          a = c2(fma(x.x, v.x, a.x), fma(x.y, v.x, a.y));
+          e = c2(fma(x.y, v.y, e.x), fma(x.x, v.y, e.y));
+          b = c2(fma(x2.x, v2.x, b.x), fma(x2.y, v2.x, b.y));
+          f = c2(fma(x2.y, v2.y, f.x), fma(x2.x, v2.y, f.y));
         }
         if (r < r1) {
           const double2 x = A[r * ld + c], v = A[r * ld + j];
-          a = c2(fma(x.x, v.x, fma(x.y, v.y, a.x)), fma(x.y, v.x, fma(-x.x, v.y, a.y)));
+          a = c2(fma(x.x, v.x, a.x), fma(x.y, v.x, a.y));
+          e = c2(fma(x.y, v.y, e.x), fma(x.x, v.y, e.y));
         }
-        sum = cadd(sum, cadd(a, b));
+        a = cadd(a, b);
+        e = cadd(e, f);
+        sum = cadd(sum, c2(a.x + e.x, a.y - e.y));
       }
     }
     for (int off = 1; off < lpc; off <<= 1)
@@ -680,18 +688,27 @@ __global__ void __launch_bounds__(256) k_qr_f64(const afq_ctx_dev c, double2* __
       const double2 alpha = A[j * ld + j];
       const double xn = y[j].x;
       double2 t = c2(0, 0), scl = c2(1, 0), beta = alpha;
+      double nib = 0.0;  // -1 / b = conj(tau) conj(scale)
       if (!(xn == 0.0 && alpha.y == 0.0)) {
         const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
         const double b = alpha.x >= 0.0 ? -nrm : nrm, dx = alpha.x - b, d2 = dx * dx + alpha.y * alpha.y;
-        // tau = (b - alpha) / b and scale = 1 / (alpha - b), a quotient per lane
-        const double num = tid == 0 ? -dx : tid == 1 ? -alpha.y : tid == 2 ? dx : -alpha.y;
-        const double q = num / (tid < 2 ? b : d2);
+        // tau = (b - alpha) / b, scale = 1 / (alpha - b) and -1 / b, a quotient per lane
+        const double num = tid == 0 ? -dx : tid == 2 ? dx : tid == 4 ? -1.0 : -alpha.y;
+        const double q = num / (tid == 2 || tid == 3 ? d2 : b);
         t = c2(__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1));
         scl = c2(__shfl_sync(0xffffffffu, q, 2), __shfl_sync(0xffffffffu, q, 3));
+        nib = __shfl_sync(0xffffffffu, q, 4);
         beta = c2(b, 0);
+        // a Newton step: its relative error is that of the whole reflector, and 1 / d2 alone has three roundings
+        const double h = alpha.y * scl.x, l = fma(alpha.y, scl.x, -h);
+        const double ex = fma(alpha.y, scl.y, fma(-dx, scl.x, 1.0)), ey = fma(-dx, scl.y, -h) - l;
+        scl = c2(scl.x + fma(scl.x, ex, -(scl.y * ey)), scl.y + fma(scl.x, ey, scl.y * ex));
       }
-      for (int i = j + 1 + tid; i < k; i += 32)
-        y[i] = cmul(cconj(t), cadd(A[j * ld + i], cmul(cconj(scl), y[i])));
+      // conj(tau) v^H a = conj(tau) a_j - sum / b
+      for (int i = j + 1 + tid; i < k; i += 32) {
+        const double2 p = cmul(cconj(t), A[j * ld + i]);
+        y[i] = c2(fma(nib, y[i].x, p.x), fma(nib, y[i].y, p.y));
+      }
       if (tid == 0) {
         rprod = cmul(rprod, beta);
         tau[j] = t;
