@@ -265,6 +265,9 @@ inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 bool is_fp64(const afq_ctx* c) { return c->d.precision == AFQ_PREC_FP64; }
 
+// The guard word of the context's tensor-core kernels
+const int* status_word(const afq_ctx* c) { return is_fp64(c) ? c->dg.status : c->tc.status; }
+
 // Green's function + overlap. FP64: G into c->green. Mixed: the 16-bit operands of the
 // force-bias, energy and exp_h1 contractions (wg) and/or the overlap.
 // chain (inside a block): the walkers are propagated next, so the same launch also forms G (mixed
@@ -322,7 +325,7 @@ int energy_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
   if (!is_fp64(c)) return afq::tc_energy(c->tc, c->dev, out, st);
   if (c->dg.has_u) {
     CHECK(energy_gemms(c, st));
-    return afq::dig_launch_energy(c->dev, c->green, c->dg.z, c->fb, out, st);
+    return afq::dig_launch_energy(c->dev, c->green, c->dg.z, c->fb, out, c->dg.status, st);
   }
   return afq::launch_energy_f64(c->dev, c->e_chunks, c->e_gchunk, c->green, c->epart, out, st);
 }
@@ -832,6 +835,14 @@ extern "C" {
 
 int afq_abi_version(void) { return AFQ_ABI_VERSION; }
 
+int afq_test_preset_status(afq_ctx* ctx, int bits, void* stream) {
+  if (!ctx || bits < 0 || bits > 255) { afq_set_error("bad argument"); return -1; }
+  // the word's low byte (little endian); the rest stays zero
+  const cudaError_t e = cudaMemsetAsync(const_cast<int*>(status_word(ctx)), bits, 1, S(stream));
+  if (e != cudaSuccess) { afq_set_error("preset status: %s", cudaGetErrorString(e)); return (int)e; }
+  return 0;
+}
+
 const char* afq_last_error(void) { return g_err; }
 
 size_t afq_workspace_size(const afq_dims* dims) {
@@ -989,7 +1000,10 @@ int afq_calc_force_bias(afq_ctx* ctx, const void* walkers_up, const void* walker
   if (!ctx || !force_bias) { afq_set_error("NULL argument"); return -1; }
   CHECK(check_walkers(ctx, walkers_up, walkers_dn));
   CHECK(green(ctx, walkers_up, walkers_dn, ctx->green, nullptr, true, S(stream)));
-  return force_bias_from_green(ctx, reinterpret_cast<double2*>(force_bias), S(stream));
+  CHECK(force_bias_from_green(ctx, reinterpret_cast<double2*>(force_bias), S(stream)));
+  if (!is_fp64(ctx)) return 0;
+  return afq::launch_poison((long)ctx->dev.nw * ctx->dev.nchol, reinterpret_cast<double2*>(force_bias),
+                            ctx->dg.status, S(stream));
 }
 
 int afq_calc_energy(afq_ctx* ctx, const void* walkers_up, const void* walkers_dn, double* energies,
@@ -1051,7 +1065,7 @@ int afq_propagate_phaseless(afq_ctx* ctx, afq_walker_state* state, const double*
       CHECK(green(ctx, state->walkers_up, state->walkers_dn, ctx->green, ovl, true, st, true));
       CHECK(energy_from_green(ctx, ctx->ene, st));
       CHECK(afq::launch_block_stats(d, ctx->ene, state->weights, state->scalars, block_energy + blk,
-                                    block_weight + blk, st));
+                                    block_weight + blk, st, status_word(ctx)));
     }
     ctx->gstate = 0;
     CHECK(sr_impl(ctx, state, zetas + sr, nullptr, st));
@@ -1226,7 +1240,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
         CHECK(afq::t_launch_energy(d, t, ctx->e_chunks, ctx->e_gchunk, ctx->green, st));
       }
       CHECK(afq::launch_block_stats(d, ctx->ene, state->weights, state->scalars, block_energy + blk,
-                                    block_weight + blk, st));
+                                    block_weight + blk, st, status_word(ctx)));
       CHECK(afq::t_launch_block_stats(d, t, ctx->ene, state->weights, state->scalars, block_energy + blk,
                                       dblock_energy + blk, dblock_weight + blk, st));
     }
@@ -1377,7 +1391,7 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
       CHECK(energy_from_green(ctx, ctx->ene, st));
       CHECK(copy_d2d(tp.ene(blk), ctx->ene, d.nw * sizeof(double2), st, "local-energy record"));
       CHECK(afq::launch_block_stats(d, ctx->ene, state->weights, state->scalars, block_energy + blk,
-                                    block_weight + blk, st));
+                                    block_weight + blk, st, status_word(ctx)));
     }
     if (!do_sr) continue;
     ctx->gstate = 0;
@@ -1511,7 +1525,7 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
     CHECK(zero(out->gh0_prop, 2 * sizeof(double), st));
     CHECK(copy_d2d(out->gh0_prop, a.scal + 1, sizeof(double), st, "h0_prop cotangent"));
   }
-  return 0;
+  return afq::launch_fold_status(state->scalars, status_word(ctx), st);
 }
 
 int afq_propagate_free(afq_ctx* ctx, afq_walker_state* state, const double* fields, double ene0, double* norms,
@@ -1519,8 +1533,9 @@ int afq_propagate_free(afq_ctx* ctx, afq_walker_state* state, const double* fiel
   if (!ctx || !fields || !norms || !normed_overlaps) { afq_set_error("NULL argument"); return -1; }
   CHECK(check_state(ctx, state));
   CHECK(check_free(ctx));
-  return free_step(ctx, state, fields, ene0, reinterpret_cast<double2*>(norms),
-                   reinterpret_cast<double2*>(normed_overlaps), S(stream));
+  CHECK(free_step(ctx, state, fields, ene0, reinterpret_cast<double2*>(norms),
+                  reinterpret_cast<double2*>(normed_overlaps), S(stream)));
+  return afq::launch_fold_status(state->scalars, status_word(ctx), S(stream));
 }
 
 int afq_propagate_free_blocks(afq_ctx* ctx, afq_walker_state* state, const double* fields, int32_t n_prop_steps,
@@ -1547,7 +1562,7 @@ int afq_propagate_free_blocks(afq_ctx* ctx, afq_walker_state* state, const doubl
     CHECK(afq::launch_free_block_stats(d.nw, ctx->ene, ovl, reinterpret_cast<double2*>(block_energy) + b,
                                        reinterpret_cast<double2*>(block_weight) + b, st));
   }
-  return 0;
+  return afq::launch_fold_status(state->scalars, status_word(ctx), st);
 }
 
 int afq_field_block(afq_ctx* ctx, afq_walker_state* state, const double* fields, int32_t n_prop_steps,
@@ -1569,7 +1584,8 @@ int afq_field_block(afq_ctx* ctx, afq_walker_state* state, const double* fields,
   CHECK(green(ctx, state->walkers_up, state->walkers_dn, ctx->green, reinterpret_cast<double2*>(state->overlaps),
               true, st));
   CHECK(energy_from_green(ctx, ctx->ene, st));
-  CHECK(afq::launch_block_stats(d, ctx->ene, state->weights, state->scalars, block_energy, block_weight, st));
+  CHECK(afq::launch_block_stats(d, ctx->ene, state->weights, state->scalars, block_energy, block_weight, st,
+                                status_word(ctx)));
   if (local_energies) CHECK(afq::launch_clamped_energies(d, ctx->ene, state->scalars, local_energies, st));
   return 0;
 }

@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
       }
     }
   }
-  if (!ok) atomicOr(status, 4);
+  if (!ok) atomicOr(status, kDigTimeout);
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -874,7 +874,7 @@ AFQ_D double2 block_sum2(double2 v, double* red) { return c2(block_sum(v.x, red)
 
 __global__ void __launch_bounds__(128) k_dig_energy(const afq_ctx_dev c, const double2* __restrict__ green,
                                                     const double2* __restrict__ z, const double2* __restrict__ coul,
-                                                    double2* __restrict__ energy) {
+                                                    double2* __restrict__ energy, const int* __restrict__ status) {
   pdl_enter();
   __shared__ double red[32];
   const size_t w = blockIdx.x;
@@ -902,7 +902,7 @@ __global__ void __launch_bounds__(128) k_dig_energy(const afq_ctx_dev c, const d
   } else {  // UHF
     e2 = cscale(csub(co, ex), 0.5);
   }
-  energy[w] = cadd(cadd(e2, e1), c2(c.h0, 0.0));
+  energy[w] = *status == 0 ? cadd(cadd(e2, e1), c2(c.h0, 0.0)) : c2(nan(""), nan(""));
 }
 
 __global__ void __launch_bounds__(128) k_dig_energy_tangent(const afq_ctx_dev c, const double2* __restrict__ green,
@@ -1227,10 +1227,10 @@ int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int te
 }
 
 int dig_launch_energy(const afq_ctx_dev& c, const double2* green, const double2* z, const double2* coul,
-                      double2* energy, cudaStream_t st) {
+                      double2* energy, const int* status, cudaStream_t st) {
   {
     ProfScope _ps(K_ENERGY_FIN, st);
-    launch_pdl(k_dig_energy, c.nw, 128, 0, st, c, green, z, coul, energy);
+    launch_pdl(k_dig_energy, c.nw, 128, 0, st, c, green, z, coul, energy, status);
   }
   return dig_err("energy");
 }

@@ -28,6 +28,7 @@ namespace afq {
 
 constexpr int kDigTile = 128;     // A rows per tile
 constexpr int kDigSegBlocks = 32; // K blocks (of 16) an accumulator may sum exactly
+constexpr int kDigTimeout = 8;    // status bit: a wait of the digit GEMM ran out
 constexpr int kDigBad = 1 << 20;  // row exponent of a row with a NaN or an infinity
 
 inline size_t dig_bytes(long rows, long K, int tr = kDigTile) {
@@ -70,9 +71,9 @@ int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D,
                cudaStream_t st);
 
 // ---- local energy from the sliced contractions -----------------------------------------
-// z [nw][ktot] = U G per spin, coul [nw][nchol] = rc . G; final sums per walker
+// z [nw][ktot] = U G per spin, coul [nw][nchol] = rc . G; final sums per walker (NaN if *status != 0)
 int dig_launch_energy(const afq_ctx_dev& c, const double2* green, const double2* z, const double2* coul,
-                      double2* energy, cudaStream_t st);
+                      double2* energy, const int* status, cudaStream_t st);
 // its tangent: dcoul [nw][nchol], the tangents of G and rot_h1
 int dig_launch_energy_tangent(const afq_ctx_dev& c, const double2* green, const double2* dgreen, const double2* z,
                               const double2* coul, const double2* dcoul, const double* drot_up,

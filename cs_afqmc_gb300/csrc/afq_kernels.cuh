@@ -57,7 +57,10 @@ template <typename WT>
 int launch_sr(const afq_ctx_dev& c, const double* zeta, double* weights, double* cum, int32_t* idx,
               void* wu, void* wd, void* wcopy, cudaStream_t st);
 int launch_block_stats(const afq_ctx_dev& c, const double2* energy, const double* weights,
-                       double* scalars, double* be, double* bw, cudaStream_t st);
+                       double* scalars, double* be, double* bw, cudaStream_t st, const int* status);
+// scalars[AFQ_S_STATUS] |= *status; NaN over out[n] where *status is not 0
+int launch_fold_status(double* scalars, const int* status, cudaStream_t st);
+int launch_poison(long n, double2* out, const int* status, cudaStream_t st);
 int launch_phaseless_begin(double* scalars, cudaStream_t st);
 int launch_clamped_energies(const afq_ctx_dev& c, const double2* energy, const double* scalars,
                             double* out, cudaStream_t st);

@@ -406,8 +406,27 @@ struct WeightArgs {
   const double2 *shift, *fbt, *ovl_new;
   double2* ovl;
   double *weights, *scalars;
-  const int* status;  // mixed path, may be NULL
+  const int* status;  // may be NULL
 };
+
+// The tensor-core pipelines' guard word joins scalars[AFQ_S_STATUS], so that callers see a wait that ran
+// out or a bad operand in the state (status may be NULL)
+AFQ_D void fold_status(double* scalars, const int* status) {
+  if (status && *status != 0) scalars[AFQ_S_STATUS] = (double)((int)scalars[AFQ_S_STATUS] | *status);
+}
+
+__global__ void k_fold_status(double* scalars, const int* status) {
+  pdl_enter();
+  fold_status(scalars, status);
+}
+
+// NaN over results that a call returns without a state to report in
+__global__ void k_poison(long n, double2* out, const int* status) {
+  pdl_enter();
+  if (*status == 0) return;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    out[i] = c2(nan(""), nan(""));
+}
 
 // One walker's new weight and overlap
 AFQ_D double weight_step(const WeightArgs& g, int w, double pcs) {
@@ -437,11 +456,9 @@ AFQ_D double weight_step(const WeightArgs& g, int w, double pcs) {
 }
 
 // pop_control_ene_shift = e_estimate - 0.1 log(sum w / nw) / dt (propagation.py:161-163)
-// status: the tensor-core pipeline's guard word, folded into scalars[AFQ_S_STATUS] so that callers
-// see a timeout or a bad operand in the state
 AFQ_D void pop_control(const WeightArgs& g, double sum) {
   g.scalars[AFQ_S_POP_CONTROL_SHIFT] = g.scalars[AFQ_S_E_ESTIMATE] - 0.1 * log(sum / (double)g.nw) / g.dt;
-  if (g.status && *g.status != 0) g.scalars[AFQ_S_STATUS] = (double)((int)g.scalars[AFQ_S_STATUS] | *g.status);
+  fold_status(g.scalars, g.status);
 }
 
 __global__ void k_weights(const WeightArgs g) {
@@ -907,8 +924,10 @@ __global__ void k_gather_slab(int slab_elems, const int32_t* __restrict__ idx,
 
 __global__ void k_block_stats(int nw, double dt, const double2* __restrict__ energy,
                               const double* __restrict__ weights, double* __restrict__ scalars,
-                              double* __restrict__ be_out, double* __restrict__ bw_out) {
+                              double* __restrict__ be_out, double* __restrict__ bw_out,
+                              const int* __restrict__ status) {
   pdl_enter();
+  if (threadIdx.x == 0) fold_status(scalars, status);
   __shared__ double red[32];
   const double e_est = scalars[AFQ_S_E_ESTIMATE];
   const double lim = sqrt(2.0 / dt);
@@ -1251,10 +1270,10 @@ int launch_sr(const afq_ctx_dev& c, const double* zeta, double* weights, double*
 }
 
 int launch_block_stats(const afq_ctx_dev& c, const double2* energy, const double* weights,
-                       double* scalars, double* be, double* bw, cudaStream_t st) {
+                       double* scalars, double* be, double* bw, cudaStream_t st, const int* status) {
   {
     ProfScope _ps(K_STATS, st);
-    launch_pdl(k_block_stats, 1, 1024, 0, st, c.nw, c.dt, energy, weights, scalars, be, bw);
+    launch_pdl(k_block_stats, 1, 1024, 0, st, c.nw, c.dt, energy, weights, scalars, be, bw, status);
   }
   return launch_err("block_stats");
 }
@@ -1275,6 +1294,22 @@ int launch_cs_outlier(double* w1, double* w2, const double* e1, const double* e2
     launch_pdl(k_cs_outlier, 1, 1024, 0, st, nw, z_thresh, w1, w2, e1, e2, sums);
   }
   return launch_err("cs_outlier");
+}
+
+int launch_fold_status(double* scalars, const int* status, cudaStream_t st) {
+  {
+    ProfScope _ps(K_STATS, st);
+    launch_pdl(k_fold_status, 1, 1, 0, st, scalars, status);
+  }
+  return launch_err("fold_status");
+}
+
+int launch_poison(long n, double2* out, const int* status, cudaStream_t st) {
+  {
+    ProfScope _ps(K_STATS, st);
+    launch_pdl(k_poison, (unsigned)std::min((n + 255) / 256, 1024l), 256, 0, st, n, out, status);
+  }
+  return launch_err("poison");
 }
 
 int launch_phaseless_begin(double* scalars, cudaStream_t st) {

@@ -106,7 +106,13 @@ enum afq_scalar_index {
   AFQ_S_N_KILLED = 2,          /* prop_data["n_killed_walkers"] */
   AFQ_S_BLOCK_ENERGY = 3,      /* last block's weighted energy */
   AFQ_S_BLOCK_WEIGHT = 4,      /* last block's total weight */
-  AFQ_S_STATUS = 5,            /* device-side guard word (0 = ok) */
+  AFQ_S_STATUS = 5,            /* device-side guard word, 0 = ok. Bits: 1, 2, 4 a wait of a mixed-precision
+                                  tensor-core kernel ran out (4 also: an off-diagonal nonzero under
+                                  mixed_config bit 15), 8 a wait of an FP64 tensor-core contraction
+                                  ran out: the results of the call are then not valid, nor are the
+                                  context's later ones. (CPMC steps: 3 = bad neighbour pair.) Calls
+                                  without a state (afq_calc_force_bias, afq_calc_energy, FP64)
+                                  return NaN instead. */
   AFQ_NSCALARS = 8
 };
 
