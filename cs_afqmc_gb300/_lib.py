@@ -139,6 +139,7 @@ _TEST_SIGS = {
                                            ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                            ctypes.c_int, _vp, _vp]),
     "afq_test_split_pairs": (ctypes.c_int, [ctypes.c_int]),
+    "afq_test_digits_smem_limit": (ctypes.c_long, []),
     "afq_test_preset_status": (ctypes.c_int, [_vp, ctypes.c_int, _vp]),
     "afq_test_gemm_digits_bytes": (ctypes.c_size_t, [ctypes.c_int] * 4),
     "afq_test_gemm_digits": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_int,

@@ -13,6 +13,7 @@
 #include <math.h>
 
 #include "afq_adjoint.cuh"
+#include "afq_launch.cuh"
 #include "afq_common.cuh"
 #include "afq_prof.cuh"
 
@@ -813,7 +814,7 @@ int a_launch_block_stats(const afq_ctx_dev& c, const AdjointBufs& a, int blk, co
 int a_launch_energy(const afq_ctx_dev& c, const AdjointBufs& a, const double2* green, cudaStream_t st) {
   const size_t smem = (2 * (size_t)c.ktot + 2 * (size_t)c.kmax * c.kmax) * sizeof(double2);
   if (int e = a_smem(smem, "energy")) return e;
-  cudaFuncSetAttribute(k_a_energy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_a_energy, smem);
   {
     ProfScope _ps(K_ENERGY, st);
     k_a_energy<<<c.nw, 256, smem, st>>>(c, green, a.ebar, a.gene);
@@ -835,7 +836,7 @@ int a_launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, const d
   const size_t km = c.kmax;
   const size_t smem = (3 * (size_t)c.norb * km + 4 * km * km) * sizeof(double2) + (size_t)c.norb * km * sizeof(double);
   if (int e = a_smem(smem, "Green")) return e;
-  cudaFuncSetAttribute(k_a_green, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_a_green, smem);
   {
     ProfScope _ps(K_GREEN, st);
     double* gu = gt ? gt[0] : nullptr;
@@ -967,7 +968,7 @@ int a_launch_rc_energy(const afq_ctx_dev& c, const AdjointBufs& a, const double2
   }
   const size_t smem = ((size_t)c.ktot + 2 * (size_t)c.kmax * c.kmax) * sizeof(double2);
   if (int e = a_smem(smem, "rot_chol")) return e;
-  cudaFuncSetAttribute(k_a_rc_energy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_a_rc_energy, smem);
   {
     ProfScope _ps(K_ENERGY, st);
     k_a_rc_energy<<<c.nchol, 256, smem, st>>>(c, green, a.ebar, a.grc);
@@ -980,7 +981,7 @@ int a_launch_qr(const afq_ctx_dev& c, const void* wold_u, const void* wold_d, co
   const size_t km = c.kmax;
   const size_t smem = (2 * (size_t)c.norb * km + 3 * km * km) * sizeof(double2);
   if (int e = a_smem(smem, "QR")) return e;
-  cudaFuncSetAttribute(k_a_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_a_qr, smem);
   {
     ProfScope _ps(K_QR, st);
     k_a_qr<<<dim3(c.nw, c.nslab), 256, smem, st>>>(c, (const double2*)wold_u, (const double2*)wold_d,
@@ -1011,7 +1012,7 @@ int a_launch_taylor(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc,
   }
   const size_t smem = 2 * (size_t)n * sizeof(double2);
   if (int e = a_smem(smem, "Taylor")) return e;
-  cudaFuncSetAttribute(k_a_taylor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_a_taylor, smem);
   {
     ProfScope _ps(K_TAYLOR, st);
     k_a_taylor<<<dim3(nwc, c.nslab), 256, smem, st>>>(c, w0, vhs, (const double2*)wu, (const double2*)wd, a.wb[0],
@@ -1030,7 +1031,7 @@ int a_launch_taylor(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc,
 int a_launch_exp_grad(const afq_ctx_dev& c, const AdjointBufs& a, int w0, int nwc, const void* wu, const void* wd,
                       cudaStream_t st) {
   const size_t esmem = 4 * 16 * (size_t)c.kmax * sizeof(double2);
-  cudaFuncSetAttribute(k_a_exp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem);
+  raise_smem_limit((const void*)k_a_exp_grad, esmem);
   const int tiles = (c.norb + 15) / 16;
   {
     ProfScope _ps(K_EXP, st);

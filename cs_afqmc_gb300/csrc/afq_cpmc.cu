@@ -11,6 +11,7 @@
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
+#include "afq_launch.cuh"
 #include "afq_prof.cuh"
 
 namespace afq {
@@ -423,7 +424,7 @@ int launch_cpmc(int norb, int n_up, int n_dn, int nw, double dt, double u, const
   d.gauss = gauss;
   const int kmax = n_up > n_dn ? n_up : n_dn;
   const size_t smem = cpmc_smem(norb, kmax);
-  cudaFuncSetAttribute(k_cpmc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_cpmc, smem);
   {
     ProfScope _ps(K_WEIGHTS, st);
     k_cpmc<<<nw, kCpmcThreads, smem, st>>>(d, mode);

@@ -1014,7 +1014,7 @@ static int launch_digits(int cls, DigGemm g, const typename Epi::Params& ep, int
   const long tiles = (long)g.mt * g.nt * g.nb * g.splits;
   const int sms = dig_sms();
   auto kfn = k_gemm_digits<Epi>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = raise_smem_limit((const void*)kfn, smem);
   if (e != cudaSuccess) {
     afq_set_error("digit GEMM: shared-memory attribute: %s", cudaGetErrorString(e));
     return (int)e;
@@ -1255,6 +1255,16 @@ int dig_launch_energy_adjoint(const afq_ctx_dev& c, const double2* z, const doub
 }
 
 }  // namespace afq
+
+extern "C" long afq_test_digits_smem_limit(void) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, (const void*)afq::k_gemm_digits<afq::EpiDigC>);
+  if (e != cudaSuccess) {
+    afq_set_error("afq_test_digits_smem_limit: %s", cudaGetErrorString(e));
+    return -(long)e;
+  }
+  return a.maxDynamicSharedSizeBytes;
+}
 
 extern "C" size_t afq_test_gemm_digits_bytes(int M, int N, int K, int tr) {
   return afq::dig_bytes(M, K) + afq::dig_bytes(N, K, tr) + afq::dig_exps(M) + afq::dig_exps(N, tr) + 1024;

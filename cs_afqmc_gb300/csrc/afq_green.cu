@@ -510,7 +510,7 @@ static int green_launch(const MixedDev& md, const float2* wu, const float2* wd, 
     return rc;
   auto kfn = k_green_mixed<OM, NT>;
   // a refused attribute surfaces as the launch error checked by the caller
-  cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)kfn, smem);
   launch_pdl(kfn, md.nw, NT, smem, st, md, wu, wd, ovl, flags);
   return 0;
 }

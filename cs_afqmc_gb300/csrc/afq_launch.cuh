@@ -34,4 +34,9 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// A kernel's limit of dynamic shared memory, raised to smem where it is lower. The limit belongs to the function, for
+// all threads of the process: one that set it to its own launch's need could lower it between another thread's
+// setting and launch, which then fails. It is only ever raised.
+cudaError_t raise_smem_limit(const void* kernel, size_t smem);
+
 }  // namespace afq

@@ -268,11 +268,11 @@ int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
   for (int s = 0; s < (both ? 1 : c.nslab); ++s) {
     if (by_warp(s)) {
       const size_t smem = both && warp_smem(1) > warp_smem(0) ? warp_smem(1) : warp_smem(s);
-      cudaFuncSetAttribute(k_qr_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      raise_smem_limit((const void*)k_qr_warp, smem);
       launch_pdl(k_qr_warp, dim3((c.nw + kQrWarps - 1) / kQrWarps, both ? 2 : 1), 32 * kQrWarps, smem, st, c, s, u, d);
     } else {
       const size_t smem = ((size_t)c.norb + 2) * c.kslab[s] * sizeof(float2);
-      cudaFuncSetAttribute(k_qr_householder, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      raise_smem_limit((const void*)k_qr_householder, smem);
       launch_pdl(k_qr_householder, c.nw, 256, smem, st, c, s, u, d);
     }
   }

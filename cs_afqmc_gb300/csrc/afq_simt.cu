@@ -9,6 +9,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "afq_common.cuh"
 #include "afq_kernels.cuh"
@@ -1132,6 +1133,17 @@ int check_smem_optin(size_t smem, const char* what) {
   return 0;
 }
 
+cudaError_t raise_smem_limit(const void* kernel, size_t smem) {
+  static std::mutex m;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= smem) return e;
+  std::lock_guard<std::mutex> lock(m);
+  e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= smem) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
 template <typename WT>
 int launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, double2* green,
                  double2* ovl, bool write_green, cudaStream_t st) {
@@ -1142,7 +1154,7 @@ int launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, double2* 
   const size_t smem = green_f64_smem(c.norb, c.kmax);
   if (int rc = check_smem_optin(smem, "green_overlap (norb x occupied orbitals too large)")) return rc;
   auto kfn = k_green_overlap<WT>;
-  cudaError_t ea = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t ea = raise_smem_limit((const void*)kfn, smem);
   if (ea != cudaSuccess) {
     afq_set_error("green_overlap: shared-memory attribute: %s", cudaGetErrorString(ea));
     return (int)ea;
@@ -1183,7 +1195,7 @@ int launch_taylor_f64(const afq_ctx_dev& c, int w0, int nwc, const double2* vhs,
   }
   size_t smem = 2 * (size_t)c.norb * c.kmax * sizeof(double2);
   auto kfn = k_taylor_f64<WT>;
-  cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)kfn, smem);
   {
     ProfScope _ps(K_TAYLOR, st);
     kfn<<<dim3(nwc, c.nslab), 256, smem, st>>>(c, w0, vhs, (WT*)wu, (WT*)wd);
@@ -1216,7 +1228,7 @@ int launch_weights(const afq_ctx_dev& c, const double2* shift, const double2* fb
 int launch_energy_f64(const afq_ctx_dev& c, int nchunks, int gchunk, const double2* green,
                       double2* epart, double2* energy, cudaStream_t st) {
   size_t smem = (size_t)c.ktot * sizeof(double2) + 2 * (size_t)c.kmax * c.kmax * sizeof(double2);
-  cudaFuncSetAttribute(k_energy_f64_part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_energy_f64_part, smem);
   {
     ProfScope _ps(K_ENERGY, st);
     k_energy_f64_part<<<dim3(c.nw, nchunks), 256, smem, st>>>(c, gchunk, green, epart);
@@ -1234,7 +1246,7 @@ int launch_qr_f64(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st, dou
   size_t smem = 0;
   for (int s = 0; s < c.nslab; ++s)
     smem = std::max(smem, ((size_t)c.norb * (c.kslab[s] | 1) + 2 * c.kslab[s]) * sizeof(double2));
-  cudaFuncSetAttribute(k_qr_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_qr_f64, smem);
   {
     ProfScope _ps(K_QR, st);
     launch_pdl(k_qr_f64, dim3(c.nw, c.nslab), 32 * std::min(8, (c.norb + 31) / 32), smem, st, c, (double2*)wu, (double2*)wd, rdiag);

@@ -700,7 +700,7 @@ int t_launch_green(const afq_ctx_dev& c, const TangentBufs& t, const void* wu, c
   const size_t smem = (2 * (size_t)c.norb * km + 2 * km * km + 2 * km * km) * sizeof(double2) +
                       (size_t)c.norb * km * sizeof(double);
   if (int e = t_smem(smem, "Green")) return e;
-  cudaFuncSetAttribute(k_t_green, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_t_green, smem);
   {
     ProfScope _ps(K_GREEN, st);
     launch_pdl(k_t_green, c.nw, 256, smem, st, c, (const double2*)wu, (const double2*)wd, t.dw[0], t.dw[1], green, dgreen,
@@ -729,7 +729,7 @@ int t_launch_taylor(const afq_ctx_dev& c, const TangentBufs& t, int w0, int nwc,
   }
   const size_t smem = 4 * (size_t)n * sizeof(double2);
   if (int e = t_smem(smem, "Taylor")) return e;
-  cudaFuncSetAttribute(k_t_taylor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_t_taylor, smem);
   {
     ProfScope _ps(K_TAYLOR, st);
     k_t_taylor<<<dim3(nwc, c.nslab), 256, smem, st>>>(c, w0, vhs, dvhs, t.dexp[0], t.dexp[1], (double2*)wu,
@@ -754,7 +754,7 @@ int t_launch_qr(const afq_ctx_dev& c, const TangentBufs& t, const void* wu, cons
   const size_t km = c.kmax;
   const size_t smem = (2 * (size_t)c.norb * km + 2 * km * km) * sizeof(double2);
   if (int e = t_smem(smem, "QR")) return e;
-  cudaFuncSetAttribute(k_t_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_t_qr, smem);
   {
     ProfScope _ps(K_QR, st);
     k_t_qr<<<dim3(c.nw, c.nslab), 256, smem, st>>>(c, t.wold[0], t.wold[1], (const double2*)wu, (const double2*)wd,
@@ -767,7 +767,7 @@ int t_launch_energy(const afq_ctx_dev& c, const TangentBufs& t, int nchunks, int
                     cudaStream_t st) {
   const size_t smem = (2 * (size_t)c.ktot + 4 * (size_t)c.kmax * c.kmax) * sizeof(double2);
   if (int e = t_smem(smem, "energy")) return e;
-  cudaFuncSetAttribute(k_t_energy_part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  raise_smem_limit((const void*)k_t_energy_part, smem);
   {
     ProfScope _ps(K_ENERGY, st);
     k_t_energy_part<<<dim3(c.nw, nchunks), 256, smem, st>>>(c, gchunk, green, t.dgreen, t.dpart, t.drc[0],

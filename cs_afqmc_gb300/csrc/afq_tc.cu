@@ -85,7 +85,7 @@ static int launch_gemm(int cls, const GemmMaps& maps, int nterms, int k_tiles, i
   constexpr int smem = gemm_smem_bytes<BNMAX, STAGES, Epi>();
   static_assert(smem <= 232448, "shared memory");
   auto kfn = k_gemm_tc<BNMAX, STAGES, Epi>;
-  cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  raise_smem_limit((const void*)kfn, smem);
   {
     ProfScope _ps(cls, st);
     launch_pdl(kfn, dim3(n_tiles, m_tiles), kGemmThreads, smem, st,
@@ -111,7 +111,7 @@ static int launch_split(int cls, const SplitMaps& maps, SplitArgs g, int num_sms
   const bool bf16 = ((g.idesc >> 7) & 1u) != 0;
   if (g_split_pairs && g.m_tiles >= 2) {
     auto kfn = k_gemm_split<Epi, 2>;
-    cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+    raise_smem_limit((const void*)kfn, kSplitSmem);
     g.idesc = ptx::idesc_f16(256, kSplitBN, bf16 ? 1 : 0);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
@@ -148,7 +148,7 @@ static int launch_split(int cls, const SplitMaps& maps, SplitArgs g, int num_sms
     return launch_check("gemm_split");
   }
   auto kfn = k_gemm_split<Epi, 1>;
-  cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+  raise_smem_limit((const void*)kfn, kSplitSmem);
   const int grid = ntiles < num_sms ? ntiles : num_sms;
   {
     ProfScope _ps(cls, st);
@@ -1357,7 +1357,7 @@ template <int NP>
 static int launch_prop_fused(const TcState& t, int s, const PropDev& pd, cudaStream_t st) {
   const size_t smem = prop_fused_smem(t.nq, t.NT[s]);
   auto kfn = k_prop_fused<NP>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit((const void*)kfn, smem);
   if (e != cudaSuccess) {
     afq_set_error("prop_fused: shared-memory attribute: %s", cudaGetErrorString(e));
     return (int)e;
@@ -1374,7 +1374,7 @@ template <int NP>
 static int launch_prop_wide(const TcState& t, int s, const PropDev& pd, cudaStream_t st) {
   const size_t smem = prop_wide_smem(t.NT[s]);
   auto kfn = k_prop_wide<NP>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit((const void*)kfn, smem);
   if (e != cudaSuccess) {
     afq_set_error("prop_wide: shared-memory attribute: %s", cudaGetErrorString(e));
     return (int)e;
@@ -1537,7 +1537,7 @@ int tc_propagate_walkers(TcState& t, const afq_ctx_dev& c, void* wu, void* wd, c
       }
       auto kfn = threads <= kTaylorMaxThreads * 3 / 4 ? k_taylor_tc<kTaylorMaxThreads * 3 / 4, kTaylorCW>
                                                       : k_taylor_tc<kTaylorMaxThreads, kTaylorCW>;
-      cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      raise_smem_limit((const void*)kfn, smem);
       {
         ProfScope _ps(K_TAYLOR, st);
         kfn<<<t.nwc < t.num_sms ? t.nwc : t.num_sms, threads, smem, st>>>(t.m_vt[s][0], t.m_vt[s][1], t.m_t0[s][0],

@@ -48,6 +48,10 @@ size_t afq_test_gemm_digits_bytes(int M, int N, int K, int tr);
 int afq_test_gemm_digits(const double* a, const double* b, double* d, int M, int N, int K, int tr,
                          void* scratch, int* status, void* stream);
 
+/* The dynamic shared memory that a launch of the complex FP64 contraction kernel may take at present,
+ * in bytes; negative: a CUDA error. */
+long afq_test_digits_smem_limit(void);
+
 /* Sets the guard word of a context's tensor-core kernels to bits (0..255), as a wait that runs out would:
  * for tests of how it is reported. */
 int afq_test_preset_status(struct afq_ctx* ctx, int bits, void* stream);
