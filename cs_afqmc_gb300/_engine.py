@@ -135,7 +135,11 @@ def _zeros(n, dtype=torch.float64):
 def engine_for(trial, ham_data: Optional[dict], wave_data: dict, walkers, *, dt: float = 1.0,
                n_exp_terms: int = 6, n_batch: int = 1, need_propagation: bool = False,
                mixed_config: int = 0) -> Engine:
-    """Find or build the engine for these walkers (shape, dtype) and intermediates."""
+    """Find or build the engine for these walkers (shape, dtype) and intermediates.
+
+    ham_data["fp64_units"] = True keeps every contraction of FP64 walkers in FP64 sums, for operands
+    graded over many orders of magnitude (localised orbitals, a nearly orthogonal trial); by default they are
+    exact to about 2^-57 of the largest elements of the rows they contract."""
     restricted = not isinstance(walkers, (list, tuple))
     w0 = walkers if restricted else walkers[0]
     nw = int(w0.shape[0])
@@ -143,6 +147,8 @@ def engine_for(trial, ham_data: Optional[dict], wave_data: dict, walkers, *, dt:
     uhf = trial.kind == "uhf"
     if uhf and restricted:
         raise _lib.AfqError("the UHF trial needs unrestricted (two-slab) walkers")
+    if prec == _lib.AFQ_PREC_FP64:  # the accuracy options of the mixed path do not apply
+        mixed_config = _lib.FP64_UNITS if ham_data is not None and ham_data.get("fp64_units") else 0
     store = ham_data if ham_data is not None else wave_data
     cache = store.setdefault(_CACHE_KEY, {})
     mo = wave_data["mo_coeff"]

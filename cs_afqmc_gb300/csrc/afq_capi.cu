@@ -143,6 +143,7 @@ int derive(const afq_dims* d, afq_ctx_dev* c, int* nw_chunk, int* e_chunks, int*
     c->kslab[1] = c->nocc_slab[1] = d->n_dn;
   }
   c->kmax = c->kslab[0] > c->kslab[1] ? c->kslab[0] : c->kslab[1];
+  c->digits = d->precision == AFQ_PREC_FP64 && !(d->mixed_config & AFQ_FP64_UNITS) ? 1 : 0;
   if (d->trial_type == AFQ_TRIAL_RHF) {
     c->nspin_g = 1;
     c->gocc[0] = d->n_up;
@@ -185,7 +186,7 @@ void dig_dims(const afq_ctx_dev& c, int nw_chunk, DigCtx* g) {
   // Z = U G costs 4 (nocc norb)^2 per walker on the tensor cores, about 1/28 of the time of the
   // same flops on the FP64 units, where the sums over f_g cost 4 nchol norb nocc^2: even at
   // norb = 28 nchol, and U takes memory, so a quarter of that.
-  g->has_u = c.norb <= 7 * c.nchol ? 1 : 0;
+  g->has_u = c.digits && c.norb <= 7 * c.nchol ? 1 : 0;
   for (int s = 0; s < 2; ++s) {
     const int on = g->has_u && s < c.nspin_g ? c.gocc[s] * c.norb : 0;
     op(g->u[s], on, on, on ? afq::dig_tr(c.nw, on, 1, kPlanSms) : 16);
@@ -195,7 +196,7 @@ void dig_dims(const afq_ctx_dev& c, int nw_chunk, DigCtx* g) {
     g->uplan[s] = afq::dig_plan(t, g->u[s].kb(), kPlanSms, 4);
   }
   afq::dig_walk_dims(c.norb, c.kslab, c.nslab, nw_chunk, &g->walk);
-  g->use_walk = c.norb <= 256 && (long)nw_chunk * g->walk.ncol * nn >= kWalkMin;
+  g->use_walk = c.digits && c.norb <= 256 && (long)nw_chunk * g->walk.ncol * nn >= kWalkMin;
 }
 
 Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chunks, size_t welem,
@@ -218,7 +219,7 @@ Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chu
   s.free_scr = L->take(4 * nw * C16);
   s.tc = L->take(d->precision == AFQ_PREC_MIXED ? afq::tc_workspace_bytes(c, nw_chunk, d->mixed_config)
                                                 : 256);
-  if (d->precision == AFQ_PREC_FP64) {
+  if (c.digits) {
     DigCtx g;
     dig_dims(c, nw_chunk, &g);
     auto take = [&](size_t (&o)[2], const afq::DigOp& op) {
@@ -265,8 +266,11 @@ inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 bool is_fp64(const afq_ctx* c) { return c->d.precision == AFQ_PREC_FP64; }
 
-// The guard word of the context's tensor-core kernels
+// The guard word of the context's tensor-core kernels (NULL without any)
 const int* status_word(const afq_ctx* c) { return is_fp64(c) ? c->dg.status : c->tc.status; }
+
+// rot_chol with rows g, both spins of a UHF trial together
+const double* rc_all(const afq_ctx* c) { return c->dev.nspin_g == 2 ? c->rccat : c->dev.rot_chol[0]; }
 
 // Green's function + overlap. FP64: G into c->green. Mixed: the 16-bit operands of the
 // force-bias, energy and exp_h1 contractions (wg) and/or the overlap.
@@ -282,9 +286,13 @@ int green(afq_ctx* c, const void* wu, const void* wd, double2* g, double2* ovl, 
   return 0;
 }
 
-// out [nw][nchol] = alpha g . rc^T (FP64), alpha = 2 (RHF, one slab) or 1
-int fb_gemm(afq_ctx* c, const double2* g, const afq::DigOp& rc, double2* out, cudaStream_t st, bool coulomb = false) {
+// out [nw][nchol] = alpha g . rc^T (FP64), alpha = 2 (RHF, one slab) or 1; rc and its digits
+int fb_gemm(afq_ctx* c, const double2* g, const double* rcd, const afq::DigOp& rc, double2* out, cudaStream_t st,
+            bool coulomb = false) {
   const afq_ctx_dev& d = c->dev;
+  if (!d.digits)
+    return afq::launch_gemm_cr(false, d.nw, d.nchol, d.ktot, g, d.ktot, rcd, d.ktot, out, d.nchol,
+                               c2(d.energy_mode == 0 && !coulomb ? 2.0 : 1.0, 0.0), st);
   CHECK(afq::dig_slice_cplx_rows(c->dg.ga, g, d.ktot, 1.0, st));
   return afq::dig_gemm_c(coulomb ? afq::K_ENERGY : afq::K_FB, c->dg.ga, rc, d.nw, d.nchol, out, d.nchol, 0,
                          d.energy_mode == 0 && !coulomb ? 1 : 0, c->dg.fb, c->dg.part, c->dg.status, st);
@@ -293,7 +301,7 @@ int fb_gemm(afq_ctx* c, const double2* g, const afq::DigOp& rc, double2* out, cu
 // The local energy's contractions of c->green: c->fb = Coulomb sums, dg.z = U G (FP64)
 int energy_gemms(afq_ctx* c, cudaStream_t st) {
   const afq_ctx_dev& d = c->dev;
-  CHECK(fb_gemm(c, c->green, c->dg.rc, c->fb, st, true));
+  CHECK(fb_gemm(c, c->green, rc_all(c), c->dg.rc, c->fb, st, true));
   for (int s = 0, off = 0; s < d.nspin_g; ++s) {
     afq::DigOp a = c->dg.ga;
     a.K = c->dg.u[s].K;
@@ -309,6 +317,8 @@ int energy_gemms(afq_ctx* c, cudaStream_t st) {
 int vhs_gemm(afq_ctx* c, const double2* x, int nwc, double2* vhs, cudaStream_t st) {
   const afq_ctx_dev& d = c->dev;
   const int nn = d.norb * d.norb;
+  if (!d.digits)
+    return afq::launch_gemm_cr(true, nwc, nn, d.nchol, x, d.nchol, c->h.chol, nn, vhs, nn, c2(0.0, sqrt(d.dt)), st);
   afq::DigOp a = c->dg.xa;
   a.rows = 2 * nwc;
   CHECK(afq::dig_slice_cplx_rows(a, x, d.nchol, sqrt(d.dt), st));
@@ -318,7 +328,7 @@ int vhs_gemm(afq_ctx* c, const double2* x, int nwc, double2* vhs, cudaStream_t s
 
 int force_bias_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
   if (!is_fp64(c)) return afq::tc_force_bias(c->tc, c->dev, out, st);
-  return fb_gemm(c, c->green, c->dg.rc, out, st);
+  return fb_gemm(c, c->green, rc_all(c), c->dg.rc, out, st);
 }
 
 int energy_from_green(afq_ctx* c, double2* out, cudaStream_t st) {
@@ -566,8 +576,10 @@ TSizes tangent_sizes(const afq_ctx_dev& c, int nw_chunk, int e_chunks, Layout* L
   s.drccat = L->take(c.nspin_g == 2 ? (size_t)c.nchol * c.ktot * sizeof(double) : 256);
   DigCtx g;
   dig_dims(c, nw_chunk, &g);
-  s.drc_d = L->take(afq::dig_bytes(g.rc.rows, g.rc.K, g.rc.tr));
-  s.drc_e = L->take(afq::dig_exps(g.rc.rows, g.rc.tr));
+  if (c.digits) {
+    s.drc_d = L->take(afq::dig_bytes(g.rc.rows, g.rc.K, g.rc.tr));
+    s.drc_e = L->take(afq::dig_exps(g.rc.rows, g.rc.tr));
+  }
   s.wk = L->off;
   if (g.use_walk) {
     for (int i = 0; i < g.walk.n_e(c.nslab); ++i) {
@@ -597,9 +609,9 @@ int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, co
                   const JvpWalk& jw, const double* fields, cudaStream_t st, bool next_g) {
   const afq_ctx_dev& d = c->dev;
   CHECK(force_bias_from_green(c, c->fb, st));
-  CHECK(fb_gemm(c, t.dgreen, c->dg.rc, t.dfb, st));
+  CHECK(fb_gemm(c, t.dgreen, rc_all(c), c->dg.rc, t.dfb, st));
   if (t.drccat) {  // orbital rotation: + alpha G dRC^T (t.dxt as scratch, rewritten below)
-    CHECK(fb_gemm(c, c->green, drc, t.dxt, st));
+    CHECK(fb_gemm(c, c->green, t.drccat, drc, t.dxt, st));
     CHECK(afq::t_launch_add((long)d.nw * d.nchol, t.dxt, t.dfb, st));
   }
   CHECK(afq::t_launch_field_shifts(d, fields, c->fb, t.dfb, c->xt, t.dxt, c->shift, t.dshift, c->fbt, t.dfbt, st));
@@ -698,8 +710,12 @@ AdjSizes adjoint_sizes(const afq_ctx_dev& c, int nw_chunk, int n_prop, int n_ene
   s.scal = L->take(8 * sizeof(double));
   s.beb = L->take((size_t)s.nblk * sizeof(double));
   s.bwb = L->take((size_t)s.nblk * sizeof(double));
+  s.dg = s.dg_end = s.part = L->off;
+  if (!c.digits) {
+    s.total = L->off;
+    return s;
+  }
   const AdjOps o = adj_ops(c, nw_chunk);
-  s.dg = L->off;
   s.cn_d = L->take(afq::dig_bytes(o.cn.rows, o.cn.K, o.cn.tr));
   s.cn_e = L->take(afq::dig_exps(o.cn.rows, o.cn.tr));
   s.rt_d = L->take(afq::dig_bytes(o.rt.rows, o.rt.K, o.rt.tr));
@@ -836,7 +852,7 @@ extern "C" {
 int afq_abi_version(void) { return AFQ_ABI_VERSION; }
 
 int afq_test_preset_status(afq_ctx* ctx, int bits, void* stream) {
-  if (!ctx || bits < 0 || bits > 255) { afq_set_error("bad argument"); return -1; }
+  if (!ctx || bits < 0 || bits > 255 || !status_word(ctx)) { afq_set_error("bad argument"); return -1; }
   // the word's low byte (little endian); the rest stays zero
   const cudaError_t e = cudaMemsetAsync(const_cast<int*>(status_word(ctx)), bits, 1, S(stream));
   if (e != cudaSuccess) { afq_set_error("preset status: %s", cudaGetErrorString(e)); return (int)e; }
@@ -932,8 +948,8 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
       return (int)e;
     }
   }
-  if (dims->precision == AFQ_PREC_FP64) {
-    dig_dims(c->dev, nwc, &c->dg);
+  if (dims->precision == AFQ_PREC_FP64) dig_dims(c->dev, nwc, &c->dg);
+  if (dev.digits) {
     auto at = [&](afq::DigOp& o, const size_t (&off)[2]) {
       o.d = reinterpret_cast<unsigned char*>(ws + off[0]);
       o.e = reinterpret_cast<int*>(ws + off[1]);
@@ -1001,7 +1017,7 @@ int afq_calc_force_bias(afq_ctx* ctx, const void* walkers_up, const void* walker
   CHECK(check_walkers(ctx, walkers_up, walkers_dn));
   CHECK(green(ctx, walkers_up, walkers_dn, ctx->green, nullptr, true, S(stream)));
   CHECK(force_bias_from_green(ctx, reinterpret_cast<double2*>(force_bias), S(stream)));
-  if (!is_fp64(ctx)) return 0;
+  if (!ctx->dev.digits) return 0;
   return afq::launch_poison((long)ctx->dev.nw * ctx->dev.nchol, reinterpret_cast<double2*>(force_bias),
                             ctx->dg.status, S(stream));
 }
@@ -1197,7 +1213,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
   afq::DigOp drc = ctx->dg.rc;
   drc.d = reinterpret_cast<unsigned char*>(tw + ts.drc_d);
   drc.e = reinterpret_cast<int*>(tw + ts.drc_e);
-  if (t.drccat) CHECK(afq::dig_slice_real_rows(drc, t.drccat, d.ktot, st));
+  if (t.drccat && d.digits) CHECK(afq::dig_slice_real_rows(drc, t.drccat, d.ktot, st));
   JvpWalk jw{ctx->dg.walk, nullptr, nullptr};
   if (ctx->dg.use_walk) {  // (the workspace was cleared above: padding is zero)
     jw.w.vd = reinterpret_cast<unsigned char*>(tw + ts.v[0]);
@@ -1233,7 +1249,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
       CHECK(afq::t_launch_green(d, t, state->walkers_up, state->walkers_dn, ctx->green, t.dgreen, ovl, t.dlo, st));
       CHECK(energy_from_green(ctx, ctx->ene, st));
       if (ctx->dg.has_u && !rot) {  // ctx->fb and dg.z are those of the energy just evaluated
-        CHECK(fb_gemm(ctx, t.dgreen, ctx->dg.rc, t.dfb, st, true));
+        CHECK(fb_gemm(ctx, t.dgreen, rc_all(ctx), ctx->dg.rc, t.dfb, st, true));
         CHECK(afq::dig_launch_energy_tangent(d, ctx->green, t.dgreen, ctx->dg.z, ctx->fb, t.dfb, t.drot[0], t.drot[1],
                                              t.dene, st));
       } else {
@@ -1423,7 +1439,7 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
   CHECK(afq::a_launch_end(blk, block_energy, block_weight, a, st));
   const int nwc = ctx->nw_chunk, nb = d.nw / nwc;
   const long nn = (long)d.norb * d.norb;
-  const double* brc = d.nspin_g == 2 ? ctx->rccat : d.rot_chol[0];
+  const double* brc = rc_all(ctx);
   AdjOps ao = adj_ops(d, nwc);
   ao.cn.d = reinterpret_cast<unsigned char*>(base + as.cn_d);
   ao.cn.e = reinterpret_cast<int*>(base + as.cn_e);
@@ -1431,9 +1447,11 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
   ao.rt.e = reinterpret_cast<int*>(base + as.rt_e);
   ao.va.d = reinterpret_cast<unsigned char*>(base + as.va_d);
   ao.va.e = reinterpret_cast<int*>(base + as.va_e);
-  CHECK(zero(base + as.dg, as.dg_end - as.dg, st));
-  CHECK(afq::dig_slice_real_rows(ao.cn, ctx->h.chol, nn, st));
-  CHECK(afq::dig_slice_real_cols(ao.rt, brc, d.ktot, st));
+  if (d.digits) {
+    CHECK(zero(base + as.dg, as.dg_end - as.dg, st));
+    CHECK(afq::dig_slice_real_rows(ao.cn, ctx->h.chol, nn, st));
+    CHECK(afq::dig_slice_real_cols(ao.rt, brc, d.ktot, st));
+  }
   const bool walk = adj_walk(d, ctx->dg);
   afq::DigOp et[2] = {ctx->dg.walk.e[0], ctx->dg.walk.e[1]};
   afq::DigVbar vb;
@@ -1498,18 +1516,29 @@ int afq_propagate_phaseless_vjp_ex(afq_ctx* ctx, afq_walker_state* state, void* 
         else
           CHECK(afq::a_launch_taylor(d, a, w0, nwc, ctx->vhs, tp.w(start, 0), tp.w(start, 1), st));
         if (cg) CHECK(afq::a_launch_chol_grad(d, a, nwc, tp.xt(step) + (size_t)w0 * d.nchol, st));
-        CHECK(afq::dig_slice_cplx_rows(ao.va, a.vbar, nn, sqrt(d.dt), st));
-        CHECK(afq::dig_gemm_c(afq::K_FB, ao.va, ao.cn, nwc, d.nchol, a.xtb + (size_t)w0 * d.nchol, d.nchol, 3, 0,
-                              ao.xtb, reinterpret_cast<double2*>(base + as.part), ctx->dg.status, st));
+        double2* xtb = a.xtb + (size_t)w0 * d.nchol;
+        if (d.digits) {
+          CHECK(afq::dig_slice_cplx_rows(ao.va, a.vbar, nn, sqrt(d.dt), st));
+          CHECK(afq::dig_gemm_c(afq::K_FB, ao.va, ao.cn, nwc, d.nchol, xtb, d.nchol, 3, 0, ao.xtb,
+                                reinterpret_cast<double2*>(base + as.part), ctx->dg.status, st));
+        } else {
+          CHECK(afq::launch_gemm_cr(false, nwc, d.nchol, (int)nn, a.vbar, nn, ctx->h.chol, nn, xtb, d.nchol,
+                                    c2(0.0, -sqrt(d.dt)), st));
+        }
       }
       CHECK(afq::a_launch_field(d, a, tp.xt(step), st));
       if (rot) {  // fb = alpha rot_chol G(W_start): rot_chol-bar += alpha Re(fb-bar^H G)
         CHECK(afq::launch_green<double>(d, tp.w(start, 0), tp.w(start, 1), ctx->green, nullptr, true, st));
         CHECK(afq::a_launch_rc_fb(d, a, ctx->green, alpha, st));
       }
-      CHECK(afq::dig_slice_cplx_rows(ctx->dg.xa, a.fbb, d.nchol, 1.0, st));
-      CHECK(afq::dig_gemm_c(afq::K_VHS, ctx->dg.xa, ao.rt, d.nw, d.ktot, a.gpend, d.ktot, 0,
-                            d.energy_mode == 0 ? 1 : 0, afq::DigPlan{1, ctx->dg.xa.kb()}, nullptr, ctx->dg.status, st));
+      if (d.digits) {
+        CHECK(afq::dig_slice_cplx_rows(ctx->dg.xa, a.fbb, d.nchol, 1.0, st));
+        CHECK(afq::dig_gemm_c(afq::K_VHS, ctx->dg.xa, ao.rt, d.nw, d.ktot, a.gpend, d.ktot, 0,
+                              d.energy_mode == 0 ? 1 : 0, afq::DigPlan{1, ctx->dg.xa.kb()}, nullptr, ctx->dg.status, st));
+      } else {
+        CHECK(afq::launch_gemm_cr(true, d.nw, d.ktot, d.nchol, a.fbb, d.nchol, brc, d.ktot, a.gpend, d.ktot,
+                                  c2(alpha, 0.0), st));
+      }
       gp = true;
       swap_slabs(a.wb, a.wb2);
       double2* t = a.lbar;

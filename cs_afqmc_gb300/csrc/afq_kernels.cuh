@@ -14,6 +14,7 @@ struct afq_ctx_dev {
   int gocc[2];
   int ktot;          // (gocc0 + (nspin_g==2 ? gocc1 : 0)) * norb
   int energy_mode;   // 0 RHF restricted, 1 RHF two-slab, 2 UHF
+  int digits;        // FP64: contractions as digit products on the tensor cores (else the FP64 units)
   double h0, h0_prop_re, h0_prop_im;
   const double* trial[2];     // [norb, nocc_s]
   const double* exp_h1[2];    // [norb, norb] per slab
@@ -36,7 +37,7 @@ int launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, double2* 
 // the same for up to 32 electrons per spin, FP64 walkers (afq_green64.cu); errors by cudaGetLastError
 int launch_green_f64(const afq_ctx_dev& c, const void* wu, const void* wd, double2* green, double2* ovl,
                      bool write_green, cudaStream_t st);
-int launch_gemm_cr(int M, int N, int K, const double2* A, long lda, const double* B,
+int launch_gemm_cr(bool b_kn, int M, int N, int K, const double2* A, long lda, const double* B,
                    long ldb, double2* C, long ldc, double2 alpha, cudaStream_t st);
 int launch_field_shifts(const afq_ctx_dev& c, const double* fields, const double2* fb,
                         double2* xt, double2* shift, double2* fbt, cudaStream_t st);

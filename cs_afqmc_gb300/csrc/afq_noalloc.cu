@@ -128,6 +128,6 @@ extern "C" int afq_calc_force_bias_noalloc(int32_t norb, int32_t nocc, int32_t n
   double2* green = static_cast<double2*>(scratch);  // every element is overwritten below
   rc = afq::launch_green<double>(c, walkers, nullptr, green, nullptr, true, st);
   if (rc) return rc;
-  return afq::launch_gemm_cr(n_walkers, nchol, c.ktot, green, c.ktot, rot_chol, c.ktot,
+  return afq::launch_gemm_cr(false, n_walkers, nchol, c.ktot, green, c.ktot, rot_chol, c.ktot,
                              reinterpret_cast<double2*>(force_bias), nchol, c2(2.0, 0.0), st);
 }

@@ -135,10 +135,13 @@ __global__ void k_green_overlap(const afq_ctx_dev c, const WT* __restrict__ w_up
 }
 
 // ======================================================================================
-// Complex x real GEMM, FP64, on the FP64 units: C[m][n] = alpha * sum_k A[m][k] * B[n][k].
-// For the entry points without a workspace; contexts use the digit GEMM (afq_digits.cuh).
+// Complex x real GEMM, FP64, on the FP64 units: C[m][n] = alpha * sum_k A[m][k] * B(k, n)
+// B_KN: B(k,n) = B[k*ldb + n]; otherwise B(k,n) = B[n*ldb + k].
+// For the entry points without a workspace and contexts that ask for the FP64 units; the others use the
+// digit GEMM (afq_digits.cuh).
 // ======================================================================================
 
+template <bool B_KN>
 __global__ void __launch_bounds__(256) k_gemm_cr(int M, int N, int K, const double2* __restrict__ A,
                                                  long lda, const double* __restrict__ B, long ldb,
                                                  double2* __restrict__ C, long ldc, double2 alpha) {
@@ -159,9 +162,15 @@ __global__ void __launch_bounds__(256) k_gemm_cr(int M, int N, int K, const doub
       int r = e >> 4, cc = e & 15;  // A: row r of 64, col cc of 16
       int gm = m0 + r, gk = k0 + cc;
       As[cc][r] = (gm < M && gk < K) ? A[(long)gm * lda + gk] : c2(0, 0);
-      int bc = e >> 4, br = e & 15;  // n col bc of 64, k row br of 16
-      int bk = k0 + br, bn = n0 + bc;
-      Bs[br][bc] = (bk < K && bn < N) ? B[(long)bn * ldb + bk] : 0.0;
+      if (B_KN) {
+        int br = e >> 6, bc = e & 63;  // k row br of 16, n col bc of 64
+        int bk = k0 + br, bn = n0 + bc;
+        Bs[br][bc] = (bk < K && bn < N) ? B[(long)bk * ldb + bn] : 0.0;
+      } else {
+        int bc = e >> 4, br = e & 15;  // n col bc of 64, k row br of 16
+        int bk = k0 + br, bn = n0 + bc;
+        Bs[br][bc] = (bk < K && bn < N) ? B[(long)bn * ldb + bk] : 0.0;
+      }
     }
     __syncthreads();
 #pragma unroll
@@ -1166,11 +1175,14 @@ int launch_green(const afq_ctx_dev& c, const void* wu, const void* wd, double2* 
   return launch_err("green_overlap");
 }
 
-int launch_gemm_cr(int M, int N, int K, const double2* A, long lda, const double* B,
+int launch_gemm_cr(bool b_kn, int M, int N, int K, const double2* A, long lda, const double* B,
                    long ldb, double2* C, long ldc, double2 alpha, cudaStream_t st) {
   dim3 grid((N + 63) / 64, (M + 63) / 64);
-  ProfScope _ps(K_FB, st);
-  k_gemm_cr<<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, alpha);
+  ProfScope _ps(b_kn ? K_VHS : K_FB, st);
+  if (b_kn)
+    k_gemm_cr<true><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, alpha);
+  else
+    k_gemm_cr<false><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, alpha);
   return launch_err("gemm_cr");
 }
 

@@ -35,10 +35,22 @@ extern "C" {
 
 #define AFQ_ABI_VERSION 1
 
+/* afq_dims.mixed_config of an AFQ_PREC_FP64 context: every contraction as sums on the FP64 units (5 to 17 times
+ * the time of a block, and a small part of the workspace); other bits are ignored there. */
+#define AFQ_FP64_UNITS (1 << 24)
+
 enum afq_walker_type { AFQ_WALKERS_RESTRICTED = 0, AFQ_WALKERS_UNRESTRICTED = 1 };
 enum afq_trial_type { AFQ_TRIAL_RHF = 0, AFQ_TRIAL_UHF = 1 };
 enum afq_precision {
-  AFQ_PREC_FP64 = 0,  /* every contraction in FP64 (the reference's arithmetic) */
+  AFQ_PREC_FP64 = 0,  /* FP64 data, sums and results. The large contractions (force bias, vhs, exchange and
+                         Coulomb sums, exp_h1 and Taylor products of large populations, their tangents and
+                         adjoints) hold every operand row as 56-bit integers relative to the row's
+                         largest element: the error of a dot product of K terms is a rounding of the result
+                         plus about sqrt(K) 2^-57 max|a| max|b|, for rows of similar elements below that of an
+                         FP64 sum, but relative to the largest elements, not to the terms: an element 2^-20 of
+                         its row's largest keeps 36 bits. For operands graded against each other over many
+                         orders of magnitude AFQ_FP64_UNITS keeps every contraction in FP64
+                         sums (the reference's arithmetic). */
   AFQ_PREC_MIXED = 1  /* BF16 tensor-core contractions with split-BF16 correction, FP32
                          walkers, FP64 determinants / weights / energy accumulation */
 };
@@ -57,7 +69,8 @@ typedef struct afq_dims {
   int32_t precision;    /* afq_precision */
   int32_t n_exp_terms;  /* Taylor terms of exp(vhs), reference default 6 */
   int32_t n_batch;      /* walker chunks for the vhs workspace (>= 1, divides n_walkers) */
-  int32_t mixed_config; /* AFQ_PREC_MIXED accuracy options; 0 = library default (767).
+  int32_t mixed_config; /* AFQ_PREC_FP64: 0 or AFQ_FP64_UNITS.
+                           AFQ_PREC_MIXED accuracy options; 0 = library default (767).
                            bits 0..7: lo (correction) terms of G / rot_chol (force bias),
                            fields / chol (vhs), walker / exp_h1 (exp_h1 products), G /
                            rot_chol (energy); bits 8..10: Taylor products with split
