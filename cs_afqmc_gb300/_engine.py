@@ -148,7 +148,9 @@ def engine_for(trial, ham_data: Optional[dict], wave_data: dict, walkers, *, dt:
     if uhf and restricted:
         raise _lib.AfqError("the UHF trial needs unrestricted (two-slab) walkers")
     if prec == _lib.AFQ_PREC_FP64:  # the accuracy options of the mixed path do not apply
-        mixed_config = _lib.FP64_UNITS if ham_data is not None and ham_data.get("fp64_units") else 0
+        # measurements have an engine of their own, which leaves out what the propagation needs
+        mixed_config = (_lib.FP64_UNITS if ham_data is not None and ham_data.get("fp64_units") else
+                        0 if need_propagation else _lib.FP64_MEASURE)
     store = ham_data if ham_data is not None else wave_data
     cache = store.setdefault(_CACHE_KEY, {})
     mo = wave_data["mo_coeff"]

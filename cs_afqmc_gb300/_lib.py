@@ -26,6 +26,7 @@ MIXED_DIAG_CHOL = 1 << 15    # every Cholesky vector diagonal: per-row exp(vhs),
 MIXED_EXPLICIT = 1 << 30     # the caller's configuration as given (no automatic diagonal path)
 MIXED_LEGACY_TAYLOR = 1 << 16  # separate exp_h1 GEMMs and Taylor kernel instead of the fused kernel
 FP64_UNITS = 1 << 24         # FP64 contexts: contractions as sums on the FP64 units
+FP64_MEASURE = 1 << 25       # FP64 contexts: overlaps, force biases and energies only
 MIXED_SYM_CHOL = 1 << 17     # every Cholesky vector symmetric: packed vhs GEMM, V mirrored on load
 
 _vp = ctypes.c_void_p

@@ -36,7 +36,8 @@ struct DigCtx {
   afq::DigPlan fb;  // K ranges of the force bias
   // exchange energy: U per spin of G (rows (i, q), K = (k, p)); has_u 0: too few vectors for it
   int has_u;
-  afq::DigOp u[2], ua[2], ub[2];  // ua, ub: rot_chol^T, at set-up only
+  afq::DigOp u[2], ua[2], ub[2];  // ua, ub: rot_chol^T, at set-up only; ua for u_strip of the i at a time
+  int u_strip;
   afq::DigPlan uplan[2];
   double2* z;     // [nw][ktot]
   double2* part;  // partial results of split K ranges
@@ -89,10 +90,10 @@ struct Layout {
 };
 
 struct Sizes {
-  // digits: [tiles, row exponents]
-  size_t dg, dg_chol[2], dg_rc[2], dg_xa[2], dg_ga[2], dg_u[2][2], dg_ua[2], dg_ub[2], dg_uend, dg_end, dg_status;
-  size_t dg_part, dg_z, dg_utmp;
-  size_t dg_e[2][2], dg_v[2], dg_x[2], dg_wt, dg_wa;
+  // digits: [tiles, row exponents]; dg .. dg_end the operands sliced once, dgw .. dgw_end the walkers'
+  size_t dg, dg_chol[2], dg_rc[2], dg_u[2][2], dg_e[2][2], dg_status, dg_end;
+  size_t dgw, dg_xa[2], dg_ga[2], dg_v[2], dg_x[2], dgw_end, dg_part, dg_z, dg_wt, dg_wa;
+  size_t dg_ua[2], dg_ub[2], dg_utmp;  // set-up of U, in the place of the walkers' scratch
   size_t green, fb, xt, shift, fbt, vhs, ovl_new, ene, epart, rccat, wcopy, sr_idx, cum, free_scr, tc, total;
 };
 
@@ -144,6 +145,7 @@ int derive(const afq_dims* d, afq_ctx_dev* c, int* nw_chunk, int* e_chunks, int*
   }
   c->kmax = c->kslab[0] > c->kslab[1] ? c->kslab[0] : c->kslab[1];
   c->digits = d->precision == AFQ_PREC_FP64 && !(d->mixed_config & AFQ_FP64_UNITS) ? 1 : 0;
+  c->measure = c->digits && (d->mixed_config & AFQ_FP64_MEASURE) ? 1 : 0;
   if (d->trial_type == AFQ_TRIAL_RHF) {
     c->nspin_g = 1;
     c->gocc[0] = d->n_up;
@@ -170,6 +172,8 @@ int derive(const afq_dims* d, afq_ctx_dev* c, int* nw_chunk, int* e_chunks, int*
 // that workspace sizes do not depend on where they are asked for.
 constexpr int kPlanSms = 152;
 constexpr long kWalkMin = 1000000;
+constexpr int kUWalkers = 4;
+constexpr size_t kUBytes = (size_t)32 << 20;
 void dig_dims(const afq_ctx_dev& c, int nw_chunk, DigCtx* g) {
   const int nn = c.norb * c.norb;
   auto op = [](afq::DigOp& o, int rows, int K, int tr) {
@@ -185,72 +189,90 @@ void dig_dims(const afq_ctx_dev& c, int nw_chunk, DigCtx* g) {
   g->fb = afq::dig_plan(tiles, g->rc.kb(), kPlanSms, 8);
   // Z = U G costs 4 (nocc norb)^2 per walker on the tensor cores, about 1/28 of the time of the
   // same flops on the FP64 units, where the sums over f_g cost 4 nchol norb nocc^2: even at
-  // norb = 28 nchol, and U takes memory, so a quarter of that.
-  g->has_u = c.digits && c.norb <= 7 * c.nchol ? 1 : 0;
+  // norb = 28 nchol, and U takes memory, so a quarter of that. U has 16 (nocc norb)^2 bytes whatever the
+  // population: above kUBytes it takes kUWalkers. An energy with it and without, 198 orbitals and 33 electrons
+  // (683 MB, 2.7 ms to form): 1 or 2 walkers 1.29 / 2.75 ms, 4 walkers 1.29 / 4.73, 64 walkers 1.3 / 54; 120 and 20
+  // (92 MB): 1 to 4 walkers 0.34 / 0.75 ms; 40 and 7 (1.3 MB): 0.07 / 0.17.
+  size_t u_bytes = 0;
+  for (int s = 0; s < c.nspin_g; ++s) u_bytes += afq::dig_bytes((long)c.gocc[s] * c.norb, (long)c.gocc[s] * c.norb, 64);
+  g->has_u = c.digits && c.norb <= 7 * c.nchol && (c.nw >= kUWalkers || u_bytes <= kUBytes) ? 1 : 0;
+  // U is formed by strips of about 1024 rows: their FP64 values would otherwise take half of what U does
+  g->u_strip = std::max(1, 1024 / c.norb);
   for (int s = 0; s < 2; ++s) {
     const int on = g->has_u && s < c.nspin_g ? c.gocc[s] * c.norb : 0;
     op(g->u[s], on, on, on ? afq::dig_tr(c.nw, on, 1, kPlanSms) : 16);
-    op(g->ua[s], on, c.nchol, afq::kDigTile);
+    op(g->ua[s], std::min(on, g->u_strip * c.norb), c.nchol, afq::kDigTile);
     op(g->ub[s], on, c.nchol, 64);
     const int t = ((2 * c.nw + afq::kDigTile - 1) / afq::kDigTile) * ((on + g->u[s].tr - 1) / g->u[s].tr);
     g->uplan[s] = afq::dig_plan(t, g->u[s].kb(), kPlanSms, 4);
   }
   afq::dig_walk_dims(c.norb, c.kslab, c.nslab, nw_chunk, &g->walk);
-  g->use_walk = c.digits && c.norb <= 256 && (long)nw_chunk * g->walk.ncol * nn >= kWalkMin;
+  g->use_walk = c.digits && !c.measure && c.norb <= 256 && (long)nw_chunk * g->walk.ncol * nn >= kWalkMin;
 }
 
 Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chunks, size_t welem,
                 Layout* L) {
   Sizes s;
   const size_t nw = c.nw, C16 = sizeof(double2);
+  s.rccat = L->take(c.nspin_g == 2 ? (size_t)c.nchol * c.ktot * sizeof(double) : 256);
+  s.tc = L->take(d->precision == AFQ_PREC_MIXED ? afq::tc_workspace_bytes(c, nw_chunk, d->mixed_config)
+                                                : 256);
+  DigCtx g;
+  if (c.digits) dig_dims(c, nw_chunk, &g);
+  auto take = [&](size_t (&o)[2], const afq::DigOp& op) {
+    o[0] = L->take(afq::dig_bytes(op.rows, op.K, op.tr));
+    o[1] = L->take(afq::dig_exps(op.rows, op.tr));
+  };
+  if (c.digits) {
+    s.dg = L->off;
+    if (!c.measure) take(s.dg_chol, g.chol);
+    take(s.dg_rc, g.rc);
+    for (int i = 0; i < 2; ++i) take(s.dg_u[i], g.u[i]);
+    for (int i = 0; g.use_walk && i < g.walk.n_e(c.nslab); ++i) take(s.dg_e[i], g.walk.e[i]);
+    s.dg_status = L->take(256);
+    s.dg_end = L->off;
+  }
+  const size_t scratch = L->off;
   s.green = L->take(nw * c.ktot * C16);
   s.fb = L->take(nw * c.nchol * C16);
   s.xt = L->take(nw * c.nchol * C16);
   s.shift = L->take(nw * C16);
   s.fbt = L->take(nw * C16);
-  s.vhs = L->take(d->precision == AFQ_PREC_FP64 ? (size_t)nw_chunk * c.norb * c.norb * C16 : 256);
+  s.vhs = L->take(d->precision == AFQ_PREC_FP64 && !c.measure ? (size_t)nw_chunk * c.norb * c.norb * C16 : 256);
   s.ovl_new = L->take(nw * C16);
   s.ene = L->take(nw * C16);
   s.epart = L->take(nw * e_chunks * 5 * C16);
-  s.rccat = L->take(c.nspin_g == 2 ? (size_t)c.nchol * c.ktot * sizeof(double) : 256);
-  s.wcopy = L->take(nw * c.norb * (c.kslab[0] + c.kslab[1]) * welem);
+  s.wcopy = L->take(c.measure ? 256 : nw * c.norb * (c.kslab[0] + c.kslab[1]) * welem);
   s.sr_idx = L->take(nw * sizeof(int32_t));
   s.cum = L->take(nw * sizeof(double));
   s.free_scr = L->take(4 * nw * C16);
-  s.tc = L->take(d->precision == AFQ_PREC_MIXED ? afq::tc_workspace_bytes(c, nw_chunk, d->mixed_config)
-                                                : 256);
   if (c.digits) {
-    DigCtx g;
-    dig_dims(c, nw_chunk, &g);
-    auto take = [&](size_t (&o)[2], const afq::DigOp& op) {
-      o[0] = L->take(afq::dig_bytes(op.rows, op.K, op.tr));
-      o[1] = L->take(afq::dig_exps(op.rows, op.tr));
-    };
-    s.dg = L->off;
-    take(s.dg_chol, g.chol);
-    take(s.dg_rc, g.rc);
-    take(s.dg_xa, g.xa);
+    s.dgw = L->off;
+    if (!c.measure) take(s.dg_xa, g.xa);
     take(s.dg_ga, g.ga);
-    for (int i = 0; i < 2; ++i) take(s.dg_u[i], g.u[i]);
-    const int big = g.ua[1].rows > g.ua[0].rows ? 1 : 0;
-    take(s.dg_ua, g.ua[big]);
-    take(s.dg_ub, g.ub[big]);
-    s.dg_uend = L->off;
-    for (int i = 0; i < g.walk.n_e(c.nslab); ++i) take(s.dg_e[i], g.walk.e[i]);
-    s.dg_v[0] = L->take(g.use_walk ? afq::dig_walk_v_bytes(g.walk) : 256);
-    s.dg_v[1] = L->take(g.use_walk ? afq::dig_walk_ve_bytes(g.walk) : 256);
-    s.dg_x[0] = L->take(g.use_walk ? afq::dig_walk_x_bytes(g.walk) : 256);
-    s.dg_x[1] = L->take(g.use_walk ? afq::dig_walk_xe_bytes(g.walk) : 256);
-    s.dg_status = L->take(256);
-    s.dg_end = L->off;
-    const size_t wt = g.use_walk ? (size_t)g.walk.chunk * c.norb * g.walk.ncol * C16 : 256;
-    s.dg_wt = L->take(wt);
-    s.dg_wa = L->take(wt);
+    if (g.use_walk) {
+      s.dg_v[0] = L->take(afq::dig_walk_v_bytes(g.walk));
+      s.dg_v[1] = L->take(afq::dig_walk_ve_bytes(g.walk));
+      s.dg_x[0] = L->take(afq::dig_walk_x_bytes(g.walk));
+      s.dg_x[1] = L->take(afq::dig_walk_xe_bytes(g.walk));
+    }
+    s.dgw_end = L->off;
+    if (g.use_walk) {
+      const size_t wt = (size_t)g.walk.chunk * c.norb * g.walk.ncol * C16;
+      s.dg_wt = L->take(wt);
+      s.dg_wa = L->take(wt);
+    }
     size_t part = afq::dig_partial_bytes(c.nw, c.nchol, g.fb.splits);
     for (int i = 0; i < 2; ++i) part = std::max(part, afq::dig_partial_bytes(c.nw, g.u[i].rows, g.uplan[i].splits));
     s.dg_part = L->take(part);
     s.dg_z = L->take(g.has_u ? nw * c.ktot * C16 : 256);
-    s.dg_utmp = L->take(g.has_u ? (size_t)g.ua[big].rows * g.ua[big].rows * sizeof(double) : 256);
+    const size_t end = L->off;
+    L->off = scratch;  // used before the walkers' scratch is
+    const int big = g.ub[1].rows > g.ub[0].rows ? 1 : 0;
+    take(s.dg_ua, g.ua[big]);
+    take(s.dg_ub, g.ub[big]);
+    s.dg_utmp = L->take((size_t)g.ua[big].rows * g.ub[big].rows * sizeof(double));
+    L->off = std::max(L->off, end);
   }
   s.total = L->off;
   return s;
@@ -348,6 +370,7 @@ int check_walkers(const afq_ctx* c, const void* wu, const void* wd) {
 
 int check_state(const afq_ctx* c, const afq_walker_state* s) {
   if (!s) { afq_set_error("state is NULL"); return -1; }
+  if (c->dev.measure) { afq_set_error("the context was created for measurements only"); return -1; }
   CHECK(check_walkers(c, s->walkers_up, s->walkers_dn));
   if (!s->weights || !s->overlaps || !s->scalars) { afq_set_error("state has NULL arrays"); return -1; }
   return 0;
@@ -954,38 +977,46 @@ int afq_ctx_create(const afq_dims* dims, const afq_hamiltonian* ham, void* works
       o.d = reinterpret_cast<unsigned char*>(ws + off[0]);
       o.e = reinterpret_cast<int*>(ws + off[1]);
     };
-    at(c->dg.chol, sz.dg_chol);
     at(c->dg.rc, sz.dg_rc);
-    at(c->dg.xa, sz.dg_xa);
     at(c->dg.ga, sz.dg_ga);
     c->dg.status = reinterpret_cast<int*>(ws + sz.dg_status);
     c->dg.part = reinterpret_cast<double2*>(ws + sz.dg_part);
     c->dg.z = reinterpret_cast<double2*>(ws + sz.dg_z);
-    int e = zero(ws + sz.dg, sz.dg_end - sz.dg, st);  // padding stays zero
-    c->dg.walk.vd = reinterpret_cast<unsigned char*>(ws + sz.dg_v[0]);
-    c->dg.walk.ve = reinterpret_cast<int*>(ws + sz.dg_v[1]);
-    c->dg.walk.xd = reinterpret_cast<unsigned char*>(ws + sz.dg_x[0]);
-    c->dg.walk.xe = reinterpret_cast<int*>(ws + sz.dg_x[1]);
     c->dg.walk.status = c->dg.status;
-    c->dg.walk_t = reinterpret_cast<double2*>(ws + sz.dg_wt);
-    c->dg.walk_acc = reinterpret_cast<double2*>(ws + sz.dg_wa);
-    for (int s = 0; s < c->dg.walk.n_e(dev.nslab); ++s) at(c->dg.walk.e[s], sz.dg_e[s]);
-    if (!e) e = afq::dig_walk_slice_e(c->dg.walk, c->dg.walk.e, dev.exp_h1, dev.nslab, false, st);
+    int e = zero(ws + sz.dg, sz.dg_end - sz.dg, st);  // padding stays zero
     for (int s = 0; s < dev.nspin_g && c->dg.has_u && !e; ++s) {
-      // U[(i,q),(k,p)] = (X X^T)[(i,p),(k,q)], X = rot_chol^T
+      // U[(i,q),(k,p)] = (X X^T)[(i,p),(k,q)], X = rot_chol^T; u_strip of the i at a time
       at(c->dg.u[s], sz.dg_u[s]);
       at(c->dg.ua[s], sz.dg_ua);
       at(c->dg.ub[s], sz.dg_ub);
       const int on = c->dg.u[s].rows;
       double* tmp = reinterpret_cast<double*>(ws + sz.dg_utmp);
-      if (s == 1) e = zero(ws + sz.dg_ua[0], sz.dg_uend - sz.dg_ua[0], st);  // the other spin's rows
-      if (!e) e = afq::dig_slice_real_cols(c->dg.ua[s], dev.rot_chol[s], on, st);
-      if (!e) e = afq::dig_slice_real_cols(c->dg.ub[s], dev.rot_chol[s], on, st);
-      if (!e) e = afq::dig_gemm_r(afq::K_PREP, c->dg.ua[s], c->dg.ub[s], on, on, tmp, on, dev.norb, c->dg.status, st);
-      if (!e) e = afq::dig_slice_real_rows(c->dg.u[s], tmp, on, st);
+      e = afq::dig_slice_real_cols(c->dg.ub[s], dev.rot_chol[s], on, st);
+      for (int r0 = 0; r0 < on && !e; r0 += c->dg.ua[s].rows) {
+        afq::DigOp a = c->dg.ua[s];
+        a.rows = std::min(a.rows, on - r0);
+        e = afq::dig_slice_real_cols(a, dev.rot_chol[s] + r0, on, st);
+        if (!e) e = afq::dig_gemm_r(afq::K_PREP, a, c->dg.ub[s], a.rows, on, tmp, on, dev.norb, c->dg.status, st);
+        if (!e) e = afq::dig_slice_real_rows(c->dg.u[s], tmp, on, st, a.rows, r0);
+      }
     }
-    if (!e) e = afq::dig_slice_real_cols(c->dg.chol, ham->chol, (long)dims->norb * dims->norb, st);
-    if (!e) e = afq::dig_slice_real_rows(c->dg.rc, dev.nspin_g == 2 ? c->rccat : ham->rot_chol_up, dev.ktot, st);
+    if (!e) e = afq::dig_slice_real_rows(c->dg.rc, rc_all(c), dev.ktot, st);
+    if (!dev.measure) {
+      at(c->dg.chol, sz.dg_chol);
+      at(c->dg.xa, sz.dg_xa);
+      if (!e) e = afq::dig_slice_real_cols(c->dg.chol, ham->chol, (long)dims->norb * dims->norb, st);
+    }
+    if (c->dg.use_walk) {
+      c->dg.walk.vd = reinterpret_cast<unsigned char*>(ws + sz.dg_v[0]);
+      c->dg.walk.ve = reinterpret_cast<int*>(ws + sz.dg_v[1]);
+      c->dg.walk.xd = reinterpret_cast<unsigned char*>(ws + sz.dg_x[0]);
+      c->dg.walk.xe = reinterpret_cast<int*>(ws + sz.dg_x[1]);
+      c->dg.walk_t = reinterpret_cast<double2*>(ws + sz.dg_wt);
+      c->dg.walk_acc = reinterpret_cast<double2*>(ws + sz.dg_wa);
+      for (int s = 0; s < c->dg.walk.n_e(dev.nslab); ++s) at(c->dg.walk.e[s], sz.dg_e[s]);
+      if (!e) e = afq::dig_walk_slice_e(c->dg.walk, c->dg.walk.e, dev.exp_h1, dev.nslab, false, st);
+    }
+    if (!e) e = zero(ws + sz.dgw, sz.dgw_end - sz.dgw, st);  // the walkers' padding, after the set-up in its place
     if (e) {
       delete c;
       return e;

@@ -14,6 +14,7 @@ struct afq_ctx_dev {
   int gocc[2];
   int ktot;          // (gocc0 + (nspin_g==2 ? gocc1 : 0)) * norb
   int energy_mode;   // 0 RHF restricted, 1 RHF two-slab, 2 UHF
+  int measure;       // no propagation operands (AFQ_FP64_MEASURE)
   int digits;        // FP64: contractions as digit products on the tensor cores (else the FP64 units)
   double h0, h0_prop_re, h0_prop_im;
   const double* trial[2];     // [norb, nocc_s]

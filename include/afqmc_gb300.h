@@ -38,6 +38,9 @@ extern "C" {
 /* afq_dims.mixed_config of an AFQ_PREC_FP64 context: every contraction as sums on the FP64 units (5 to 17 times
  * the time of a block, and a small part of the workspace); other bits are ignored there. */
 #define AFQ_FP64_UNITS (1 << 24)
+/* ... without AFQ_FP64_UNITS: a context for afq_calc_overlap, afq_calc_force_bias and afq_calc_energy only, whose
+ * workspace leaves out the sliced Cholesky vectors and the propagation's buffers; calls with a state are refused. */
+#define AFQ_FP64_MEASURE (1 << 25)
 
 enum afq_walker_type { AFQ_WALKERS_RESTRICTED = 0, AFQ_WALKERS_UNRESTRICTED = 1 };
 enum afq_trial_type { AFQ_TRIAL_RHF = 0, AFQ_TRIAL_UHF = 1 };
@@ -69,7 +72,7 @@ typedef struct afq_dims {
   int32_t precision;    /* afq_precision */
   int32_t n_exp_terms;  /* Taylor terms of exp(vhs), reference default 6 */
   int32_t n_batch;      /* walker chunks for the vhs workspace (>= 1, divides n_walkers) */
-  int32_t mixed_config; /* AFQ_PREC_FP64: 0 or AFQ_FP64_UNITS.
+  int32_t mixed_config; /* AFQ_PREC_FP64: 0, AFQ_FP64_UNITS or AFQ_FP64_MEASURE.
                            AFQ_PREC_MIXED accuracy options; 0 = library default (767).
                            bits 0..7: lo (correction) terms of G / rot_chol (force bias),
                            fields / chol (vhs), walker / exp_h1 (exp_h1 products), G /
@@ -133,7 +136,11 @@ typedef struct afq_ctx afq_ctx;
 
 /* ---- context ------------------------------------------------------------------------ */
 
-/* Bytes of device workspace a context with these sizes needs. Returns 0 on bad sizes. */
+/* Bytes of device workspace a context with these sizes needs. Returns 0 on bad sizes.
+ * AFQ_PREC_FP64 without AFQ_FP64_UNITS: 16 bytes per element of chol, of rot_chol and, from 4 walkers on or up to 32 MB,
+ * of the (nocc norb)^2 exchange matrix of each spin of the trial, whatever the population; and per walker about
+ * 32 bytes per element of vhs (for 160 MB or 152 walkers of them at a time, whichever is more) and the complex
+ * arrays. Contexts do not share them. */
 size_t afq_workspace_size(const afq_dims* dims);
 
 /* Create a context. `workspace` must hold afq_workspace_size(dims) bytes (256-B aligned)
