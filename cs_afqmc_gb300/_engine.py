@@ -169,14 +169,21 @@ def engine_for(trial, ham_data: Optional[dict], wave_data: dict, walkers, *, dt:
             return tuple(ident(y) for y in x)
         return (id(x), x.data_ptr() if isinstance(x, torch.Tensor) else None)
 
+    def versions(x):
+        if isinstance(x, (list, tuple)):
+            return tuple(versions(y) for y in x)
+        return x._version if isinstance(x, torch.Tensor) and not x.is_inference() else None
+
     key = (nw, restricted, prec, float(dt) if have_prop else None, n_exp_terms, n_batch,
            int(mixed_config),
            ident(mo),
            ident(ham_data.get("rot_chol")) if ham_data is not None else None,
            ident(ham_data.get("exp_h1")) if have_prop else None,
            ident(ham_data.get("chol")) if ham_data is not None else None)
+    # contexts keep converted copies of these: one of a tensor that was changed in place since is stale
+    held = versions([mo] + [None if ham_data is None else ham_data.get(k) for k in ("rot_chol", "exp_h1", "chol")])
     eng = cache.get(key)
-    if eng is not None:
+    if eng is not None and eng.held == held:
         return eng
     norb = trial.norb
     nelec = trial.nelec
@@ -234,6 +241,7 @@ def engine_for(trial, ham_data: Optional[dict], wave_data: dict, walkers, *, dt:
     eng = Engine(norb=norb, nelec=nelec, nchol=nchol, n_walkers=nw, restricted=restricted, uhf=uhf,
                  precision=prec, dt=dt, n_exp_terms=n_exp_terms, n_batch=n_batch, arrays=a, h0=h0,
                  h0_prop=h0p, mixed_config=mixed_config)
+    eng.held = held
     cache[key] = eng
     return eng
 

@@ -90,7 +90,9 @@ typedef struct afq_dims {
 /* Hamiltonian and trial intermediates built by hamiltonian.build_measurement_intermediates
  * and build_propagation_intermediates (hamiltonian.py:49-81 -> wavefunctions.py:602-619,
  * 817-841; propagation.py:292-325, 464-509). Device pointers; the caller keeps them alive
- * for the context's lifetime. The trial must be real (float64 mo_coeff). */
+ * for the context's lifetime and their contents unchanged: chol, rot_chol and exp_h1 are read once, by
+ * afq_ctx_create (the context keeps converted copies), the others at every call, so that a changed Hamiltonian
+ * needs a new context. The trial must be real (float64 mo_coeff). */
 typedef struct afq_hamiltonian {
   double h0;
   double h0_prop_re, h0_prop_im;  /* -h0 - sum(mf_shifts^2)/2 */
