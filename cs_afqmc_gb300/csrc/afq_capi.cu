@@ -41,7 +41,9 @@ struct DigCtx {
   afq::DigPlan uplan[2];
   double2* z;     // [nw][ktot]
   double2* part;  // partial results of split K ranges
-  int use_walk;   // Taylor products on the digit GEMM (walk), else k_taylor_f64
+  // operands of the Taylor products on the digit GEMM (walk) are there; used by the steps, by forward mode (by
+  // reverse mode wherever they are there); else the FP64 units
+  int use_walk, walk_fwd, walk_jvp;
   afq::DigWalk walk;
   double2 *walk_t, *walk_acc;  // [chunk][norb * (k0 + k1)]
   int* status;
@@ -171,7 +173,6 @@ int derive(const afq_dims* d, afq_ctx_dev* c, int* nw_chunk, int* e_chunks, int*
 // Shapes of the sliced FP64 operands (no pointers). The plan assumes the full part's 152 SMs, so
 // that workspace sizes do not depend on where they are asked for.
 constexpr int kPlanSms = 152;
-constexpr long kWalkMin = 1000000;
 constexpr int kUWalkers = 4;
 constexpr size_t kUBytes = (size_t)32 << 20;
 void dig_dims(const afq_ctx_dev& c, int nw_chunk, DigCtx* g) {
@@ -207,7 +208,21 @@ void dig_dims(const afq_ctx_dev& c, int nw_chunk, DigCtx* g) {
     g->uplan[s] = afq::dig_plan(t, g->u[s].kb(), kPlanSms, 4);
   }
   afq::dig_walk_dims(c.norb, c.kslab, c.nslab, nw_chunk, &g->walk);
-  g->use_walk = c.digits && !c.measure && c.norb <= 256 && (long)nw_chunk * g->walk.ncol * nn >= kWalkMin;
+  // Taylor products on digits or on the FP64 units. Digits take 0.1 ms a step (14 launches) and then 0.3 to 1 us a
+  // walker; the units up to kTaylorSmall a time that grows with q = norb^2 electrons, 0.3 us a walker at 20 x 5 and 2.2
+  // at 40 x 12, above it several times that. Two steps in us, digits / units: 20 x 5 (q 2000), 50, 400 and 2000 walkers
+  // 206 / 53, 372 / 135, 1296 / 610; 28 x 7 (5488) 203 / 121, 369 / 304, 1283 / 1380; 32 x 8 (8192) 196 / 144, 362 / 395,
+  // 1283 / 1811; 40 x 7 (11200) 227 / 212, 447 / 580; 64 x 4 (16384) 236 / 240, 502 / 684; 60 x 10 (36000), 8 walkers
+  // 263 / 753.
+  const long q = (long)nn * c.kmax;
+  const bool can = c.digits && !c.measure && c.norb <= 256;
+  g->walk_fwd = can && (c.norb * c.kmax > afq::kTaylorSmall || q >= 14000 || (q >= 7500 && nw_chunk * c.nslab >= 200));
+  // Forward mode, the whole call of three steps, 50 and 1000 walkers: 24 x 6 (3456) 2.37 / 2.02, 5.52 / 5.34 ms; 28 x 7
+  // 2.46 / 2.29, 5.87 / 6.86; 24 x 12 (6912) 2.71 / 2.72, 7.54 / 9.81.
+  g->walk_jvp = can && q >= 5000;
+  // Reverse mode, 50, 200 and 1000 walkers: 20 x 5 3.18 / 2.95, 3.63 / 3.73, 7.21 / 8.26 ms; 28 x 7 3.41 / 3.45, 4.02 /
+  // 4.55, 8.03 / 10.84.
+  g->use_walk = can && (q >= 5000 || (long)nw_chunk * g->walk.ncol * nn >= 1000000);
 }
 
 Sizes sizes_for(const afq_dims* d, const afq_ctx_dev& c, int nw_chunk, int e_chunks, size_t welem,
@@ -396,7 +411,7 @@ int walk_exp(const afq::DigWalk& w, const afq_ctx_dev& d, const afq::DigOp* E, c
 // W <- E exp(V) E W (propagation.py:67-92) of nwc walkers from w0 on, FP64
 int taylor_fp64(afq_ctx* c, int w0, int nwc, const double2* vhs, void* wu, void* wd, cudaStream_t st) {
   const afq_ctx_dev& d = c->dev;
-  if (!c->dg.use_walk) return afq::launch_taylor_f64<double>(d, w0, nwc, vhs, wu, wd, st);
+  if (!c->dg.walk_fwd) return afq::launch_taylor_f64<double>(d, w0, nwc, vhs, wu, wd, st);
   const afq::DigWalk& w = c->dg.walk;
   const afq::WalkVec T = walk_buf(d, c->dg.walk_t), A = walk_buf(d, c->dg.walk_acc);
   for (int k = 0; k < nwc; k += w.chunk) {
@@ -604,7 +619,7 @@ TSizes tangent_sizes(const afq_ctx_dev& c, int nw_chunk, int e_chunks, Layout* L
     s.drc_e = L->take(afq::dig_exps(g.rc.rows, g.rc.tr));
   }
   s.wk = L->off;
-  if (g.use_walk) {
+  if (g.walk_jvp) {
     for (int i = 0; i < g.walk.n_e(c.nslab); ++i) {
       s.de[i][0] = L->take(afq::dig_bytes(g.walk.e[i].rows, c.norb));
       s.de[i][1] = L->take(afq::dig_exps(g.walk.e[i].rows));
@@ -643,7 +658,7 @@ int propagate_jvp(afq_ctx* c, afq_walker_state* s, const afq::TangentBufs& t, co
     const int w0 = b * c->nw_chunk;
     CHECK(vhs_gemm(c, c->xt + (size_t)w0 * d.nchol, c->nw_chunk, c->vhs, st));
     CHECK(vhs_gemm(c, t.dxt + (size_t)w0 * d.nchol, c->nw_chunk, t.dvhs, st));
-    if (c->dg.use_walk)
+    if (c->dg.walk_jvp)
       CHECK(taylor_jvp(c, t, jw.w, jw.t, jw.a, w0, c->nw_chunk, c->vhs, s->walkers_up, s->walkers_dn, st));
     else
       CHECK(afq::t_launch_taylor(d, t, w0, c->nw_chunk, c->vhs, t.dvhs, s->walkers_up, s->walkers_dn, st));
@@ -1246,7 +1261,7 @@ int afq_propagate_phaseless_jvp_ex(afq_ctx* ctx, afq_walker_state* state, const 
   drc.e = reinterpret_cast<int*>(tw + ts.drc_e);
   if (t.drccat && d.digits) CHECK(afq::dig_slice_real_rows(drc, t.drccat, d.ktot, st));
   JvpWalk jw{ctx->dg.walk, nullptr, nullptr};
-  if (ctx->dg.use_walk) {  // (the workspace was cleared above: padding is zero)
+  if (ctx->dg.walk_jvp) {  // (the workspace was cleared above: padding is zero)
     jw.w.vd = reinterpret_cast<unsigned char*>(tw + ts.v[0]);
     jw.w.ve = reinterpret_cast<int*>(tw + ts.v[1]);
     jw.w.xd = reinterpret_cast<unsigned char*>(tw + ts.x[0]);

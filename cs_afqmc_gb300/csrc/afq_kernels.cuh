@@ -25,6 +25,9 @@ struct afq_ctx_dev {
 };
 
 namespace afq {
+// largest slab (norb x electrons) of the FP64 Taylor kernel with four lanes per element
+constexpr int kTaylorSmall = 512;
+
 // dynamic shared memory of the FP64 Green's-function / overlap kernel (k_green_overlap)
 inline size_t green_f64_smem(int norb, int kmax) {
   return (size_t)norb * kmax * 16 + (size_t)kmax * 2 * kmax * 16 + (size_t)norb * kmax * 8;

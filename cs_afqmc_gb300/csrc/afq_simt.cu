@@ -328,10 +328,10 @@ __global__ void __launch_bounds__(256) k_taylor_f64(const afq_ctx_dev c, int w0,
   }
 }
 
-// The same for small slabs (norb * k <= 512): four lanes per element, each a quarter of the sum
-// over q, so that a product of a few hundred elements is a few dependent FMAs long instead of norb
-// (norb 20, 5 electrons, 50 walkers: 44 us with an element per thread).
-constexpr int kTaylorSmall = 512;
+// The same for small slabs (norb * k <= kTaylorSmall, what its static shared memory holds): four lanes per element,
+// each a quarter of the sum over q, so that a product of a few hundred elements is a few dependent FMAs long
+// instead of norb. A step against an element per thread: 16 x 3 electrons, 50 walkers 38 -> 13 us; 20 x 5, 50 walkers
+// 44 -> 27, 400 walkers 130 -> 68; 32 x 8 98 -> 72; 40 x 12 195 -> 169; 64 x 8 323 -> 233.
 
 __global__ void __launch_bounds__(256) k_taylor_small(const afq_ctx_dev c, int w0, const double2* __restrict__ vhs,
                                                       double2* __restrict__ w_up, double2* __restrict__ w_dn) {

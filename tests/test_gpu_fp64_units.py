@@ -52,6 +52,10 @@ PLANS = {
     "V cotangents in two segments, stacked": dict(kind="uhf", restricted=False, norb=40, nelec=(28, 27), nchol=30, nw=12),
     "V cotangents in two segments": dict(kind="uhf", restricted=False, norb=70, nelec=(30, 26), nchol=30, nw=6),
     "batches": dict(kind="uhf", restricted=False, norb=66, nelec=(9, 8), nchol=60, nw=48, n_batch=2),
+    "steps on the units, reverse mode on digits": dict(kind="uhf", restricted=False, norb=20, nelec=(5, 4), nchol=24, nw=400),
+    "derivatives on digits": dict(kind="rhf", restricted=False, norb=28, nelec=(7, 7), nchol=24, nw=30),
+    "all on digits from 200 slabs on": dict(kind="uhf", restricted=False, norb=33, nelec=(7, 6), nchol=30, nw=100),
+    "all on digits, few walkers": dict(kind="rhf", restricted=True, norb=47, nelec=(12, 12), nchol=30, nw=3),
     "one walker": dict(kind="rhf", restricted=False, norb=33, nelec=(6, 6), nchol=50, nw=1),
 }
 
