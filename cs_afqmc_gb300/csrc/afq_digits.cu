@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(kDigThreads, 1)
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&accempty[buf]);
-          const int er = g.ea[(size_t)(w.batch * g.a_bt + w.m) * kDigTile + r] + ep.shift;
+          const int er = g.ea[(size_t)(w.batch * g.a_bt + w.m) * kDigTile + r] + Epi::shift(ep);
           const int* eb = g.eb + (size_t)(w.batch * g.b_bt + w.n) * tr + col0;
 #pragma unroll
           for (int c0 = 0; c0 < 16; c0 += 4)
@@ -731,6 +731,7 @@ struct EpiDigC {
     long ldc, split_stride;
     int rot, shift;  // C = i^rot 2^shift D
   };
+  AFQ_D static int shift(const Params& p) { return p.shift; }
   AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
     const int m = (w.m * kDigTile + r) >> 1, odd = r & 1, n0 = w.n * p.tr + col0;
 #pragma unroll
@@ -756,8 +757,9 @@ struct EpiDigR {
     double* d;
     int M, N, tr;
     long ldd;
-    int shift, swap;
+    int swap;
   };
+  AFQ_D static int shift(const Params&) { return 0; }
   AFQ_D static void store(const Params& p, const DigWhere& w, int r, int col0, const double (&v)[4]) {
     const int m = w.m * kDigTile + r, n0 = w.n * p.tr + col0;
     if (m >= p.M) return;
@@ -776,15 +778,14 @@ struct EpiDigR {
 };
 
 // Products of DigWalk: row p of tile m, columns 2c and 2c + 1 of one walker.
-// These also take the digit products with i + j = 8 (into the last accumulator, whose integer is
-// then rounded once): exp_h1 is nearly diagonal and a column of a walker has a few large entries,
+// These also take the digit products with i + j = 8 (into the last accumulator, which then holds two weights and may
+// round): exp_h1 is nearly diagonal and a column of a walker has a few large entries,
 // so the scale of a dot product can be far above its value. Walkers after a step, against
 // extended precision: 1.7e-16 at norb 33, 2.1e-16 at norb 120; the FP64 units: 3.5e-16, 6.2e-16.
 struct WalkParams {
   WalkOut o;
   int n, o0, ncol, tr, only;  // only: the slab to store (-1: both)
   int stack, pair;            // stacked rows; V (the two row halves make one result) or E (a slab each)
-  int shift;
 };
 
 struct EpiWalk {
@@ -1054,7 +1055,8 @@ int dig_tr(int M, int N, int kb, int sms) {
 }
 
 // The count of K ranges that gives the fewest (rounds of tiles over the SMs) x (K blocks per
-// range + 2 for a range's epilogue).
+// range + 2 for a segment's epilogue; the contractions of a two-step block of 512 walkers in 60 orbitals take 315 us with 2
+// or 6 and 335 with none, other sizes the same with all three).
 DigPlan dig_plan(int tiles, int kb, int sms, int max_splits) {
   DigPlan best{1, kb};
   long cost = -1;
@@ -1096,7 +1098,7 @@ int dig_gemm_c(int cls, const DigOp& A, const DigOp& B, int M, int N, double2* C
 int dig_gemm_r(int cls, const DigOp& A, const DigOp& B, int M, int N, double* D, long ldd, int swap,
                int* status, cudaStream_t st) {
   DigGemm g = dig_args(A, B);
-  EpiDigR::Params ep{D, M, N, B.tr, ldd, 0, swap};
+  EpiDigR::Params ep{D, M, N, B.tr, ldd, swap};
   return launch_digits<EpiDigR>(cls, g, ep, status, st);
 }
 
@@ -1110,7 +1112,9 @@ void dig_walk_dims(int norb, const int* k, int nslab, int nw, DigWalk* d) {
   d->mt = (norb + kDigTile - 1) / kDigTile;
   d->nt = (2 * d->ncol + 63) / 64;
   d->tr = ((2 * d->ncol + d->nt - 1) / d->nt + 15) / 16 * 16;
-  // V digits of a chunk: at most 160 MB, whole rounds of the 152 SMs where it is cut
+  // V digits of a chunk: at most 160 MB or 152 walkers, whichever is more (171 MB at 129 orbitals, 304 at 256), in whole
+  // rounds of the full part's 152 SMs. Two steps with chunks of 40, 160 and 640 MB: 2000 walkers in 60 orbitals 2.81, 2.28
+  // and 2.12 ms; 1216 in 120 5.77, 4.83 and 4.26; 304 in 200 5.63, 5.65 and 5.61.
   const size_t per = (size_t)d->mt * kDigTile * d->kbv() * 256;
   const long most = std::max<long>((long)((160u << 20) / per) / 152 * 152, 152);
   d->chunk = nw < most ? nw : (int)most;
@@ -1167,7 +1171,7 @@ int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut
   g.tr = d.tr;
   g.splits = 1;
   g.kps = g.kb;
-  WalkParams ep{o, d.n, d.o[0], d.ncol, d.tr, d.stack || e < 0 || d.o[1] == 0 ? -1 : e, d.stack, d.stack && e < 0, 0};
+  WalkParams ep{o, d.n, d.o[0], d.ncol, d.tr, d.stack || e < 0 || d.o[1] == 0 ? -1 : e, d.stack, d.stack && e < 0};
   return launch_digits<EpiWalk>(cls, g, ep, d.status, st);
 }
 
@@ -1222,7 +1226,7 @@ int dig_walk_vbar(const DigWalk& d, const DigVbar& v, const double2* tay, int te
   g.kps = g.kb;
   WalkOut o;  // [norb][norb] per walker: one slab of norb columns
   o.out = WalkVec{{vbar, nullptr}, (size_t)d.n * d.n};
-  WalkParams ep{o, d.n, d.n, d.n, v.tr, -1, 0, 0, 0};
+  WalkParams ep{o, d.n, d.n, d.n, v.tr, -1, 0, 0};
   return launch_digits<EpiWalk>(K_TAYLOR, g, ep, d.status, st);
 }
 

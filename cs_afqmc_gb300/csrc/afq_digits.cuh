@@ -6,11 +6,20 @@
 // 59, 2012, with digits of a fixed weight). A digit times its weight is exact in BF16, a
 // product of two is exact in FP32, and the sum of all products with i + j = c over up to 512
 // terms of K is an integer below 2^24 in units of 2^(-14-7c) for c <= 5: the tensor core's FP32
-// accumulator never rounds it. One accumulator per c = 0..7 (36 of the 64 digit products;
-// the others are below 2^-70) is therefore exact, the eight are combined in 64-bit integer
-// arithmetic, and the only rounding of a dot product is the final one to FP64 (plus the
-// remainders, 2^-57 of the row's largest element each). A plain FP64 sum of K terms rounds K
-// times.
+// accumulator never rounds it. There is one accumulator per c = 0..7, 36 of the 64 digit products; those of
+// c = 6 and 7 can pass 2^24 (35847 x 512 and 38038 x 512 at most) and then round to a few units of 2^-56
+// and 2^-63. The eight are combined in 64-bit integer arithmetic and rounded to FP64.
+//
+// Error of a dot product of up to 512 terms, with 2^ea, 2^eb the scales of its two rows (at most twice
+// their largest elements): the rounding of the result; per term the two remainders, 2^-57 2^(ea + eb) each at most, and
+// the seven products with i + j = 8 (plus less from the others), 2^-58 each at most: altogether below K 2^(ea + eb - 54), for
+// terms of no common sign about sqrt(K) 2^(ea + eb - 58). More terms come in segments of 512, and
+// contractions cut into K ranges in ranges, whose results are added in FP64.
+// A plain FP64 sum rounds K times at the size of its partial sums: for rows of similar elements (Gaussian: 3.2e-16 of the
+// result against 0.9e-16) and for Cholesky vectors that fall by 1e5 against flat fields (4.5e-16, 1.5e-16) it is further
+// off. But the digits' error is relative to the rows' largest elements, not to the terms: one large element that meets a zero
+// with the others 1e-4 leaves 2e-13, rows that fall and rise against each other by 1e6 1e-11. Contexts can ask for the
+// FP64 units instead (AFQ_FP64_UNITS).
 //
 // Why: this part does FP64 at 1.04 TFLOP/s (DGEMM) and BF16 at 1.9 PFLOP/s, so 36 tensor-core
 // products cost about 2 % of the FP64 ones; integer instructions combine the accumulators
@@ -55,7 +64,7 @@ int dig_slice_real_cols(const DigOp& op, const double* src, long ld, cudaStream_
 // ---- contractions ---------------------------------------------------------------------
 // C[m][n] (complex, ldc) = i^rot 2^shift sum_k A[m][k] B[n][k]: A sliced by
 // dig_slice_cplx_rows, B real. part: split partials when the K range is cut (see
-// dig_gemm_plan); may be NULL when the plan has one split.
+// dig_plan); may be NULL when the plan has one split.
 struct DigPlan {
   int splits, kps;  // K ranges computed independently, K blocks per range
 };
@@ -148,7 +157,9 @@ int dig_walk_slice_e(const DigWalk& d, const DigOp* e, const double* const* exp_
 int dig_walk_mul(int cls, const DigWalk& d, int e, const DigOp* E, const WalkOut& o, int nw, cudaStream_t st);
 // B columns per tile for an output of 2 M x N with kb K blocks: 64 where the tiles (times up to
 // eight K ranges) reach half of the SMs, else 32, so that small problems still spread out; never
-// more than N needs.
+// more than N needs. The contractions of a two-step block in us, with 32 / with 64 / by the rule: 20 orbitals, 50 and 500
+// walkers 87 / 109 / 87, 90 / 114 / 102; 60 orbitals, 64 and 512 walkers 135 / 158 / 134, 464 / 315 / 315; 80 orbitals, 256
+// walkers 576 / 367 / 391; 120 orbitals, 16 and 256 walkers 476 / 391 / 424, 1716 / 1036 / 1035.
 int dig_tr(int M, int N, int kb, int sms);
 
 }  // namespace afq
