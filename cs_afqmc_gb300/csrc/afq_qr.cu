@@ -12,8 +12,8 @@ namespace afq {
 // with the comb's teeth, and a weight that moves by one FP32 rounding exchanges a whole walker wherever a
 // tooth lies that close (64 sites, 2048 walkers: with the slab in registers and its column sums split over
 // eight row groups, one of twelve populations came out with another walker). So a
-// column is summed as it always was, which costs 64 x 28 electrons, 2048 slabs 131 -> 254 us; 120 x 20, 1024 slabs
-// 114 -> 131; 198 x 33, 256 slabs 161 -> 215; 60 x 10 and 60 x 8, 512 walkers 16 -> 30.
+// column is summed as it always was, which costs 64 x 28 electrons, 2048 slabs 131 -> 174 us; 120 x 20, 1024 slabs
+// 114 -> 127; 198 x 33, 256 slabs 161 -> 215; 60 x 10 and 60 x 8, 512 walkers 16 -> 30.
 
 // v y of a rank-1 update and -tau v of a column of Q (the compiler's contractions of the first version)
 AFQ_D float2 qr_vy(float2 v, float2 y) {
@@ -47,7 +47,9 @@ AFQ_D void qr_reflector(float2 alpha, float xn, float2& tau, float2& scl, float2
 // warp-level synchronisation. Column sums (the reflector applied to the trailing columns) are owned by
 // lanes per column (qr_colsum); the rank-1 updates by lane = row. The squared norm below the diagonal
 // is accumulated as a float pair.
-constexpr int kQrWarps = 4;
+// Slabs per CTA: one of four waits for room for all four (64 x 28, 2048 slabs: 12 instead of 14 on an SM and a second,
+// nearly empty wave, 254 us instead of 174).
+constexpr int kQrWarps = 1;
 
 __host__ __device__ constexpr int qr_ld(int k) { return k | 1; }
 
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(32 * kQrWarps) k_qr_warp(const afq_ctx_dev c, 
   }
 }
 
-// Slabs of more than 32 columns, or too long for four to share a CTA: one CTA per (walker, slab).
+// Slabs of more than 32 columns, or too long for four to share an SM: one CTA per (walker, slab).
 AFQ_D float warp_sumf(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -262,7 +264,8 @@ int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
   auto warp_smem = [&](int s) {
     return kQrWarps * ((size_t)c.norb * qr_ld(c.kslab[s]) + 64) * sizeof(float2);
   };
-  auto by_warp = [&](int s) { return c.kslab[s] <= 32 && warp_smem(s) <= 227 * 1024; };
+  // longer slabs would leave an SM fewer than four warps
+  auto by_warp = [&](int s) { return c.kslab[s] <= 32 && 4 / kQrWarps * warp_smem(s) <= 227 * 1024; };
   const bool both = c.nslab == 2 && by_warp(0) && by_warp(1);  // one launch for both slabs
   ProfScope _ps(K_QR, st);
   for (int s = 0; s < (both ? 1 : c.nslab); ++s) {
