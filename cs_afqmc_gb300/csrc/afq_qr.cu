@@ -264,8 +264,10 @@ int launch_qr_f32(const afq_ctx_dev& c, void* wu, void* wd, cudaStream_t st) {
   auto warp_smem = [&](int s) {
     return kQrWarps * ((size_t)c.norb * qr_ld(c.kslab[s]) + 64) * sizeof(float2);
   };
-  // longer slabs would leave an SM fewer than four warps
-  auto by_warp = [&](int s) { return c.kslab[s] <= 32 && 4 / kQrWarps * warp_smem(s) <= 227 * 1024; };
+  // longer slabs would leave an SM fewer than four warps; the second slab follows the first into the block form (the two
+  // forms sum a column in different orders)
+  auto fits = [&](int s) { return c.kslab[s] <= 32 && 4 / kQrWarps * warp_smem(s) <= 227 * 1024; };
+  auto by_warp = [&](int s) { return fits(0) && fits(s); };
   const bool both = c.nslab == 2 && by_warp(0) && by_warp(1);  // one launch for both slabs
   ProfScope _ps(K_QR, st);
   for (int s = 0; s < (both ? 1 : c.nslab); ++s) {

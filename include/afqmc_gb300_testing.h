@@ -52,6 +52,8 @@ int afq_test_gemm_digits(const double* a, const double* b, double* d, int M, int
  * in bytes; negative: a CUDA error. */
 long afq_test_digits_smem_limit(void);
 
+struct afq_ctx;
+
 /* Sets the guard word of a context's tensor-core kernels to bits (0..255), as a wait that runs out would:
  * for tests of how it is reported. */
 int afq_test_preset_status(struct afq_ctx* ctx, int bits, void* stream);

@@ -30,14 +30,14 @@ def parts(w):
     return np.ascontiguousarray(w.real.astype(F)), np.ascontiguousarray(w.imag.astype(F))
 
 
-def determinant(c, w):
+def determinant(c, w, widest):
     """det(C^T W) of every walker as the elimination rounds it; the product of the pivots in FP64."""
     n, o = c.shape
     c, (wx, wy), nw = c.astype(F), parts(w), w.shape[0]
     s = [np.zeros((nw, o, o), F), np.zeros((nw, o, o), F)]
     for p in range(n):
         s = [fma(c[p][None, :, None], x[:, p, None, :], t) for x, t in zip((wx, wy), s)]
-    mask = np.uint32(31 if o <= 32 else 63)
+    mask = np.uint32(31 if widest <= 32 else 63)  # row index in the low bits of the pivot key
     used, rows, piv, at = np.zeros((nw, o), bool), [], [], np.arange(nw)
     for j in range(o):
         mag = np.abs(s[0][:, :, j]) + np.abs(s[1][:, :, j])
@@ -74,7 +74,7 @@ def test_overlaps_round_as_sums_in_order(norb, n_up, n_dn):
     ovl = to_np(case.trial.calc_overlap(case.gpu_walkers(), case.wave_data))
     want = 1.0
     for c, w in zip(case.sys.mo_coeff, case.walkers0):
-        want = want * determinant(np.asarray(c)[:, : w.shape[2]], w.astype(np.complex64))
+        want = want * determinant(np.asarray(c)[:, : w.shape[2]], w.astype(np.complex64), max(n_up, n_dn))
     # the pivots are the same numbers; 70 FP64 products of them
     assert np.max(np.abs(ovl - want) / np.abs(want)) < 70 * 2.3e-16
 
@@ -171,9 +171,9 @@ def householder_q(w, by_warp):
     return x + 1j * y
 
 
-# above 32 columns, or where four slabs do not fit a block's shared memory, a block takes a slab
+# above 32 columns, or where four slabs do not fit a block's shared memory, a block takes a slab, and the second one too
 @pytest.mark.parametrize("norb,n_up,n_dn", [(2, 1, 1), (9, 5, 1), (20, 3, 2), (40, 12, 9), (64, 28, 17), (90, 32, 16),
-                                            (130, 33, 4), (170, 40, 37), (256, 17, 27)])
+                                            (130, 33, 4), (170, 40, 37), (256, 17, 27), (140, 30, 35)])
 def test_qr_rounds_as_sums_in_order(norb, n_up, n_dn):
     from tests.helpers import Case, to_np
 
@@ -184,5 +184,5 @@ def test_qr_rounds_as_sums_in_order(norb, n_up, n_dn):
     pg = case.prop.orthonormalize_walkers(pg)
     for w, q in zip(before, pg["walkers"]):
         k = w.shape[2]
-        by_warp = k <= 32 and 32 * (norb * (k | 1) + 64) <= 227 * 1024
+        by_warp = all(j <= 32 and 32 * (norb * (j | 1) + 64) <= 227 * 1024 for j in (n_up, k))
         assert np.array_equal(householder_q(w, by_warp), to_np(q)), k
